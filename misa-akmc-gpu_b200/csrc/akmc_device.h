@@ -13,6 +13,9 @@ constexpr int kMaxV = AKMC_MAX_SECTOR_VACANCIES;  // vacancies per block and sec
 constexpr int kNoAllocMaxBlocks = AKMC_NOALLOC_MAX_BLOCKS;
 constexpr int kJumpN = 76;                        // |N(s) u N(t)| - 2 sites per jump
 constexpr int kRefreshN = 78;                     // density refresh sites per jump
+constexpr int kTermN = 302;                       // distinct energy terms of a vacancy's 8 jumps (Geometry)
+constexpr int kTermSlots = 312;                   // + own and target embedding values, and a zero term
+constexpr int kFootSlots = 256;                   // lanes that compute them
 constexpr int kShellNb = 58;                      // neighbours within the 5-shell cutoff
 constexpr int kNbrStride = 32;  // words per block of RoundArgs::nbr (one 128-byte line)
 constexpr int kFlowSlots = 64;                    // vacancies held in one domain block's area
@@ -37,7 +40,22 @@ struct Geometry {
   int32_t nbr[2][kShellNb];          // EAM shell neighbours (sh in sh_s)
   int32_t jump[2][8][kJumpN];        // EAM dE site list of jump b, order (dz, dy, dX)
   int32_t refresh[2][8][kRefreshN];  // density refresh list of jump b (incl. s and t)
+  // The dE terms of the 8 jumps, each formed once.  Site j of jump b contributes
+  // [F(rho_j + f_X(sj) - f_X(tj)) - F(rho_j)] + phi_XY(sj) - phi_XY(tj), which depends on the jump
+  // only through the moving species X and the shell of j around the target: for one X the 8 x 76
+  // entries of the jump lists hold 302 distinct terms, over 144 sites.  They are formed by 251 lanes
+  // of 256, two F evaluations each: a site of m terms takes (m + 2) / 2 consecutive lanes of one
+  // warp, the first of which (the leader) evaluates F(rho_j) and one term's F, the others two terms' F.
+  int32_t foot_site[2][kFootSlots];  // the lane's site by x parity of the vacancy: packed (dX, dy, dz)
+  int32_t foot_out[kFootSlots];      // term written from F evaluation A | B << 10 (kFootNone: none) |
+                                     // leader lane << 20 | raw << 25 (F(A) itself is written to kTermN + raw - 1:
+                                     // 1 the vacancy's own site, 2 + b the target of jump b)
+  int32_t foot_shells[kFootSlots];   // (sh_s * 8 + sh_t) of evaluation A | B << 8 (0: F(rho_j) itself)
+  uint8_t foot_refresh[8][kFootSlots];  // (sh_s * 8 + sh_t) by which jump b onto the vacancy's site changed
+                                        // the lane's site (0: unchanged)
+  uint16_t term[2][8][kJumpN];       // jump list entry -> term
 };
+constexpr int kFootNone = 1023;
 
 // Per-potential tables.
 struct Potential {

@@ -6,11 +6,10 @@
 //              the block's active sector, append it to the block's list;
 //   k_hop      one CTA per active block: stage the sector plus a 2-cell halo (occupancy
 //              bytes and the int32 density cache) into shared memory and run the hop
-//              loop there.  Evaluator warp w evaluates jump directions w, w + kEvalWarps,
-//              ... of a vacancy (its 32 lanes split the 76 sites of a jump); the control
-//              warp forms the ordered total, selects, performs the hop and keeps the
-//              vacancy list and the clock; each hop writes its two occupancy bytes and 78
-//              densities through to global memory;
+//              loop there.  Warp w evaluates jump directions w, w + W, ... of a vacancy (its
+//              32 lanes split the 76 sites of a jump); every warp forms the ordered total and
+//              selects for itself, and the hop's updates are spread over the warps; each hop
+//              writes its two occupancy bytes and 78 densities through to global memory;
 //   k_finalize one thread per block: clock of blocks without vacancies, next round.
 // Concurrently active sectors are at least 4 cells apart, so the staged regions of
 // different blocks never overlap and no atomics are needed on the lattice.
@@ -39,21 +38,25 @@ constexpr int kSweepVisits = AKMC_SWEEP_VISITS;
 #define AKMC_SWEEP_SLEEP_NS 256
 #endif
 enum : int { kPairBond = 0, kEam64 = 1, kEam32 = 2 };  // energy kinds, one kernel instance each
-// CTA shape: W warps evaluate the 8 jump directions (warp w takes jumps w, w + W, ...), one
-// more warp controls the hop loop.  The hop kernels are built for W = 8 (one jump per warp) and
-// W = 4 (two jumps per warp, two CTAs per SM); a context picks one (akmc_context_config).
+// CTA shape: W warps.  EAM: all of them form a vacancy's dE terms (Geometry::foot_*, 256 lanes' worth),
+// two sum its 8 jumps, and the hop's other work (write-through, ordered list, clock, random draws) is spread
+// over the rest.  Pair bond: one warp evaluates a vacancy.  The hop kernels are built for W = 8 and W = 4;
+// a context picks one (akmc_context_config).  One 8-warp CTA per SM: a hop is a chain of dependent
+// instructions, so its latency is what counts, and two CTAs per SM (128 registers a thread instead of 255,
+// so spills in the loop, and the other CTA's sweeps and hops on the same issue slots) measured slower: 40.6
+// against 33.5 ms for 1024 rounds of the 256^3 lattice end to end, 30.2 against 27.7 ms for 256 rounds of
+// 512 boxes.
 template <int W>
 struct Shape {
   static_assert(8 % W == 0, "whole jump directions per warp");
   static constexpr int kEvalWarps = W;
   static constexpr int kJumpsPerWarp = 8 / W;
-  static constexpr int kThreads = 32 * (W + 1);
-  static constexpr int kCtl = 32 * W;  // control thread: first lane of the control warp
-  // CTAs per SM the register budget is cut for: two 5-warp CTAs fit (10 warps, at most 3 per SM
-  // partition), two 9-warp ones would cut a thread to 96 registers.
+  static constexpr int kThreads = 32 * W;
+  static constexpr int kCtl = 32 * (W - 1);  // control thread: first lane of the last warp, which also draws ahead
+  static constexpr int kClk = W == 8 ? 192 : 96;  // the thread that runs the sector's clock
+  static constexpr int kOrdWarp = W == 8 ? 4 : 3;  // the warp that keeps the ordered list
   static constexpr int kCtasPerSm = W <= 4 ? 2 : 1;
 };
-constexpr int kMaxThreads = Shape<8>::kThreads;
 // The shape's constants under their short names inside a kernel or device function of shape W.
 #define AKMC_SHAPE(W)                                         \
   constexpr int kEvalWarps = Shape<W>::kEvalWarps;            \
@@ -145,6 +148,13 @@ __device__ __forceinline__ void make_region(const BlockDev& B, const JobDev& J, 
   R.nt = R.tma ? R.n : R.LXt * R.ey * R.ez;
 }
 
+// Rounds with vacancies a CTA can take in one sweep (a sweep finds a few).
+constexpr int kMaxTake = 64;
+constexpr int kTermSets = 2;
+constexpr int kZeroTerm = kTermSlots - 1;  // a term that is always 0
+// Draws of the two random streams made ahead of their use: a ring of two batches.
+constexpr int kDrawBatch = 8, kDrawRing = 2 * kDrawBatch;
+
 // Shared-memory working set of one CTA (followed by the staged region).
 struct Smem {
   double b1[25], b2[25];
@@ -155,23 +165,23 @@ struct Smem {
   int32_t dfq[4 * 64];          // f_X(shell s) - f_X(shell t) in Q.24, index X*64 + s*8 + t
   int32_t fq1[4];               // f_X at the first shell
   int32_t d1[2][8];             // 1nn local offsets by x parity
-  int32_t w1[2][8];             // 1nn packed (dx, dy, dz)
   int32_t d2[6];
-  int32_t jl[2][8][kJumpN];     // int16 local offset | (s*8+t) << 16
-  int32_t rl[2][8][kRefreshN];  // packed (dx, dy, dz) | (s*8+t) << 24
+  uint8_t rf[8][kFootSlots];    // Geometry::foot_refresh
+  // dE terms of a vacancy's jumps (Geometry::foot_out), of two vacancies at a time: FP64 a double
+  // each (0.0: a vacancy's site), FP32-comp (term, 1.0f for an atom's site); then its own and its
+  // targets' embedding values (FP32-comp: the F cells, in fx).  The pair-bond loop keeps its path here.
+  alignas(16) double term[kTermSets][kTermSlots];
+  float4 fx[kTermSets][9];
   int32_t vidx[kMaxV];          // vacancy table index of record k
-  // Vacancy records in two sets: a hop selected from set c writes set c ^ 1 (see run_block).
-  int32_t vloc[2][kMaxV], vlid[2][kMaxV];               // local site, global site id
-  int16_t vcx[2][kMaxV], vcy[2][kMaxV], vcz[2][kMaxV];  // local coordinates (x in doubled sites)
-  int32_t vgx[2][kMaxV], vgy[2][kMaxV], vgz[2][kMaxV];  // global coordinates
-  uint8_t vact[2][kMaxV];       // vacancy still inside the active sector
-  // the same record packed for the selection, which every warp reads: (local site, local x, y,
-  // z) and (global x, y, z, site id), two 16-byte loads instead of seven
-  alignas(16) int4 vpk[2][kMaxV][2];
-  int32_t ord[2][kMaxV];        // the active vacancies in z-y-x order (ascending site id)
+  // Vacancy record k: (local site, local x, y, z) and (global x, y, z, site id), x in doubled
+  // sites.  A hop's record and rates are written after its middle barrier, when every warp has
+  // selected from the old ones.
+  alignas(16) int4 vpk[kMaxV][2];
+  alignas(16) double rates[kMaxV][8];
+  alignas(8) uint8_t vX[kMaxV][8];  // code of jump b's target atom (0: the target is a vacancy)
+  uint8_t vact[kMaxV];          // vacancy still inside the active sector
+  int32_t ord[2][kMaxV];        // the active vacancies in z-y-x order (ascending site id), in two sets
   int32_t nord[2];
-  uint8_t vX[2][kMaxV][8];      // code of jump b's target atom (0: the target is a vacancy)
-  alignas(16) double rates[2][kMaxV][8];
   // F-table window, two planes: FP64 (c0, c1) x kFWin then (c2, c3) x kFWin;
   // FP32 (hi, lo, c1, c2) x kFWin then c3 x kFWin
   alignas(16) unsigned char fwin[kFWin * 32];
@@ -180,29 +190,30 @@ struct Smem {
   uint32_t mbar_phase, mbst_phase;
   int32_t win_pot;                             // potential (and precision) the window holds
   int32_t tab_key[2];                          // potential, kind and region strides the tables hold
-  // hop-loop control, written by the control thread, in slots of the iteration parity
-  double ctl_u[2];         // the selection's uniform, drawn ahead
-  int32_t ctl_stop[2];     // the sector's window is reached (or the hop cap): no more selections
-  uint64_t xsn[2][4];      // selection stream after the uniform drawn ahead
   int32_t ctl_ok;          // the region's copies arrived
-  int32_t fin;             // record set that holds the block's vacancies after run_block
-  uint64_t xs[4], xt[4];  // the block's selection / residence-time streams while it runs
+  int32_t ctl_stop;        // the sector's window is reached (or the hop cap): no more selections
+  // the block's selection (0) and residence-time (1) streams: running state, the draws made
+  // ahead, the state after each, and what the draws stand for (uniform, -ln uniform)
+  uint64_t str[2][4];
+  uint64_t raw[2][kDrawRing], sts[kDrawRing][2][4];
+  double du[kDrawRing], dl[kDrawRing];
   // asynchronous schedule (k_flow)
   int8_t flow_lag[8][27];
-  int32_t flow_cand[kMaxThreads];
+  int32_t flow_cand[kMaxTake];
   int32_t flow_ncand, flow_stop, flow_progress, flow_more;
   int32_t fv[kFlowSlots], fslot[kFlowSlots], fnv;  // the sector's vacancies and their slots
   int32_t fsite[kFlowSlots];                        // their sites
-  int64_t flow_cr[kMaxThreads], flow_ct[kMaxThreads];  // round and target of each round handed over
-  unsigned long long flow_cvv[kMaxThreads];             // its block's vacancy-slot valid bits
+  int64_t flow_cr[kMaxTake], flow_ct[kMaxTake];        // round and target of each round handed over
+  unsigned long long flow_cvv[kMaxTake];                // its block's vacancy-slot valid bits
   int64_t cur_r, cur_t;   // the block's round and target for its next chained round
   int32_t bc0[3], bc1[3];  // the running block's area and its job's block count, kept for the
   int32_t bnb;             // post-round updates (a reload after the round's stores is an L2 trip)
   int64_t hops_out;       // the block's hop count after run_block
-  // run_block's control thread: hops at the start, hops, n_act sum and evaluations of the
-  // block-round, the sector's clock and its threshold
+  // run_block's clock thread: hops at the start, hops, n_act sum and evaluations of the
+  // block-round, selections made, the sector's clock and its threshold
   int64_t c_hop0, c_nh, c_nact, c_evals;
-  double c_time, c_thr;
+  int32_t c_sel, c_path;
+  double c_time;
   double c_nu, c_kT;  // the job's attempt frequency and kT (the rates' constants)
   double c_rkT;       // RN(1 / kT): the rates' exponent arguments without a division
   double pre_evo;         // the active sector's clock, read while the region's copies fly
@@ -302,7 +313,6 @@ __device__ void load_tables(Smem& sm, const Potential& P, const Geometry& G, con
   if (tid < 16) {
     const int32_t w = G.nn1[tid >> 3][tid & 7];
     sm.d1[tid >> 3][tid & 7] = local_delta(w, R);
-    sm.w1[tid >> 3][tid & 7] = w;
   }
   if (tid < 6) sm.d2[tid] = local_delta(G.nn2[tid], R);
   if (eam) {
@@ -315,20 +325,13 @@ __device__ void load_tables(Smem& sm, const Potential& P, const Geometry& G, con
       else sm.dphi32[i] = pf[hs] - pf[ht];
       if (i < 4 * 64) sm.dfq[i] = P.fq[i >> 6][hs] - P.fq[i >> 6][ht];
     }
-    for (int i = tid; i < 2 * 8 * kJumpN; i += kThreads) {
-      const int32_t w = __ldg(&G.jump[0][0][0] + i);
-      (&sm.jl[0][0][0])[i] = (local_delta(w, R) & 0xffff) | ((unpack_sh_s(w) * 8 + unpack_sh_t(w)) << 16);
-    }
-    for (int i = tid; i < 2 * 8 * kRefreshN; i += kThreads) {
-      const int32_t w = __ldg(&G.refresh[0][0][0] + i);
-      (&sm.rl[0][0][0])[i] = (w & 0xffffff) | ((unpack_sh_s(w) * 8 + unpack_sh_t(w)) << 24);
-    }
+    for (int i = tid; i < 8 * kFootSlots / 4; i += kThreads)
+      reinterpret_cast<uint32_t*>(&sm.rf[0][0])[i] = __ldg(reinterpret_cast<const uint32_t*>(&G.foot_refresh[0][0]) + i);
+    if (tid < kTermSets) sm.term[tid][kZeroTerm] = 0.0;
   }
 }
 
 __device__ __forceinline__ int sdelta(int32_t e) { return static_cast<int16_t>(e & 0xffff); }
-__device__ __forceinline__ int jshells(int32_t e) { return (e >> 16) & 63; }
-__device__ __forceinline__ int rshells(int32_t e) { return (e >> 24) & 63; }
 
 // Cells outside the shared-memory window (rare): global memory, range-checked.
 __device__ __noinline__ double F64_far(const double2* g64lo, const double2* g64hi, unsigned int* status, int32_t r,
@@ -397,162 +400,286 @@ __device__ __forceinline__ FCell32 cell32(const FTab& T, int32_t r) {
   return c;
 }
 
-// Rates of vacancy k of record set `set`, all 8 jumps, CTA-collective (no barrier inside; the
-// caller synchronises before the rates are read).  Warp b evaluates jump b.
-//  pair-bond: lanes 0..3 run the four bond counts of VacRatesSolver::deltaE
-//             (vacancy_rates_solver.cpp:45-116), each summed in the reference order;
-//  EAM:       lane q sums sites i = q, q+32, q+64 of the jump's list; the 32 partials
-//             merge by a xor butterfly (16, 8, 4, 2, 1), then the moving atom's own
-//             embedding change is added.
-// l is the vacancy's local site (its record's vloc), d1b[p] jump b's 1nn offset for x parity p.
-template <int KIND>
-__device__ void eval_vacancy(Smem& sm, int set, const uint8_t* occ_s, const int32_t* rho_s, int k, int l, int b,
-                             const int32_t (&d1b)[2], const FTab& FT, const JobC& jc, const int32_t (&jr)[2][3],
-                             double* de_out) {
-  const int lane = threadIdx.x & 31;
-  const int q = lane;
-  const int p = l & 1;
-  const int tl = l + (p ? d1b[1] : d1b[0]);
-  const uint8_t Xc = occ_s[tl];
+// The rate of a jump with energy change dE of atom Xc (0: the target is a vacancy), into the record of
+// vacancy k and jump b.
+__device__ __forceinline__ void put_rate(Smem& sm, int k, int b, uint8_t Xc, double dE, double* de_out) {
   const bool avail = is_atom(Xc);
-  double dE = 0.0;
-#ifdef AKMC_PHASE_PROFILE
-  long long tev = clock64();
-#endif
-  if (KIND == kPairBond) {
-    double energy = 0.0;
-    if (avail && q < 4) {
-      const bool at_t = (q & 1) != 0;
-      const int center = at_t ? tl : l;
-      const int pc = at_t ? (p ^ 1) : p;
-      const uint8_t src = (q == 0 || q == 3) ? static_cast<uint8_t>(kV) : Xc;
-      const int ovr = q == 2 ? tl : (q == 3 ? l : -1);
-      const uint8_t ovr_code = q == 2 ? static_cast<uint8_t>(kV) : Xc;
-      const int si = bond_index(src);
-      for (int b2 = 0; b2 < 8; ++b2) {
-        const int nb = center + sm.d1[pc][b2];
-        const uint8_t o = nb == ovr ? ovr_code : occ_s[nb];
-        energy += sm.b1[bond_index(o) * 5 + si];
-      }
+  sm.rates[k][b] = avail ? arrhenius_rk(sm.c_nu, sm.c_kT, sm.c_rkT, Xc, dE) : 0.0;
+  sm.vX[k][b] = avail ? Xc : 0;
+  if (de_out) de_out[k * 8 + b] = avail ? dE : 0.0;  // akmc_calculate only
+}
+
+// Pair bond: the rates of vacancy k at local site l, by one warp.  Lanes 4 b + 0..3 run the four bond
+// counts of VacRatesSolver::deltaE (vacancy_rates_solver.cpp:45-116) for jump b, each summed in the
+// reference order.
+__device__ __forceinline__ void pair_rates(Smem& sm, const uint8_t* occ_s, int k, int l, double* de_out) {
+  const int lane = threadIdx.x & 31, b = lane >> 2, q = lane & 3;
+  const int p = l & 1;
+  const int tl = l + sm.d1[p][b];
+  const uint8_t Xc = occ_s[tl];
+  const bool at_t = (q & 1) != 0;
+  const int center = at_t ? tl : l;
+  const int pc = at_t ? (p ^ 1) : p;
+  const uint8_t src = (q == 0 || q == 3) ? static_cast<uint8_t>(kV) : Xc;
+  const int ovr = q == 2 ? tl : (q == 3 ? l : -1);
+  const uint8_t ovr_code = q == 2 ? static_cast<uint8_t>(kV) : Xc;
+  const int si = bond_index(src);
+  double energy = 0.0;
 #pragma unroll
-      for (int b2 = 0; b2 < 6; ++b2) {
-        if (!((0x2F >> b2) & 1)) continue;  // PeriodLatticeList::get2nnStatus
-        const int nb = center + sm.d2[b2];
-        const uint8_t o = nb == ovr ? ovr_code : occ_s[nb];
-        energy += sm.b2[bond_index(o) * 5 + si];
-      }
+  for (int b2 = 0; b2 < 8; ++b2) {
+    const int nb = center + sm.d1[pc][b2];
+    const uint8_t o = nb == ovr ? ovr_code : occ_s[nb];
+    energy += sm.b1[bond_index(o) * 5 + si];
+  }
+#pragma unroll
+  for (int b2 = 0; b2 < 6; ++b2) {
+    if (!((0x2F >> b2) & 1)) continue;  // PeriodLatticeList::get2nnStatus
+    const int nb = center + sm.d2[b2];
+    const uint8_t o = nb == ovr ? ovr_code : occ_s[nb];
+    energy += sm.b2[bond_index(o) * 5 + si];
+  }
+  const double pair = energy + __shfl_down_sync(kFull, energy, 1);  // q0: e_before, q2: e_after
+  const double after = __shfl_down_sync(kFull, pair, 2);
+  if (q == 0) put_rate(sm, k, b, Xc, after - pair, de_out);
+}
+
+// A lane's share of the dE terms (Geometry::foot_*): its site's local offset (x parity 0 in the low half,
+// 1 in the high), the terms it writes, the shell pairs of its two evaluations and their density changes
+// for a moving Fe atom.
+struct Slot {
+  int32_t off, out, sh, dA, dB;
+};
+
+// FP32 F cell at density r: the node and the polynomial part of dF32.
+struct F32Val {
+  float hi, lo, q;
+};
+__device__ __forceinline__ F32Val F32part(const FCell32& c, int32_t r) {
+  const float p = static_cast<float>(r & kRhoFracMask) * 0x1p-17f;
+  F32Val v;
+  v.hi = c.hi;
+  v.lo = c.lo;
+  v.q = fma_f(fma_f(c.c3, p, c.c2), p, c.c1) * p;
+  return v;
+}
+// F(r1) - F(r0) from the two parts: dF32's sums.
+__device__ __forceinline__ float F32diff(const F32Val& a1, const F32Val& a0) {
+  const float node = (a1.hi - a0.hi) + (a1.lo - a0.lo);
+  return node + (a1.q - a0.q);
+}
+
+// One slot of the dE terms of the vacancy at local site l for moving Fe atoms, into term set `set`;
+// all 32 lanes of a warp.  With REFRESH the vacancy has just come here from local site `from` by jump
+// b of an atom X, and the slot's leader first brings its site's density up to date (the 78 density
+// deltas of the hop all lie on the slots' sites; no other warp touches them before the next barrier).
+// `inside`: the vacancy is still in its sector; one that left it needs no terms, and some of its sites lie
+// past the region's 2-cell halo (the refreshed ones never do).
+// What bounds this: two to four 16-byte reads of random F cells a lane (about 10 shared-memory
+// wavefronts a warp and read).  Each jump's 76 sites evaluated on their own took 1232 F evaluations a
+// vacancy; the shared terms take 447.
+template <int KIND, bool REFRESH>
+__device__ __forceinline__ void foot_terms(Smem& sm, int set, const uint8_t* occ_s, int32_t* rho_s, int l, const Slot& c,
+                                           int slot, const FTab& FT, int b, int X, int from, bool inside) {
+  const int lane = threadIdx.x & 31;
+  const int lead = (c.out >> 20) & 31;
+  int j = l + ((l & 1) ? c.off >> 16 : sdelta(c.off));
+  int code = 0;
+  if (REFRESH) {
+    code = sm.rf[b][slot];
+    if (!inside && !code) j = l;  // outside the staged halo: only the deltas are wanted
+  }
+  uint8_t o = occ_s[j];
+  int32_t r = rho_s[j];
+  if (REFRESH) {
+    r += sm.dfq[atom_index(static_cast<uint8_t>(X)) * 64 + code];  // code 0: + 0
+    if (j == from) o = static_cast<uint8_t>(X);
+    __syncwarp();
+    if (code && lead == lane) rho_s[j] = r;
+  }
+  const int32_t rA = r + c.dA, rB = r + c.dB;
+  const bool win = static_cast<unsigned>((rA >> kRhoCellShift) - FT.kw0) < static_cast<unsigned>(kFWin) &&
+                   static_cast<unsigned>((rB >> kRhoCellShift) - FT.kw0) < static_cast<unsigned>(kFWin);
+  const int outA = c.out & 1023, outB = (c.out >> 10) & 1023, raw = (c.out >> 25) & 15;
+  const int hA = c.sh & 63, hB = (c.sh >> 8) & 63;
+  const bool atom = o != kV;
+  const int y = atom ? atom_index(o) * 64 : 0;
+  if (KIND == kEam64) {
+    double FA, FB;
+    if (win) {
+      FA = F64win(FT, rA);
+      FB = F64win(FT, rB);
+    } else {
+      FA = F64(FT, rA);
+      FB = F64(FT, rB);
     }
-    const double pair = energy + __shfl_down_sync(kFull, energy, 1);  // q0: e_before, q2: e_after
-    const double after = __shfl_down_sync(kFull, pair, 2);
-    dE = after - pair;
-  } else if (KIND == kEam64) {
-    double acc = 0.0, EX = 0.0;
-    const int X = atom_index(Xc);  // read only when avail
-    if (avail) {
-      // gather: this lane's sites (q, q+32, q+64 of the jump's list; lanes 12..31 have two),
-      // their occupancy, densities and shell codes, and the moving atom's own two densities
-      uint8_t o[3];
-      int32_t r0[3], r1[3];
-      int h[3];
-      bool in[3];
-#pragma unroll
-      for (int u = 0; u < 3; ++u) {
-        in[u] = q + 32 * u < kJumpN;
-        const int32_t e = p ? jr[1][u] : jr[0][u];  // 0 outside the list: the vacancy's own site
-        const int j = l + sdelta(e);
-        h[u] = jshells(e);
-        o[u] = occ_s[j];
-        r0[u] = rho_s[j];
-        r1[u] = r0[u] + sm.dfq[X * 64 + h[u]];
-      }
-      const int32_t rx1 = rho_s[l] - sm.fq1[X], rx0 = rho_s[tl];
-      // every cell inside the shared-memory window (nearly always): one straight run of loads
-      // and polynomials; otherwise the general path, which reads far cells from global memory
-      bool win = static_cast<unsigned>((rx1 >> kRhoCellShift) - FT.kw0) < static_cast<unsigned>(kFWin) &&
-                 static_cast<unsigned>((rx0 >> kRhoCellShift) - FT.kw0) < static_cast<unsigned>(kFWin);
-#pragma unroll
-      for (int u = 0; u < 3; ++u)
-        win = win && (!in[u] || (static_cast<unsigned>((r0[u] >> kRhoCellShift) - FT.kw0) < static_cast<unsigned>(kFWin) &&
-                                 static_cast<unsigned>((r1[u] >> kRhoCellShift) - FT.kw0) < static_cast<unsigned>(kFWin)));
-      double t[3];
-      if (win) {
-        EX = F64win(FT, rx1) - F64win(FT, rx0);
-#pragma unroll
-        for (int u = 0; u < 3; ++u) t[u] = in[u] ? F64win(FT, r1[u]) - F64win(FT, r0[u]) : 0.0;
-      } else {
-        EX = F64(FT, rx1) - F64(FT, rx0);
-#pragma unroll
-        for (int u = 0; u < 3; ++u) t[u] = in[u] ? F64(FT, r1[u]) - F64(FT, r0[u]) : 0.0;
-      }
-      // site term (F(r+d) - F(r)) + (phi_s - phi_t), summed in list order
-#pragma unroll
-      for (int u = 0; u < 3; ++u)
-        if (in[u] && o[u] != kV) acc += t[u] + sm.dphi64[(X * 4 + atom_index(o[u])) * 64 + h[u]];
-    }
-#pragma unroll
-    EVAL_T(0);
-    for (int m = 16; m >= 1; m >>= 1) acc = acc + __shfl_xor_sync(kFull, acc, m);
-    EVAL_T(1);
-    if (avail && q == 0) dE = EX + acc;
-    EVAL_T(2);
+    const double F0 = __shfl_sync(kFull, FA, lead);
+    const double tA = (FA - F0) + sm.dphi64[y + hA], tB = (FB - F0) + sm.dphi64[y + hB];
+    double* const T = sm.term[set];
+    if (outA != kFootNone) T[outA] = atom ? tA : 0.0;
+    if (outB != kFootNone) T[outB] = atom ? tB : 0.0;
+    if (raw) T[kTermN + raw - 1] = FA;
   } else {
+    F32Val a, bb;
+    if (win) {
+      a = F32part(cell32win(FT, rA), rA);
+      bb = F32part(cell32win(FT, rB), rB);
+    } else {
+      a = F32part(cell32(FT, rA), rA);
+      bb = F32part(cell32(FT, rB), rB);
+    }
+    F32Val f0;
+    f0.hi = __shfl_sync(kFull, a.hi, lead);
+    f0.lo = __shfl_sync(kFull, a.lo, lead);
+    f0.q = __shfl_sync(kFull, a.q, lead);
+    const float tA = F32diff(a, f0) + sm.dphi32[y + hA], tB = F32diff(bb, f0) + sm.dphi32[y + hB];
+    float2* const T = reinterpret_cast<float2*>(sm.term[set]);
+    if (outA != kFootNone) T[outA] = make_float2(tA, atom ? 1.f : 0.f);
+    if (outB != kFootNone) T[outB] = make_float2(tB, atom ? 1.f : 0.f);
+    if (raw) sm.fx[set][raw - 1] = make_float4(a.hi, a.lo, a.q, 0.f);
+  }
+}
+
+// Rates of jumps 4 half .. 4 half + 3 of vacancy k at local site l from term set `set`, by one warp, for
+// Fe targets and vacant ones; the other atoms' jumps are left to solute_rate.  Eight lanes take a jump:
+// lane sub the partial sums sub + 8 g (g = 0..3) of the 32 interleaved ones (entries i = q, q + 32, q + 64
+// of the jump's list; ix: their terms, 10 bits each), merged in the order of the 32-lane xor butterfly
+// (16, 8, 4, 2, 1).  A vacancy's site adds 0.0, which leaves every partial sum as it is: a sum that
+// starts at a term (never -0.0) cannot become -0.0.
+template <int KIND>
+__device__ __forceinline__ void jump_rates(Smem& sm, int set, const uint8_t* occ_s, int k, int l, int half,
+                                           const int32_t (&ix)[2][4], double* de_out) {
+  const int lane = threadIdx.x & 31, b = 4 * half + (lane >> 3);
+  const int p = l & 1;
+  const uint8_t Xc = occ_s[l + sm.d1[p][b]];
+  const int32_t w0 = p ? ix[1][0] : ix[0][0], w1 = p ? ix[1][1] : ix[0][1], w2 = p ? ix[1][2] : ix[0][2],
+                w3 = p ? ix[1][3] : ix[0][3];
+  const int i[10] = {w0 & 1023, (w0 >> 10) & 1023, (w0 >> 20) & 1023, w1 & 1023, (w1 >> 10) & 1023,
+                     (w1 >> 20) & 1023, w2 & 1023, (w2 >> 10) & 1023, (w2 >> 20) & 1023, w3 & 1023};
+  double dE;
+  if (KIND == kEam64) {
+    const double* T = sm.term[set];
+    double t[10];
+#pragma unroll
+    for (int q = 0; q < 10; ++q) t[q] = T[i[q]];
+    const double EX = T[kTermN] - T[kTermN + 1 + b];
+    const double g0 = (t[0] + t[1]) + t[2], g1 = (t[3] + t[4]) + t[5], g2 = t[6] + t[7], g3 = t[8] + t[9];
+    double x = (g0 + g2) + (g1 + g3);
+#pragma unroll
+    for (int m = 4; m >= 1; m >>= 1) x = x + __shfl_xor_sync(kFull, x, m);
+    dE = EX + x;
+  } else {
+    const float2* T = reinterpret_cast<const float2*>(sm.term[set]);
+    float2 t[10];
+#pragma unroll
+    for (int q = 0; q < 10; ++q) t[q] = T[i[q]];
+    const float4 f1 = sm.fx[set][0], f0 = sm.fx[set][1 + b];
+    const F32Val e1 = {f1.x, f1.y, f1.z}, e0 = {f0.x, f0.y, f0.z};
+    const float EX = F32diff(e1, e0);
+    Comp32 g[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      g[q].s = g[q].c = 0.f;
+      const int first = q < 2 ? 3 * q : 6 + 2 * (q - 2), n = q < 2 ? 3 : 2;
+#pragma unroll
+      for (int v = 0; v < 3; ++v)
+        if (v < n && t[first + v].y != 0.f) kahan_add(g[q], t[first + v].x);
+    }
+    Comp32 x = comp_merge(comp_merge(g[0], g[2]), comp_merge(g[1], g[3]));
+#pragma unroll
+    for (int m = 4; m >= 1; m >>= 1) {
+      Comp32 o;
+      o.s = __shfl_xor_sync(kFull, x.s, m);
+      o.c = __shfl_xor_sync(kFull, x.c, m);
+      x = comp_merge(x, o);
+    }
+    dE = static_cast<double>(EX + (x.s - x.c));
+  }
+  if ((lane & 7) == 0 && (Xc == kFe || !is_atom(Xc))) put_rate(sm, k, b, Xc, dE, de_out);
+}
+
+// Rate of jump b of vacancy k at local site l with a solute target (the shared terms are those of a
+// moving Fe atom), by one warp; nothing for other targets.  Lane q sums sites i = q, q + 32, q + 64 of the
+// jump's list (jl: the list's packed entries); the 32 partials merge by a xor butterfly (16, 8, 4, 2, 1),
+// then the moving atom's own embedding change is added.
+template <int KIND>
+__device__ __forceinline__ void solute_rate(Smem& sm, const uint8_t* occ_s, const int32_t* rho_s, int k, int l, int b,
+                                            const Region& R, const Geometry& G, const FTab& FT, double* de_out) {
+  const int q = threadIdx.x & 31;
+  const int p = l & 1;
+  const int tl = l + sm.d1[p][b];
+  const uint8_t Xc = occ_s[tl];
+  if (Xc == kFe || !is_atom(Xc)) return;  // uniform
+  const int X = atom_index(Xc);
+  uint8_t o[3];
+  int32_t r0[3], r1[3];
+  int h[3];
+  bool in[3];
+#pragma unroll
+  for (int u = 0; u < 3; ++u) {
+    in[u] = q + 32 * u < kJumpN;
+    const int32_t e = in[u] ? __ldg(&G.jump[p][b][q + 32 * u]) : 0;  // outside the list: the vacancy's own site
+    const int j = l + local_delta(e, R);
+    h[u] = unpack_sh_s(e) * 8 + unpack_sh_t(e);
+    o[u] = occ_s[j];
+    r0[u] = rho_s[j];
+    r1[u] = r0[u] + sm.dfq[X * 64 + h[u]];
+  }
+  const int32_t rx1 = rho_s[l] - sm.fq1[X], rx0 = rho_s[tl];
+  // every cell inside the shared-memory window (nearly always): one straight run of loads
+  // and polynomials; otherwise the general path, which reads far cells from global memory
+  bool win = static_cast<unsigned>((rx1 >> kRhoCellShift) - FT.kw0) < static_cast<unsigned>(kFWin) &&
+             static_cast<unsigned>((rx0 >> kRhoCellShift) - FT.kw0) < static_cast<unsigned>(kFWin);
+#pragma unroll
+  for (int u = 0; u < 3; ++u)
+    win = win && (!in[u] || (static_cast<unsigned>((r0[u] >> kRhoCellShift) - FT.kw0) < static_cast<unsigned>(kFWin) &&
+                             static_cast<unsigned>((r1[u] >> kRhoCellShift) - FT.kw0) < static_cast<unsigned>(kFWin)));
+  double dE;
+  if (KIND == kEam64) {
+    double t[3], EX;
+    if (win) {
+      EX = F64win(FT, rx1) - F64win(FT, rx0);
+#pragma unroll
+      for (int u = 0; u < 3; ++u) t[u] = in[u] ? F64win(FT, r1[u]) - F64win(FT, r0[u]) : 0.0;
+    } else {
+      EX = F64(FT, rx1) - F64(FT, rx0);
+#pragma unroll
+      for (int u = 0; u < 3; ++u) t[u] = in[u] ? F64(FT, r1[u]) - F64(FT, r0[u]) : 0.0;
+    }
+    // site term (F(r+d) - F(r)) + (phi_s - phi_t), summed in list order
+    double acc = 0.0;
+#pragma unroll
+    for (int u = 0; u < 3; ++u)
+      if (in[u] && o[u] != kV) acc += t[u] + sm.dphi64[(X * 4 + atom_index(o[u])) * 64 + h[u]];
+#pragma unroll
+    for (int m = 16; m >= 1; m >>= 1) acc = acc + __shfl_xor_sync(kFull, acc, m);
+    dE = EX + acc;
+  } else {
+    float t[3], EX;
+    if (win) {
+      EX = dF32(cell32win(FT, rx1), cell32win(FT, rx0), rx1, rx0);
+#pragma unroll
+      for (int u = 0; u < 3; ++u) t[u] = in[u] ? dF32(cell32win(FT, r1[u]), cell32win(FT, r0[u]), r1[u], r0[u]) : 0.f;
+    } else {
+      EX = dF32(cell32(FT, rx1), cell32(FT, rx0), rx1, rx0);
+#pragma unroll
+      for (int u = 0; u < 3; ++u) t[u] = in[u] ? dF32(cell32(FT, r1[u]), cell32(FT, r0[u]), r1[u], r0[u]) : 0.f;
+    }
     Comp32 acc;
     acc.s = 0.f;
     acc.c = 0.f;
-    const int X = atom_index(Xc);  // read only when avail
-    if (avail) {
-      uint8_t o[3];
-      int32_t r0[3], r1[3];
-      int h[3];
-      bool in[3];
 #pragma unroll
-      for (int u = 0; u < 3; ++u) {
-        in[u] = q + 32 * u < kJumpN;
-        const int32_t e = p ? jr[1][u] : jr[0][u];
-        const int j = l + sdelta(e);
-        h[u] = jshells(e);
-        o[u] = occ_s[j];
-        r0[u] = rho_s[j];
-        r1[u] = r0[u] + sm.dfq[X * 64 + h[u]];
-      }
-      bool win = true;
-#pragma unroll
-      for (int u = 0; u < 3; ++u)
-        win = win && (!in[u] || (static_cast<unsigned>((r0[u] >> kRhoCellShift) - FT.kw0) < static_cast<unsigned>(kFWin) &&
-                                 static_cast<unsigned>((r1[u] >> kRhoCellShift) - FT.kw0) < static_cast<unsigned>(kFWin)));
-      float t[3];
-      if (win) {
-#pragma unroll
-        for (int u = 0; u < 3; ++u) t[u] = in[u] ? dF32(cell32win(FT, r1[u]), cell32win(FT, r0[u]), r1[u], r0[u]) : 0.f;
-      } else {
-#pragma unroll
-        for (int u = 0; u < 3; ++u) t[u] = in[u] ? dF32(cell32(FT, r1[u]), cell32(FT, r0[u]), r1[u], r0[u]) : 0.f;
-      }
-#pragma unroll
-      for (int u = 0; u < 3; ++u)
-        if (in[u] && o[u] != kV) kahan_add(acc, t[u] + sm.dphi32[(X * 4 + atom_index(o[u])) * 64 + h[u]]);
-    }
+    for (int u = 0; u < 3; ++u)
+      if (in[u] && o[u] != kV) kahan_add(acc, t[u] + sm.dphi32[(X * 4 + atom_index(o[u])) * 64 + h[u]]);
 #pragma unroll
     for (int m = 16; m >= 1; m >>= 1) {
-      Comp32 o;
-      o.s = __shfl_xor_sync(kFull, acc.s, m);
-      o.c = __shfl_xor_sync(kFull, acc.c, m);
-      acc = comp_merge(acc, o);
+      Comp32 v;
+      v.s = __shfl_xor_sync(kFull, acc.s, m);
+      v.c = __shfl_xor_sync(kFull, acc.c, m);
+      acc = comp_merge(acc, v);
     }
-    if (avail && q == 0) {
-      const int32_t r1 = rho_s[l] - sm.fq1[X];
-      const int32_t r0 = rho_s[tl];
-      const float EX = dF32(cell32(FT, r1), cell32(FT, r0), r1, r0);
-      const float dEf = EX + (acc.s - acc.c);
-      dE = static_cast<double>(dEf);
-    }
+    dE = static_cast<double>(EX + (acc.s - acc.c));
   }
-  if (q == 0) {
-    sm.rates[set][k][b] = avail ? arrhenius_rk(sm.c_nu, sm.c_kT, sm.c_rkT, Xc, dE) : 0.0;
-    sm.vX[set][k][b] = avail ? Xc : 0;
-    if (de_out) de_out[k * 8 + b] = avail ? dE : 0.0;  // akmc_calculate only
-  }
-  if (KIND == kEam64) EVAL_T(3);
+  if (q == 0) put_rate(sm, k, b, Xc, dE, de_out);
 }
 
 // Bulk staging of a region (R.bulk): the bulk-copy unit moves whole rows, R.bo occupancy bytes
@@ -632,59 +759,40 @@ __device__ __forceinline__ void stage_tensor(const Region& R, const void* tmaps,
   } while (0)
 #endif
 
-// Hop-loop sub-phases (builds with -DAKMC_PHASE_PROFILE -DAKMC_HOP_PROFILE=1): thread 0 (an
-// evaluator) adds its cycles per stage into counters 16..19, the control thread into 20..22,
-// and counts the iterations in 23.  With -DAKMC_HOP_PROFILE=2 thread 0's four counters split
-// the perform stage instead (HOP_P).
-#if defined(AKMC_PHASE_PROFILE) && defined(AKMC_HOP_PROFILE)
-#define HOP_T(k)                                                                                           \
-  do {                                                                                                     \
-    if (threadIdx.x == 0 || threadIdx.x == kCtl) {                                                         \
-      const long long t_ = clock64();                                                                      \
-      atomicAdd(a.counters + (threadIdx.x == 0 ? 16 : 20) + (k), static_cast<unsigned long long>(t_ - thp)); \
-      thp = t_;                                                                                            \
-    }                                                                                                      \
-  } while (0)
-#else
-#define HOP_T(k) \
-  do {           \
-  } while (0)
-#endif
-#if defined(AKMC_PHASE_PROFILE) && defined(AKMC_HOP_PROFILE) && AKMC_HOP_PROFILE == 2
-#define HOP_P(k)                                                                       \
-  do {                                                                                 \
-    if (threadIdx.x == 0) {                                                            \
-      const long long t_ = clock64();                                                  \
-      atomicAdd(a.counters + 16 + (k), static_cast<unsigned long long>(t_ - thp));     \
-      thp = t_;                                                                        \
-    }                                                                                  \
-  } while (0)
-#undef HOP_T
-#define HOP_T(k)                                                                       \
-  do {                                                                                 \
-    if (threadIdx.x == 0) thp = clock64();                                             \
-  } while (0)
-#else
-#define HOP_P(k) \
-  do {           \
-  } while (0)
-#endif
+// Advances the running state of stream lane (0 selection, 1 residence time) by one draw into ring
+// slot `slot`: the raw draw and the state after it.  Called by lanes 0 and 1 of one warp.
+__device__ __forceinline__ void draw_ahead(Smem& sm, uint64_t (&x)[4], int lane, int slot) {
+  sm.raw[lane][slot] = xoshiro_next(x);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) sm.sts[slot][lane][i] = x[i];
+}
+// What a batch's draws stand for, one draw a lane: the selection uniform in [0, 1) (lanes 0-7) and
+// -ln of the residence-time uniform in (0, 1] (lanes 8-15; sublattice.inl:118-120).
+__device__ __forceinline__ void draw_values(Smem& sm, int lane, int slot0) {
+  if (lane < kDrawBatch) {
+    sm.du[slot0 + lane] = static_cast<double>(sm.raw[0][slot0 + lane] >> 11) * 0x1p-53;
+  } else if (lane < 2 * kDrawBatch) {
+    const int k = slot0 + lane - kDrawBatch;
+    sm.dl[k] = -port_log(static_cast<double>((sm.raw[1][k] >> 11) + 1) * 0x1p-53);
+  }
+}
 
-// The hop loop of one block's active sector (or one per-hop API step), CTA-collective.
+// The hop loop of one block's active sector (or, with API, one per-hop API step), CTA-collective.
 // round_now is the block's round (its completed rounds), read by the caller.
-// The evaluator warps evaluate rates (warp w: jumps w, w + kEvalWarps, ...) and refresh
-// densities; the control warp keeps the ordered vacancy list, selects, performs the occupancy
-// swap and runs the clock.
 // vlist holds the ids of the cnt_in vacancies inside the sector (any order).  Returns
 // false, uniformly, when the sector's clock is already past its window: nothing ran and
 // the vacancy arrays of sm were not filled.
-template <int KIND, int W>
-__device__ bool run_block(const RoundArgs& a, int gb, Smem& sm, uint8_t* occ_s, int32_t* rho_s,
-                          const int32_t* vlist, int cnt_in, int64_t round_now, bool flowpre = false) {
+//
+// Every warp selects for itself, all lanes alike (the ordered sums are deterministic, so no broadcast
+// is needed); the hop's updates are spread over the warps.
+template <int KIND, int W, bool API>
+__device__ __forceinline__ bool run_block(const RoundArgs& a, int gb, Smem& sm, uint8_t* occ_s, int32_t* rho_s,
+                                          const int32_t* vlist, int cnt_in, int64_t round_now, bool flowpre = false) {
   AKMC_SHAPE(W);
+  constexpr int kClk = Shape<W>::kClk, kOrdWarp = Shape<W>::kOrdWarp;
+  constexpr bool eam = KIND != kPairBond;
   const int tid = threadIdx.x;
   const int lane = tid & 31, warp = tid >> 5;
-  const bool evaluator = warp < kEvalWarps;
 #ifdef AKMC_PHASE_PROFILE
   long long tph = clock64();
 #endif
@@ -694,15 +802,14 @@ __device__ bool run_block(const RoundArgs& a, int gb, Smem& sm, uint8_t* occ_s, 
   BlockDev& B = a.blocks[gb];
   const JobDev& J = a.jobs[B.job];
   const Potential& P = a.pots[J.pot];
-  const bool eam = KIND != kPairBond;
   // the block record, the lattice and the vacancy table are read at L2 (__ldcg): under the
   // asynchronous schedule another SM may have written them since this SM last looked
-  const int sec = a.mode == kModeRound ? sector_of_round(round_now) : a.api_sector;
+  const int sec = API ? a.api_sector : sector_of_round(round_now);
   // flowpre (k_flow): the caller issued a bulk region's copies on mbar_st already, and left the
-  // sector's clock (sm.pre_evo), the streams (sm.xs, sm.xt) and the vacancies' sites (sm.fsite)
-  // in shared memory, read while the copies were in flight
+  // sector's clock (sm.pre_evo), the block's hops (sm.hops_out), the streams (sm.str) and the
+  // vacancies' sites (sm.fsite) in shared memory, read while the copies were in flight
   double thr = 0.0;
-  if (a.mode == kModeRound) {
+  if (!API) {
     const int64_t step = round_now >> 3;
     thr = static_cast<double>(step + 1) * J.window - (flowpre ? sm.pre_evo : __ldcg(&B.evo[sec]));
     if (!(0.0 < thr)) {  // sector_time stays 0 (sublattice.inl:82)
@@ -735,8 +842,8 @@ __device__ bool run_block(const RoundArgs& a, int gb, Smem& sm, uint8_t* occ_s, 
   // F-table window: one bulk copy issued by the control thread, overlapped with the staging
   const int win_key = J.pot * 2 + (KIND == kEam32 ? 1 : 0);
   const bool need_win = eam && sm.win_pot != win_key;
-  // the shell tables and neighbour lists depend on the potential, the kind and the region's
-  // row strides only: kept from the CTA's previous block when those match
+  // the shell tables depend on the potential, the kind and the region's row strides only: kept
+  // from the CTA's previous block when those match
   const int tab0 = J.pot * 4 + KIND, tab1 = R.LX | (R.LY << 16);
   const bool need_tab = sm.tab_key[0] != tab0 || sm.tab_key[1] != tab1;
   const int nrows = R.LY * R.LZ;
@@ -772,7 +879,7 @@ __device__ bool run_block(const RoundArgs& a, int gb, Smem& sm, uint8_t* occ_s, 
 #endif
   AKMC_STAGE_T(1);
 
-  // stage the region: warp w takes rows w, w+9, ...; kStageRows rows of loads are issued
+  // stage the region: warp w takes rows w, w + W, ...; kStageRows rows of loads are issued
   // before any shared-memory store so they are all in flight (rows hold <= 64 sites)
   if (!R.bulk) {
     // row positions of the region's x span (the halo holds the sites past either end)
@@ -833,48 +940,74 @@ __device__ bool run_block(const RoundArgs& a, int gb, Smem& sm, uint8_t* occ_s, 
     const int z = t / jc.sy;
     const int lx = X - R.ox, ly = y - R.oy, lz = z - R.oz;
     sm.vidx[tid] = v;
-    sm.vloc[0][tid] = lx + R.LX * (ly + R.LY * lz);
-    sm.vlid[0][tid] = s;
-    sm.vcx[0][tid] = static_cast<int16_t>(lx);
-    sm.vcy[0][tid] = static_cast<int16_t>(ly);
-    sm.vcz[0][tid] = static_cast<int16_t>(lz);
-    sm.vgx[0][tid] = X;
-    sm.vgy[0][tid] = y;
-    sm.vgz[0][tid] = z;
-    sm.vact[0][tid] = 1;
-    sm.vpk[0][tid][0] = make_int4(lx + R.LX * (ly + R.LY * lz), lx, ly, lz);
-    sm.vpk[0][tid][1] = make_int4(X, y, z, s);
+    sm.vact[tid] = 1;
+    sm.vpk[tid][0] = make_int4(lx + R.LX * (ly + R.LY * lz), lx, ly, lz);
+    sm.vpk[tid][1] = make_int4(X, y, z, s);
+  }
+  if (!API && !flowpre && tid >= kCtl && tid < kCtl + 8) {
+    const int q = tid - kCtl;
+    sm.str[q >> 2][q & 3] = q < 4 ? __ldcg(&B.xs[q]) : __ldcg(&B.xt[q - 4]);
+  }
+  // this lane's share of the dE terms and of the jump sums, in registers, read while the copies fly
+  Slot sl[kJumpsPerWarp];
+  int32_t ix[2][4];
+  if (eam) {
+    const Geometry& G = *a.geo;
+#pragma unroll
+    for (int q = 0; q < kJumpsPerWarp; ++q) {
+      const int slot = tid + kThreads * q;
+      const int d0 = local_delta(__ldg(&G.foot_site[0][slot]), R), d1 = local_delta(__ldg(&G.foot_site[1][slot]), R);
+      sl[q].off = (d0 & 0xffff) | (d1 << 16);
+      sl[q].out = __ldg(&G.foot_out[slot]);
+      sl[q].sh = __ldg(&G.foot_shells[slot]);
+      const int hA = sl[q].sh & 63, hB = (sl[q].sh >> 8) & 63;
+      sl[q].dA = __ldg(&P.fq[0][hA >> 3]) - __ldg(&P.fq[0][hA & 7]);
+      sl[q].dB = __ldg(&P.fq[0][hB >> 3]) - __ldg(&P.fq[0][hB & 7]);
+    }
+    // the jump sums are taken by the even and odd warps of a pair (jump_rates)
+    const int b = 4 * (warp & 1) + (lane >> 3), sub = lane & 7;
+#pragma unroll
+    for (int p = 0; p < 2; ++p) {
+      auto t = [&](int i) -> int32_t { return i < kJumpN ? __ldg(&G.term[p][b][i]) : kZeroTerm; };
+      ix[p][0] = t(sub) | t(sub + 32) << 10 | t(sub + 64) << 20;
+      ix[p][1] = t(sub + 8) | t(sub + 40) << 10 | t(sub + 72) << 20;
+      ix[p][2] = t(sub + 16) | t(sub + 48) << 10 | t(sub + 24) << 20;
+      ix[p][3] = t(sub + 56);
+    }
   }
   __syncthreads();
   AKMC_STAGE_T(3);
   AKMC_PHASE(0);
-  if (tid == kCtl) {
+  if (tid < cnt) {
     // z-y-x scan order of ABVIModel::calcRates = ascending site id inside a sector
-    for (int i = 0; i < cnt; ++i) {
-      int j = i;
-      while (j > 0 && sm.vlid[0][sm.ord[0][j - 1]] > sm.vlid[0][i]) {
-        sm.ord[0][j] = sm.ord[0][j - 1];
-        --j;
-      }
-      sm.ord[0][j] = i;
+    const int s = sm.vpk[tid][1].w;
+    int rank = 0;
+    for (int i = 0; i < cnt; ++i) rank += sm.vpk[i][1].w < s ? 1 : 0;
+    sm.ord[0][rank] = tid;
+  }
+  if (!API && warp == kEvalWarps - 1) {  // the first batch of draws
+    if (lane < 2) {
+      uint64_t x[4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) x[i] = sm.str[lane][i];
+#pragma unroll 1
+      for (int k = 0; k < kDrawBatch; ++k) draw_ahead(sm, x, lane, k);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) sm.str[lane][i] = x[i];
     }
+    __syncwarp();
+    draw_values(sm, lane, 0);
+  }
+  if (tid == 64) {
     sm.nord[0] = cnt;
-    uint64_t x[4];
-    for (int i = 0; i < 4; ++i) {
-      if (flowpre) {
-        x[i] = sm.xs[i];
-      } else {
-        x[i] = __ldcg(&B.xs[i]);
-        sm.xs[i] = x[i];
-        sm.xt[i] = __ldcg(&B.xt[i]);
-      }
-    }
-    // the first selection's uniform, drawn ahead; the stream moves on only if a selection uses it
-    sm.ctl_u[0] = a.mode == kModeRound ? uniform_co(x) : 0.0;
-    for (int i = 0; i < 4; ++i) sm.xsn[0][i] = x[i];
-    sm.ctl_stop[0] = 0;
     sm.ctl_ok = 1;
-    sm.fin = 0;
+    sm.c_hop0 = flowpre ? sm.hops_out : __ldcg(&B.hops);
+    sm.c_nh = 0;
+    sm.c_nact = 0;
+    sm.c_evals = cnt;
+    sm.c_sel = 0;
+    sm.ctl_stop = 0;
+    sm.c_time = 0.0;
     if (need_win) {
       if (mbar_wait(&sm.mbar, sm.mbar_phase)) {
         sm.mbar_phase ^= 1u;
@@ -899,406 +1032,546 @@ __device__ bool run_block(const RoundArgs& a, int gb, Smem& sm, uint8_t* occ_s, 
   __syncthreads();
   AKMC_PHASE(1);
   if (!sm.ctl_ok) return true;
-  // this lane's entries of its warp's jump lists, both x parities
-  int32_t jr[kJumpsPerWarp][2][3];
-#pragma unroll
-  for (int jj = 0; jj < kJumpsPerWarp; ++jj)
-#pragma unroll
-    for (int u = 0; u < 3; ++u) {
-      const int i = lane + 32 * u;
-      const bool in = eam && evaluator && i < kJumpN;
-      const int b = warp + kEvalWarps * jj;
-      jr[jj][0][u] = in ? sm.jl[0][b][i] : 0;
-      jr[jj][1][u] = in ? sm.jl[1][b][i] : 0;
-    }
-  // and its jumps' 1nn offsets, both x parities
-  int32_t d1r[kJumpsPerWarp][2];
-#pragma unroll
-  for (int jj = 0; jj < kJumpsPerWarp; ++jj) {
-    const int b = evaluator ? warp + kEvalWarps * jj : 0;
-    d1r[jj][0] = sm.d1[0][b];
-    d1r[jj][1] = sm.d1[1][b];
-  }
-  double* const de_out = a.mode == kModeCalc ? a.api_de : nullptr;
-  const int D = eam ? 4 : 3;  // a hop changes the rates of vacancies within D cells of its origin
+  double* const de_out = API && a.mode == kModeCalc ? a.api_de : nullptr;
+  constexpr int D = eam ? 4 : 3;  // a hop changes the rates of vacancies within D cells of its origin
 
-  // first evaluation: every vacancy of the sector, into record set 0
-  if (evaluator) {
-    for (int k = 0; k < cnt; ++k) {
-      const int l = sm.vloc[0][k];
-#pragma unroll
-      for (int jj = 0; jj < kJumpsPerWarp; ++jj)
-        eval_vacancy<KIND>(sm, 0, occ_s, rho_s, k, l, warp + kEvalWarps * jj, d1r[jj], FT, jc, jr[jj], de_out);
+  // Density site i of 78 of a hop: jump b of parity p from the site with local index s and global
+  // coordinates (gX, gY, gZ).  UPDATE: the delta of moving atom X is applied first; the density is
+  // written through.
+  auto refresh = [&](int i, int p, int b, int s, int X, int gX, int gY, int gZ, bool update) {
+    const int32_t e = __ldg(&a.geo->refresh[p][b][i]);
+    const int j = s + local_delta(e, R);
+    int32_t v = rho_s[j];
+    if (update) {
+      v += sm.dfq[atom_index(static_cast<uint8_t>(X)) * 64 + unpack_sh_s(e) * 8 + unpack_sh_t(e)];
+      rho_s[j] = v;
     }
-  }
-  __syncthreads();
-  AKMC_PHASE(2);
-
-  // Hop loop, one CTA barrier per hop.  The vacancy records, the ordered list, the rates and the
-  // jump targets come in two sets: a hop selected from set c writes set n = c ^ 1, which the next
-  // hop reads, so no write of a hop meets a read of the same hop.  Every warp selects for itself
-  // (the ordered sum and the scan are deterministic: every warp finds the same hop), then:
-  //  - the evaluator warps perform it (occupancy swap, the 78 density deltas, set n), meet at a
-  //    named barrier, and evaluate the vacancies the hop made dirty into set n;
-  //  - the control warp runs the hop's clock, writes its event, decides whether the sector's
-  //    window is reached and draws the next selection's uniform, into the control slots of the
-  //    next iteration (indexed by iteration parity).
-  // A selection that finds no jump (u * total reached no running sum) advances the clock only and
-  // keeps set c.
-  // the control thread's running values live in shared memory (sm.c_*): held in registers they
-  // would be live in every thread across the loop
-  if (tid == kCtl) {
-    sm.c_hop0 = __ldcg(&B.hops);
-    sm.c_nh = 0;
-    sm.c_nact = 0;
-    sm.c_evals = cnt;
-    sm.c_time = 0.0;
-    sm.c_thr = thr;
-  }
-  int c = 0;   // record set of the current selection
-  int it = 0;  // iteration parity: control slots
-  // vacancy k of record set `set` lies within D cells of the cell (qx, qy, qz) and in the sector
-  auto dirty = [&](int set, int k, int qx, int qy, int qz) -> bool {
-    return sm.vact[set][k] && abs((sm.vcx[set][k] >> 1) - qx) <= D && abs(sm.vcy[set][k] - qy) <= D &&
-           abs(sm.vcz[set][k] - qz) <= D;
+    const int gx = wrap1(gX + unpack_dx(e), jc.sx), gy = wrap1(gY + unpack_dy(e), jc.sy),
+              gz = wrap1(gZ + unpack_dz(e), jc.sz);
+    lattice_put(jc.rho + static_cast<int64_t>(jc.px) * (gy + static_cast<int64_t>(jc.sy) * gz), jc.sx, gx, v);
   };
-#if defined(AKMC_PHASE_PROFILE) && defined(AKMC_HOP_PROFILE)
-  long long thp = clock64();
-#endif
-  while (true) {
-    // the active count and the first active vacancy, read with the loop's stop word
-    const int nord = sm.nord[c];
-    const int k0 = sm.ord[c][0];
-    if (sm.ctl_stop[it]) break;
-    const int n = c ^ 1;
-    // With one active vacancy (nearly every sector at these dilutions) that vacancy is the one
-    // that hops: its record is read while lane 0 selects (k0 is any value when nord != 1).
-    const int kq = nord == 1 ? k0 : 0;
-    const int4 pa = sm.vpk[c][kq][0], pb = sm.vpk[c][kq][1];
-    int s = pa.x;
-    int vx2 = pa.y, qy = pa.z, qz = pa.w;
-    int sX = pb.x, sY = pb.y, sZ = pb.z;
-    // [1] selection: lane 0 of every warp forms the ordered total (ABVIModel::calcRates,
-    // kmc.cpp:68-115), then finds the first of the same running sums above u * total
-    // (ABVIModel::select, kmc.cpp:242-309).  Jumps onto a vacancy hold 0.0, which leaves a
-    // positive sum unchanged.  With one active vacancy the running sums of the total's pass stay
-    // in registers (its 8 rates read in four 16-byte loads) and are compared afterwards,
-    // independently of one another, instead of being formed a second time.
-    int isel = -1, stop = 0;
-    double total = 0.0, u = 0.0;
-    if (lane == 0) {
-      double pv[8];
-      if (nord == 1) {
-        const double2* r2 = reinterpret_cast<const double2*>(sm.rates[c][kq]);
-        const double2 a0 = r2[0], a1 = r2[1], a2 = r2[2], a3 = r2[3];
-        pv[0] = total + a0.x;
-        pv[1] = pv[0] + a0.y;
-        pv[2] = pv[1] + a1.x;
-        pv[3] = pv[2] + a1.y;
-        pv[4] = pv[3] + a2.x;
-        pv[5] = pv[4] + a2.y;
-        pv[6] = pv[5] + a3.x;
-        pv[7] = pv[6] + a3.y;
-        total = pv[7];
-      } else {
-        for (int i = 0; i < nord; ++i) {
-          const double* r = sm.rates[c][sm.ord[c][i]];
+  // Occupancy o of the site (gX, gY, gZ), written through.
+  auto put_occ = [&](int gX, int gY, int gZ, uint8_t o) {
+    lattice_put(jc.occ + static_cast<int64_t>(jc.px) * (gY + static_cast<int64_t>(jc.sy) * gZ), jc.sx, gX, o);
+  };
+  auto in_sector = [&](int lx, int ly, int lz) -> bool {
+    return (lx >> 1) >= R.hx && (lx >> 1) < R.hx + R.w[0] && ly >= 2 && ly < 2 + R.w[1] && lz >= 2 && lz < 2 + R.w[2];
+  };
+  // The ordered total of one vacancy's rates and its selection (ABVIModel::calcRates, kmc.cpp:68-115,
+  // and select, kmc.cpp:242-309), alike in every lane of the calling warps: lane q also forms the running
+  // sum through jump q (adding 0.0 to a non-negative sum leaves it as it is), and the first running sum
+  // above u * total wins.  Jumps onto a vacancy hold 0.0.  Returns the lanes above u * total.
+  auto select_one = [&](const double2 (&r2)[4], double u, double& total) -> unsigned {
+    const double rr[8] = {r2[0].x, r2[0].y, r2[1].x, r2[1].y, r2[2].x, r2[2].y, r2[3].x, r2[3].y};
+    double t = 0.0, x = 0.0;
 #pragma unroll
-          for (int bb = 0; bb < 8; ++bb) total += r[bb];
-        }
-      }
-      if (a.mode == kModeCalc) {
+    for (int q = 0; q < 8; ++q) {
+      t += rr[q];
+      x += q <= lane ? rr[q] : 0.0;
+    }
+    total = t;
+    const double expected = u * t;  // ModelAdapter::selectAndPerform
+    return __ballot_sync(kFull, lane < 8 && x > expected);
+  };
+  // The clock thread: the selection used draw `it`; advances the sector's clock and decides
+  // whether its window is reached.  Returns the residence time.
+  auto clock_step = [&](int it, double total, bool hop, int n_act) -> double {
+    const double dt = sm.dl[it & (kDrawRing - 1)] / total;
+    const double t = sm.c_time + dt;
+    int stop = t < thr ? 0 : 1;
+    sm.c_time = t;
+    sm.c_sel = it + 1;
+    if (hop) {
+      sm.c_nact += n_act;
+      const int64_t nh = sm.c_nh + 1;
+      sm.c_nh = nh;
+      if (nh >= a.hop_cap) {
+        atomicOr(a.status, kErrHopCap);
         stop = 1;
-      } else if (total == 0.0 || fabs(total) < DBL_EPSILON) {  // sublattice.inl:108-112
-        stop = 2;
-      } else {
-        u = a.mode == kModeSelectPerform ? a.api_u : sm.ctl_u[it];
-        const double expected = u * total;  // ModelAdapter::selectAndPerform
-        if (nord == 1) {
+      }
+    }
+    sm.ctl_stop = stop;
+    return dt;
+  };
+  // The event record of the hop just counted (hop index c_hop0 + c_nh - 1).
+  auto log_event = [&](int from, int to, int X, double u, double total, double dt, int n_act, int nd) {
+    const unsigned long long slot = atomicAdd(a.log_count, 1ull);
+    if (slot < static_cast<unsigned long long>(a.log_cap)) {
+      akmc_event* e = a.log + slot;
+      e->round = round_now;
+      e->hop = sm.c_hop0 + sm.c_nh - 1;
+      e->from_site = from;
+      e->to_site = to;
+      e->block = B.local_id;
+      e->species = X;
+      e->u = u;
+      e->total = total;
+      e->dt = dt;
+      e->n_act = n_act;
+      e->n_dirty = nd;
+      e->job = B.job;
+      e->reserved = 0;
+    } else {
+      atomicOr(a.status, kErrLogOverflow);
+    }
+  };
+  // One draw of each stream ahead of its use, a batch after the one in use; the batch's values when
+  // it is complete.  Iteration `it`, by the last warp.
+  auto draw_step = [&](int it) {
+    if (lane < 2) {
+      uint64_t x[4];
 #pragma unroll
-          for (int q = 7; q >= 0; --q)
-            if (pv[q] > expected) isel = q;
-        } else {
-          double acc = 0.0;
-          for (int i = 0; i < nord && isel < 0; ++i) {
-            const double* r = sm.rates[c][sm.ord[c][i]];
-            for (int bb = 0; bb < 8; ++bb) {
-              acc += r[bb];
-              if (acc > expected) {
-                isel = i * 8 + bb;
-                break;
-              }
-            }
-          }
-        }
+      for (int i = 0; i < 4; ++i) x[i] = sm.str[lane][i];
+      draw_ahead(sm, x, lane, (it + kDrawBatch) & (kDrawRing - 1));
+#pragma unroll
+      for (int i = 0; i < 4; ++i) sm.str[lane][i] = x[i];
+    }
+    if ((it & (kDrawBatch - 1)) == kDrawBatch - 1) {
+      __syncwarp();
+      draw_values(sm, lane, (it + 1) & (kDrawRing - 1));
+    }
+  };
+
+  if (!API && cnt == 1 && !eam) {
+    // One vacancy, pair bond: warp 0 runs the whole hop loop without a CTA barrier (32 lanes hold the 4
+    // bond counts of all 8 jumps); warp 1 draws ahead, a batch at a time.  Only occupancies change: the
+    // path is kept and its sites written through when the loop ends (or the list is full).
+    int2* const path = reinterpret_cast<int2*>(&sm.term[0][0]);  // (local site, site id)
+    constexpr int kPath = 512;
+    static_assert(kPath * sizeof(int2) <= sizeof(sm.term), "the path fits in the term sets");
+    auto put_path = [&](int n, int t0, int nt) {
+      for (int i = t0; i < n; i += nt) {
+        const int2 e = path[i];
+        const int t = e.y / jc.sx;
+        put_occ(e.y % jc.sx, t % jc.sy, t / jc.sy, occ_s[e.x]);
       }
-    }
-    isel = __shfl_sync(kFull, isel, 0);
-    stop = __shfl_sync(kFull, stop, 0);
-    HOP_T(0);
-    if (stop) {
-      if (tid == kCtl) {
-        if (stop == 1) {  // akmc_calculate: the sector's vacancies with their jump rates
-          *a.api_total = total;
-          for (int i = 0; i < cnt; ++i) {
-            a.api_sites[i] = sm.vact[c][i] ? sm.vlid[c][i] : -1;
-            for (int bb = 0; bb < 8; ++bb) a.api_rates[i * 8 + bb] = sm.rates[c][i][bb];
-          }
-          *a.api_count = cnt;
-        } else {
-          if (a.mode == kModeSelectPerform) {
-            a.api_event->from_site = -1;
-            a.api_event->total = total;
-          }
-          sm.c_time = sm.c_thr;
+    };
+    if (warp == 1) {
+      // batch n is ready at the n-th meeting of the two warps; warp 0 leaves at the one it names
+      for (int n = 1;; ++n) {
+        if (lane < 2) {
+          uint64_t x[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) x[i] = sm.str[lane][i];
+#pragma unroll 1
+          for (int k = 0; k < kDrawBatch; ++k) draw_ahead(sm, x, lane, (n * kDrawBatch + k) & (kDrawRing - 1));
+#pragma unroll
+          for (int i = 0; i < 4; ++i) sm.str[lane][i] = x[i];
         }
+        __syncwarp();
+        draw_values(sm, lane, (n * kDrawBatch) & (kDrawRing - 1));
+        asm volatile("bar.sync 2, 64;" ::: "memory");
+        if (*reinterpret_cast<volatile int32_t*>(&sm.ctl_stop) == n) break;
       }
-      break;
-    }
-    // the selected jump: vacancy ksel of set c, direction bsel, atom X
-    const bool hop = isel >= 0;
-    const int bsel = hop ? (isel & 7) : 0;
-    int ksel = kq;
-    if (nord != 1) {  // several active vacancies: the selected one's record
-      ksel = hop ? sm.ord[c][isel >> 3] : 0;
-      const int4 qa = sm.vpk[c][ksel][0], qb = sm.vpk[c][ksel][1];
-      s = qa.x;
-      vx2 = qa.y;
-      qy = qa.z;
-      qz = qa.w;
-      sX = qb.x;
-      sY = qb.y;
-      sZ = qb.z;
-    }
-    const int p = s & 1;
-    const int X = hop ? sm.vX[c][ksel][bsel] : 0;
-    const int32_t wg = sm.w1[p][bsel];
-    const int snew = s + sm.d1[p][bsel];  // the vacancy's local site after the hop
-    const int qx = vx2 >> 1;
-    const int nlx = vx2 + unpack_dx(wg), nly = qy + unpack_dy(wg), nlz = qz + unpack_dz(wg);
-    const bool nact = (nlx >> 1) >= R.hx && (nlx >> 1) < R.hx + R.w[0] && nly >= 2 && nly < 2 + R.w[1] &&
-                      nlz >= 2 && nlz < 2 + R.w[2];
-    const int ngx = wrap1(sX + unpack_dx(wg), jc.sx), ngy = wrap1(sY + unpack_dy(wg), jc.sy),
-              ngz = wrap1(sZ + unpack_dz(wg), jc.sz);
-    const int32_t to_g = ngx + jc.sx * (ngy + jc.sy * ngz);
-    HOP_P(0);
-    if (evaluator) {
-      if (hop) {
-        // [2] perform (ABVIModel::perform, kmc.cpp:358-396) on the staged region, written
-        // through, and set n: items 0..77 the density deltas, 78 the occupancy swap, 79 the
-        // ordered list, then one record and 8 rates per vacancy.  With 8 evaluator warps no warp
-        // holds two kinds of item (a warp runs its kinds one after another): warps 0-2 the
-        // deltas, warp 3 the swap, warp 4 the list, warps 5-7 the records and rates.
-        const int nitems = kRefreshN + 2 + 9 * cnt;
-        int i0 = tid, lim = nitems, step = kCtl;
-        if (kEvalWarps == 8) {
-          static_assert(kRefreshN <= 96, "three warps of density deltas");
-          if (tid < 96) {
-            lim = kRefreshN;
-          } else if (tid == 96 || tid == 128) {
-            i0 = tid == 96 ? kRefreshN : kRefreshN + 1;
-            lim = i0 + 1;
-          } else if (tid >= 160) {
-            i0 = kRefreshN + 2 + (tid - 160);
-            step = 96;
-          } else {
-            lim = 0;
-          }
+    } else if (warp == 0) {
+      const int4 pa = sm.vpk[0][0], pb = sm.vpk[0][1];
+      int s = pa.x, lx = pa.y, ly = pa.z, lz = pa.w, gX = pb.x, gY = pb.y, gZ = pb.z, gid = pb.w;
+      double time = 0.0;
+      int64_t nh = 0, evals = 1;
+      int it = 0, np = 1, meets = 0;
+      if (lane == 0) path[0] = make_int2(s, gid);
+      for (;; ++it) {
+        if (it > 0 && (it & (kDrawBatch - 1)) == 0) {  // the next batch of draws
+          asm volatile("bar.sync 2, 64;" ::: "memory");
+          ++meets;
         }
-        for (int i = i0; i < lim; i += step) {
-          if (i < kRefreshN) {
-            if (eam) {
-              const int32_t e = sm.rl[p][bsel][i];
-              const int j = s + local_delta(e, R);
-              const int32_t v = rho_s[j] + sm.dfq[atom_index(static_cast<uint8_t>(X)) * 64 + rshells(e)];
-              rho_s[j] = v;
-              const int gx = wrap1(sX + unpack_dx(e), jc.sx), gy = wrap1(sY + unpack_dy(e), jc.sy),
-                        gz = wrap1(sZ + unpack_dz(e), jc.sz);
-              lattice_put(jc.rho + static_cast<int64_t>(jc.px) * (gy + static_cast<int64_t>(jc.sy) * gz), jc.sx, gx, v);
-            }
-          } else if (i == kRefreshN) {
+        pair_rates(sm, occ_s, 0, s, nullptr);
+        __syncwarp();
+        const double2* r = reinterpret_cast<const double2*>(sm.rates[0]);
+        const double2 r2[4] = {r[0], r[1], r[2], r[3]};
+        const uint64_t vX = *reinterpret_cast<const uint64_t*>(sm.vX[0]);
+        const double u = sm.du[it & (kDrawRing - 1)];
+        double total;
+        const unsigned above = select_one(r2, u, total);
+        if (total == 0.0 || fabs(total) < DBL_EPSILON) {  // sublattice.inl:108-112
+          time = thr;
+          break;
+        }
+        const double dt = sm.dl[it & (kDrawRing - 1)] / total;
+        time += dt;
+        bool stop = !(time < thr);
+        if (above) {  // else: a selection that finds no jump advances the clock only
+          const int b = __ffs(static_cast<int>(above)) - 1;
+          const int X = static_cast<int>((vX >> (8 * b)) & 0xff);
+          const int p = s & 1;
+          // 1nn offset b of parity p (LatListMeta::getIdBy1nnOffset order)
+          const int dX = (b & 4) ? 1 : -1, dy = ((b >> 1) & 1) - 1 + p, dz = (b & 1) - 1 + p;
+          lx += dX;
+          ly += dy;
+          lz += dz;
+          gX = wrap1(gX + dX, jc.sx);
+          gY = wrap1(gY + dy, jc.sy);
+          gZ = wrap1(gZ + dz, jc.sz);
+          const int snew = s + dX + R.LX * (dy + R.LY * dz);
+          const int nid = gX + jc.sx * (gY + jc.sy * gZ);
+          const bool nact = in_sector(lx, ly, lz);
+          nh += 1;
+          evals += nact ? 1 : 0;
+          __syncwarp();
+          if (lane == 0) {
             occ_s[snew] = kV;
             occ_s[s] = static_cast<uint8_t>(X);
-            lattice_put(jc.occ + static_cast<int64_t>(jc.px) * (ngy + static_cast<int64_t>(jc.sy) * ngz), jc.sx, ngx,
-                        static_cast<uint8_t>(kV));
-            lattice_put(jc.occ + static_cast<int64_t>(jc.px) * (sY + static_cast<int64_t>(jc.sy) * sZ), jc.sx, sX,
-                        static_cast<uint8_t>(X));
-          } else if (i == kRefreshN + 1) {
-            // the hopped vacancy leaves its place in the ordered list and re-enters at its new
-            // site id if it is still inside the sector
-            const int pos = isel >> 3;
-            int m = 0;
-            for (int q = 0; q < nord; ++q)
-              if (q != pos) sm.ord[n][m++] = sm.ord[c][q];
-            if (nact) {
-              int j = m;
-              while (j > 0 && sm.vlid[c][sm.ord[n][j - 1]] > to_g) {
-                sm.ord[n][j] = sm.ord[n][j - 1];
-                --j;
-              }
-              sm.ord[n][j] = ksel;
-              ++m;
+            path[np] = make_int2(snew, nid);
+            if (a.log_cap > 0) {
+              sm.c_nh = nh;
+              log_event(gid, nid, X, u, total, dt, 1, nact ? 1 : 0);
             }
-            sm.nord[n] = m;
-          } else if (i < kRefreshN + 2 + cnt) {
-            const int k = i - kRefreshN - 2;
-            if (k == ksel) {
-              sm.vloc[n][k] = snew;
-              sm.vlid[n][k] = to_g;
-              sm.vcx[n][k] = static_cast<int16_t>(nlx);
-              sm.vcy[n][k] = static_cast<int16_t>(nly);
-              sm.vcz[n][k] = static_cast<int16_t>(nlz);
-              sm.vgx[n][k] = ngx;
-              sm.vgy[n][k] = ngy;
-              sm.vgz[n][k] = ngz;
-              sm.vact[n][k] = nact ? 1 : 0;
-              sm.vpk[n][k][0] = make_int4(snew, nlx, nly, nlz);
-              sm.vpk[n][k][1] = make_int4(ngx, ngy, ngz, to_g);
-            } else {
-              sm.vloc[n][k] = sm.vloc[c][k];
-              sm.vlid[n][k] = sm.vlid[c][k];
-              sm.vcx[n][k] = sm.vcx[c][k];
-              sm.vcy[n][k] = sm.vcy[c][k];
-              sm.vcz[n][k] = sm.vcz[c][k];
-              sm.vgx[n][k] = sm.vgx[c][k];
-              sm.vgy[n][k] = sm.vgy[c][k];
-              sm.vgz[n][k] = sm.vgz[c][k];
-              sm.vact[n][k] = sm.vact[c][k];
-              sm.vpk[n][k][0] = sm.vpk[c][k][0];
-              sm.vpk[n][k][1] = sm.vpk[c][k][1];
-            }
-          } else {
-            // rates of vacancy q / 8, jump q % 8 carried over; the dirty ones are overwritten below
-            const int q = i - kRefreshN - 2 - cnt;
-            (&sm.rates[n][0][0])[q] = (&sm.rates[c][0][0])[q];
-            (&sm.vX[n][0][0])[q] = (&sm.vX[c][0][0])[q];
+          }
+          __syncwarp();
+          s = snew;
+          gid = nid;
+          if (++np == kPath) {  // the list is full: write it through and start over from here
+            put_path(np, lane, 32);
+            __syncwarp();
+            if (lane == 0) path[0] = make_int2(s, gid);
+            np = 1;
+          }
+          if (nh >= a.hop_cap) {
+            if (lane == 0) atomicOr(a.status, kErrHopCap);
+            stop = true;
+          }
+          if (!nact && !stop) {  // the sector is empty now: its clock jumps to the window
+            time = thr;
+            stop = true;
           }
         }
-        HOP_P(1);
-        asm volatile("bar.sync 1, %0;" ::"n"(kCtl) : "memory");  // the evaluator warps only
-        HOP_P(2);
-        HOP_T(1);
-        // [3] + [4] the vacancies within D cells of the hop's origin, evaluated into set n
-        // (the hopped vacancy alone: dirty while it stays inside the sector, at its new site)
-        for (int base = 0; base < cnt; base += 32) {
-          const int k = base + lane;
-          unsigned m = cnt == 1 ? (nact ? 1u : 0u) : __ballot_sync(kFull, k < cnt && dirty(n, k, qx, qy, qz));
-          while (m) {
-            const int kk = base + __ffs(m) - 1;
-            m &= m - 1;
-            const int l = cnt == 1 ? snew : sm.vloc[n][kk];
-#pragma unroll
-            for (int jj = 0; jj < kJumpsPerWarp; ++jj)
-              eval_vacancy<KIND>(sm, n, occ_s, rho_s, kk, l, warp + kEvalWarps * jj, d1r[jj], FT, jc, jr[jj], nullptr);
-          }
-        }
-        HOP_T(2);
-      }
-    } else {  // control warp: the hop's clock and event, the next iteration's decision and uniform
-      int nd = 0;
-      if (hop && cnt == 1) {
-        nd = nact ? 1 : 0;
-      } else if (hop) {
-        // the dirty count, from set c with the hopped vacancy at its new cell
-        for (int base = 0; base < cnt; base += 32) {
-          const int k = base + lane;
-          const bool d = k < cnt && (k == ksel ? nact : dirty(c, k, qx, qy, qz));
-          nd += __popc(__ballot_sync(kFull, d));
+        if (stop) {
+          ++it;
+          break;
         }
       }
       if (lane == 0) {
-        const int nx = it ^ 1;
-        int nstop = 0;
-        if (a.mode == kModeSelectPerform) {  // the per-hop entry point stops after one selection
-          akmc_event* e = a.api_event;
-          e->round = 0;
-          e->hop = sm.c_hop0;
-          e->from_site = hop ? sm.vlid[c][ksel] : -1;
-          e->to_site = hop ? to_g : -1;
-          e->block = B.local_id;
-          e->species = X;
-          e->u = u;
-          e->total = total;
-          e->dt = 0.0;
-          e->n_act = nord;
-          e->n_dirty = nd;
-          e->job = B.job;
-          e->reserved = 0;
-          if (hop) {
-            sm.c_nh = 1;
-            sm.c_evals += nd;
-            sm.c_nact += nord;
-          }
-          nstop = 1;
+        sm.vpk[0][0] = make_int4(s, lx, ly, lz);
+        sm.vpk[0][1] = make_int4(gX, gY, gZ, gid);
+        sm.c_time = time;
+        sm.c_sel = it;
+        sm.c_nh = nh;
+        sm.c_nact = nh;
+        sm.c_evals = evals;
+        sm.c_path = np;
+        // the next meeting is warp 1's last
+        *reinterpret_cast<volatile int32_t*>(&sm.ctl_stop) = meets + 1;
+      }
+      __syncwarp();
+      asm volatile("bar.sync 2, 64;" ::: "memory");
+    }
+    __syncthreads();
+    put_path(sm.c_path, tid, kThreads);
+  } else if (!API && cnt == 1) {
+    // One vacancy, EAM (nearly every block-round at dilute concentrations): its record lives in
+    // registers, alike in every thread.  A hop is two phases, a CTA barrier after each:
+    //  A  warps 0 and 1: the 8 jump sums and rates from the dE terms; the others: jumps with a solute
+    //     target, then what the last hop left to do off the chain (its clock, the draws ahead, the
+    //     write-through of its 78 densities and two occupancies);
+    //  B  every warp selects, then the density deltas and dE terms at the vacancy's new site.
+    constexpr int kWt0 = kEvalWarps == 8 ? 96 : 64, kWtN = kEvalWarps == 8 ? 96 : 64;  // write-through threads
+    const int4 pa = sm.vpk[0][0], pb = sm.vpk[0][1];
+    int s = pa.x, lx = pa.y, ly = pa.z, lz = pa.w, gX = pb.x, gY = pb.y, gZ = pb.z, gid = pb.w;
+#pragma unroll
+    for (int q = 0; q < kJumpsPerWarp; ++q)
+      foot_terms<KIND, false>(sm, 0, occ_s, rho_s, s, sl[q], tid + kThreads * q, FT, 0, 0, 0, true);
+    __syncthreads();
+    // the last selection: its uniform, total, jump, atom, origin
+    bool hop = false, nact = true;
+    int b = 0, X = 0, os = 0, oX = 0, oY = 0, oZ = 0, oid = 0;
+    double u = 0.0, total = 0.0;
+    for (int it = 0;; ++it) {
+      if (nact) {
+        if (warp < 2) {
+          jump_rates<KIND>(sm, 0, occ_s, 0, s, warp, ix, nullptr);
         } else {
-          // the selection used the uniform drawn ahead: the stream moves on
-          for (int i = 0; i < 4; ++i) sm.xs[i] = sm.xsn[it][i];
-          const double u2 = uniform_oc(sm.xt);  // sublattice.inl:118-120
-          const double dt = -port_log(u2) / total;
-          sm.c_time += dt;
+#pragma unroll 1
+          for (int q = warp - 2; q < 8; q += kEvalWarps - 2) solute_rate<KIND>(sm, occ_s, rho_s, 0, s, q, R, *a.geo, FT, nullptr);
+        }
+      }
+      if (it > 0 && warp >= 2) {
+        if (tid == kClk) {
+          const double dt = clock_step(it - 1, total, hop, 1);
           if (hop) {
-            sm.c_nh += 1;
-            sm.c_evals += nd;
-            sm.c_nact += nord;
-            if (a.log_cap > 0) {
-              const unsigned long long slot = atomicAdd(a.log_count, 1ull);
-              if (slot < static_cast<unsigned long long>(a.log_cap)) {
-                akmc_event* e = a.log + slot;
-                e->round = round_now;
-                e->hop = sm.c_hop0 + sm.c_nh - 1;
-                e->from_site = sm.vlid[c][ksel];
-                e->to_site = to_g;
-                e->block = B.local_id;
-                e->species = X;
-                e->u = u;
-                e->total = total;
-                e->dt = dt;
-                e->n_act = nord;
-                e->n_dirty = nd;
-                e->job = B.job;
-                e->reserved = 0;
-              } else {
-                atomicOr(a.status, kErrLogOverflow);
-              }
-            }
-          }
-          if (!(sm.c_time < sm.c_thr)) nstop = 1;
-          if (sm.c_nh >= a.hop_cap) {
-            atomicOr(a.status, kErrHopCap);
-            nstop = 1;
-          }
-          if (!nstop) {  // the next selection's uniform, committed only if a selection uses it
-            uint64_t x[4] = {sm.xs[0], sm.xs[1], sm.xs[2], sm.xs[3]};
-            sm.ctl_u[nx] = uniform_co(x);
-            for (int i = 0; i < 4; ++i) sm.xsn[nx][i] = x[i];
+            sm.c_evals += nact ? 1 : 0;
+            if (a.log_cap > 0) log_event(oid, gid, X, u, total, dt, 1, nact ? 1 : 0);
           }
         }
-        sm.ctl_stop[nx] = nstop;
+        if (hop) {
+          if (tid >= kWt0 && tid < kWt0 + kWtN)
+            for (int i = tid - kWt0; i < kRefreshN; i += kWtN) refresh(i, os & 1, b, os, X, oX, oY, oZ, false);
+          if (tid == kCtl) put_occ(gX, gY, gZ, kV);
+          if (tid == kCtl + 1) put_occ(oX, oY, oZ, static_cast<uint8_t>(X));
+        }
+        if (warp == kEvalWarps - 1) draw_step(it - 1);
       }
-      HOP_T(1);
+      __syncthreads();
+      AKMC_PHASE(2);
+      if (it > 0 && sm.ctl_stop) break;
+      if (!nact) {  // the sector is empty now: its clock jumps to the window
+        if (tid == kClk) sm.c_time = thr;
+        break;
+      }
+      const double2* r = reinterpret_cast<const double2*>(sm.rates[0]);
+      const double2 r2[4] = {r[0], r[1], r[2], r[3]};
+      const uint64_t vX = *reinterpret_cast<const uint64_t*>(sm.vX[0]);
+      u = sm.du[it & (kDrawRing - 1)];
+      const unsigned above = select_one(r2, u, total);
+      if (total == 0.0 || fabs(total) < DBL_EPSILON) {  // sublattice.inl:108-112
+        if (tid == kClk) sm.c_time = thr;
+        break;
+      }
+      hop = above != 0;  // else: a selection that finds no jump advances the clock only
+      if (hop) {
+        b = __ffs(static_cast<int>(above)) - 1;
+        X = static_cast<int>((vX >> (8 * b)) & 0xff);
+        os = s;
+        oX = gX;
+        oY = gY;
+        oZ = gZ;
+        oid = gid;
+        const int p = s & 1;
+        // 1nn offset b of parity p (LatListMeta::getIdBy1nnOffset order)
+        const int dX = (b & 4) ? 1 : -1, dy = ((b >> 1) & 1) - 1 + p, dz = (b & 1) - 1 + p;
+        s += dX + R.LX * (dy + R.LY * dz);
+        lx += dX;
+        ly += dy;
+        lz += dz;
+        nact = in_sector(lx, ly, lz);
+        // perform (ABVIModel::perform, kmc.cpp:358-396) on the staged region
+        if (tid == kCtl) {
+          occ_s[s] = kV;
+          occ_s[os] = static_cast<uint8_t>(X);
+        }
+#pragma unroll
+        for (int q = 0; q < kJumpsPerWarp; ++q)
+          foot_terms<KIND, true>(sm, 0, occ_s, rho_s, s, sl[q], tid + kThreads * q, FT, b, X, os, nact);
+        gX = wrap1(gX + dX, jc.sx);
+        gY = wrap1(gY + dy, jc.sy);
+        gZ = wrap1(gZ + dz, jc.sz);
+        gid = gX + jc.sx * (gY + jc.sy * gZ);
+      }
+      __syncthreads();
+      AKMC_PHASE(5);
     }
-    __syncthreads();  // set n (or c), the clock's decision and the next uniform visible
-    HOP_T(threadIdx.x == 0 ? 3 : 2);
-    HOP_P(3);
-#if defined(AKMC_PHASE_PROFILE) && defined(AKMC_HOP_PROFILE)
-    if (tid == 0) atomicAdd(a.counters + 23, 1ull);
-#endif
-    AKMC_PHASE(5);
-    if (hop) c = n;
-    it ^= 1;
+    if (tid == 0) {
+      sm.vpk[0][0] = make_int4(s, lx, ly, lz);
+      sm.vpk[0][1] = make_int4(gX, gY, gZ, gid);
+    }
+  } else {
+    // vacancy k lies within D cells of the cell (qx, qy, qz) and in the sector
+    auto dirty = [&](int k, int qx, int qy, int qz) -> bool {
+      const int4 v = sm.vpk[k][0];
+      return sm.vact[k] && abs((v.y >> 1) - qx) <= D && abs(v.z - qy) <= D && abs(v.w - qz) <= D;
+    };
+    int c = 0;  // set of the ordered list in use
+    int ksel = -1, snew = 0;
+    // vacancies to evaluate: all of them at first, then those the last hop made dirty
+    unsigned m0 = cnt >= 32 ? kFull : (1u << cnt) - 1u, m1 = cnt > 32 ? (cnt >= 64 ? kFull : (1u << (cnt - 32)) - 1u) : 0u;
+    for (int it = 0;; ++it) {
+      auto next = [&]() -> int {  // takes one vacancy off the masks, -1 when there is none
+        if (m0) {
+          const int k = __ffs(static_cast<int>(m0)) - 1;
+          m0 &= m0 - 1;
+          return k;
+        }
+        if (m1) {
+          const int k = 31 + __ffs(static_cast<int>(m1));
+          m1 &= m1 - 1;
+          return k;
+        }
+        return -1;
+      };
+      auto site = [&](int k) -> int { return k == ksel ? snew : sm.vpk[k][0].x; };
+      if (!eam) {  // a warp takes a vacancy
+        for (int n = 0;; ++n) {
+          const int k = next();
+          if (k < 0) break;
+          if (n % kEvalWarps == warp) pair_rates(sm, occ_s, k, site(k), de_out);
+        }
+      } else {
+        // two vacancies at a time: their dE terms by all warps, a barrier, then the jump sums of the
+        // first by warps 0 and 1 and of the second by warps 2 and 3, solute targets by the last warps
+        while (m0 | m1) {
+          const int ka = next(), kb = next();
+          const int la = site(ka), lb = kb >= 0 ? site(kb) : la;
+#pragma unroll
+          for (int q = 0; q < kJumpsPerWarp; ++q)
+            foot_terms<KIND, false>(sm, 0, occ_s, rho_s, la, sl[q], tid + kThreads * q, FT, 0, 0, 0, true);
+          if (kb >= 0)
+#pragma unroll
+            for (int q = 0; q < kJumpsPerWarp; ++q)
+              foot_terms<KIND, false>(sm, 1, occ_s, rho_s, lb, sl[q], tid + kThreads * q, FT, 0, 0, 0, true);
+          __syncthreads();
+          if (warp < 4) {
+            if (warp < 2) jump_rates<KIND>(sm, 0, occ_s, ka, la, warp & 1, ix, de_out);
+            else if (kb >= 0) jump_rates<KIND>(sm, 1, occ_s, kb, lb, warp & 1, ix, de_out);
+          }
+          constexpr int kw = kEvalWarps == 8 ? 4 : 0;
+          if (warp >= kw) {
+#pragma unroll 1
+            for (int n = warp - kw; n < (kb >= 0 ? 16 : 8); n += kEvalWarps - kw)
+              solute_rate<KIND>(sm, occ_s, rho_s, n < 8 ? ka : kb, n < 8 ? la : lb, n & 7, R, *a.geo, FT, de_out);
+          }
+          if (m0 | m1) __syncthreads();  // the term sets are written again
+        }
+      }
+      __syncthreads();
+      AKMC_PHASE(2);
+      // ordered total over the z-y-x sorted list; lane i keeps the running sum through its vacancy
+      // (i or i + 32 of the list)
+      const int nord = sm.nord[c];
+      double total = 0.0, s0 = 0.0, s1 = 0.0;
+      for (int i = 0; i < nord; ++i) {
+        const double2* r2 = reinterpret_cast<const double2*>(sm.rates[sm.ord[c][i]]);
+        const double2 a0 = r2[0], a1 = r2[1], a2 = r2[2], a3 = r2[3];
+        total += a0.x;
+        total += a0.y;
+        total += a1.x;
+        total += a1.y;
+        total += a2.x;
+        total += a2.y;
+        total += a3.x;
+        total += a3.y;
+        if (i == lane) s0 = total;
+        if (i == lane + 32) s1 = total;
+      }
+      if (API && a.mode == kModeCalc) {  // akmc_calculate: the sector's vacancies with their jump rates
+        if (tid < cnt) a.api_sites[tid] = sm.vpk[tid][1].w;
+        for (int i = tid; i < 8 * cnt; i += kThreads) a.api_rates[i] = (&sm.rates[0][0])[i];
+        if (tid == kClk) {
+          *a.api_total = total;
+          *a.api_count = cnt;
+        }
+        break;
+      }
+      if (total == 0.0 || fabs(total) < DBL_EPSILON) {  // sublattice.inl:108-112
+        if (tid == kClk) {
+          if (API) {
+            a.api_event->from_site = -1;
+            a.api_event->total = total;
+          } else {
+            sm.c_time = thr;
+          }
+        }
+        break;
+      }
+      const double u = API ? a.api_u : sm.du[it & (kDrawRing - 1)];
+      const double expected = u * total;  // ModelAdapter::selectAndPerform
+      // the first vacancy whose running sum is above u * total (the sums never fall), then the jump
+      const unsigned f0 = __ballot_sync(kFull, lane < nord && s0 > expected);
+      const unsigned f1 = __ballot_sync(kFull, lane + 32 < nord && s1 > expected);
+      const bool hop = (f0 | f1) != 0;
+      const int pos = f0 ? __ffs(static_cast<int>(f0)) - 1 : f1 ? 31 + __ffs(static_cast<int>(f1)) : 0;
+      double x = 0.0;
+      if (pos > 0) x = __shfl_sync(kFull, pos <= 32 ? s0 : s1, (pos - 1) & 31);
+      ksel = sm.ord[c][pos];
+      {
+        const double2* r2 = reinterpret_cast<const double2*>(sm.rates[ksel]);
+        const double2 a0 = r2[0], a1 = r2[1], a2 = r2[2], a3 = r2[3];
+        const double rr[8] = {a0.x, a0.y, a1.x, a1.y, a2.x, a2.y, a3.x, a3.y};
+#pragma unroll
+        for (int q = 0; q < 8; ++q) x += q <= lane ? rr[q] : 0.0;
+      }
+      const unsigned above = __ballot_sync(kFull, lane < 8 && x > expected);
+      const int b = hop ? __ffs(static_cast<int>(above)) - 1 : 0;
+      const int X = sm.vX[ksel][b];
+      const int4 pa = sm.vpk[ksel][0], pb = sm.vpk[ksel][1];
+      const int s = pa.x, p = s & 1;
+      const int qx = pa.y >> 1, qy = pa.z, qz = pa.w;  // the hop's origin cell
+      const int dX = (b & 4) ? 1 : -1, dy = ((b >> 1) & 1) - 1 + p, dz = (b & 1) - 1 + p;
+      const int nlx = pa.y + dX, nly = qy + dy, nlz = qz + dz;
+      snew = s + dX + R.LX * (dy + R.LY * dz);
+      const bool nact = in_sector(nlx, nly, nlz);
+      const int nX = wrap1(pb.x + dX, jc.sx), nY = wrap1(pb.y + dy, jc.sy), nZ = wrap1(pb.z + dz, jc.sz);
+      const int32_t nid = nX + jc.sx * (nY + jc.sy * nZ);
+      double dt = 0.0;
+      if (warp < 3) {
+        if (eam && hop && tid < kRefreshN) refresh(tid, p, b, s, X, pb.x, pb.y, pb.z, true);
+      } else {
+        if (tid == 96 && hop) {
+          occ_s[snew] = kV;
+          occ_s[s] = static_cast<uint8_t>(X);
+          put_occ(nX, nY, nZ, kV);
+          put_occ(pb.x, pb.y, pb.z, static_cast<uint8_t>(X));
+        }
+        if (warp == kOrdWarp && hop) {
+          // the hopped vacancy leaves its place in the ordered list and re-enters at its new site
+          // id if it is still inside the sector; every other one moves by at most one place
+          int less = 0;
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const int i = lane + 32 * h;
+            const bool other = i < nord && i != pos;
+            const int k = other ? sm.ord[c][i] : 0;
+            const bool before = other && sm.vpk[k][1].w < nid;
+            less += __popc(__ballot_sync(kFull, before));
+            if (other) sm.ord[c ^ 1][i - (i > pos ? 1 : 0) + (nact && !before ? 1 : 0)] = k;
+          }
+          if (lane == 0) {
+            if (nact) sm.ord[c ^ 1][less] = ksel;
+            sm.nord[c ^ 1] = nord - 1 + (nact ? 1 : 0);
+          }
+        }
+        if (tid == kClk) {
+          if (API) {
+            if (hop) {
+              sm.c_nh = 1;
+              sm.c_nact += nord;
+            }
+            sm.ctl_stop = 1;  // the per-hop entry point stops after one selection
+          } else {
+            dt = clock_step(it, total, hop, nord);
+          }
+        }
+        if (!API && warp == kEvalWarps - 1) draw_step(it);
+      }
+      __syncthreads();
+      AKMC_PHASE(4);
+      if (hop) {
+        m0 = __ballot_sync(kFull, lane < cnt && (lane == ksel ? nact : dirty(lane, qx, qy, qz)));
+        if (cnt > 32) m1 = __ballot_sync(kFull, lane + 32 < cnt && (lane + 32 == ksel ? nact : dirty(lane + 32, qx, qy, qz)));
+        c ^= 1;
+        if (tid == 96) {
+          sm.vpk[ksel][0] = make_int4(snew, nlx, nly, nlz);
+          sm.vpk[ksel][1] = make_int4(nX, nY, nZ, nid);
+          sm.vact[ksel] = nact ? 1 : 0;
+        }
+      }
+      if (tid == kClk && hop) {
+        const int nd = __popc(m0) + __popc(m1);
+        sm.c_evals += nd;
+        if (!API && a.log_cap > 0) log_event(pb.w, nid, X, u, total, dt, nord, nd);
+      }
+      if (API && tid == kClk) {
+        akmc_event* e = a.api_event;
+        e->round = 0;
+        e->hop = sm.c_hop0;
+        e->from_site = hop ? pb.w : -1;
+        e->to_site = hop ? nid : -1;
+        e->block = B.local_id;
+        e->species = hop ? X : 0;
+        e->u = u;
+        e->total = total;
+        e->dt = 0.0;
+        e->n_act = nord;
+        e->n_dirty = hop ? __popc(m0) + __popc(m1) : 0;
+        e->job = B.job;
+        e->reserved = 0;
+      }
+      if (sm.ctl_stop) break;
+    }
   }
   __syncthreads();
   AKMC_PHASE(6);
-  if (tid == 0) sm.fin = c;  // every thread holds the same c
-  if (a.mode == kModeCalc) return true;
+  if (API && a.mode == kModeCalc) return true;
   if (tid == kCtl) {
     const int64_t nh = sm.c_nh;
-    if (a.mode == kModeRound) {
+    if (!API) {
       // (k_flow read the clock while the region's copies flew: no second round trip)
       B.evo[sec] = (flowpre ? sm.pre_evo : __ldcg(&B.evo[sec])) + sm.c_time;
-      for (int i = 0; i < 4; ++i) {
-        B.xs[i] = sm.xs[i];
-        B.xt[i] = sm.xt[i];
+      const int n = sm.c_sel;  // draws the selections used: the streams move on by as many
+      if (n > 0) {
+        const int slot = (n - 1) & (kDrawRing - 1);
+        for (int i = 0; i < 4; ++i) {
+          B.xs[i] = sm.sts[slot][0][i];
+          B.xt[i] = sm.sts[slot][1][i];
+        }
       }
     }
     B.hops = sm.c_hop0 + nh;
@@ -1318,7 +1591,7 @@ __device__ bool run_block(const RoundArgs& a, int gb, Smem& sm, uint8_t* occ_s, 
     sm.acc[5] += static_cast<unsigned long long>(nh * (eam ? 2 + kRefreshN : 2));
   }
   // the lattice was written through at every hop; only the vacancy positions remain
-  if (tid < cnt) a.vac_site[sm.vidx[tid]] = sm.vlid[c][tid];
+  if (tid < cnt) a.vac_site[sm.vidx[tid]] = sm.vpk[tid][1].w;
   return true;
 }
 
@@ -1335,18 +1608,17 @@ __device__ __forceinline__ void carve(uint8_t* smem, int nreg, Smem*& sm, uint8_
 __device__ void dispatch_block(const RoundArgs& a, int gb, uint8_t* smem) {
   const BlockDev& B = a.blocks[gb];
   const JobDev& J = a.jobs[B.job];
-  const int sec = a.mode == kModeRound ? sector_of_round(B.round) : a.api_sector;
   Region R;
-  make_region(B, J, sec, R);
+  make_region(B, J, a.api_sector, R);
   Smem* sm;
   uint8_t* occ_s;
   int32_t* rho_s;
   carve(smem, R.n, sm, occ_s, rho_s);
   const int32_t* vl = a.blk_list + static_cast<int64_t>(gb) * kMaxV;
   const int cnt = min(B.cnt, kMaxV);
-  if (J.model == AKMC_MODEL_PAIRBOND) run_block<kPairBond, 8>(a, gb, *sm, occ_s, rho_s, vl, cnt, B.round);
-  else if (J.precision == AKMC_FP32C) run_block<kEam32, 8>(a, gb, *sm, occ_s, rho_s, vl, cnt, B.round);
-  else run_block<kEam64, 8>(a, gb, *sm, occ_s, rho_s, vl, cnt, B.round);
+  if (J.model == AKMC_MODEL_PAIRBOND) run_block<kPairBond, 8, true>(a, gb, *sm, occ_s, rho_s, vl, cnt, B.round);
+  else if (J.precision == AKMC_FP32C) run_block<kEam32, 8, true>(a, gb, *sm, occ_s, rho_s, vl, cnt, B.round);
+  else run_block<kEam64, 8, true>(a, gb, *sm, occ_s, rho_s, vl, cnt, B.round);
 }
 
 __global__ void k_bucket(RoundArgs a) {
@@ -1436,7 +1708,7 @@ __global__ void __launch_bounds__(Shape<W>::kThreads, Shape<W>::kCtasPerSm) k_ho
     uint8_t* occ_s;
     int32_t* rho_s;
     carve(smem, R.n, sm, occ_s, rho_s);
-    run_block<KIND, W>(a, gb, *sm, occ_s, rho_s, a.blk_list + static_cast<int64_t>(gb) * kMaxV, min(B.cnt, kMaxV),
+    run_block<KIND, W, false>(a, gb, *sm, occ_s, rho_s, a.blk_list + static_cast<int64_t>(gb) * kMaxV, min(B.cnt, kMaxV),
                        B.round);
   }
   cta_flush<W>(a, smem);
@@ -1779,7 +2051,7 @@ __device__ bool flow_advance(const RoundArgs& a, BlockDev& B, const JobDev& J, i
 template <int KIND, int W>
 __global__ void __launch_bounds__(Shape<W>::kThreads, Shape<W>::kCtasPerSm) k_flow(RoundArgs a) {
   AKMC_SHAPE(W);
-  const int kFlowTake = a.flow_take > 0 && a.flow_take < kThreads ? a.flow_take : kThreads;
+  const int kFlowTake = a.flow_take > 0 && a.flow_take < kMaxTake ? a.flow_take : kMaxTake;
   extern __shared__ __align__(16) uint8_t smem[];
   Smem* sm0 = reinterpret_cast<Smem*>(smem);
   const int tid = threadIdx.x;
@@ -1943,8 +2215,8 @@ __global__ void __launch_bounds__(Shape<W>::kThreads, Shape<W>::kCtasPerSm) k_fl
           const int q = tid - kFlowSlots;
           if (q == 0) sm->hops_out = __ldcg(&B.hops);  // run_block replaces it if the round runs
           else if (q == 1) sm->pre_evo = __ldcg(&B.evo[sec]);
-          else if (q < 6) sm->xs[q - 2] = __ldcg(&B.xs[q - 2]);
-          else sm->xt[q - 6] = __ldcg(&B.xt[q - 6]);
+          else if (q < 6) sm->str[0][q - 2] = __ldcg(&B.xs[q - 2]);
+          else sm->str[1][q - 6] = __ldcg(&B.xt[q - 6]);
         }
         __syncthreads();
         const int cnt = sm->fnv;
@@ -1954,7 +2226,7 @@ __global__ void __launch_bounds__(Shape<W>::kThreads, Shape<W>::kCtasPerSm) k_fl
           tw = clock64();
         }
 #endif
-        const bool ran = run_block<KIND, W>(a, gb, *sm, occ_s, rho_s, sm->fv, cnt, r, true);
+        const bool ran = run_block<KIND, W, false>(a, gb, *sm, occ_s, rho_s, sm->fv, cnt, r, true);
 #ifdef AKMC_PHASE_PROFILE
         if (tid == 0) tw = clock64();
 #endif
@@ -1967,12 +2239,12 @@ __global__ void __launch_bounds__(Shape<W>::kThreads, Shape<W>::kCtasPerSm) k_fl
         if (ran && tid < cnt) {
           // a vacancy still inside the block's area keeps its owner and slot (its site updated);
           // only one that left it needs the owner lookup
-          const int f = sm->fin;
-          const int cx = sm->vgx[f][tid] >> 1, cy = sm->vgy[f][tid], cz = sm->vgz[f][tid];
+          const int4 g = sm->vpk[tid][1];
+          const int cx = g.x >> 1, cy = g.y, cz = g.z;
           const int* c0 = sm->bc0;
           const int* c1 = sm->bc1;
           const bool inside = cx >= c0[0] && cx < c1[0] && cy >= c0[1] && cy < c1[1] && cz >= c0[2] && cz < c1[2];
-          const int32_t site = sm->vlid[f][tid];
+          const int32_t site = g.w;
           int osec = 0, o = gb;
           if (inside)
             osec = (cx - c0[0] >= (c1[0] - c0[0]) / 2 ? 1 : 0) | (cy - c0[1] >= (c1[1] - c0[1]) / 2 ? 2 : 0) |

@@ -76,6 +76,7 @@ void build_geometry(Geometry& g, int nsh) {
           }
     }
   }
+  build_terms(g, nsh);
 }
 
 void pairbond_tables(double b1[5][5], double b2[5][5]) {

@@ -11,6 +11,8 @@ namespace akmc {
 
 int shells_within(double lattice_const, double cutoff);
 void build_geometry(Geometry& g, int nshells);
+// The foot_* and term tables of a geometry whose jump lists are filled (called by build_geometry).
+void build_terms(Geometry& g, int nsh);
 void pairbond_tables(double b1[5][5], double b2[5][5]);
 void cell_coefs(const double* F, int n, int k, double c[4]);
 int eam_johnson(uint64_t seed, double lattice_const, double cutoff, akmc_eam_tables* out, double params[4][5]);
