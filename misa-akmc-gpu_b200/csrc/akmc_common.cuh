@@ -97,12 +97,9 @@ AK_HD double rint_d(double x) {
 // 1/i! + r/(i+1)!, then r^2, r^4, r^8), and scaling by 2^k through the exponent field.  The
 // dependent chain of the polynomial is 6 operations instead of Horner's 14 (a rate is one long
 // FP64 chain per jump); max error 0.92 ulp against a correctly rounded exp over the range used.
-AK_HD double port_exp(double x) {
-  if (x != x) return x;
-  if (x > 709.782712893384) return bits_to_double(0x7ff0000000000000ULL);
-  if (x < -745.1332191019412) return 0.0;
+AK_HD double exp_poly(double x, int& k) {  // x = k ln2 + r: k and e^r
   const double kd = rint_d(x * 0x1.71547652b82fep+0);
-  const int k = static_cast<int>(kd);
+  k = static_cast<int>(kd);
   double r = fma_d(-kd, 0x1.62e42fee00000p-1, x);
   r = fma_d(-kd, 0x1.a39ef35793c76p-33, r);
   const double r2 = r * r, r4 = r2 * r2, r8 = r4 * r4;
@@ -114,7 +111,18 @@ AK_HD double port_exp(double x) {
   const double p1213 = fma_d(0x1.6124613a86d09p-33, r, 0x1.1eed8eff8d898p-29);  // 1/12!, 1/13!
   const double t0 = fma_d(p45, r2, p23), t1 = fma_d(p89, r2, p67), t2 = fma_d(p1213, r2, p1011);
   const double T = fma_d(t2, r8, fma_d(t1, r4, t0));
-  const double p = 1.0 + fma_d(r2, T, r);
+  return 1.0 + fma_d(r2, T, r);
+}
+AK_HD double port_exp(double x) {
+  int k;
+  if (x < 700.0 && x > -700.0) {  // nearly every argument: 2^k is a normal number
+    const double p = exp_poly(x, k);
+    return p * bits_to_double(static_cast<uint64_t>(k + 1023) << 52);
+  }
+  if (x != x) return x;
+  if (x > 709.782712893384) return bits_to_double(0x7ff0000000000000ULL);
+  if (x < -745.1332191019412) return 0.0;
+  const double p = exp_poly(x, k);
   if (k > 1023) return p * bits_to_double(2046ULL << 52) * bits_to_double(static_cast<uint64_t>(k) << 52);
   if (k < -1022) return p * bits_to_double(1ULL << 52) * bits_to_double(static_cast<uint64_t>(k + 2045) << 52);
   return p * bits_to_double(static_cast<uint64_t>(k + 1023) << 52);
@@ -182,10 +190,10 @@ AK_HD double div_rn_recip(double a, double b, double y) {
   return fma_d(r1, y, q1);
 }
 
-// arrhenius() with the exponent argument -Ea / kT formed by div_rn_recip (rkT = RN(1 / kT)):
-// the same bits.
-AK_HD double arrhenius_rk(double nu, double kT, double rkT, uint8_t moving, double dE) {
-  const double Ea = e0_of(moving) + dE / 2;
+// arrhenius() with the exponent argument -Ea / kT formed by div_rn_recip (rkT = RN(1 / kT)) and the moving
+// atom's e0 given: the same bits.
+AK_HD double arrhenius_rk(double nu, double kT, double rkT, double e0, double dE) {
+  const double Ea = e0 + dE / 2;
   return nu * port_exp(div_rn_recip(-Ea, kT, rkT));
 }
 

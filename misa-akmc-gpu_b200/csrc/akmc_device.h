@@ -14,7 +14,7 @@ constexpr int kNoAllocMaxBlocks = AKMC_NOALLOC_MAX_BLOCKS;
 constexpr int kJumpN = 76;                        // |N(s) u N(t)| - 2 sites per jump
 constexpr int kRefreshN = 78;                     // density refresh sites per jump
 constexpr int kTermN = 302;                       // distinct energy terms of a vacancy's 8 jumps (Geometry)
-constexpr int kTermSlots = 312;                   // + own and target embedding values, and a zero term
+constexpr int kTermSlots = 313;                   // + own and target embedding values, a zero, a trash term
 constexpr int kFootSlots = 256;                   // lanes that compute them
 constexpr int kShellNb = 58;                      // neighbours within the 5-shell cutoff
 constexpr int kNbrStride = 32;  // words per block of RoundArgs::nbr (one 128-byte line)

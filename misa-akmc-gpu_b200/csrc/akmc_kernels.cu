@@ -151,22 +151,35 @@ __device__ __forceinline__ void make_region(const BlockDev& B, const JobDev& J, 
 // Rounds with vacancies a CTA can take in one sweep (a sweep finds a few).
 constexpr int kMaxTake = 64;
 constexpr int kTermSets = 2;
-constexpr int kZeroTerm = kTermSlots - 1;  // a term that is always 0
+constexpr int kZeroTerm = kTermSlots - 2;  // a term that is always 0
+constexpr int kTrashTerm = kTermSlots - 1;  // written by the evaluations that belong to no term, never read
+// A lane's share of the dE terms (Geometry::foot_*): its site's local offset by x parity of the vacancy, the
+// terms its two F evaluations give, their shell pairs and density changes for a moving Fe atom.
+struct alignas(16) Slot {
+  int32_t off[2];
+  int32_t tA, tB;  // kTrashTerm: none
+  int32_t hA, hB;
+  int32_t dA, dB;
+};
 // Draws of the two random streams made ahead of their use: a ring of two batches.
 constexpr int kDrawBatch = 8, kDrawRing = 2 * kDrawBatch;
 
 // Shared-memory working set of one CTA (followed by the staged region).
 struct Smem {
-  double b1[25], b2[25];
+  double e0[9];                 // migration energy prefactor by the moving atom's code
+  double b1[9 * 5], b2[9 * 5];  // pair-bond energies by the neighbour's code and the source's bond index
   union {                       // phi_XY(shell s) - phi_XY(shell t), index (X*4+Y)*64 + s*8 + t,
     double dphi64[4 * 4 * 64];  // in the precision of the kernel's kind
     float dphi32[4 * 4 * 64];
   };
   int32_t dfq[4 * 64];          // f_X(shell s) - f_X(shell t) in Q.24, index X*64 + s*8 + t
   int32_t fq1[4];               // f_X at the first shell
-  int32_t d1[2][8];             // 1nn local offsets by x parity
-  int32_t d2[6];
+  // 1nn b by x parity p at 8 p + b: (local offset, dX, dy, dz)
+  alignas(16) int4 d1[16];
   uint8_t rf[8][kFootSlots];    // Geometry::foot_refresh
+  int32_t rl[2][8][kRefreshN];  // Geometry::refresh: packed (dx, dy, dz) and shells
+  alignas(16) Slot slot[kFootSlots];  // a lane's share of the dE terms
+  alignas(16) int4 ix[64][2];         // a lane's share of the jump sums (jump_rates), by x parity
   // dE terms of a vacancy's jumps (Geometry::foot_out), of two vacancies at a time: FP64 a double
   // each (0.0: a vacancy's site), FP32-comp (term, 1.0f for an atom's site); then its own and its
   // targets' embedding values (FP32-comp: the F cells, in fx).  The pair-bond loop keeps its path here.
@@ -306,32 +319,55 @@ __device__ void load_tables(Smem& sm, const Potential& P, const Geometry& G, con
   AKMC_SHAPE(W);
   const bool eam = kind != kPairBond;
   const int tid = threadIdx.x;
-  if (tid < 25) {
-    sm.b1[tid] = P.b1[tid / 5][tid % 5];
-    sm.b2[tid] = P.b2[tid / 5][tid % 5];
-  }
   if (tid < 16) {
     const int32_t w = G.nn1[tid >> 3][tid & 7];
-    sm.d1[tid >> 3][tid & 7] = local_delta(w, R);
+    sm.d1[tid] = make_int4(local_delta(w, R), unpack_dx(w), unpack_dy(w), unpack_dz(w));
   }
-  if (tid < 6) sm.d2[tid] = local_delta(G.nn2[tid], R);
-  if (eam) {
-    if (tid < 4) sm.fq1[tid] = P.fq[tid][1];
-    for (int i = tid; i < 4 * 4 * 64; i += kThreads) {
-      const int xy = i >> 6, hs = (i >> 3) & 7, ht = i & 7;
-      const double* ph = &P.phi64[0][0][0] + xy * 8;
-      const float* pf = &P.phi32[0][0][0] + xy * 8;
-      if (kind == kEam64) sm.dphi64[i] = ph[hs] - ph[ht];
-      else sm.dphi32[i] = pf[hs] - pf[ht];
-      if (i < 4 * 64) sm.dfq[i] = P.fq[i >> 6][hs] - P.fq[i >> 6][ht];
+  if (tid < 9) sm.e0[tid] = e0_of(static_cast<uint8_t>(tid));
+  if (!eam) {
+    if (tid < 45) {  // codes 0, 1, 2, 4, 8 have a bond index; the other rows are never read
+      const int code = tid / 5, i = tid % 5;
+      const bool used = (code & (code - 1)) == 0;
+      sm.b1[tid] = used ? P.b1[bond_index(static_cast<uint8_t>(code))][i] : 0.0;
+      sm.b2[tid] = used ? P.b2[bond_index(static_cast<uint8_t>(code))][i] : 0.0;
     }
-    for (int i = tid; i < 8 * kFootSlots / 4; i += kThreads)
-      reinterpret_cast<uint32_t*>(&sm.rf[0][0])[i] = __ldg(reinterpret_cast<const uint32_t*>(&G.foot_refresh[0][0]) + i);
-    if (tid < kTermSets) sm.term[tid][kZeroTerm] = 0.0;
+    return;
   }
+  if (tid < 4) sm.fq1[tid] = P.fq[tid][1];
+  for (int i = tid; i < 4 * 4 * 64; i += kThreads) {
+    const int xy = i >> 6, hs = (i >> 3) & 7, ht = i & 7;
+    const double* ph = &P.phi64[0][0][0] + xy * 8;
+    const float* pf = &P.phi32[0][0][0] + xy * 8;
+    if (kind == kEam64) sm.dphi64[i] = ph[hs] - ph[ht];
+    else sm.dphi32[i] = pf[hs] - pf[ht];
+    if (i < 4 * 64) sm.dfq[i] = P.fq[i >> 6][hs] - P.fq[i >> 6][ht];
+  }
+  for (int i = tid; i < 8 * kFootSlots / 4; i += kThreads)
+    reinterpret_cast<uint32_t*>(&sm.rf[0][0])[i] = __ldg(reinterpret_cast<const uint32_t*>(&G.foot_refresh[0][0]) + i);
+  for (int i = tid; i < 2 * 8 * kRefreshN; i += kThreads) (&sm.rl[0][0][0])[i] = __ldg(&G.refresh[0][0][0] + i);
+  for (int i = tid; i < kFootSlots; i += kThreads) {
+    Slot c;
+    c.off[0] = local_delta(__ldg(&G.foot_site[0][i]), R);
+    c.off[1] = local_delta(__ldg(&G.foot_site[1][i]), R);
+    const int out = __ldg(&G.foot_out[i]), sh = __ldg(&G.foot_shells[i]);
+    const int tA = out & 1023, tB = (out >> 10) & 1023;
+    c.tA = (tA == kFootNone ? kTrashTerm : tA) | (out >> 20) << 10;  // leader lane and raw in the high bits
+    c.tB = tB == kFootNone ? kTrashTerm : tB;
+    c.hA = sh & 63;
+    c.hB = (sh >> 8) & 63;
+    c.dA = P.fq[0][c.hA >> 3] - P.fq[0][c.hA & 7];
+    c.dB = P.fq[0][c.hB >> 3] - P.fq[0][c.hB & 7];
+    sm.slot[i] = c;
+  }
+  for (int i = tid; i < 128; i += kThreads) {  // lane (i / 2) of a pair of warps, parity i % 2
+    const int p = i & 1, lane = (i >> 1) & 31, b = 4 * (i >> 6) + (lane >> 3), sub = lane & 7;
+    auto t = [&](int k) -> int32_t { return k < kJumpN ? __ldg(&G.term[p][b][k]) : kZeroTerm; };
+    sm.ix[i >> 1][p] = make_int4(t(sub) | t(sub + 32) << 10 | t(sub + 64) << 20, t(sub + 8) | t(sub + 40) << 10 | t(sub + 72) << 20,
+                                 t(sub + 16) | t(sub + 48) << 10 | t(sub + 24) << 20, t(sub + 56));
+  }
+  if (tid < kTermSets) sm.term[tid][kZeroTerm] = 0.0;
 }
 
-__device__ __forceinline__ int sdelta(int32_t e) { return static_cast<int16_t>(e & 0xffff); }
 
 // Cells outside the shared-memory window (rare): global memory, range-checked.
 __device__ __noinline__ double F64_far(const double2* g64lo, const double2* g64hi, unsigned int* status, int32_t r,
@@ -403,52 +439,48 @@ __device__ __forceinline__ FCell32 cell32(const FTab& T, int32_t r) {
 // The rate of a jump with energy change dE of atom Xc (0: the target is a vacancy), into the record of
 // vacancy k and jump b.
 __device__ __forceinline__ void put_rate(Smem& sm, int k, int b, uint8_t Xc, double dE, double* de_out) {
-  const bool avail = is_atom(Xc);
-  sm.rates[k][b] = avail ? arrhenius_rk(sm.c_nu, sm.c_kT, sm.c_rkT, Xc, dE) : 0.0;
-  sm.vX[k][b] = avail ? Xc : 0;
-  if (de_out) de_out[k * 8 + b] = avail ? dE : 0.0;  // akmc_calculate only
+  const double rate = arrhenius_rk(sm.c_nu, sm.c_kT, sm.c_rkT, sm.e0[Xc], dE);
+  sm.rates[k][b] = Xc ? rate : 0.0;
+  sm.vX[k][b] = Xc;
+  if (de_out) de_out[k * 8 + b] = Xc ? dE : 0.0;  // akmc_calculate only
 }
 
 // Pair bond: the rates of vacancy k at local site l, by one warp.  Lanes 4 b + 0..3 run the four bond
 // counts of VacRatesSolver::deltaE (vacancy_rates_solver.cpp:45-116) for jump b, each summed in the
-// reference order.
-__device__ __forceinline__ void pair_rates(Smem& sm, const uint8_t* occ_s, int k, int l, double* de_out) {
+// reference order.  A single warp runs this on the hop loop's chain, so it counts instructions: the bond
+// tables are indexed by occupancy code, and the neighbours of both x parities are the same offsets from a
+// corner (ly, lyz: the row and plane pitch).
+__device__ __forceinline__ void pair_rates(Smem& sm, const uint8_t* occ_s, int k, int l, int ly, int lyz, double* de_out) {
   const int lane = threadIdx.x & 31, b = lane >> 2, q = lane & 3;
   const int p = l & 1;
-  const int tl = l + sm.d1[p][b];
+  const int tl = l + sm.d1[8 * p + b].x;
   const uint8_t Xc = occ_s[tl];
   const bool at_t = (q & 1) != 0;
-  const int center = at_t ? tl : l;
-  const int pc = at_t ? (p ^ 1) : p;
-  const uint8_t src = (q == 0 || q == 3) ? static_cast<uint8_t>(kV) : Xc;
-  const int ovr = q == 2 ? tl : (q == 3 ? l : -1);
-  const uint8_t ovr_code = q == 2 ? static_cast<uint8_t>(kV) : Xc;
-  const int si = bond_index(src);
+  const uint8_t* c = occ_s + (at_t ? tl : l);
+  const int src = (q == 0 || q == 3) ? 0 : 32 - __clz(Xc);  // bond index of V, or of the moving atom
+  // after the hop (q = 2, 3) the other end of the jump, neighbour b or its opposite, holds the other one
+  const int over = q == 2 ? b : q == 3 ? 7 - b : 8;
+  const int over_code = q == 2 ? 0 : Xc;
+  const uint8_t* corner = c - ((p ^ (at_t ? 1 : 0)) ? 0 : ly + lyz);
+  const double* t1 = sm.b1 + src;
+  const double* t2 = sm.b2 + src;
   double energy = 0.0;
 #pragma unroll
-  for (int b2 = 0; b2 < 8; ++b2) {
-    const int nb = center + sm.d1[pc][b2];
-    const uint8_t o = nb == ovr ? ovr_code : occ_s[nb];
-    energy += sm.b1[bond_index(o) * 5 + si];
+  for (int b2 = 0; b2 < 8; ++b2) {  // 1nn order: dX, then dy, then dz rising
+    int o = corner[((b2 & 4) ? 1 : -1) + ((b2 & 2) ? ly : 0) + ((b2 & 1) ? lyz : 0)];
+    o = b2 == over ? over_code : o;
+    energy += t1[o * 5];
   }
-#pragma unroll
-  for (int b2 = 0; b2 < 6; ++b2) {
-    if (!((0x2F >> b2) & 1)) continue;  // PeriodLatticeList::get2nnStatus
-    const int nb = center + sm.d2[b2];
-    const uint8_t o = nb == ovr ? ovr_code : occ_s[nb];
-    energy += sm.b2[bond_index(o) * 5 + si];
-  }
+  // 2nn -x, -y, -z, +z, +x (PeriodLatticeList::get2nn2 order under the mask of get2nnStatus)
+  energy += t2[c[-2] * 5];
+  energy += t2[c[-ly] * 5];
+  energy += t2[c[-lyz] * 5];
+  energy += t2[c[lyz] * 5];
+  energy += t2[c[2] * 5];
   const double pair = energy + __shfl_down_sync(kFull, energy, 1);  // q0: e_before, q2: e_after
   const double after = __shfl_down_sync(kFull, pair, 2);
   if (q == 0) put_rate(sm, k, b, Xc, after - pair, de_out);
 }
-
-// A lane's share of the dE terms (Geometry::foot_*): its site's local offset (x parity 0 in the low half,
-// 1 in the high), the terms it writes, the shell pairs of its two evaluations and their density changes
-// for a moving Fe atom.
-struct Slot {
-  int32_t off, out, sh, dA, dB;
-};
 
 // FP32 F cell at density r: the node and the polynomial part of dF32.
 struct F32Val {
@@ -474,35 +506,33 @@ __device__ __forceinline__ float F32diff(const F32Val& a1, const F32Val& a0) {
 // deltas of the hop all lie on the slots' sites; no other warp touches them before the next barrier).
 // `inside`: the vacancy is still in its sector; one that left it needs no terms, and some of its sites lie
 // past the region's 2-cell halo (the refreshed ones never do).
-// What bounds this: two to four 16-byte reads of random F cells a lane (about 10 shared-memory
-// wavefronts a warp and read).  Each jump's 76 sites evaluated on their own took 1232 F evaluations a
-// vacancy; the shared terms take 447.
+// What bounds this: the instructions of one chain (a hop waits for it), and four 16-byte reads of random F
+// cells a lane (about 10 shared-memory wavefronts a warp and read).  Each jump's 76 sites evaluated on their
+// own took 1232 F evaluations a vacancy; the shared terms take 447.
 template <int KIND, bool REFRESH>
 __device__ __forceinline__ void foot_terms(Smem& sm, int set, const uint8_t* occ_s, int32_t* rho_s, int l, const Slot& c,
                                            int slot, const FTab& FT, int b, int X, int from, bool inside) {
-  const int lane = threadIdx.x & 31;
-  const int lead = (c.out >> 20) & 31;
-  int j = l + ((l & 1) ? c.off >> 16 : sdelta(c.off));
+  const int lead = (c.tA >> 10) & 31, raw = c.tA >> 15;
+  int j = l + ((l & 1) ? c.off[1] : c.off[0]);
   int code = 0;
   if (REFRESH) {
     code = sm.rf[b][slot];
     if (!inside && !code) j = l;  // outside the staged halo: only the deltas are wanted
   }
-  uint8_t o = occ_s[j];
+  int o = occ_s[j];
   int32_t r = rho_s[j];
   if (REFRESH) {
     r += sm.dfq[atom_index(static_cast<uint8_t>(X)) * 64 + code];  // code 0: + 0
-    if (j == from) o = static_cast<uint8_t>(X);
+    if (j == from) o = X;
     __syncwarp();
-    if (code && lead == lane) rho_s[j] = r;
+    if (code && lead == (threadIdx.x & 31)) rho_s[j] = r;
   }
   const int32_t rA = r + c.dA, rB = r + c.dB;
-  const bool win = static_cast<unsigned>((rA >> kRhoCellShift) - FT.kw0) < static_cast<unsigned>(kFWin) &&
-                   static_cast<unsigned>((rB >> kRhoCellShift) - FT.kw0) < static_cast<unsigned>(kFWin);
-  const int outA = c.out & 1023, outB = (c.out >> 10) & 1023, raw = (c.out >> 25) & 15;
-  const int hA = c.sh & 63, hB = (c.sh >> 8) & 63;
+  static_assert((kFWin & (kFWin - 1)) == 0, "one test for both cells");
+  const bool win = static_cast<unsigned>(((rA >> kRhoCellShift) - FT.kw0) | ((rB >> kRhoCellShift) - FT.kw0)) <
+                   static_cast<unsigned>(kFWin);
   const bool atom = o != kV;
-  const int y = atom ? atom_index(o) * 64 : 0;
+  const int y = atom ? atom_index(static_cast<uint8_t>(o)) * 64 : 0;
   if (KIND == kEam64) {
     double FA, FB;
     if (win) {
@@ -513,10 +543,10 @@ __device__ __forceinline__ void foot_terms(Smem& sm, int set, const uint8_t* occ
       FB = F64(FT, rB);
     }
     const double F0 = __shfl_sync(kFull, FA, lead);
-    const double tA = (FA - F0) + sm.dphi64[y + hA], tB = (FB - F0) + sm.dphi64[y + hB];
+    const double tA = (FA - F0) + sm.dphi64[y + c.hA], tB = (FB - F0) + sm.dphi64[y + c.hB];
     double* const T = sm.term[set];
-    if (outA != kFootNone) T[outA] = atom ? tA : 0.0;
-    if (outB != kFootNone) T[outB] = atom ? tB : 0.0;
+    T[c.tA & 1023] = atom ? tA : 0.0;
+    T[c.tB] = atom ? tB : 0.0;
     if (raw) T[kTermN + raw - 1] = FA;
   } else {
     F32Val a, bb;
@@ -531,10 +561,11 @@ __device__ __forceinline__ void foot_terms(Smem& sm, int set, const uint8_t* occ
     f0.hi = __shfl_sync(kFull, a.hi, lead);
     f0.lo = __shfl_sync(kFull, a.lo, lead);
     f0.q = __shfl_sync(kFull, a.q, lead);
-    const float tA = F32diff(a, f0) + sm.dphi32[y + hA], tB = F32diff(bb, f0) + sm.dphi32[y + hB];
+    const float tA = F32diff(a, f0) + sm.dphi32[y + c.hA], tB = F32diff(bb, f0) + sm.dphi32[y + c.hB];
     float2* const T = reinterpret_cast<float2*>(sm.term[set]);
-    if (outA != kFootNone) T[outA] = make_float2(tA, atom ? 1.f : 0.f);
-    if (outB != kFootNone) T[outB] = make_float2(tB, atom ? 1.f : 0.f);
+    const float on = atom ? 1.f : 0.f;
+    T[c.tA & 1023] = make_float2(tA, on);
+    T[c.tB] = make_float2(tB, on);
     if (raw) sm.fx[set][raw - 1] = make_float4(a.hi, a.lo, a.q, 0.f);
   }
 }
@@ -547,12 +578,12 @@ __device__ __forceinline__ void foot_terms(Smem& sm, int set, const uint8_t* occ
 // starts at a term (never -0.0) cannot become -0.0.
 template <int KIND>
 __device__ __forceinline__ void jump_rates(Smem& sm, int set, const uint8_t* occ_s, int k, int l, int half,
-                                           const int32_t (&ix)[2][4], double* de_out) {
+                                           const int4 (&ix)[2], double* de_out) {
   const int lane = threadIdx.x & 31, b = 4 * half + (lane >> 3);
   const int p = l & 1;
-  const uint8_t Xc = occ_s[l + sm.d1[p][b]];
-  const int32_t w0 = p ? ix[1][0] : ix[0][0], w1 = p ? ix[1][1] : ix[0][1], w2 = p ? ix[1][2] : ix[0][2],
-                w3 = p ? ix[1][3] : ix[0][3];
+  const uint8_t Xc = occ_s[l + sm.d1[8 * p + b].x];
+  const int32_t w0 = p ? ix[1].x : ix[0].x, w1 = p ? ix[1].y : ix[0].y, w2 = p ? ix[1].z : ix[0].z,
+                w3 = p ? ix[1].w : ix[0].w;
   const int i[10] = {w0 & 1023, (w0 >> 10) & 1023, (w0 >> 20) & 1023, w1 & 1023, (w1 >> 10) & 1023,
                      (w1 >> 20) & 1023, w2 & 1023, (w2 >> 10) & 1023, (w2 >> 20) & 1023, w3 & 1023};
   double dE;
@@ -594,7 +625,7 @@ __device__ __forceinline__ void jump_rates(Smem& sm, int set, const uint8_t* occ
     }
     dE = static_cast<double>(EX + (x.s - x.c));
   }
-  if ((lane & 7) == 0 && (Xc == kFe || !is_atom(Xc))) put_rate(sm, k, b, Xc, dE, de_out);
+  if ((lane & 7) == 0 && Xc <= kFe) put_rate(sm, k, b, Xc, dE, de_out);
 }
 
 // Rate of jump b of vacancy k at local site l with a solute target (the shared terms are those of a
@@ -606,9 +637,9 @@ __device__ __forceinline__ void solute_rate(Smem& sm, const uint8_t* occ_s, cons
                                             const Region& R, const Geometry& G, const FTab& FT, double* de_out) {
   const int q = threadIdx.x & 31;
   const int p = l & 1;
-  const int tl = l + sm.d1[p][b];
+  const int tl = l + sm.d1[8 * p + b].x;
   const uint8_t Xc = occ_s[tl];
-  if (Xc == kFe || !is_atom(Xc)) return;  // uniform
+  if (Xc <= kFe) return;  // uniform: Fe, or a vacancy
   const int X = atom_index(Xc);
   uint8_t o[3];
   int32_t r0[3], r1[3];
@@ -948,33 +979,6 @@ __device__ __forceinline__ bool run_block(const RoundArgs& a, int gb, Smem& sm, 
     const int q = tid - kCtl;
     sm.str[q >> 2][q & 3] = q < 4 ? __ldcg(&B.xs[q]) : __ldcg(&B.xt[q - 4]);
   }
-  // this lane's share of the dE terms and of the jump sums, in registers, read while the copies fly
-  Slot sl[kJumpsPerWarp];
-  int32_t ix[2][4];
-  if (eam) {
-    const Geometry& G = *a.geo;
-#pragma unroll
-    for (int q = 0; q < kJumpsPerWarp; ++q) {
-      const int slot = tid + kThreads * q;
-      const int d0 = local_delta(__ldg(&G.foot_site[0][slot]), R), d1 = local_delta(__ldg(&G.foot_site[1][slot]), R);
-      sl[q].off = (d0 & 0xffff) | (d1 << 16);
-      sl[q].out = __ldg(&G.foot_out[slot]);
-      sl[q].sh = __ldg(&G.foot_shells[slot]);
-      const int hA = sl[q].sh & 63, hB = (sl[q].sh >> 8) & 63;
-      sl[q].dA = __ldg(&P.fq[0][hA >> 3]) - __ldg(&P.fq[0][hA & 7]);
-      sl[q].dB = __ldg(&P.fq[0][hB >> 3]) - __ldg(&P.fq[0][hB & 7]);
-    }
-    // the jump sums are taken by the even and odd warps of a pair (jump_rates)
-    const int b = 4 * (warp & 1) + (lane >> 3), sub = lane & 7;
-#pragma unroll
-    for (int p = 0; p < 2; ++p) {
-      auto t = [&](int i) -> int32_t { return i < kJumpN ? __ldg(&G.term[p][b][i]) : kZeroTerm; };
-      ix[p][0] = t(sub) | t(sub + 32) << 10 | t(sub + 64) << 20;
-      ix[p][1] = t(sub + 8) | t(sub + 40) << 10 | t(sub + 72) << 20;
-      ix[p][2] = t(sub + 16) | t(sub + 48) << 10 | t(sub + 24) << 20;
-      ix[p][3] = t(sub + 56);
-    }
-  }
   __syncthreads();
   AKMC_STAGE_T(3);
   AKMC_PHASE(0);
@@ -1032,6 +1036,15 @@ __device__ __forceinline__ bool run_block(const RoundArgs& a, int gb, Smem& sm, 
   __syncthreads();
   AKMC_PHASE(1);
   if (!sm.ctl_ok) return true;
+  // this lane's share of the dE terms and of the jump sums (taken by the even and odd warps of a pair)
+  Slot sl[kJumpsPerWarp];
+  int4 ix[2];
+  if (eam) {
+#pragma unroll
+    for (int q = 0; q < kJumpsPerWarp; ++q) sl[q] = sm.slot[tid + kThreads * q];
+    ix[0] = sm.ix[tid & 63][0];
+    ix[1] = sm.ix[tid & 63][1];
+  }
   double* const de_out = API && a.mode == kModeCalc ? a.api_de : nullptr;
   constexpr int D = eam ? 4 : 3;  // a hop changes the rates of vacancies within D cells of its origin
 
@@ -1039,7 +1052,7 @@ __device__ __forceinline__ bool run_block(const RoundArgs& a, int gb, Smem& sm, 
   // coordinates (gX, gY, gZ).  UPDATE: the delta of moving atom X is applied first; the density is
   // written through.
   auto refresh = [&](int i, int p, int b, int s, int X, int gX, int gY, int gZ, bool update) {
-    const int32_t e = __ldg(&a.geo->refresh[p][b][i]);
+    const int32_t e = sm.rl[p][b][i];
     const int j = s + local_delta(e, R);
     int32_t v = rho_s[j];
     if (update) {
@@ -1054,24 +1067,30 @@ __device__ __forceinline__ bool run_block(const RoundArgs& a, int gb, Smem& sm, 
   auto put_occ = [&](int gX, int gY, int gZ, uint8_t o) {
     lattice_put(jc.occ + static_cast<int64_t>(jc.px) * (gY + static_cast<int64_t>(jc.sy) * gZ), jc.sx, gX, o);
   };
+  // local coordinates inside the sector
+  const int slx = 2 * R.hx, swx = 2 * R.w[0];
   auto in_sector = [&](int lx, int ly, int lz) -> bool {
-    return (lx >> 1) >= R.hx && (lx >> 1) < R.hx + R.w[0] && ly >= 2 && ly < 2 + R.w[1] && lz >= 2 && lz < 2 + R.w[2];
+    return static_cast<unsigned>(lx - slx) < static_cast<unsigned>(swx) &&
+           static_cast<unsigned>(ly - 2) < static_cast<unsigned>(R.w[1]) &&
+           static_cast<unsigned>(lz - 2) < static_cast<unsigned>(R.w[2]);
   };
   // The ordered total of one vacancy's rates and its selection (ABVIModel::calcRates, kmc.cpp:68-115,
-  // and select, kmc.cpp:242-309), alike in every lane of the calling warps: lane q also forms the running
-  // sum through jump q (adding 0.0 to a non-negative sum leaves it as it is), and the first running sum
-  // above u * total wins.  Jumps onto a vacancy hold 0.0.  Returns the lanes above u * total.
-  auto select_one = [&](const double2 (&r2)[4], double u, double& total) -> unsigned {
-    const double rr[8] = {r2[0].x, r2[0].y, r2[1].x, r2[1].y, r2[2].x, r2[2].y, r2[3].x, r2[3].y};
-    double t = 0.0, x = 0.0;
-#pragma unroll
-    for (int q = 0; q < 8; ++q) {
-      t += rr[q];
-      x += q <= lane ? rr[q] : 0.0;
-    }
-    total = t;
-    const double expected = u * t;  // ModelAdapter::selectAndPerform
-    return __ballot_sync(kFull, lane < 8 && x > expected);
+  // and select, kmc.cpp:242-309), alike in every lane: the first of the running sums above u * total wins.
+  // Jumps onto a vacancy hold 0.0.  Returns the jump, -1 for none.
+  auto select_one = [&](const double2 (&r2)[4], double u, double& total) -> int {
+    const double v0 = r2[0].x, v1 = v0 + r2[0].y, v2 = v1 + r2[1].x, v3 = v2 + r2[1].y, v4 = v3 + r2[2].x,
+                 v5 = v4 + r2[2].y, v6 = v5 + r2[3].x, v7 = v6 + r2[3].y;
+    total = v7;
+    const double expected = u * v7;  // ModelAdapter::selectAndPerform
+    int b = v7 > expected ? 7 : -1;
+    b = v6 > expected ? 6 : b;
+    b = v5 > expected ? 5 : b;
+    b = v4 > expected ? 4 : b;
+    b = v3 > expected ? 3 : b;
+    b = v2 > expected ? 2 : b;
+    b = v1 > expected ? 1 : b;
+    b = v0 > expected ? 0 : b;
+    return b;
   };
   // The clock thread: the selection used draw `it`; advances the sector's clock and decides
   // whether its window is reached.  Returns the residence time.
@@ -1175,34 +1194,30 @@ __device__ __forceinline__ bool run_block(const RoundArgs& a, int gb, Smem& sm, 
           asm volatile("bar.sync 2, 64;" ::: "memory");
           ++meets;
         }
-        pair_rates(sm, occ_s, 0, s, nullptr);
+        pair_rates(sm, occ_s, 0, s, R.LX, R.LX * R.LY, nullptr);
         __syncwarp();
         const double2* r = reinterpret_cast<const double2*>(sm.rates[0]);
         const double2 r2[4] = {r[0], r[1], r[2], r[3]};
-        const uint64_t vX = *reinterpret_cast<const uint64_t*>(sm.vX[0]);
         const double u = sm.du[it & (kDrawRing - 1)];
         double total;
-        const unsigned above = select_one(r2, u, total);
-        if (total == 0.0 || fabs(total) < DBL_EPSILON) {  // sublattice.inl:108-112
+        const int b = select_one(r2, u, total);
+        if (fabs(total) < DBL_EPSILON) {  // sublattice.inl:108-112
           time = thr;
           break;
         }
         const double dt = sm.dl[it & (kDrawRing - 1)] / total;
         time += dt;
         bool stop = !(time < thr);
-        if (above) {  // else: a selection that finds no jump advances the clock only
-          const int b = __ffs(static_cast<int>(above)) - 1;
-          const int X = static_cast<int>((vX >> (8 * b)) & 0xff);
-          const int p = s & 1;
-          // 1nn offset b of parity p (LatListMeta::getIdBy1nnOffset order)
-          const int dX = (b & 4) ? 1 : -1, dy = ((b >> 1) & 1) - 1 + p, dz = (b & 1) - 1 + p;
-          lx += dX;
-          ly += dy;
-          lz += dz;
-          gX = wrap1(gX + dX, jc.sx);
-          gY = wrap1(gY + dy, jc.sy);
-          gZ = wrap1(gZ + dz, jc.sz);
-          const int snew = s + dX + R.LX * (dy + R.LY * dz);
+        if (b >= 0) {  // else: a selection that finds no jump advances the clock only
+          const int X = sm.vX[0][b];
+          const int4 d = sm.d1[8 * (s & 1) + b];
+          lx += d.y;
+          ly += d.z;
+          lz += d.w;
+          gX = wrap1(gX + d.y, jc.sx);
+          gY = wrap1(gY + d.z, jc.sy);
+          gZ = wrap1(gZ + d.w, jc.sz);
+          const int snew = s + d.x;
           const int nid = gX + jc.sx * (gY + jc.sy * gZ);
           const bool nact = in_sector(lx, ly, lz);
           nh += 1;
@@ -1271,34 +1286,45 @@ __device__ __forceinline__ bool run_block(const RoundArgs& a, int gb, Smem& sm, 
     for (int q = 0; q < kJumpsPerWarp; ++q)
       foot_terms<KIND, false>(sm, 0, occ_s, rho_s, s, sl[q], tid + kThreads * q, FT, 0, 0, 0, true);
     __syncthreads();
-    // the last selection: its uniform, total, jump, atom, origin
+    // the last selection: its uniform, total, jump, atom and origin; g*: the vacancy's global record,
+    // kept by the warps that write (not 0 and 1)
     bool hop = false, nact = true;
-    int b = 0, X = 0, os = 0, oX = 0, oY = 0, oZ = 0, oid = 0;
+    int b = 0, X = 0, os = 0;
+    int4 d = make_int4(0, 0, 0, 0);
     double u = 0.0, total = 0.0;
     for (int it = 0;; ++it) {
-      if (nact) {
-        if (warp < 2) {
-          jump_rates<KIND>(sm, 0, occ_s, 0, s, warp, ix, nullptr);
-        } else {
+      if (warp < 2) {
+        if (nact) jump_rates<KIND>(sm, 0, occ_s, 0, s, warp, ix, nullptr);
+      } else {
+        if (nact) {
 #pragma unroll 1
           for (int q = warp - 2; q < 8; q += kEvalWarps - 2) solute_rate<KIND>(sm, occ_s, rho_s, 0, s, q, R, *a.geo, FT, nullptr);
         }
-      }
-      if (it > 0 && warp >= 2) {
-        if (tid == kClk) {
-          const double dt = clock_step(it - 1, total, hop, 1);
+        if (it > 0) {
+          const int oX = gX, oY = gY, oZ = gZ, oid = gid;
           if (hop) {
-            sm.c_evals += nact ? 1 : 0;
-            if (a.log_cap > 0) log_event(oid, gid, X, u, total, dt, 1, nact ? 1 : 0);
+            gX = wrap1(gX + d.y, jc.sx);
+            gY = wrap1(gY + d.z, jc.sy);
+            gZ = wrap1(gZ + d.w, jc.sz);
+            gid = gX + jc.sx * (gY + jc.sy * gZ);
           }
+          if (tid == kClk) {
+            const double dt = clock_step(it - 1, total, hop, 1);
+            if (hop) {
+              sm.c_evals += nact ? 1 : 0;
+              if (a.log_cap > 0) log_event(oid, gid, X, u, total, dt, 1, nact ? 1 : 0);
+            }
+          }
+          if (hop) {
+            if (tid >= kWt0 && tid < kWt0 + kWtN)
+              for (int i = tid - kWt0; i < kRefreshN; i += kWtN) refresh(i, os & 1, b, os, X, oX, oY, oZ, false);
+            if (tid == kCtl || tid == kCtl + 1) {
+              const bool to = tid == kCtl;
+              put_occ(to ? gX : oX, to ? gY : oY, to ? gZ : oZ, to ? static_cast<uint8_t>(kV) : static_cast<uint8_t>(X));
+            }
+          }
+          if (warp == kEvalWarps - 1) draw_step(it - 1);
         }
-        if (hop) {
-          if (tid >= kWt0 && tid < kWt0 + kWtN)
-            for (int i = tid - kWt0; i < kRefreshN; i += kWtN) refresh(i, os & 1, b, os, X, oX, oY, oZ, false);
-          if (tid == kCtl) put_occ(gX, gY, gZ, kV);
-          if (tid == kCtl + 1) put_occ(oX, oY, oZ, static_cast<uint8_t>(X));
-        }
-        if (warp == kEvalWarps - 1) draw_step(it - 1);
       }
       __syncthreads();
       AKMC_PHASE(2);
@@ -1309,29 +1335,22 @@ __device__ __forceinline__ bool run_block(const RoundArgs& a, int gb, Smem& sm, 
       }
       const double2* r = reinterpret_cast<const double2*>(sm.rates[0]);
       const double2 r2[4] = {r[0], r[1], r[2], r[3]};
-      const uint64_t vX = *reinterpret_cast<const uint64_t*>(sm.vX[0]);
       u = sm.du[it & (kDrawRing - 1)];
-      const unsigned above = select_one(r2, u, total);
-      if (total == 0.0 || fabs(total) < DBL_EPSILON) {  // sublattice.inl:108-112
+      const int sel = select_one(r2, u, total);
+      if (fabs(total) < DBL_EPSILON) {  // sublattice.inl:108-112
         if (tid == kClk) sm.c_time = thr;
         break;
       }
-      hop = above != 0;  // else: a selection that finds no jump advances the clock only
+      hop = sel >= 0;  // else: a selection that finds no jump advances the clock only
       if (hop) {
-        b = __ffs(static_cast<int>(above)) - 1;
-        X = static_cast<int>((vX >> (8 * b)) & 0xff);
+        b = sel;
+        X = sm.vX[0][b];
+        d = sm.d1[8 * (s & 1) + b];
         os = s;
-        oX = gX;
-        oY = gY;
-        oZ = gZ;
-        oid = gid;
-        const int p = s & 1;
-        // 1nn offset b of parity p (LatListMeta::getIdBy1nnOffset order)
-        const int dX = (b & 4) ? 1 : -1, dy = ((b >> 1) & 1) - 1 + p, dz = (b & 1) - 1 + p;
-        s += dX + R.LX * (dy + R.LY * dz);
-        lx += dX;
-        ly += dy;
-        lz += dz;
+        s += d.x;
+        lx += d.y;
+        ly += d.z;
+        lz += d.w;
         nact = in_sector(lx, ly, lz);
         // perform (ABVIModel::perform, kmc.cpp:358-396) on the staged region
         if (tid == kCtl) {
@@ -1341,15 +1360,11 @@ __device__ __forceinline__ bool run_block(const RoundArgs& a, int gb, Smem& sm, 
 #pragma unroll
         for (int q = 0; q < kJumpsPerWarp; ++q)
           foot_terms<KIND, true>(sm, 0, occ_s, rho_s, s, sl[q], tid + kThreads * q, FT, b, X, os, nact);
-        gX = wrap1(gX + dX, jc.sx);
-        gY = wrap1(gY + dy, jc.sy);
-        gZ = wrap1(gZ + dz, jc.sz);
-        gid = gX + jc.sx * (gY + jc.sy * gZ);
       }
       __syncthreads();
       AKMC_PHASE(5);
     }
-    if (tid == 0) {
+    if (tid == 64) {
       sm.vpk[0][0] = make_int4(s, lx, ly, lz);
       sm.vpk[0][1] = make_int4(gX, gY, gZ, gid);
     }
@@ -1382,7 +1397,7 @@ __device__ __forceinline__ bool run_block(const RoundArgs& a, int gb, Smem& sm, 
         for (int n = 0;; ++n) {
           const int k = next();
           if (k < 0) break;
-          if (n % kEvalWarps == warp) pair_rates(sm, occ_s, k, site(k), de_out);
+          if (n % kEvalWarps == warp) pair_rates(sm, occ_s, k, site(k), R.LX, R.LX * R.LY, de_out);
         }
       } else {
         // two vacancies at a time: their dE terms by all warps, a barrier, then the jump sums of the
@@ -1440,7 +1455,7 @@ __device__ __forceinline__ bool run_block(const RoundArgs& a, int gb, Smem& sm, 
         }
         break;
       }
-      if (total == 0.0 || fabs(total) < DBL_EPSILON) {  // sublattice.inl:108-112
+      if (fabs(total) < DBL_EPSILON) {  // sublattice.inl:108-112
         if (tid == kClk) {
           if (API) {
             a.api_event->from_site = -1;
@@ -1474,11 +1489,11 @@ __device__ __forceinline__ bool run_block(const RoundArgs& a, int gb, Smem& sm, 
       const int4 pa = sm.vpk[ksel][0], pb = sm.vpk[ksel][1];
       const int s = pa.x, p = s & 1;
       const int qx = pa.y >> 1, qy = pa.z, qz = pa.w;  // the hop's origin cell
-      const int dX = (b & 4) ? 1 : -1, dy = ((b >> 1) & 1) - 1 + p, dz = (b & 1) - 1 + p;
-      const int nlx = pa.y + dX, nly = qy + dy, nlz = qz + dz;
-      snew = s + dX + R.LX * (dy + R.LY * dz);
+      const int4 d = sm.d1[8 * p + b];
+      const int nlx = pa.y + d.y, nly = qy + d.z, nlz = qz + d.w;
+      snew = s + d.x;
       const bool nact = in_sector(nlx, nly, nlz);
-      const int nX = wrap1(pb.x + dX, jc.sx), nY = wrap1(pb.y + dy, jc.sy), nZ = wrap1(pb.z + dz, jc.sz);
+      const int nX = wrap1(pb.x + d.y, jc.sx), nY = wrap1(pb.y + d.z, jc.sy), nZ = wrap1(pb.z + d.w, jc.sz);
       const int32_t nid = nX + jc.sx * (nY + jc.sy * nZ);
       double dt = 0.0;
       if (warp < 3) {
