@@ -33,6 +33,12 @@ constexpr int kStageRows = 4;  // rows of the staged region each warp has in fli
 #define AKMC_SWEEP_VISITS 1
 #endif
 constexpr int kSweepVisits = AKMC_SWEEP_VISITS;
+// CTAs that look after a block at a time: a sweep visits at most nblocks * kSweepWatch / CTAs blocks (and one
+// per thread).  More only makes the visits wait on one another: with every thread of every CTA visiting, a
+// context of a few hundred blocks had each of its round words read hundreds of thousands of times a sweep.
+// 512 rounds of 180 blocks: 23.5 ms so, 11.7 with 16, 11.8 with 8, 13.1 with 4 (then blocks wait for a visit:
+// 56 and 113 ms with 2 and 1); 4096 blocks: the same from 8 on.
+constexpr int kSweepWatch = 16;
 // Nanoseconds a k_flow CTA sleeps after a sweep that moved no block on (0: none).
 #ifndef AKMC_SWEEP_SLEEP_NS
 #define AKMC_SWEEP_SLEEP_NS 256
@@ -2076,6 +2082,7 @@ __global__ void __launch_bounds__(Shape<W>::kThreads, Shape<W>::kCtasPerSm) k_fl
     sm0->flow_lag[i / 27][o] = static_cast<int8_t>(flow_lag(i / 27, o % 3 - 1, (o / 3) % 3 - 1, o / 9 - 1));
   }
   const int nb = a.nblocks;
+  const int watch = max(1, min(kThreads, static_cast<int>((static_cast<int64_t>(nb) * kSweepWatch) / gridDim.x)));
   int cursor = static_cast<int>((static_cast<int64_t>(blockIdx.x) * nb) / gridDim.x);
   const uint64_t t_begin = globaltimer_ns();  // a time-boxed launch takes no new round after its budget
   if (tid == 0) sm0->flow_stop = 0;
@@ -2107,8 +2114,8 @@ __global__ void __launch_bounds__(Shape<W>::kThreads, Shape<W>::kCtasPerSm) k_fl
     // while the sweep lasts as long as its slowest visit (one that takes a block)
 #pragma unroll 1
     for (int vis = 0; vis < kSweepVisits; ++vis) {
-      const int off = tid + vis * kThreads;
-      if (off >= nb) break;
+      const int off = tid + vis * watch;
+      if (tid >= watch || off >= nb) break;
       int gb = cursor + off;
       if (gb >= nb) gb -= nb;
       BlockDev& B = a.blocks[gb];
@@ -2324,7 +2331,7 @@ __global__ void __launch_bounds__(Shape<W>::kThreads, Shape<W>::kCtasPerSm) k_fl
     if (tid == 0) t_hop += clock64() - t0;
 #endif
     if (AKMC_SWEEP_SLEEP_NS > 0 && !sm0->flow_progress) __nanosleep(AKMC_SWEEP_SLEEP_NS);
-    cursor += kSweepVisits * kThreads;
+    cursor += kSweepVisits * watch;
     if (cursor >= nb) cursor %= nb;
   }
   cta_flush<W>(a, smem);
