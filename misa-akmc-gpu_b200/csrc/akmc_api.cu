@@ -130,10 +130,7 @@ struct akmc_ctx {
   bool flow_ok = false;  // more than one block, and every block area starts with few enough vacancies
   int flow_grid = 0;
   unsigned long long* d_fstate = nullptr;
-  unsigned long long* d_vclaim = nullptr;
-  unsigned long long* d_vvalid = nullptr;
-  int32_t* d_vslot = nullptr;
-  int32_t* d_vsite = nullptr;
+  unsigned long long* d_vslot = nullptr;
   int32_t* d_vcount = nullptr;
   int32_t* d_nbr = nullptr;
   unsigned char* d_tmaps = nullptr;  // per job slot: two 128-byte tensor maps
@@ -215,14 +212,12 @@ void free_device(akmc_ctx* ctx) {
   ctx->ev.clear();
   dfree(ctx->stream, ctx->d_vac_count);
   ctx->d_vac_count = nullptr;
-  void* flow_ptrs[] = {ctx->d_fstate, ctx->d_vclaim, ctx->d_vvalid, ctx->d_vslot, ctx->d_vsite,
-                       ctx->d_vcount, ctx->d_nbr,    ctx->d_vsec,   ctx->d_flow};
+  void* flow_ptrs[] = {ctx->d_fstate, ctx->d_vslot, ctx->d_vcount, ctx->d_nbr, ctx->d_vsec, ctx->d_flow};
   for (void* p : flow_ptrs) dfree(ctx->stream, p);
   ctx->d_fstate = nullptr;
-  ctx->d_vclaim = ctx->d_vvalid = nullptr;
-  ctx->d_vslot = ctx->d_vcount = ctx->d_nbr = ctx->d_flow = nullptr;
+  ctx->d_vslot = nullptr;
+  ctx->d_vcount = ctx->d_nbr = ctx->d_flow = nullptr;
   ctx->d_vsec = nullptr;
-  ctx->d_vsite = nullptr;
   dfree(ctx->stream, ctx->d_tmaps);
   ctx->d_tmaps = nullptr;
   dfree(ctx->stream, ctx->d_cl);
@@ -634,6 +629,8 @@ akmc_status setup_job(akmc_ctx* ctx, int32_t ji, JobDev& J, BlockDev* hb, int32_
   J.max_rounds = j.cfg.max_rounds;
   J.nu = j.cfg.attempt_freq;
   J.kT = kBoltzmann * j.cfg.temperature;
+  J.rkT = 1.0 / J.kT;
+  J.fwin0 = ctx->pots[static_cast<size_t>(j.pot)].P.fwin0;
   J.window = j.cfg.sector_window;
   for (int b = 0; b < j.nblocks; ++b) {
     BlockDev& B = hb[b];
@@ -890,10 +887,7 @@ AKMC_API akmc_status akmc_prepare(akmc_ctx* ctx) {
   CK(dalloc(ctx->stream, &ctx->d_counters, 24));
   CK(dalloc(ctx->stream, &ctx->d_vac_count, 1));
   CK(dalloc(ctx->stream, &ctx->d_fstate, ncap));
-  CK(dalloc(ctx->stream, &ctx->d_vclaim, ncap));
-  CK(dalloc(ctx->stream, &ctx->d_vvalid, ncap));
   CK(dalloc(ctx->stream, &ctx->d_vslot, ncap * kFlowSlots));
-  CK(dalloc(ctx->stream, &ctx->d_vsite, ncap * kFlowSlots));
   CK(dalloc(ctx->stream, &ctx->d_vcount, ncap));
   CK(dalloc(ctx->stream, &ctx->d_nbr, ncap * kNbrStride));
   CK(dalloc(ctx->stream, &ctx->d_vsec, ncap));
@@ -966,10 +960,7 @@ AKMC_API akmc_status akmc_prepare(akmc_ctx* ctx) {
   a.api_sites = ctx->d_api_sites;
   a.api_count = ctx->d_api_count;
   a.fstate = ctx->d_fstate;
-  a.vclaim = ctx->d_vclaim;
-  a.vvalid = ctx->d_vvalid;
   a.vslot = ctx->d_vslot;
-  a.vsite = ctx->d_vsite;
   a.vcount = ctx->d_vcount;
   a.nbr = ctx->d_nbr;
   a.vsec = ctx->d_vsec;

@@ -115,17 +115,19 @@ struct JobDev {
                       // that does not wrap in y or z is staged by one tensor copy per array through
                       // the job's tensor maps (RoundArgs::tmaps)
   int32_t tbox[3];    // the box: the job's widest region, x rounded out as the bulk form rounds it
-  int32_t pad_tbox;
+  int32_t fwin0;      // Potential::fwin0 of its potential
   int32_t nb[3];      // domain blocks per dimension
   int32_t block0;     // first global block
   int32_t nblocks;
   int32_t model, precision, pot;
   int32_t done;
-  int32_t bulk;       // 1: regions that do not wrap in x are staged by bulk copies of whole rows
+  int32_t bulk;       // 1: region rows are staged by 16-byte copies
   int64_t round;
   int64_t hops;
   int64_t hop_budget, max_rounds;
   double nu, kT, window;
+  double rkT;         // RN(1 / kT): the rates' exponent arguments without a division
+  double pad;         // a multiple of 16 bytes: copied in 16-byte words
 };
 
 struct BlockDev {
@@ -181,10 +183,8 @@ struct RoundArgs {
   int64_t hop_cap;
   // asynchronous round schedule (k_flow)
   unsigned long long* fstate;   // per block: rounds completed << 1, | 1 while a thread or CTA holds it
-  unsigned long long* vclaim;   // per block: slots of vslot taken
-  unsigned long long* vvalid;   // per block: slots of vslot holding a vacancy id
-  int32_t* vslot;               // per block: kFlowSlots ids of the vacancies in its area
-  int32_t* vsite;               // per block: their sites (kept with the ids by whoever moves them)
+  unsigned long long* vslot;    // per block, kFlowSlots words: id << 32 | site of each vacancy in its area
+                                // (all bits set: a free slot)
   int32_t* vcount;              // per block: fill counter while the slots are rebuilt
   unsigned int* vsec;           // per block: bit s set while a vacancy of its area lies in sector s
   const void* tmaps;            // per job slot: two 128-byte tensor maps (occupancy, densities)

@@ -17,7 +17,9 @@
 
 #include <cfloat>
 #include <algorithm>
+#include <cstddef>
 #include <cstdint>
+#include <utility>
 
 #include "akmc_device.h"
 
@@ -91,25 +93,24 @@ struct Region {
   int ey, ez;         // rows of the region in y and z (LY, LZ: the pitch, the job's box with tma)
   int tma;            // staged by one tensor copy per array
   int hx;             // cells before the sector in x within the pitch (the 2-cell halo, plus xo / 2)
-  int bulk;           // rows staged by bulk copies: bo occupancy bytes and br densities each
+  int bulk;           // rows staged by 16-byte copies: bo occupancy bytes and br densities each
   int bo, br;
 };
 
-// The staged region of a block's sector: the sector and a 2-cell halo.  Rows are staged
-// whole by the bulk-copy unit when the job allows it (J.bulk: rows of a multiple of 16 sites,
-// 16-byte aligned arrays, shared memory sized for the wider rows): each row's span is rounded
-// out to 16-site boundaries from its unwrapped origin R.ox (which may lie before the row or run
-// past its end: the sector never wraps, its halo may), so every copy starts on a 16-byte
-// boundary.  A span that crosses the row's end (or starts before it) is copied as two pieces,
-// each inside the row; the span must not be longer than the row.
-__device__ __forceinline__ void make_region(const BlockDev& B, const JobDev& J, int sec, Region& R) {
+// The staged region of a block's sector: the sector and a 2-cell halo.  With J.bulk (shared memory sized for
+// the wider rows) each row's span is rounded out to 16-site boundaries from its unwrapped origin R.ox (which may
+// lie before the row or run past its end: the sector never wraps, its halo may; the row's halo entries hold the
+// sites past either end), so that copies of 16 bytes start on 16-byte boundaries in both arrays.
+__device__ __forceinline__ void make_region(const int32_t (&c0)[3], const int32_t (&c1)[3], const JobDev& J, int sec,
+                                            Region& R) {
+#pragma unroll
   for (int d = 0; d < 3; ++d) {
-    const int half = (B.c1[d] - B.c0[d]) / 2;
+    const int half = (c1[d] - c0[d]) / 2;
     if ((sec >> d) & 1) {
-      R.slo[d] = B.c0[d] + half;
-      R.w[d] = B.c1[d] - B.c0[d] - half;
+      R.slo[d] = c0[d] + half;
+      R.w[d] = c1[d] - c0[d] - half;
     } else {
-      R.slo[d] = B.c0[d];
+      R.slo[d] = c0[d];
       R.w[d] = half;
     }
   }
@@ -155,7 +156,17 @@ __device__ __forceinline__ void make_region(const BlockDev& B, const JobDev& J, 
 }
 
 // Rounds with vacancies a CTA can take in one sweep (a sweep finds a few).
-constexpr int kMaxTake = 64;
+constexpr int kMaxTake = 16;
+// A block's round handed to the CTA with what the block record holds for it: read by the thread that took the
+// block (k_flow's sweep), in flight together, so that the CTA itself waits for no record.
+struct alignas(16) Round {
+  int64_t r, t;        // the round and the launch's target
+  int64_t hops;        // the block's hops so far
+  double evo;          // the active sector's clock
+  uint64_t str[2][4];  // selection and residence-time streams
+  int32_t gb, job, local;
+  int32_t c0[3], c1[3];  // block cells
+};
 constexpr int kTermSets = 2;
 constexpr int kZeroTerm = kTermSlots - 2;  // a term that is always 0
 constexpr int kTrashTerm = kTermSlots - 1;  // written by the evaluations that belong to no term, never read
@@ -216,26 +227,17 @@ struct Smem {
   uint64_t str[2][4];
   uint64_t raw[2][kDrawRing], sts[kDrawRing][2][4];
   double du[kDrawRing], dl[kDrawRing];
-  // asynchronous schedule (k_flow)
-  int8_t flow_lag[8][27];
-  int32_t flow_cand[kMaxTake];
+  Round round[kMaxTake];   // rounds handed over by a sweep; [0] alone in the other kernels
+  JobDev job;              // the job of the running block (job_key: its index), copied when it changes
+  int32_t job_key;
+  int32_t fnv;             // vacancies of the running sector
+  int32_t fslot[kFlowSlots];  // and their slots (k_flow)
   int32_t flow_ncand, flow_stop, flow_progress, flow_more;
-  int32_t fv[kFlowSlots], fslot[kFlowSlots], fnv;  // the sector's vacancies and their slots
-  int32_t fsite[kFlowSlots];                        // their sites
-  int64_t flow_cr[kMaxTake], flow_ct[kMaxTake];        // round and target of each round handed over
-  unsigned long long flow_cvv[kMaxTake];                // its block's vacancy-slot valid bits
-  int64_t cur_r, cur_t;   // the block's round and target for its next chained round
-  int32_t bc0[3], bc1[3];  // the running block's area and its job's block count, kept for the
-  int32_t bnb;             // post-round updates (a reload after the round's stores is an L2 trip)
-  int64_t hops_out;       // the block's hop count after run_block
-  // run_block's clock thread: hops at the start, hops, n_act sum and evaluations of the
-  // block-round, selections made, the sector's clock and its threshold
-  int64_t c_hop0, c_nh, c_nact, c_evals;
+  // run_block's clock thread: hops, n_act sum and evaluations of the block-round, selections made, the
+  // sector's clock
+  int64_t c_nh, c_nact, c_evals;
   int32_t c_sel, c_path;
   double c_time;
-  double c_nu, c_kT;  // the job's attempt frequency and kT (the rates' constants)
-  double c_rkT;       // RN(1 / kT): the rates' exponent arguments without a division
-  double pre_evo;         // the active sector's clock, read while the region's copies fly
   // device counters summed per CTA and added once when the kernel ends (per-round atomics on
   // the same addresses from every CTA queue up); hops of the current job likewise
   unsigned long long acc[6];  // counters 0 (hops), 1, 3, 4, 5, 6
@@ -283,9 +285,6 @@ struct FTab {
   int kw0;
   const Potential* pot;      // the full tables (far cells), read on the rare path only
   unsigned int* status;
-#ifdef AKMC_PHASE_PROFILE
-  unsigned long long* prof;  // sub-phase cycles of the evaluation
-#endif
 };
 
 // Job constants of the running block, held in registers (the job record sits in global
@@ -295,21 +294,6 @@ struct JobC {
   int32_t* rho;
   int sx, sy, sz, px;
 };
-
-#if defined(AKMC_PHASE_PROFILE) && !defined(AKMC_FLOW_PROFILE) && !defined(AKMC_HOP_PROFILE)
-#define EVAL_T(i)                                                                       \
-  do {                                                                                  \
-    if (threadIdx.x == 0) {                                                             \
-      const long long t_ = clock64();                                                   \
-      atomicAdd(FT.prof + (i), static_cast<unsigned long long>(t_ - tev));              \
-      tev = t_;                                                                         \
-    }                                                                                   \
-  } while (0)
-#else
-#define EVAL_T(i) \
-  do {            \
-  } while (0)
-#endif
 
 __device__ __forceinline__ int local_delta(int32_t w, const Region& R) {
   return unpack_dx(w) + R.LX * (unpack_dy(w) + R.LY * unpack_dz(w));
@@ -445,7 +429,7 @@ __device__ __forceinline__ FCell32 cell32(const FTab& T, int32_t r) {
 // The rate of a jump with energy change dE of atom Xc (0: the target is a vacancy), into the record of
 // vacancy k and jump b.
 __device__ __forceinline__ void put_rate(Smem& sm, int k, int b, uint8_t Xc, double dE, double* de_out) {
-  const double rate = arrhenius_rk(sm.c_nu, sm.c_kT, sm.c_rkT, sm.e0[Xc], dE);
+  const double rate = arrhenius_rk(sm.job.nu, sm.job.kT, sm.job.rkT, sm.e0[Xc], dE);
   sm.rates[k][b] = Xc ? rate : 0.0;
   sm.vX[k][b] = Xc;
   if (de_out) de_out[k * 8 + b] = Xc ? dE : 0.0;  // akmc_calculate only
@@ -719,210 +703,80 @@ __device__ __forceinline__ void solute_rate(Smem& sm, const uint8_t* occ_s, cons
   if (q == 0) put_rate(sm, k, b, Xc, dE, de_out);
 }
 
-// Bulk staging of a region (R.bulk): the bulk-copy unit moves whole rows, R.bo occupancy bytes
-// and R.br densities from the row's 16-site boundary R.ox (unwrapped; the row's halo holds the
-// sites past either end), into shared rows of pitch R.LX; thread t0 + k nt issues row
-// t0 + k nt, one copy per array.  The barrier is armed for the bytes of every row (stage_bytes).
-__device__ __forceinline__ void stage_rows(const Region& R, const uint8_t* occ, const int32_t* rho, int px, int sy, int sz,
-                                           bool eam, uint8_t* occ_s, int32_t* rho_s, uint64_t* bar, int t0, int nt) {
-  asm volatile("fence.proxy.async;" ::: "memory");  // generic accesses before, copies after
-  const int nrows = R.ey * R.ez;
-  for (int row = t0; row < nrows; row += nt) {
-    const int ly = row % R.ey, lz = row / R.ey;
-    const int gy = wrap1(R.oy + ly, sy), gz = wrap1(R.oz + lz, sz);
-    const int64_t first = static_cast<int64_t>(px) * (gy + static_cast<int64_t>(sy) * gz) + kHaloL + R.ox;
-    const int l = R.LX * (ly + R.LY * lz);  // the shared row (pitch LX, LY)
-    bulk_copy(occ_s + l, occ + first, static_cast<uint32_t>(R.bo), bar);
-    if (eam) bulk_copy(rho_s + l, rho + first, static_cast<uint32_t>(4 * R.br), bar);
-  }
-}
-// Bytes the bulk staging of region R moves (the barrier's transaction count).
-__device__ __forceinline__ uint32_t stage_bytes(const Region& R, bool eam) {
-  if (R.tma) return static_cast<uint32_t>(R.n) * (eam ? 5u : 1u);
-  return static_cast<uint32_t>(R.ey * R.ez) * static_cast<uint32_t>(R.bo + (eam ? 4 * R.br : 0));
-}
-// Tensor staging of a region (R.tma): one 3D tile copy per array of the job's box from entry
-// (kHaloL + R.ox, R.oy, R.oz) of the lattice (x a multiple of 16 entries: 16-byte aligned in both
-// arrays), into shared memory laid out with the box as pitch.  Parts of the box past the region
-// are staged too and never read; parts past the array are filled with zeros.  One thread issues
-// both copies.
-__device__ __forceinline__ void stage_tensor(const Region& R, const void* tmaps, int job, bool eam, uint8_t* occ_s,
-                                             int32_t* rho_s, uint64_t* bar) {
-  asm volatile("fence.proxy.async;" ::: "memory");  // generic accesses before, copies after
-  const unsigned char* m = static_cast<const unsigned char*>(tmaps) + static_cast<size_t>(job) * 256;
-  const int x = kHaloL + R.ox, y = R.oy, z = R.oz;
-  asm volatile(
-      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(
-          smem_u32(occ_s)),
-      "l"(m), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar))
-      : "memory");
-  if (eam)
-    asm volatile(
-        "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(
-            smem_u32(rho_s)),
-        "l"(m + 128), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar))
-        : "memory");
+// The CTA's copy of job `job`'s record (constant while a launch runs); CTA-wide, uniform.
+__device__ __forceinline__ void load_job(Smem& sm, const RoundArgs& a, int job) {
+  if (sm.job_key == job) return;
+  __syncthreads();  // every thread has read the key; the previous job's readers are done
+  static_assert(sizeof(JobDev) % 16 == 0, "copied in 16-byte words");
+  if (threadIdx.x < sizeof(JobDev) / 16)
+    reinterpret_cast<int4*>(&sm.job)[threadIdx.x] = __ldcg(reinterpret_cast<const int4*>(a.jobs + job) + threadIdx.x);
+  if (threadIdx.x == 0) sm.job_key = job;
+  __syncthreads();
 }
 
-// Phase profile (builds with -DAKMC_PHASE_PROFILE): thread 0 accumulates the cycles
-// between consecutive CTA barriers into counters[8 + phase].
-#ifdef AKMC_PHASE_PROFILE
-#define AKMC_PHASE(i)                                                                           \
-  do {                                                                                          \
-    if (threadIdx.x == 0) {                                                                     \
-      const long long t_ = clock64();                                                           \
-      atomicAdd(a.counters + 8 + (i), static_cast<unsigned long long>(t_ - tph));               \
-      tph = t_;                                                                                 \
-    }                                                                                           \
-  } while (0)
-#else
-#define AKMC_PHASE(i) \
-  do {              \
-  } while (0)
-#endif
-// Staging sub-phases (builds with -DAKMC_FLOW_PROFILE): counters 16..19.
-#ifdef AKMC_FLOW_PROFILE
-#define AKMC_STAGE_T(k)                                                                         \
-  do {                                                                                          \
-    if (threadIdx.x == 0) {                                                                     \
-      const long long t_ = clock64();                                                           \
-      atomicAdd(a.counters + 16 + (k), static_cast<unsigned long long>(t_ - tsub));             \
-      tsub = t_;                                                                                \
-    }                                                                                           \
-  } while (0)
-#else
-#define AKMC_STAGE_T(k) \
-  do {                \
-  } while (0)
-#endif
-
-// Advances the running state of stream lane (0 selection, 1 residence time) by one draw into ring
-// slot `slot`: the raw draw and the state after it.  Called by lanes 0 and 1 of one warp.
-__device__ __forceinline__ void draw_ahead(Smem& sm, uint64_t (&x)[4], int lane, int slot) {
-  sm.raw[lane][slot] = xoshiro_next(x);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) sm.sts[slot][lane][i] = x[i];
-}
-// What a batch's draws stand for, one draw a lane: the selection uniform in [0, 1) (lanes 0-7) and
-// -ln of the residence-time uniform in (0, 1] (lanes 8-15; sublattice.inl:118-120).
-__device__ __forceinline__ void draw_values(Smem& sm, int lane, int slot0) {
-  if (lane < kDrawBatch) {
-    sm.du[slot0 + lane] = static_cast<double>(sm.raw[0][slot0 + lane] >> 11) * 0x1p-53;
-  } else if (lane < 2 * kDrawBatch) {
-    const int k = slot0 + lane - kDrawBatch;
-    sm.dl[k] = -port_log(static_cast<double>((sm.raw[1][k] >> 11) + 1) * 0x1p-53);
-  }
-}
-
-// The hop loop of one block's active sector (or, with API, one per-hop API step), CTA-collective.
-// round_now is the block's round (its completed rounds), read by the caller.
-// vlist holds the ids of the cnt_in vacancies inside the sector (any order).  Returns
-// false, uniformly, when the sector's clock is already past its window: nothing ran and
-// the vacancy arrays of sm were not filled.
-//
-// Every warp selects for itself, all lanes alike (the ordered sums are deterministic, so no broadcast
-// is needed); the hop's updates are spread over the warps.
-template <int KIND, int W, bool API>
-__device__ __forceinline__ bool run_block(const RoundArgs& a, int gb, Smem& sm, uint8_t* occ_s, int32_t* rho_s,
-                                          const int32_t* vlist, int cnt_in, int64_t round_now, bool flowpre = false) {
+// Issues the copies of a region into shared memory (CTA-wide, no wait: stage_wait).  A region that does not
+// wrap in y or z is one tensor copy per array of the job's box from entry (kHaloL + R.ox, R.oy, R.oz) of the
+// lattice (x a multiple of 16 entries: 16-byte aligned in both arrays), laid out with the box as pitch; parts of
+// the box past the region are staged too and never read, parts past the array are filled with zeros.  The others
+// go row by row, 16 bytes a copy (cp.async), half a warp a row where its copies fit: one bulk copy per row and
+// array measured 15 cycles each through the copy unit, 5.9K cycles for the 14 x 14 rows of a 20-cell block.
+template <int KIND, int W>
+__device__ __forceinline__ void stage_region(Smem& sm, const RoundArgs& a, const Region& R, uint8_t* occ_s, int32_t* rho_s) {
   AKMC_SHAPE(W);
-  constexpr int kClk = Shape<W>::kClk, kOrdWarp = Shape<W>::kOrdWarp;
   constexpr bool eam = KIND != kPairBond;
-  const int tid = threadIdx.x;
-  const int lane = tid & 31, warp = tid >> 5;
-#ifdef AKMC_PHASE_PROFILE
-  long long tph = clock64();
-#endif
-#ifdef AKMC_FLOW_PROFILE
-  long long tsub = clock64();
-#endif
-  BlockDev& B = a.blocks[gb];
-  const JobDev& J = a.jobs[B.job];
-  const Potential& P = a.pots[J.pot];
-  // the block record, the lattice and the vacancy table are read at L2 (__ldcg): under the
-  // asynchronous schedule another SM may have written them since this SM last looked
-  const int sec = API ? a.api_sector : sector_of_round(round_now);
-  // flowpre (k_flow): the caller issued a bulk region's copies on mbar_st already, and left the
-  // sector's clock (sm.pre_evo), the block's hops (sm.hops_out), the streams (sm.str) and the
-  // vacancies' sites (sm.fsite) in shared memory, read while the copies were in flight
-  double thr = 0.0;
-  if (!API) {
-    const int64_t step = round_now >> 3;
-    thr = static_cast<double>(step + 1) * J.window - (flowpre ? sm.pre_evo : __ldcg(&B.evo[sec]));
-    if (!(0.0 < thr)) {  // sector_time stays 0 (sublattice.inl:82)
-      if (flowpre && tid == kCtl) {  // copies already issued complete first: the buffer is reused next
-        Region R0;
-        make_region(B, J, sec, R0);
-        if (R0.bulk) {
-          if (mbar_wait(&sm.mbar_st, sm.mbst_phase)) sm.mbst_phase ^= 1u;
-          else atomicOr(a.status, kErrTimeout);
-        }
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const JobDev& J = sm.job;
+  if (R.tma) {
+    if (tid == kCtl) {
+      bulk_expect(&sm.mbar_st, static_cast<uint32_t>(R.n) * (eam ? 5u : 1u));
+      asm volatile("fence.proxy.async;" ::: "memory");  // generic accesses before, copies after
+      const unsigned char* m = static_cast<const unsigned char*>(a.tmaps) + static_cast<size_t>(sm.job_key) * 256;
+      const int x = kHaloL + R.ox, y = R.oy, z = R.oz;
+      asm volatile(
+          "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(
+              smem_u32(occ_s)),
+          "l"(m), "r"(x), "r"(y), "r"(z), "r"(smem_u32(&sm.mbar_st))
+          : "memory");
+      if (eam)
+        asm volatile(
+            "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(
+                smem_u32(rho_s)),
+            "l"(m + 128), "r"(x), "r"(y), "r"(z), "r"(smem_u32(&sm.mbar_st))
+            : "memory");
+    }
+  } else if (R.bulk) {
+    const int no = R.bo >> 4, nc = no + (eam ? R.br >> 2 : 0);  // 16-byte copies of a row
+    const int per = nc <= 16 ? 2 : 1;                           // rows a warp takes at a time (nc <= 32)
+    const int c = per == 2 ? lane & 15 : lane, sub = per == 2 ? lane >> 4 : 0;
+    const int nrows = R.ey * R.ez;
+    int row = warp * per + sub;
+    int lz = row / R.ey, ly = row - lz * R.ey;
+    const int step = kThreads / 32 * per, dz = step / R.ey, dy = step - dz * R.ey;
+    for (; row < nrows; row += step) {
+      const int gy = wrap1(R.oy + ly, J.sy), gz = wrap1(R.oz + lz, J.sz);
+      const int64_t first = static_cast<int64_t>(J.px) * (gy + static_cast<int64_t>(J.sy) * gz) + kHaloL + R.ox;
+      const int l = R.LX * (ly + R.LY * lz);  // the shared row (pitch LX, LY)
+      if (c < nc) {
+        const bool o = c < no;
+        const void* src = o ? static_cast<const void*>(J.occ + first + 16 * c) : static_cast<const void*>(J.rho + first + 4 * (c - no));
+        const uint32_t dst = o ? smem_u32(occ_s + l + 16 * c) : smem_u32(rho_s + l + 4 * (c - no));
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(dst), "l"(src) : "memory");
       }
-      return false;
+      ly += dy;
+      lz += dz;
+      if (ly >= R.ey) {
+        ly -= R.ey;
+        ++lz;
+      }
     }
-  }
-  JobC jc;
-  jc.occ = J.occ;
-  jc.rho = J.rho;
-  jc.sx = J.sx;
-  jc.sy = J.sy;
-  jc.sz = J.sz;
-  jc.px = J.px;
-
-  Region R;
-  make_region(B, J, sec, R);
-  if (tid == 0) {  // before the barrier below; the evaluations read them
-    sm.c_nu = J.nu;
-    sm.c_kT = J.kT;
-    sm.c_rkT = 1.0 / J.kT;
-  }
-  // F-table window: one bulk copy issued by the control thread, overlapped with the staging
-  const int win_key = J.pot * 2 + (KIND == kEam32 ? 1 : 0);
-  const bool need_win = eam && sm.win_pot != win_key;
-  // the shell tables depend on the potential, the kind and the region's row strides only: kept
-  // from the CTA's previous block when those match
-  const int tab0 = J.pot * 4 + KIND, tab1 = R.LX | (R.LY << 16);
-  const bool need_tab = sm.tab_key[0] != tab0 || sm.tab_key[1] != tab1;
-  const int nrows = R.LY * R.LZ;
-  if (R.bulk && !flowpre && tid == kCtl)  // armed before any copy is issued (after the barrier below)
-    bulk_expect(&sm.mbar_st, stage_bytes(R, eam));
-  __syncthreads();  // every thread has read win_pot and tab_key; the previous item's readers are done
-  AKMC_STAGE_T(0);
-  if (need_win && tid == kCtl) {
-    if (KIND == kEam32) {
-      bulk_expect(&sm.mbar, kFWin * 20u);
-      bulk_copy(sm.fwin, P.F32a + P.fwin0, kFWin * 16u, &sm.mbar);
-      bulk_copy(sm.fwin + kFWin * 16, P.F32b + P.fwin0, kFWin * 4u, &sm.mbar);
-    } else {
-      bulk_expect(&sm.mbar, kFWin * 32u);
-      bulk_copy(sm.fwin, P.F64lo + P.fwin0, kFWin * 16u, &sm.mbar);
-      bulk_copy(sm.fwin + kFWin * 16, P.F64hi + P.fwin0, kFWin * 16u, &sm.mbar);
-    }
-  }
-  if (need_tab) {
-    load_tables<W>(sm, P, *a.geo, R, KIND);
-    if (tid == 0) {
-      sm.tab_key[0] = tab0;
-      sm.tab_key[1] = tab1;
-    }
-  }
-  FTab FT;
-  FT.win = sm.fwin;
-  FT.kw0 = P.fwin0;
-  FT.pot = &P;
-  FT.status = a.status;
-#ifdef AKMC_PHASE_PROFILE
-  FT.prof = a.counters + 16;
-#endif
-  AKMC_STAGE_T(1);
-
-  // stage the region: warp w takes rows w, w + W, ...; kStageRows rows of loads are issued
-  // before any shared-memory store so they are all in flight (rows hold <= 64 sites)
-  if (!R.bulk) {
-    // row positions of the region's x span (the halo holds the sites past either end)
+  } else {
+    // row loads, where shared memory cannot hold the rounded rows: warp w takes rows w, w + W, ...;
+    // kStageRows rows of loads are issued before any shared-memory store so they are all in flight (rows hold
+    // <= 64 sites; the halo holds the sites past either end)
     const int gx0 = kHaloL + R.ox + lane, gx1 = gx0 + 32;
     const bool has0 = lane < R.LX, has1 = lane + 32 < R.LX;
     constexpr int kW = kThreads / 32;
+    const int nrows = R.LY * R.LZ;
     for (int row0 = warp; row0 < nrows; row0 += kStageRows * kW) {
       uint8_t ov[kStageRows][2];
       int32_t rv[kStageRows][2];
@@ -931,15 +785,15 @@ __device__ __forceinline__ bool run_block(const RoundArgs& a, int gb, Smem& sm, 
         const int row = row0 + kW * k;
         if (row < nrows) {
           const int ly = row % R.LY, lz = row / R.LY;
-          const int gy = wrap1(R.oy + ly, jc.sy), gz = wrap1(R.oz + lz, jc.sz);
-          const int64_t base = static_cast<int64_t>(jc.px) * (gy + static_cast<int64_t>(jc.sy) * gz);
+          const int gy = wrap1(R.oy + ly, J.sy), gz = wrap1(R.oz + lz, J.sz);
+          const int64_t base = static_cast<int64_t>(J.px) * (gy + static_cast<int64_t>(J.sy) * gz);
           if (has0) {
-            ov[k][0] = __ldcg(jc.occ + base + gx0);
-            if (eam) rv[k][0] = __ldcg(jc.rho + base + gx0);
+            ov[k][0] = __ldcg(J.occ + base + gx0);
+            if (eam) rv[k][0] = __ldcg(J.rho + base + gx0);
           }
           if (has1) {
-            ov[k][1] = __ldcg(jc.occ + base + gx1);
-            if (eam) rv[k][1] = __ldcg(jc.rho + base + gx1);
+            ov[k][1] = __ldcg(J.occ + base + gx1);
+            if (eam) rv[k][1] = __ldcg(J.rho + base + gx1);
           }
         }
       }
@@ -959,89 +813,173 @@ __device__ __forceinline__ bool run_block(const RoundArgs& a, int gb, Smem& sm, 
         }
       }
     }
-  } else if (!flowpre) {
-    if (R.tma) {
-      if (tid == kCtl) stage_tensor(R, a.tmaps, B.job, eam, occ_s, rho_s, &sm.mbar_st);
+  }
+}
+
+// Vacancy record k of the running sector: vacancy v at site s = (X, y, z).
+__device__ __forceinline__ void put_record(Smem& sm, const Region& R, int k, int v, int32_t s, int X, int y, int z) {
+  const int lx = X - R.ox, ly = y - R.oy, lz = z - R.oz;
+  sm.vidx[k] = v;
+  sm.vact[k] = 1;
+  sm.vpk[k][0] = make_int4(lx + R.LX * (ly + R.LY * lz), lx, ly, lz);
+  sm.vpk[k][1] = make_int4(X, y, z, s);
+}
+
+// Phase profile (builds with -DAKMC_PHASE_PROFILE): thread 0 accumulates the cycles
+// between consecutive CTA barriers into counters[8 + phase].
+#ifdef AKMC_PHASE_PROFILE
+#define AKMC_PHASE(i)                                                                           \
+  do {                                                                                          \
+    if (threadIdx.x == 0) {                                                                     \
+      const long long t_ = clock64();                                                           \
+      atomicAdd(a.counters + 8 + (i), static_cast<unsigned long long>(t_ - tph));               \
+      tph = t_;                                                                                 \
+    }                                                                                           \
+  } while (0)
+#else
+#define AKMC_PHASE(i) \
+  do {              \
+  } while (0)
+#endif
+// Advances the running state of stream lane (0 selection, 1 residence time) by one draw into ring
+// slot `slot`: the raw draw and the state after it.  Called by lanes 0 and 1 of one warp.
+__device__ __forceinline__ void draw_ahead(Smem& sm, uint64_t (&x)[4], int lane, int slot) {
+  sm.raw[lane][slot] = xoshiro_next(x);
+#pragma unroll
+  for (int i = 0; i < 4; ++i) sm.sts[slot][lane][i] = x[i];
+}
+// What a batch's draws stand for, one draw a lane: the selection uniform in [0, 1) (lanes 0-7) and
+// -ln of the residence-time uniform in (0, 1] (lanes 8-15; sublattice.inl:118-120).
+__device__ __forceinline__ void draw_values(Smem& sm, int lane, int slot0) {
+  if (lane < kDrawBatch) {
+    sm.du[slot0 + lane] = static_cast<double>(sm.raw[0][slot0 + lane] >> 11) * 0x1p-53;
+  } else if (lane < 2 * kDrawBatch) {
+    const int k = slot0 + lane - kDrawBatch;
+    sm.dl[k] = -port_log(static_cast<double>((sm.raw[1][k] >> 11) + 1) * 0x1p-53);
+  }
+}
+
+// The hop loop of the active sector of one block, round C (or, with API, one per-hop API step), CTA-collective.
+// Before the call, after a CTA barrier that ended all earlier use of shared memory: sm.job holds the block's
+// job, the region's copies are issued (stage_region), and threads outside the last warp have written the records
+// of the sector's sm.fnv vacancies (put_record, any order).  Returns, uniformly, the number of vacancies, or -1
+// when the sector's clock is already past its window: nothing ran.
+//
+// Every warp selects for itself, all lanes alike (the ordered sums are deterministic, so no broadcast
+// is needed); the hop's updates are spread over the warps.
+template <int KIND, int W, bool API>
+__device__ __forceinline__ int run_block(const RoundArgs& a, Smem& sm, Round& C, const Region& R, uint8_t* occ_s,
+                                         int32_t* rho_s, int sec) {
+  AKMC_SHAPE(W);
+  constexpr int kClk = Shape<W>::kClk, kOrdWarp = Shape<W>::kOrdWarp;
+  constexpr bool eam = KIND != kPairBond;
+  const int tid = threadIdx.x;
+  const int lane = tid & 31, warp = tid >> 5;
+#ifdef AKMC_PHASE_PROFILE
+  long long tph = clock64();
+#endif
+  const JobDev& J = sm.job;
+  const int64_t round_now = C.r;
+  const double thr = API ? 0.0 : static_cast<double>((round_now >> 3) + 1) * J.window - C.evo;
+  const bool runs = API || 0.0 < thr;  // else sector_time stays 0 (sublattice.inl:82)
+  const Potential& P = a.pots[J.pot];
+  JobC jc;
+  jc.occ = J.occ;
+  jc.rho = J.rho;
+  jc.sx = J.sx;
+  jc.sy = J.sy;
+  jc.sz = J.sz;
+  jc.px = J.px;
+  // F-table window: one bulk copy per plane issued by the control thread, overlapped with the staging
+  const int win_key = J.pot * 2 + (KIND == kEam32 ? 1 : 0);
+  const bool need_win = eam && runs && sm.win_pot != win_key;
+  // the shell tables depend on the potential, the kind and the region's row strides only: kept
+  // from the CTA's previous block when those match
+  const int tab0 = J.pot * 4 + KIND, tab1 = R.LX | (R.LY << 16);
+  const bool need_tab = runs && (sm.tab_key[0] != tab0 || sm.tab_key[1] != tab1);
+  if (need_win && tid == kCtl) {
+    if (KIND == kEam32) {
+      bulk_expect(&sm.mbar, kFWin * 20u);
+      bulk_copy(sm.fwin, P.F32a + J.fwin0, kFWin * 16u, &sm.mbar);
+      bulk_copy(sm.fwin + kFWin * 16, P.F32b + J.fwin0, kFWin * 4u, &sm.mbar);
     } else {
-      stage_rows(R, jc.occ, jc.rho, jc.px, jc.sy, jc.sz, eam, occ_s, rho_s, &sm.mbar_st, tid, kThreads);
+      bulk_expect(&sm.mbar, kFWin * 32u);
+      bulk_copy(sm.fwin, P.F64lo + J.fwin0, kFWin * 16u, &sm.mbar);
+      bulk_copy(sm.fwin + kFWin * 16, P.F64hi + J.fwin0, kFWin * 16u, &sm.mbar);
     }
   }
-  AKMC_STAGE_T(2);
-  const int cnt = cnt_in;
-  if (tid < cnt) {
-    const int v = vlist[tid];
-    const int s = flowpre ? sm.fsite[tid] : __ldcg(&a.vac_site[v]);
-    const int X = s % jc.sx;
-    const int t = s / jc.sx;
-    const int y = t % jc.sy;
-    const int z = t / jc.sy;
-    const int lx = X - R.ox, ly = y - R.oy, lz = z - R.oz;
-    sm.vidx[tid] = v;
-    sm.vact[tid] = 1;
-    sm.vpk[tid][0] = make_int4(lx + R.LX * (ly + R.LY * lz), lx, ly, lz);
-    sm.vpk[tid][1] = make_int4(X, y, z, s);
-  }
-  if (!API && !flowpre && tid >= kCtl && tid < kCtl + 8) {
-    const int q = tid - kCtl;
-    sm.str[q >> 2][q & 3] = q < 4 ? __ldcg(&B.xs[q]) : __ldcg(&B.xt[q - 4]);
-  }
-  __syncthreads();
-  AKMC_STAGE_T(3);
-  AKMC_PHASE(0);
-  if (tid < cnt) {
-    // z-y-x scan order of ABVIModel::calcRates = ascending site id inside a sector
-    const int s = sm.vpk[tid][1].w;
-    int rank = 0;
-    for (int i = 0; i < cnt; ++i) rank += sm.vpk[i][1].w < s ? 1 : 0;
-    sm.ord[0][rank] = tid;
-  }
-  if (!API && warp == kEvalWarps - 1) {  // the first batch of draws
-    if (lane < 2) {
-      uint64_t x[4];
+  if (need_tab) load_tables<W>(sm, P, *a.geo, R, KIND);
+  FTab FT;
+  FT.win = sm.fwin;
+  FT.kw0 = J.fwin0;
+  FT.pot = &P;
+  FT.status = a.status;
+  if (warp == kEvalWarps - 1) {
+    if (!API) {  // the first batch of draws, while the others order the vacancies and the copies fly
+      if (lane < 2) {
+        uint64_t x[4];
 #pragma unroll
-      for (int i = 0; i < 4; ++i) x[i] = sm.str[lane][i];
+        for (int i = 0; i < 4; ++i) x[i] = C.str[lane][i];
 #pragma unroll 1
-      for (int k = 0; k < kDrawBatch; ++k) draw_ahead(sm, x, lane, k);
+        for (int k = 0; k < kDrawBatch; ++k) draw_ahead(sm, x, lane, k);
 #pragma unroll
-      for (int i = 0; i < 4; ++i) sm.str[lane][i] = x[i];
+        for (int i = 0; i < 4; ++i) sm.str[lane][i] = x[i];
+      }
+      __syncwarp();
+      draw_values(sm, lane, 0);
     }
-    __syncwarp();
-    draw_values(sm, lane, 0);
-  }
-  if (tid == 64) {
-    sm.nord[0] = cnt;
-    sm.ctl_ok = 1;
-    sm.c_hop0 = flowpre ? sm.hops_out : __ldcg(&B.hops);
-    sm.c_nh = 0;
-    sm.c_nact = 0;
-    sm.c_evals = cnt;
-    sm.c_sel = 0;
-    sm.ctl_stop = 0;
-    sm.c_time = 0.0;
-    if (need_win) {
-      if (mbar_wait(&sm.mbar, sm.mbar_phase)) {
-        sm.mbar_phase ^= 1u;
-        sm.win_pot = win_key;
-      } else {
-        atomicOr(a.status, kErrTimeout);
-        mbar_wait(&sm.mbar, sm.mbar_phase);  // bounded second wait for the copy in flight
-        sm.win_pot = -1;
-        sm.ctl_ok = 0;
+  } else {
+    asm volatile("bar.sync 3, %0;" ::"n"(kThreads - 32) : "memory");  // the records, written by these warps
+    const int n = sm.fnv;
+    if (tid < n) {
+      // z-y-x scan order of ABVIModel::calcRates = ascending site id inside a sector
+      const int s = sm.vpk[tid][1].w;
+      int rank = 0;
+      for (int i = 0; i < n; ++i) rank += sm.vpk[i][1].w < s ? 1 : 0;
+      sm.ord[0][rank] = tid;
+    }
+    if (tid == 64) {
+      sm.nord[0] = n;
+      sm.ctl_ok = 1;
+      sm.ctl_stop = 0;
+      sm.c_nh = 0;
+      sm.c_nact = 0;
+      sm.c_evals = n;
+      sm.c_sel = 0;
+      sm.c_time = 0.0;
+      if (need_win) {
+        if (mbar_wait(&sm.mbar, sm.mbar_phase)) {
+          sm.mbar_phase ^= 1u;
+          sm.win_pot = win_key;
+        } else {
+          atomicOr(a.status, kErrTimeout);
+          mbar_wait(&sm.mbar, sm.mbar_phase);  // bounded second wait for the copy in flight
+          sm.win_pot = -1;
+          sm.ctl_ok = 0;
+        }
+      }
+      if (R.tma) {
+        if (mbar_wait(&sm.mbar_st, sm.mbst_phase)) {
+          sm.mbst_phase ^= 1u;
+        } else {
+          atomicOr(a.status, kErrTimeout);
+          if (mbar_wait(&sm.mbar_st, sm.mbst_phase)) sm.mbst_phase ^= 1u;  // bounded second wait
+          sm.ctl_ok = 0;
+        }
       }
     }
-    if (R.bulk) {  // the region's rows
-      if (mbar_wait(&sm.mbar_st, sm.mbst_phase)) {
-        sm.mbst_phase ^= 1u;
-      } else {
-        atomicOr(a.status, kErrTimeout);
-        if (mbar_wait(&sm.mbar_st, sm.mbst_phase)) sm.mbst_phase ^= 1u;  // bounded second wait
-        sm.ctl_ok = 0;
-      }
-    }
   }
+  asm volatile("cp.async.wait_all;" ::: "memory");  // this thread's copies of the region's rows
+  AKMC_PHASE(0);
   __syncthreads();
   AKMC_PHASE(1);
-  if (!sm.ctl_ok) return true;
+  if (need_tab && tid == 0) {
+    sm.tab_key[0] = tab0;
+    sm.tab_key[1] = tab1;
+  }
+  if (!runs) return -1;
+  const int cnt = sm.fnv;
+  if (!sm.ctl_ok) return cnt;
   // this lane's share of the dE terms and of the jump sums (taken by the even and odd warps of a pair)
   Slot sl[kJumpsPerWarp];
   int4 ix[2];
@@ -1118,23 +1056,23 @@ __device__ __forceinline__ bool run_block(const RoundArgs& a, int gb, Smem& sm, 
     sm.ctl_stop = stop;
     return dt;
   };
-  // The event record of the hop just counted (hop index c_hop0 + c_nh - 1).
+  // The event record of the hop just counted (hop index C.hops + c_nh - 1).
   auto log_event = [&](int from, int to, int X, double u, double total, double dt, int n_act, int nd) {
     const unsigned long long slot = atomicAdd(a.log_count, 1ull);
     if (slot < static_cast<unsigned long long>(a.log_cap)) {
       akmc_event* e = a.log + slot;
       e->round = round_now;
-      e->hop = sm.c_hop0 + sm.c_nh - 1;
+      e->hop = C.hops + sm.c_nh - 1;
       e->from_site = from;
       e->to_site = to;
-      e->block = B.local_id;
+      e->block = C.local;
       e->species = X;
       e->u = u;
       e->total = total;
       e->dt = dt;
       e->n_act = n_act;
       e->n_dirty = nd;
-      e->job = B.job;
+      e->job = C.job;
       e->reserved = 0;
     } else {
       atomicOr(a.status, kErrLogOverflow);
@@ -1562,17 +1500,17 @@ __device__ __forceinline__ bool run_block(const RoundArgs& a, int gb, Smem& sm, 
       if (API && tid == kClk) {
         akmc_event* e = a.api_event;
         e->round = 0;
-        e->hop = sm.c_hop0;
+        e->hop = C.hops;
         e->from_site = hop ? pb.w : -1;
         e->to_site = hop ? nid : -1;
-        e->block = B.local_id;
+        e->block = C.local;
         e->species = hop ? X : 0;
         e->u = u;
         e->total = total;
         e->dt = 0.0;
         e->n_act = nord;
         e->n_dirty = hop ? __popc(m0) + __popc(m1) : 0;
-        e->job = B.job;
+        e->job = C.job;
         e->reserved = 0;
       }
       if (sm.ctl_stop) break;
@@ -1580,27 +1518,33 @@ __device__ __forceinline__ bool run_block(const RoundArgs& a, int gb, Smem& sm, 
   }
   __syncthreads();
   AKMC_PHASE(6);
-  if (API && a.mode == kModeCalc) return true;
-  if (tid == kCtl) {
-    const int64_t nh = sm.c_nh;
+  if (API && a.mode == kModeCalc) return cnt;
+  // The lattice was written through at every hop (or at the end of the pair-bond loop); the vacancy positions,
+  // the block's record and the counters remain.
+  if (tid < cnt) a.vac_site[sm.vidx[tid]] = sm.vpk[tid][1].w;
+  if (tid == 0) {
+    BlockDev& B = a.blocks[C.gb];
     if (!API) {
-      // (k_flow read the clock while the region's copies flew: no second round trip)
-      B.evo[sec] = (flowpre ? sm.pre_evo : __ldcg(&B.evo[sec])) + sm.c_time;
+      B.evo[sec] = C.evo + sm.c_time;
       const int n = sm.c_sel;  // draws the selections used: the streams move on by as many
       if (n > 0) {
         const int slot = (n - 1) & (kDrawRing - 1);
+#pragma unroll
         for (int i = 0; i < 4; ++i) {
-          B.xs[i] = sm.sts[slot][0][i];
-          B.xt[i] = sm.sts[slot][1][i];
+          B.xs[i] = C.str[0][i] = sm.sts[slot][0][i];
+          B.xt[i] = C.str[1][i] = sm.sts[slot][1][i];
         }
       }
     }
-    B.hops = sm.c_hop0 + nh;
-    sm.hops_out = sm.c_hop0 + nh;
-    if (sm.acc_job != B.job) {
+    C.hops += sm.c_nh;
+    B.hops = C.hops;
+  }
+  if (tid == 32) {
+    const int64_t nh = sm.c_nh;
+    if (sm.acc_job != C.job) {
       if (sm.acc_job >= 0 && sm.acc_job_hops)
         atomicAdd(reinterpret_cast<unsigned long long*>(&a.jobs[sm.acc_job].hops), sm.acc_job_hops);
-      sm.acc_job = B.job;
+      sm.acc_job = C.job;
       sm.acc_job_hops = 0;
     }
     sm.acc_job_hops += static_cast<unsigned long long>(nh);
@@ -1611,9 +1555,7 @@ __device__ __forceinline__ bool run_block(const RoundArgs& a, int gb, Smem& sm, 
     sm.acc[4] += static_cast<unsigned long long>(R.nt);
     sm.acc[5] += static_cast<unsigned long long>(nh * (eam ? 2 + kRefreshN : 2));
   }
-  // the lattice was written through at every hop; only the vacancy positions remain
-  if (tid < cnt) a.vac_site[sm.vidx[tid]] = sm.vpk[tid][1].w;
-  return true;
+  return cnt;
 }
 
 // The region's arrays after Smem, each starting on a 128-byte boundary of the shared window
@@ -1626,20 +1568,46 @@ __device__ __forceinline__ void carve(uint8_t* smem, int nreg, Smem*& sm, uint8_
   occ_s = occ_of(rho_s, nreg);
 }
 
-__device__ void dispatch_block(const RoundArgs& a, int gb, uint8_t* smem) {
+// One block whose sector's vacancies k_bucket listed (k_hop, k_api_block), CTA-wide.
+template <int KIND, int W, bool API>
+__device__ __forceinline__ void listed_block(const RoundArgs& a, int gb, int sec, uint8_t* smem) {
+  Smem& sm0 = *reinterpret_cast<Smem*>(smem);
+  const int tid = threadIdx.x;
   const BlockDev& B = a.blocks[gb];
-  const JobDev& J = a.jobs[B.job];
+  __syncthreads();  // the previous block's readers are done
+  Round& C = sm0.round[0];
+  if (tid == 0) {
+    C.gb = gb;
+    C.job = B.job;
+    C.local = B.local_id;
+    C.r = B.round;
+    C.hops = B.hops;
+    C.evo = B.evo[sec];
+    sm0.fnv = min(B.cnt, kMaxV);
+  } else if (tid >= 32 && tid < 35) {
+    C.c0[tid - 32] = B.c0[tid - 32];
+    C.c1[tid - 32] = B.c1[tid - 32];
+  } else if (tid >= 64 && tid < 72) {
+    const int q = tid - 64;
+    C.str[q >> 2][q & 3] = q < 4 ? B.xs[q] : B.xt[q - 4];
+  }
+  __syncthreads();
+  load_job(sm0, a, C.job);
   Region R;
-  make_region(B, J, a.api_sector, R);
+  make_region(C.c0, C.c1, sm0.job, sec, R);
   Smem* sm;
   uint8_t* occ_s;
   int32_t* rho_s;
   carve(smem, R.n, sm, occ_s, rho_s);
-  const int32_t* vl = a.blk_list + static_cast<int64_t>(gb) * kMaxV;
-  const int cnt = min(B.cnt, kMaxV);
-  if (J.model == AKMC_MODEL_PAIRBOND) run_block<kPairBond, 8, true>(a, gb, *sm, occ_s, rho_s, vl, cnt, B.round);
-  else if (J.precision == AKMC_FP32C) run_block<kEam32, 8, true>(a, gb, *sm, occ_s, rho_s, vl, cnt, B.round);
-  else run_block<kEam64, 8, true>(a, gb, *sm, occ_s, rho_s, vl, cnt, B.round);
+  stage_region<KIND, W>(*sm, a, R, occ_s, rho_s);
+  if (tid < sm->fnv) {
+    const JobDev& J = sm->job;
+    const int v = a.blk_list[static_cast<int64_t>(gb) * kMaxV + tid];
+    const int32_t s = a.vac_site[v];
+    const int t = s / J.sx;
+    put_record(*sm, R, tid, v, s, s - t * J.sx, t % J.sy, t / J.sy);
+  }
+  run_block<KIND, W, API>(a, *sm, C, R, occ_s, rho_s, sec);
 }
 
 __global__ void k_bucket(RoundArgs a) {
@@ -1680,6 +1648,8 @@ __device__ void init_cta_smem(uint8_t* smem) {
   Smem* sm = reinterpret_cast<Smem*>(smem);
   if (threadIdx.x == 0) {
     sm->win_pot = -1;
+    sm->job_key = -1;
+    sm->fnv = 0;
     sm->tab_key[0] = sm->tab_key[1] = -1;
     sm->mbar_phase = 0;
     sm->mbst_phase = 0;
@@ -1723,14 +1693,7 @@ __global__ void __launch_bounds__(Shape<W>::kThreads, Shape<W>::kCtasPerSm) k_ho
     const int gb = a.active[item];
     const BlockDev& B = a.blocks[gb];
     if (job_kind(a.jobs[B.job]) != KIND) continue;
-    Region R;
-    make_region(B, a.jobs[B.job], sector_of_round(B.round), R);
-    Smem* sm;
-    uint8_t* occ_s;
-    int32_t* rho_s;
-    carve(smem, R.n, sm, occ_s, rho_s);
-    run_block<KIND, W, false>(a, gb, *sm, occ_s, rho_s, a.blk_list + static_cast<int64_t>(gb) * kMaxV, min(B.cnt, kMaxV),
-                       B.round);
+    listed_block<KIND, W, false>(a, gb, sector_of_round(B.round), smem);
   }
   cta_flush<W>(a, smem);
 }
@@ -1758,11 +1721,6 @@ __global__ void __launch_bounds__(Shape<W>::kThreads, Shape<W>::kCtasPerSm) k_ho
 // straight away when it holds no other round of the sweep (its hop budget is checked here, at
 // each time-step boundary).
 
-__device__ __forceinline__ unsigned long long ld_acquire_u64(const unsigned long long* p) {
-  unsigned long long v;
-  asm volatile("ld.acquire.gpu.global.b64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
-  return v;
-}
 __device__ __forceinline__ uint64_t globaltimer_ns() {
   uint64_t t;
   asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
@@ -1773,11 +1731,6 @@ __device__ __forceinline__ void fence_acq_rel() { asm volatile("fence.acq_rel.gp
 __device__ __forceinline__ void st_release_u64(unsigned long long* p, unsigned long long v) {
   asm volatile("st.release.gpu.global.b64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
 }
-#ifdef AKMC_PUBLISH_FENCE
-__device__ __forceinline__ void st_relaxed_u64(unsigned long long* p, unsigned long long v) {
-  asm volatile("st.relaxed.gpu.global.b64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
-}
-#endif
 __device__ __forceinline__ unsigned long long ld_relaxed_u64(const unsigned long long* p) {
   unsigned long long v;
   asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(v) : "l"(p));
@@ -1789,18 +1742,20 @@ __device__ __forceinline__ unsigned int ld_relaxed_u32(const unsigned int* p) {
   return v;
 }
 
-// Rounds back to the latest earlier round of the neighbour at offset (dx, dy, dz) whose
-// region meets this round's (phase = round mod 8), 0 if none ever does.  Per dimension a
-// +1 neighbour's regions meet ours only between our high half and its low half (block
-// edges >= 8 cells, halos of 2), a -1 neighbour's only between our low half and its high.
-__device__ int flow_lag(int phase, int dx, int dy, int dz) {
-  const int now = sector_of_round(phase);
-  const int d[3] = {dx, dy, dz};
+// Rounds back to the latest earlier round of the neighbour at offset o = (dz+1)*9 + (dy+1)*3 + dx+1 whose
+// region meets this round's (phase = round mod 8), 0 if none ever does.  Per dimension a +1 neighbour's regions
+// meet ours only between our high half and its low half (block edges >= 8 cells, halos of 2), a -1 neighbour's
+// only between our low half and its high half.
+__host__ __device__ constexpr int flow_sector(int phase) {
+  constexpr int ring[8] = {0, 7, 2, 5, 3, 4, 1, 6};  // sector_of_round
+  return ring[phase & 7];
+}
+__host__ __device__ constexpr int flow_lag(int phase, int o) {
+  const int d[3] = {o % 3 - 1, (o / 3) % 3 - 1, o / 9 - 1};
   for (int k = 1; k <= 8; ++k) {
-    const int then = sector_of_round(phase + 8 - k);
-    bool meet = true;
+    bool meet = o != 13;
     for (int a = 0; a < 3; ++a) {
-      const int hn = (now >> a) & 1, ht = (then >> a) & 1;
+      const int hn = (flow_sector(phase) >> a) & 1, ht = (flow_sector(phase + 8 - k) >> a) & 1;
       if (d[a] == 1) meet = meet && hn == 1 && ht == 0;
       if (d[a] == -1) meet = meet && hn == 0 && ht == 1;
     }
@@ -1842,7 +1797,8 @@ __device__ int budget_gate(const RoundArgs& a, const JobDev& J, int64_t b) {
 
 // Flags word of a block's row of RoundArgs::nbr: the energy kind (kNbrFree for a free block
 // slot) and whether the job's hop budget gates its rounds at time-step boundaries (budget_gate).
-constexpr int kNbrFree = 3, kNbrKindMask = 3, kNbrGate = 4;
+// kNbrSolo: a single-block job, whose rounds wait for no other block.
+constexpr int kNbrFree = 3, kNbrKindMask = 3, kNbrGate = 4, kNbrSolo = 8;
 
 // The neighbours' completed rounds relative to round r0 (P[o] = rounds - r0, clamped to
 // +-2^30; the block itself never holds it back: 2^30), read with relaxed loads, all in flight at
@@ -1878,30 +1834,28 @@ __device__ __forceinline__ void flow_snapshot(const RoundArgs& a, int gb, const 
   }
 }
 
-// Whether a snapshot relative to r0 lets round r0 + d run (the neighbours' rounds it waits for
-// are complete).
-__device__ __forceinline__ bool flow_ready(const int32_t (&P)[27], int64_t r0, int d, const int8_t (*lag)[27]) {
-  const int ph = static_cast<int>((r0 + d) & 7);
-  bool ok = true;
-#pragma unroll
-  for (int o = 0; o < 27; ++o) {
-    const int k = lag[ph][o];
-    if (k && P[o] < d - k + 1) ok = false;
-  }
-  return ok;
+// Rounds from r0 on that a snapshot relative to r0 lets run: the smallest d <= D such that some neighbour has
+// not completed the round that r0 + d waits for.  Round r0 + d, of phase (r0 + d) mod 8, waits for a neighbour
+// with lag k to have completed d - k + 1 rounds past r0; so for each phase (first reached after e rounds) and
+// neighbour, the first round held back is e + 8 max(0, floor((P + k + 7 - e) / 8)).  56 pairs of a phase and a
+// neighbour with a lag, five instructions each, for any number of rounds.
+template <int I>
+__device__ __forceinline__ int flow_limit_pair(const int32_t (&P)[27], const int (&e)[8], int D) {
+  constexpr int o = I / 8, ph = I % 8, k = flow_lag(ph, o);
+  if constexpr (k > 0) D = min(D, e[ph] + 8 * max(0, (P[o] + (k + 7) - e[ph]) >> 3));
+  return D;
 }
-
-__device__ __forceinline__ bool site_in_sector(const BlockDev& B, const JobDev& J, int sec, int32_t s) {
-  const int X = s % J.sx;
-  const int t = s / J.sx;
-  const int c[3] = {X >> 1, t % J.sy, t / J.sy};
-  for (int d = 0; d < 3; ++d) {
-    const int half = (B.c1[d] - B.c0[d]) / 2;
-    const int lo = (sec >> d) & 1 ? B.c0[d] + half : B.c0[d];
-    const int hi = (sec >> d) & 1 ? B.c1[d] : B.c0[d] + half;
-    if (c[d] < lo || c[d] >= hi) return false;
-  }
-  return true;
+template <int... I>
+__device__ __forceinline__ int flow_limit_all(const int32_t (&P)[27], const int (&e)[8], int D,
+                                              std::integer_sequence<int, I...>) {
+  ((D = flow_limit_pair<I>(P, e, D)), ...);
+  return D;
+}
+__device__ __forceinline__ int flow_limit(const int32_t (&P)[27], int64_t r0, int D) {
+  int e[8];
+#pragma unroll
+  for (int k = 0; k < 8; ++k) e[k] = (k - static_cast<int>(r0)) & 7;
+  return flow_limit_all(P, e, D, std::make_integer_sequence<int, 27 * 8>{});
 }
 
 // Block whose area holds site s (the reference's rank split, as k_bucket) and the sector of that
@@ -1922,73 +1876,73 @@ __device__ __noinline__ int owner_sector(const JobDev& J, int32_t s, int* sec) {
   return J.block0 + k[0] + J.nb[0] * (k[1] + J.nb[1] * k[2]);
 }
 
-// Puts vacancy v into block o's slots: claim a free slot, write the id, then mark it valid.
+// A block's vacancy slot: the vacancy's id and site in one word, so that one store or compare-and-swap moves it.
+constexpr unsigned long long kNoVacancy = ~0ull;
+__device__ __forceinline__ unsigned long long slot_word(int v, int32_t site) {
+  return static_cast<unsigned long long>(static_cast<uint32_t>(v)) << 32 | static_cast<uint32_t>(site);
+}
+// Puts vacancy v into a free slot of block o, then marks its sector occupied.  The word becomes readable as a
+// whole; a round of o that can see the vacancy waits for this block's round, which is published after both.
 __device__ void flow_give(const RoundArgs& a, int o, int v, int32_t site, int osec) {
-  for (int tries = 0; tries < 4 * kFlowSlots; ++tries) {
-    const unsigned long long m = *reinterpret_cast<volatile unsigned long long*>(&a.vclaim[o]);
-    if (m == ~0ull) break;
-    const int slot = __ffsll(static_cast<long long>(~m)) - 1;
-    const unsigned long long bit = 1ull << slot;
-    if (atomicOr(&a.vclaim[o], bit) & bit) continue;  // taken meanwhile
-    a.vslot[static_cast<int64_t>(o) * kFlowSlots + slot] = v;
-    a.vsite[static_cast<int64_t>(o) * kFlowSlots + slot] = site;
-    fence_acq_rel();
-    atomicOr(&a.vvalid[o], bit);
-    atomicOr(&a.vsec[o], 1u << osec);
-    return;
+  unsigned long long* const slots = a.vslot + static_cast<int64_t>(o) * kFlowSlots;
+  for (int k = 0; k < kFlowSlots; ++k) {
+    const int i = (v + k) & (kFlowSlots - 1);
+    if (atomicCAS(slots + i, kNoVacancy, slot_word(v, site)) == kNoVacancy) {
+      atomicOr(&a.vsec[o], 1u << osec);
+      return;
+    }
   }
   atomicOr(a.status, kErrVacOverflow);
 }
 
 // Publishes the block's completed rounds (rn) and keeps (keep = 1) or frees the lease, with
 // one release store.  Release is cumulative: writes of other threads of the CTA that a barrier
-// ordered before this call are released too.  (-DAKMC_PUBLISH_FENCE: a fence and a relaxed
-// store instead, the form measured before.)  `reached`: this lease holder moved the
+// ordered before this call are released too.  `reached`: this lease holder moved the
 // block onto its target (each block is counted once).
 __device__ __forceinline__ void flow_publish(const RoundArgs& a, int gb, int64_t rn, int keep, bool reached,
                                              int kind) {
-#ifdef AKMC_PUBLISH_FENCE
-  fence_acq_rel();
-  st_relaxed_u64(&a.fstate[gb], (static_cast<unsigned long long>(rn) << 1) | static_cast<unsigned long long>(keep));
-#else
   st_release_u64(&a.fstate[gb], (static_cast<unsigned long long>(rn) << 1) | static_cast<unsigned long long>(keep));
-#endif
   if (reached) atomicAdd(&a.flow_done[kind], 1);
 }
 
-// Lease held, one thread, the block at round r0: runs the block's ready rounds whose sectors
-// hold no vacancy (the clock jumps to the window, sublattice.inl:108-112), up to 64 in one
-// batch, and leaves the block's round in *rn (the caller publishes it).  A round is ready when
-// the snapshot of the neighbours' round counters (the sweep's, Pin, or one read here with all
-// loads in flight together) already covers it, and the vacancy slots read after the snapshot
-// hold every vacancy those rounds can see (a round that could bring one into such a sector
-// overlaps it, so it is in the snapshot).  Returns true when it stops at a ready round with vacancies, false when the next
-// round is not ready or the target is reached.  *reached: this call moved the block onto its
-// target (by running rounds, or by a budget moving the target down to r0); false for a block
-// that was at its target already (a stale sweep read).
-__device__ bool flow_advance(const RoundArgs& a, BlockDev& B, const JobDev& J, int gb, const int8_t (*lag)[27],
-                             int64_t r0, const int32_t (*Pin)[27], int64_t* rn, bool* reached, int64_t* tgt,
-                             unsigned long long* vv = nullptr) {
+// Lease held, one thread, block gb of job `job` at round r0, with its next D rounds ready (flow_limit; 64 for a
+// single-block job): runs the ready rounds whose sectors hold no vacancy (the clock jumps to the window,
+// sublattice.inl:108-112), up to 64 in one batch, and leaves the block's round in *rn (the caller publishes it).
+// The sector mask read after the snapshot holds every vacancy those rounds can see (a round that could bring one
+// into such a sector overlaps it, so it is in the snapshot).  Returns true when it stops at a ready round with
+// vacancies, which is then described in *C (C null: in the next entry of sm.round, false when `take` are full);
+// false when the next round is not ready or the target is reached.  *reached: this call moved the block onto
+// its target (by running rounds, or by a budget moving the target down to r0); false for a block that was at its
+// target already (a stale sweep read).
+__device__ __forceinline__ bool flow_advance(const RoundArgs& a, Smem& sm, int gb, int job, int64_t r0, int D, Round* C,
+                                             int take, int64_t* rn, bool* reached) {
+  BlockDev& B = a.blocks[gb];
+  const JobDev& J = a.jobs[job];
   *rn = r0;
   *reached = false;
-  // one round of loads, all in flight together: the target, the job's constants, the block's
-  // hops and clocks and its vacancy slots (the lease is held: nothing else writes them but gives)
+  // one round of loads, all in flight together: the block's record (the lease is held: nothing else writes it),
+  // its sector mask and the job's constants
+  static_assert(sizeof(BlockDev) % 16 == 0 && offsetof(BlockDev, evo) % 16 == 0 && offsetof(BlockDev, xs) % 16 == 0 &&
+                    offsetof(BlockDev, c0) == 8 && offsetof(BlockDev, c1) == 20,
+                "16-byte reads of the record");
+  const int4* head = reinterpret_cast<const int4*>(&B);
+  const int4 h0 = __ldcg(head), h1 = __ldcg(head + 1);  // job, local id, c0[0..1] | c0[2], c1
   const int64_t t_old = __ldcg(&B.target);
   const int64_t hops = __ldcg(&B.hops);  // empty rounds add none
+  double2 ev[4];
+  ulonglong2 st[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    ev[k] = __ldcg(reinterpret_cast<const double2*>(B.evo) + k);
+    st[k] = __ldcg(reinterpret_cast<const ulonglong2*>(B.xs) + k);
+  }
+  const unsigned occ_sec = __ldcg(&a.vsec[gb]);
   const int nbl = J.nblocks;
   const int64_t budget = J.hop_budget;
   const double window = J.window;
   double evo[8];
 #pragma unroll
-  for (int k = 0; k < 8; ++k) evo[k] = __ldcg(&B.evo[k]);
-  // sectors holding a vacancy (the slots' sector mask)
-  unsigned occ_sec = __ldcg(&a.vsec[gb]);
-  // and, for the round this call may hand over, the valid bits of the block's vacancy slots, read
-  // last and with acquire: the slots' ids and sites (written before a give sets its bit) are read
-  // after it, by the CTA's threads past a barrier.  Every vacancy that can lie in the round's
-  // sector came with a round this lease's snapshot covers; only the lease holder clears bits.
-  if (vv) *vv = ld_acquire_u64(&a.vvalid[gb]);
-  *tgt = t_old;
+  for (int k = 0; k < 8; ++k) evo[k] = k & 1 ? ev[k >> 1].y : ev[k >> 1].x;
   if (r0 >= t_old) return false;
   // a single-block job with a hop budget ends at the end of the first time step at which its
   // hops reached the budget: once they have, its target moves down to the next boundary at or
@@ -2002,49 +1956,31 @@ __device__ bool flow_advance(const RoundArgs& a, BlockDev& B, const JobDev& J, i
       B.budget_end = 1;
     }
   }
-  *tgt = target;
   if (r0 >= target) {
     *reached = true;
     return false;
   }
-  // the sweep's snapshot, taken before the lease and fenced after it (rounds only grow, so an
-  // earlier snapshot is a safe one), or a fresh one
-  int32_t P[27];
-  if (Pin) {
-#pragma unroll
-    for (int o = 0; o < 27; ++o) P[o] = (*Pin)[o];
-  } else if (J.nblocks == 1) {  // every neighbour is the block itself: nothing to wait for
-#pragma unroll
-    for (int o = 0; o < 27; ++o) P[o] = kAhead;
-  } else {
-    int y[28];
-    flow_row(a, gb, y);
-    flow_snapshot(a, gb, y, r0, P);
-    fence_acq_rel();
-    occ_sec = __ldcg(&a.vsec[gb]);  // with the vacancies those rounds gave the block
-  }
-  const int64_t last = min(target, r0 + 64);
+  const int64_t last = min(target, r0 + D);
   int64_t r = r0;
-  bool stop_full = false;
+  bool full = false;
+  double e = 0.0;
   while (r < last) {
-    if (!flow_ready(P, r0, static_cast<int>(r - r0), lag)) break;
     const int g = budget_gate(a, J, r);
     if (g == 0) break;
     if (g == 2) {  // the job ends at this boundary: the block's target moves down to it
       B.target = r;
       B.budget_end = 1;
       target = r;
-      *tgt = r;
       break;
     }
     const int sec = sector_of_round(r);
-    if ((occ_sec >> sec) & 1u) {
-      stop_full = true;
-      break;
-    }
-    double e = evo[0];
+    e = evo[0];
 #pragma unroll
     for (int k = 1; k < 8; ++k) e = k == sec ? evo[k] : e;
+    if ((occ_sec >> sec) & 1u) {
+      full = true;
+      break;
+    }
     const double thr = static_cast<double>((r >> 3) + 1) * window - e;
     double sector_time = 0.0;
     if (sector_time < thr) sector_time = thr;
@@ -2060,8 +1996,31 @@ __device__ bool flow_advance(const RoundArgs& a, BlockDev& B, const JobDev& J, i
   }
   *rn = r;
   *reached = r == target;  // the lease holder alone moves the target
-  *tgt = target;
-  return stop_full;
+  if (!full) return false;
+  if (!C) {
+    const int i = atomicAdd(&sm.flow_ncand, 1);
+    if (i >= take) return false;
+    C = &sm.round[i];
+  }
+  C->r = r;
+  C->t = target;
+  C->hops = hops;
+  C->evo = e;
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    C->str[k >> 1][2 * (k & 1)] = st[k].x;
+    C->str[k >> 1][2 * (k & 1) + 1] = st[k].y;
+  }
+  C->gb = gb;
+  C->job = job;
+  C->local = h0.y;
+  C->c0[0] = h0.z;
+  C->c0[1] = h0.w;
+  C->c0[2] = h1.x;
+  C->c1[0] = h1.y;
+  C->c1[1] = h1.z;
+  C->c1[2] = h1.w;
+  return true;
 }
 
 // Rounds with vacancies a CTA takes per sweep: a.flow_take (0: every ready round its threads
@@ -2072,20 +2031,16 @@ __device__ bool flow_advance(const RoundArgs& a, BlockDev& B, const JobDev& J, i
 template <int KIND, int W>
 __global__ void __launch_bounds__(Shape<W>::kThreads, Shape<W>::kCtasPerSm) k_flow(RoundArgs a) {
   AKMC_SHAPE(W);
-  const int kFlowTake = a.flow_take > 0 && a.flow_take < kMaxTake ? a.flow_take : kMaxTake;
+  const int take = a.flow_take > 0 && a.flow_take < kMaxTake ? a.flow_take : kMaxTake;
   extern __shared__ __align__(16) uint8_t smem[];
-  Smem* sm0 = reinterpret_cast<Smem*>(smem);
+  Smem& sm0 = *reinterpret_cast<Smem*>(smem);
   const int tid = threadIdx.x;
   init_cta_smem(smem);
-  for (int i = tid; i < 8 * 27; i += kThreads) {
-    const int o = i % 27;
-    sm0->flow_lag[i / 27][o] = static_cast<int8_t>(flow_lag(i / 27, o % 3 - 1, (o / 3) % 3 - 1, o / 9 - 1));
-  }
   const int nb = a.nblocks;
   const int watch = max(1, min(kThreads, static_cast<int>((static_cast<int64_t>(nb) * kSweepWatch) / gridDim.x)));
   int cursor = static_cast<int>((static_cast<int64_t>(blockIdx.x) * nb) / gridDim.x);
   const uint64_t t_begin = globaltimer_ns();  // a time-boxed launch takes no new round after its budget
-  if (tid == 0) sm0->flow_stop = 0;
+  if (tid == 0) sm0.flow_stop = 0;
 #ifdef AKMC_PHASE_PROFILE
   long long t_sweep = 0, t_hop = 0, n_sweep = 0, n_full = 0, t0 = 0;
 #endif
@@ -2094,11 +2049,11 @@ __global__ void __launch_bounds__(Shape<W>::kThreads, Shape<W>::kCtasPerSm) k_fl
     if (tid == 0) t0 = clock64();
 #endif
     if (tid == 0) {
-      sm0->flow_ncand = 0;
-      sm0->flow_progress = 0;
+      sm0.flow_ncand = 0;
+      sm0.flow_progress = 0;
     }
     __syncthreads();
-    if (sm0->flow_stop) break;  // decided during the previous sweep
+    if (sm0.flow_stop) break;  // decided during the previous sweep
     // thread 0 reads the launch's progress and status while the sweep's visits are in flight,
     // and decides after its own visit whether the CTA stops after this sweep's rounds
     int need = 0, done = 0;
@@ -2109,7 +2064,7 @@ __global__ void __launch_bounds__(Shape<W>::kThreads, Shape<W>::kCtasPerSm) k_fl
       st = *reinterpret_cast<volatile unsigned*>(a.status);
     }
 
-    // sweep: thread tid looks after blocks (cursor + tid + k kThreads) mod nb, k < kSweepVisits,
+    // sweep: thread tid looks after blocks (cursor + tid + k watch) mod nb, k < kSweepVisits,
     // until it takes one: a visit that finds nothing to do ends after one or two round trips,
     // while the sweep lasts as long as its slowest visit (one that takes a block)
 #pragma unroll 1
@@ -2118,20 +2073,21 @@ __global__ void __launch_bounds__(Shape<W>::kThreads, Shape<W>::kCtasPerSm) k_fl
       if (tid >= watch || off >= nb) break;
       int gb = cursor + off;
       if (gb >= nb) gb -= nb;
-      BlockDev& B = a.blocks[gb];
       // one round of loads decides whether to look closer: the block's word, target, job, and its
       // row of the neighbour table with the flags (energy kind, free slot)
       int y[28];
       flow_row(a, gb, y);
       const unsigned long long w = ld_relaxed_u64(&a.fstate[gb]);
-      const int64_t t0 = __ldcg(&B.target);
-      const int bj = __ldcg(&B.job);
+      const int64_t t0 = __ldcg(&a.blocks[gb].target);
+      const int bj = __ldcg(&a.blocks[gb].job);
       const int64_t r = static_cast<int64_t>(w >> 1);
-      int32_t P[27];
       bool ok = (y[27] & kNbrKindMask) == KIND && !(w & 1ull) && r < t0;
-      if (ok) {  // a second: the neighbours' rounds
+      int D = 64;  // ready rounds from r on
+      if (ok && !(y[27] & kNbrSolo)) {  // a second: the neighbours' rounds
+        int32_t P[27];
         flow_snapshot(a, gb, y, r, P);
-        ok = flow_ready(P, r, 0, sm0->flow_lag);
+        D = flow_limit(P, r, 64);
+        ok = D > 0;
       }
       // a multi-block job with a hop budget: its round at a time-step boundary waits for the job's
       // other blocks (a job that ends there is taken, to mark it)
@@ -2139,23 +2095,11 @@ __global__ void __launch_bounds__(Shape<W>::kThreads, Shape<W>::kCtasPerSm) k_fl
       // the lease, then one fence: the snapshot's and the word's reads become acquires
       if (ok && atomicCAS(&a.fstate[gb], w, w | 1ull) == w) {
         fence_acq_rel();
-        const JobDev& J = a.jobs[bj];
-        int64_t rn = r, tgt = 0;
-        int keep = 0;
+        int64_t rn = r;
         bool reached = false;
-        unsigned long long vv = 0;
-        if (flow_advance(a, B, J, gb, sm0->flow_lag, r, &P, &rn, &reached, &tgt, &vv)) {
-          const int i = atomicAdd(&sm0->flow_ncand, 1);
-          if (i < kFlowTake) {
-            sm0->flow_cand[i] = gb;
-            sm0->flow_cvv[i] = vv;
-            sm0->flow_cr[i] = rn;
-            sm0->flow_ct[i] = tgt;
-            keep = 1;
-          }
-        }
-        if (rn > r) sm0->flow_progress = 1;
-        flow_publish(a, gb, rn, keep, reached, KIND);
+        const bool keep = flow_advance(a, sm0, gb, bj, r, D, nullptr, take, &rn, &reached);
+        if (rn > r) sm0.flow_progress = 1;
+        flow_publish(a, gb, rn, keep ? 1 : 0, reached, KIND);
         break;
       }
     }
@@ -2166,7 +2110,7 @@ __global__ void __launch_bounds__(Shape<W>::kThreads, Shape<W>::kCtasPerSm) k_fl
         atomicOr(a.status, kErrTimeout);
         stop = 1;
       }
-      sm0->flow_stop = stop;
+      sm0.flow_stop = stop;
     }
     __syncthreads();
 #ifdef AKMC_PHASE_PROFILE
@@ -2180,140 +2124,91 @@ __global__ void __launch_bounds__(Shape<W>::kThreads, Shape<W>::kCtasPerSm) k_fl
 
     // the hop loop for each round handed over; a single-block job's next rounds follow while
     // the launch's target allows (empty ones in between run on thread 0)
-    const int ncand = min(sm0->flow_ncand, kFlowTake);
+    const int ncand = min(sm0.flow_ncand, take);
     for (int c = 0; c < ncand; ++c) {
-      const int gb = sm0->flow_cand[c];
-      // the round and target the sweep left (a chained round: the previous link's)
-      int64_t r = sm0->flow_cr[c], target = sm0->flow_ct[c];
-      for (int link = 0;; ++link) {
+      Round& C = sm0.round[c];
+      while (true) {
 #ifdef AKMC_PHASE_PROFILE
         long long tw = clock64();
 #endif
-        BlockDev& B = a.blocks[gb];
-        const JobDev& J = a.jobs[B.job];
         // the thread that found this round ready read the neighbours' round counters and then
         // fenced (an acquire), and a CTA barrier followed: every thread's reads come after the
         // rounds it waits for (shared data is read at L2)
-        const int sec = sector_of_round(r);
+        load_job(sm0, a, C.job);
+        const int gb = C.gb, sec = sector_of_round(C.r);
         Region R;
-        make_region(B, J, sec, R);
+        make_region(C.c0, C.c1, sm0.job, sec, R);
         Smem* sm;
         uint8_t* occ_s;
         int32_t* rho_s;
         carve(smem, R.n, sm, occ_s, rho_s);
-        if (tid == 0) {
-          sm->fnv = 0;
-#pragma unroll
-          for (int d = 0; d < 3; ++d) {
-            sm->bc0[d] = B.c0[d];
-            sm->bc1[d] = B.c1[d];
+        unsigned long long word = kNoVacancy;  // the block's vacancy slots, read while the region's copies are issued
+        if (tid < kFlowSlots) word = __ldcg(a.vslot + static_cast<int64_t>(gb) * kFlowSlots + tid);
+        stage_region<KIND, W>(*sm, a, R, occ_s, rho_s);
+        if (tid < kFlowSlots && word != kNoVacancy) {
+          const int32_t s = static_cast<int32_t>(word & 0xffffffffu);
+          const int t = s / sm->job.sx, X = s - t * sm->job.sx, z = t / sm->job.sy, y = t - z * sm->job.sy;
+          if (static_cast<unsigned>((X >> 1) - R.slo[0]) < static_cast<unsigned>(R.w[0]) &&
+              static_cast<unsigned>(y - R.slo[1]) < static_cast<unsigned>(R.w[1]) &&
+              static_cast<unsigned>(z - R.slo[2]) < static_cast<unsigned>(R.w[2])) {
+            const int i = atomicAdd(&sm->fnv, 1);
+            sm->fslot[i] = tid;
+            put_record(*sm, R, i, static_cast<int>(word >> 32), s, X, y, z);
           }
-          sm->bnb = J.nblocks;
         }
-        if (R.bulk && tid == kCtl) bulk_expect(&sm->mbar_st, stage_bytes(R, KIND != kPairBond));
-        __syncthreads();  // the previous round's readers are done; the copies' barrier is armed
-        // the region's bulk copies first: the slots, clocks and streams are read while they fly
-        if (R.tma) {
-          if (tid == kCtl) stage_tensor(R, a.tmaps, B.job, KIND != kPairBond, occ_s, rho_s, &sm->mbar_st);
-        } else if (R.bulk) {
-          stage_rows(R, J.occ, J.rho, J.px, J.sy, J.sz, KIND != kPairBond, occ_s, rho_s, &sm->mbar_st, tid, kThreads);
-        }
-        if (tid < kFlowSlots) {
-          // the sweep read the valid bits when it handed the round over; a chained round reads them
-          const unsigned long long m = link == 0 ? sm0->flow_cvv[c] : ld_acquire_u64(&a.vvalid[gb]);
-          if ((m >> tid) & 1ull) {
-            const int v = __ldcg(&a.vslot[static_cast<int64_t>(gb) * kFlowSlots + tid]);
-            const int32_t st = __ldcg(&a.vsite[static_cast<int64_t>(gb) * kFlowSlots + tid]);
-            if (site_in_sector(B, J, sec, st)) {
-              const int i = atomicAdd(&sm->fnv, 1);
-              sm->fv[i] = v;
-              sm->fsite[i] = st;
-              sm->fslot[i] = tid;
-            }
-          }
-        } else if (tid < kFlowSlots + 10) {
-          // the block's hops, the sector's clock and the two streams, one value per thread, while
-          // the control thread issues the copies
-          const int q = tid - kFlowSlots;
-          if (q == 0) sm->hops_out = __ldcg(&B.hops);  // run_block replaces it if the round runs
-          else if (q == 1) sm->pre_evo = __ldcg(&B.evo[sec]);
-          else if (q < 6) sm->str[0][q - 2] = __ldcg(&B.xs[q - 2]);
-          else sm->str[1][q - 6] = __ldcg(&B.xt[q - 6]);
-        }
-        __syncthreads();
-        const int cnt = sm->fnv;
 #ifdef AKMC_PHASE_PROFILE
         if (tid == 0) {
           atomicAdd(a.counters + 12, static_cast<unsigned long long>(clock64() - tw));  // [4] before the hop loop
           tw = clock64();
         }
 #endif
-        const bool ran = run_block<KIND, W, false>(a, gb, *sm, occ_s, rho_s, sm->fv, cnt, r, true);
+        const int cnt = run_block<KIND, W, false>(a, *sm, C, R, occ_s, rho_s, sec);
+        const bool ran = cnt >= 0;
 #ifdef AKMC_PHASE_PROFILE
         if (tid == 0) tw = clock64();
 #endif
-        // the sector's vacancies move: its bit of the block's sector mask goes, and comes back
-        // below for each one still in the block (with the bit of the sector it is in now)
-        if (ran && tid == 0) atomicAnd(&a.vsec[gb], ~(1u << sector_of_round(r)));
-        __syncthreads();
-        // vacancies carried into a neighbour's area change owner (only if the round ran:
-        // otherwise nothing moved and the vacancy arrays of sm hold another round's data)
+        // Vacancies carried into a neighbour's area change owner, the others' sites and sectors are kept up to
+        // date (only if the round ran).  The sector's bit of the block's mask goes first and comes back for
+        // each vacancy still in it.  With one vacancy, thread 0 does it all and publishes the round.
+        if (ran && tid == 0) atomicAnd(&a.vsec[gb], ~(1u << sec));
+        if (ran && cnt > 1) __syncthreads();
         if (ran && tid < cnt) {
-          // a vacancy still inside the block's area keeps its owner and slot (its site updated);
-          // only one that left it needs the owner lookup
           const int4 g = sm->vpk[tid][1];
           const int cx = g.x >> 1, cy = g.y, cz = g.z;
-          const int* c0 = sm->bc0;
-          const int* c1 = sm->bc1;
-          const bool inside = cx >= c0[0] && cx < c1[0] && cy >= c0[1] && cy < c1[1] && cz >= c0[2] && cz < c1[2];
-          const int32_t site = g.w;
+          const bool inside = cx >= C.c0[0] && cx < C.c1[0] && cy >= C.c0[1] && cy < C.c1[1] && cz >= C.c0[2] && cz < C.c1[2];
+          unsigned long long* const own = a.vslot + static_cast<int64_t>(gb) * kFlowSlots + sm->fslot[tid];
           int osec = 0, o = gb;
           if (inside)
-            osec = (cx - c0[0] >= (c1[0] - c0[0]) / 2 ? 1 : 0) | (cy - c0[1] >= (c1[1] - c0[1]) / 2 ? 2 : 0) |
-                   (cz - c0[2] >= (c1[2] - c0[2]) / 2 ? 4 : 0);
+            osec = (cx - C.c0[0] >= (C.c1[0] - C.c0[0]) / 2 ? 1 : 0) | (cy - C.c0[1] >= (C.c1[1] - C.c0[1]) / 2 ? 2 : 0) |
+                   (cz - C.c0[2] >= (C.c1[2] - C.c0[2]) / 2 ? 4 : 0);
           else
-            o = owner_sector(J, site, &osec);
+            o = owner_sector(sm->job, g.w, &osec);
           if (o == gb) {
-            a.vsite[static_cast<int64_t>(gb) * kFlowSlots + sm->fslot[tid]] = site;
+            *reinterpret_cast<volatile unsigned long long*>(own) = slot_word(sm->vidx[tid], g.w);
             atomicOr(&a.vsec[gb], 1u << osec);
           } else {
-            flow_give(a, o, sm->vidx[tid], site, osec);
-            const unsigned long long bit = 1ull << sm->fslot[tid];
-            atomicAnd(&a.vvalid[gb], ~bit);
-            fence_acq_rel();
-            atomicAnd(&a.vclaim[gb], ~bit);
+            flow_give(a, o, sm->vidx[tid], g.w, osec);
+            *reinterpret_cast<volatile unsigned long long*>(own) = kNoVacancy;
           }
         }
-        __syncthreads();
+        if (ran && cnt > 1) __syncthreads();
         if (tid == 0) {
-#ifdef AKMC_FLOW_PROFILE
-          const long long q0 = clock64();
-#endif
-          // round r ran (it was below the target when handed over); the target is the lease
+          // round C.r ran (it was below the target when handed over); the target is the lease
           // holder's to move, and it is this CTA
-          int64_t rn = r + 1, tgt = target;
-          if ((rn & 7) == 0) B.hops_at[(rn >> 3) & 1] = sm->hops_out;
-          bool more = false, reached = rn >= target;
+          int64_t rn = C.r + 1;
+          if ((rn & 7) == 0) a.blocks[gb].hops_at[(rn >> 3) & 1] = C.hops;
+          bool more = false, reached = rn >= C.t;
           const bool in_time =
               a.time_budget_ns <= 0 || globaltimer_ns() - t_begin < static_cast<uint64_t>(a.time_budget_ns);
-          if (!reached && sm->bnb == 1 && c + 1 == ncand && in_time) {
+          if (!reached && sm->job.nblocks == 1 && c + 1 == ncand && in_time) {
             // a single-block job: its next rounds wait for nothing, so keep the lease and run on
             // -- when no other round this CTA took in the sweep is waiting for it
-            more = flow_advance(a, B, J, gb, sm0->flow_lag, r + 1, nullptr, &rn, &reached, &tgt);
+            more = flow_advance(a, *sm, gb, C.job, rn, 64, &C, 0, &rn, &reached);
           }
-#ifdef AKMC_FLOW_PROFILE
-          const long long q1 = clock64();
-#endif
           sm->flow_progress = 1;
           sm->flow_more = more;
-          sm->cur_r = rn;
-          sm->cur_t = tgt;
+          sm->fnv = 0;
           flow_publish(a, gb, rn, more ? 1 : 0, reached, KIND);
-#ifdef AKMC_FLOW_PROFILE
-          atomicAdd(a.counters + 20, static_cast<unsigned long long>(q1 - q0));
-          atomicAdd(a.counters + 21, static_cast<unsigned long long>(clock64() - q1));
-          atomicAdd(a.counters + 23, static_cast<unsigned long long>(q0 - tw));
-#endif
         }
         __syncthreads();
 #ifdef AKMC_PHASE_PROFILE
@@ -2322,20 +2217,18 @@ __global__ void __launch_bounds__(Shape<W>::kThreads, Shape<W>::kCtasPerSm) k_fl
           atomicAdd(a.counters + 15, static_cast<unsigned long long>(clock64() - tw));  // [7] after the hop loop
         }
 #endif
-        if (!sm0->flow_more) break;
-        r = sm0->cur_r;
-        target = sm0->cur_t;
+        if (!sm0.flow_more) break;
       }
     }
 #ifdef AKMC_PHASE_PROFILE
     if (tid == 0) t_hop += clock64() - t0;
 #endif
-    if (AKMC_SWEEP_SLEEP_NS > 0 && !sm0->flow_progress) __nanosleep(AKMC_SWEEP_SLEEP_NS);
+    if (AKMC_SWEEP_SLEEP_NS > 0 && !sm0.flow_progress) __nanosleep(AKMC_SWEEP_SLEEP_NS);
     cursor += kSweepVisits * watch;
     if (cursor >= nb) cursor %= nb;
   }
   cta_flush<W>(a, smem);
-#if defined(AKMC_PHASE_PROFILE) && !defined(AKMC_FLOW_PROFILE) && !defined(AKMC_HOP_PROFILE)
+#ifdef AKMC_PHASE_PROFILE
   if (tid == 0) {  // scheduler profile: [12] sweep cycles, [13] hop-loop cycles, [14] sweeps, [15] full rounds
     atomicAdd(a.counters + 20, static_cast<unsigned long long>(t_sweep));
     atomicAdd(a.counters + 21, static_cast<unsigned long long>(t_hop));
@@ -2352,8 +2245,6 @@ __global__ void k_flow_prep(RoundArgs a) {
   if (gb >= a.nblocks) return;
   BlockDev& B = a.blocks[gb];
   B.cnt = 0;
-  a.vclaim[gb] = 0;
-  a.vvalid[gb] = 0;
   a.vcount[gb] = 0;
   a.vsec[gb] = 0;
   int32_t* row = a.nbr + static_cast<int64_t>(gb) * kNbrStride;
@@ -2366,7 +2257,7 @@ __global__ void k_flow_prep(RoundArgs a) {
   }
   const JobDev& J = a.jobs[B.job];
   for (int o = 0; o < 27; ++o) row[o] = flow_neighbour(J, B.local_id, o);
-  row[27] = job_kind(J) | (J.hop_budget > 0 && J.nblocks > 1 ? kNbrGate : 0);
+  row[27] = job_kind(J) | (J.nblocks == 1 ? kNbrSolo : J.hop_budget > 0 ? kNbrGate : 0);
   // up to flow_rounds of the block's remaining rounds (hop budgets are checked by the kernel,
   // at time-step boundaries); a block sitting at a boundary records its hops there
   int64_t L = B.remaining < a.flow_rounds ? B.remaining : a.flow_rounds;
@@ -2392,10 +2283,7 @@ __global__ void k_flow_slots(RoundArgs a) {
     atomicOr(a.status, kErrVacOverflow);
     return;
   }
-  a.vslot[static_cast<int64_t>(o) * kFlowSlots + slot] = v;
-  a.vsite[static_cast<int64_t>(o) * kFlowSlots + slot] = a.vac_site[v];
-  atomicOr(&a.vclaim[o], 1ull << slot);
-  atomicOr(&a.vvalid[o], 1ull << slot);
+  a.vslot[static_cast<int64_t>(o) * kFlowSlots + slot] = slot_word(v, a.vac_site[v]);
   atomicOr(&a.vsec[o], 1u << osec);
 }
 
@@ -2473,7 +2361,10 @@ __global__ void __launch_bounds__(Shape<8>::kThreads, 1) k_api_block(RoundArgs a
     return;
   }
   init_cta_smem(smem);
-  dispatch_block(a, J.block0, smem);
+  const int kind = job_kind(J);
+  if (kind == kPairBond) listed_block<kPairBond, 8, true>(a, J.block0, a.api_sector, smem);
+  else if (kind == kEam32) listed_block<kEam32, 8, true>(a, J.block0, a.api_sector, smem);
+  else listed_block<kEam64, 8, true>(a, J.block0, a.api_sector, smem);
   cta_flush<8>(a, smem);
 }
 __global__ void k_api_reset(RoundArgs a) {
@@ -2748,6 +2639,7 @@ int launch_flow(const RoundArgs& a, int grid, size_t smem, void* stream, void* e
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   cudaMemsetAsync(a.flow_need, 0, 3 * sizeof(int32_t), st);
   cudaMemsetAsync(a.flow_done, 0, 3 * sizeof(int32_t), st);
+  cudaMemsetAsync(a.vslot, 0xff, static_cast<size_t>(a.nblocks) * kFlowSlots * sizeof(unsigned long long), st);
   k_flow_prep<<<(a.nblocks + 127) / 128, 128, 0, st>>>(a);
   if (a.nvac > 0) k_flow_slots<<<(a.nvac + 127) / 128, 128, 0, st>>>(a);
   if (ev0) cudaEventRecord(static_cast<cudaEvent_t>(ev0), st);
