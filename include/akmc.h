@@ -135,7 +135,7 @@ typedef struct akmc_context_config {
   /* Launch shape of the hop kernels (autotuned by akmc_b200.autotune): eval_warps = warps that
    * evaluate a vacancy's 8 jumps, 8 (one jump each, one CTA per SM; 0 = 8) or 4 (two jumps each,
    * two CTAs per SM); flow_take = rounds with vacancies a CTA of the dependency-driven schedule
-   * takes per sweep (0: all it finds).  Results do not depend on either. */
+   * takes per sweep (0: chosen by the kernel).  Results do not depend on either. */
   int32_t eval_warps;
   int32_t flow_take;
 } akmc_context_config;

@@ -135,7 +135,7 @@ struct akmc_ctx {
   int32_t* d_nbr = nullptr;
   unsigned char* d_tmaps = nullptr;  // per job slot: two 128-byte tensor maps
   unsigned int* d_vsec = nullptr;
-  int32_t* d_flow = nullptr;  // flow_need[3], flow_done[3]
+  int32_t* d_flow = nullptr;  // flow_need[3], flow_done[3], flow_idle
   // cluster statistics scratch: list, parent, size (one int32 per site of the largest job
   // measured so far), then n_list, the isolated count and the histogram
   int32_t* d_cl = nullptr;
@@ -899,7 +899,7 @@ AKMC_API akmc_status akmc_prepare(akmc_ctx* ctx) {
     CK(cudaMemcpyAsync(ctx->d_tmaps, tm.data(), tm.size(), cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));  // tm leaves scope
   }
-  CK(dalloc(ctx->stream, &ctx->d_flow, 6));
+  CK(dalloc(ctx->stream, &ctx->d_flow, 7));
   CK(dalloc(ctx->stream, &ctx->d_log_count, 1));
   CK(dalloc(ctx->stream, &ctx->d_api_total, 1));
   CK(dalloc(ctx->stream, &ctx->d_api_event, 1));
@@ -967,6 +967,7 @@ AKMC_API akmc_status akmc_prepare(akmc_ctx* ctx) {
   a.tmaps = ctx->d_tmaps;
   a.flow_need = ctx->d_flow;
   a.flow_done = ctx->d_flow + 3;
+  a.flow_idle = ctx->d_flow + 6;
   a.flow_take = ctx->cfg.flow_take;
   a.eval_warps = ctx->cfg.eval_warps;
   refresh_job_set(ctx);

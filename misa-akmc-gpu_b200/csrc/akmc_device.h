@@ -192,6 +192,7 @@ struct RoundArgs {
                                 // o = (dz+1)*9 + (dy+1)*3 + dx+1) and a flags word (k_flow_prep)
   int32_t* flow_need;           // per energy kind: blocks with rounds to run in this launch
   int32_t* flow_done;           // per energy kind: blocks that reached their target
+  int32_t* flow_idle;           // CTAs of the launch whose last sweep found no round to run
   int64_t flow_rounds;          // rounds this launch adds to every unfinished block
   int64_t flow_sweep_limit;     // sweeps per CTA before the launch gives up (kErrTimeout)
   int64_t time_budget_ns;       // > 0: the launch takes no new round after this long (akmc_run_for)

@@ -1937,6 +1937,7 @@ __device__ __forceinline__ bool flow_advance(const RoundArgs& a, Smem& sm, int g
     st[k] = __ldcg(reinterpret_cast<const ulonglong2*>(B.xs) + k);
   }
   const unsigned occ_sec = __ldcg(&a.vsec[gb]);
+  const int nidle = __ldcg(a.flow_idle);
   const int nbl = J.nblocks;
   const int64_t budget = J.hop_budget;
   const double window = J.window;
@@ -1998,8 +1999,18 @@ __device__ __forceinline__ bool flow_advance(const RoundArgs& a, Smem& sm, int g
   *reached = r == target;  // the lease holder alone moves the target
   if (!full) return false;
   if (!C) {
+    // Rounds a CTA takes per sweep: `take` when the context sets it.  Else every one its threads find while nearly
+    // all CTAs have rounds to run (512 boxes: 22.5 ms for 256 rounds; 25.0 with two, 28.2 with one), but two
+    // while more than 1 in 8 found none in their last sweep (1024 rounds of the 256^3 lattice: 28.1 against 29.7
+    // ms with all) and one while more than half did (64 boxes: 12.7 against 14.1 ms): an idle CTA runs a round
+    // sooner than this one, which runs its own one after another.
+    const int ctas = static_cast<int>(gridDim.x);
+    const int most = a.flow_take > 0 || nidle * 8 <= ctas ? take : nidle * 2 > ctas ? 1 : 2;
     const int i = atomicAdd(&sm.flow_ncand, 1);
-    if (i >= take) return false;
+    if (i >= most) {
+      if (i < take) sm.round[i].gb = -1;  // an entry left out
+      return false;
+    }
     C = &sm.round[i];
   }
   C->r = r;
@@ -2023,15 +2034,11 @@ __device__ __forceinline__ bool flow_advance(const RoundArgs& a, Smem& sm, int g
   return true;
 }
 
-// Rounds with vacancies a CTA takes per sweep: a.flow_take (0: every ready round its threads
-// found).  Measured on the 256^3 lattice and the 512 batched boxes: taking every ready round
-// found, one round per block at a time, beats taking one per sweep (others left to idle CTAs)
-// and beats chaining up to 8 rounds of one block of a multi-block job.  Single-block jobs chain:
-// their next round waits for nothing.
 template <int KIND, int W>
 __global__ void __launch_bounds__(Shape<W>::kThreads, Shape<W>::kCtasPerSm) k_flow(RoundArgs a) {
   AKMC_SHAPE(W);
-  const int take = a.flow_take > 0 && a.flow_take < kMaxTake ? a.flow_take : kMaxTake;
+  const int take = a.flow_take > 0 ? min(a.flow_take, kMaxTake) : kMaxTake;
+  bool idle = false;  // thread 0: the CTA is counted in flow_idle
   extern __shared__ __align__(16) uint8_t smem[];
   Smem& sm0 = *reinterpret_cast<Smem*>(smem);
   const int tid = threadIdx.x;
@@ -2099,7 +2106,8 @@ __global__ void __launch_bounds__(Shape<W>::kThreads, Shape<W>::kCtasPerSm) k_fl
         bool reached = false;
         const bool keep = flow_advance(a, sm0, gb, bj, r, D, nullptr, take, &rn, &reached);
         if (rn > r) sm0.flow_progress = 1;
-        flow_publish(a, gb, rn, keep ? 1 : 0, reached, KIND);
+        // a round handed over with none run before it: the word holds it and the lease already
+        if (!keep || rn > r) flow_publish(a, gb, rn, keep ? 1 : 0, reached, KIND);
         break;
       }
     }
@@ -2125,9 +2133,13 @@ __global__ void __launch_bounds__(Shape<W>::kThreads, Shape<W>::kCtasPerSm) k_fl
     // the hop loop for each round handed over; a single-block job's next rounds follow while
     // the launch's target allows (empty ones in between run on thread 0)
     const int ncand = min(sm0.flow_ncand, take);
+    if (tid == 0 && (ncand == 0) != idle) {
+      idle = ncand == 0;
+      atomicAdd(a.flow_idle, idle ? 1 : -1);
+    }
     for (int c = 0; c < ncand; ++c) {
       Round& C = sm0.round[c];
-      while (true) {
+      while (C.gb >= 0) {
 #ifdef AKMC_PHASE_PROFILE
         long long tw = clock64();
 #endif
@@ -2637,8 +2649,7 @@ int launch_flow_begin(const RoundArgs& a, int64_t n, void* stream) {
 
 int launch_flow(const RoundArgs& a, int grid, size_t smem, void* stream, void* ev0, void* ev1) {
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  cudaMemsetAsync(a.flow_need, 0, 3 * sizeof(int32_t), st);
-  cudaMemsetAsync(a.flow_done, 0, 3 * sizeof(int32_t), st);
+  cudaMemsetAsync(a.flow_need, 0, 7 * sizeof(int32_t), st);  // and flow_done, flow_idle behind it
   cudaMemsetAsync(a.vslot, 0xff, static_cast<size_t>(a.nblocks) * kFlowSlots * sizeof(unsigned long long), st);
   k_flow_prep<<<(a.nblocks + 127) / 128, 128, 0, st>>>(a);
   if (a.nvac > 0) k_flow_slots<<<(a.nvac + 127) / 128, 128, 0, st>>>(a);
