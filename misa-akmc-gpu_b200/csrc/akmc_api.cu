@@ -143,6 +143,8 @@ struct akmc_ctx {
   unsigned long long* d_cl_misc = nullptr;
   // whole-context lattice transfers: staging buffer, chunk table, per-job vacancy counts,
   // density tiles of the EAM jobs (built at the first transfer)
+  uint8_t* d_stage1 = nullptr;  // one lattice on its way into its device rows (load_lattice)
+  int64_t stage1_sites = 0;
   uint8_t* d_stage = nullptr;
   SiteChunk* d_chunks = nullptr;
   int32_t* d_job_counts = nullptr;
@@ -190,6 +192,28 @@ void dfree(cudaStream_t s, void* p) {
   if (p) cudaFreeAsync(p, s);
 }
 
+// A job's lattice into its device rows: one plain copy into a staging buffer of the context (kept, and grown when
+// a larger lattice comes), then a kernel that lays the rows out with their halos.  With collect it also fills the
+// job's slice of the vacancy table (akmc_load_occupancy).  A strided copy straight into the rows measured 1.8 ms
+// for 131 x 117 rows of 300 sites, this 0.1 ms.
+akmc_status load_lattice(akmc_ctx* ctx, int32_t job, uint8_t* d_occ, const uint8_t* occ, bool collect) {
+  const HostJob& j = ctx->jobs[static_cast<size_t>(job)];
+  if (ctx->stage1_sites < j.nsites) {
+    dfree(ctx->stream, ctx->d_stage1);
+    ctx->d_stage1 = nullptr;
+    ctx->stage1_sites = 0;
+    CK(dalloc(ctx->stream, &ctx->d_stage1, static_cast<size_t>(j.nsites)));
+    ctx->stage1_sites = j.nsites;
+  }
+  CK(cudaMemcpyAsync(ctx->d_stage1, occ, static_cast<size_t>(j.nsites), cudaMemcpyHostToDevice, ctx->stream));
+  const int e = launch_load_lattice(ctx->d_stage1, d_occ, 2 * static_cast<int32_t>(j.cfg.box[0]),
+                                    j.cfg.box[1] * j.cfg.box[2], collect ? ctx->d_vac_site + j.vac0 : nullptr,
+                                    collect ? ctx->d_vac_job + j.vac0 : nullptr, job, static_cast<int32_t>(j.nvac),
+                                    ctx->d_vac_count, ctx->d_status, ctx->stream);
+  if (e) return fail(ctx, AKMC_ECUDA, std::string("load lattice: ") + cuda_name(e));
+  return AKMC_OK;
+}
+
 akmc_status check_status(akmc_ctx* ctx) {
   unsigned int st = 0;
   CK(cudaMemcpyAsync(&st, ctx->d_status, sizeof(st), cudaMemcpyDeviceToHost, ctx->stream));
@@ -220,6 +244,9 @@ void free_device(akmc_ctx* ctx) {
   ctx->d_vsec = nullptr;
   dfree(ctx->stream, ctx->d_tmaps);
   ctx->d_tmaps = nullptr;
+  dfree(ctx->stream, ctx->d_stage1);
+  ctx->d_stage1 = nullptr;
+  ctx->stage1_sites = 0;
   dfree(ctx->stream, ctx->d_cl);
   dfree(ctx->stream, ctx->d_cl_misc);
   ctx->d_cl = nullptr;
@@ -305,16 +332,7 @@ void job_box(const HostJob& j, int32_t box[3]) {
 // of a multiple of 16 sites (lattice_pitch), so a region's rows start on 16-byte boundaries.
 bool bulk_rows(const HostJob&) { return true; }
 
-// Plain copies between a job's host lattice (rows of sx entries) and the main part of its device
-// rows (pitch px, after the kHaloL halo entries); a host-to-device copy refreshes the halos.
-template <typename T>
-cudaError_t lattice_upload(T* dev, const T* host, int64_t sx, int64_t nrows, cudaStream_t st) {
-  const int64_t px = lattice_pitch(static_cast<int32_t>(sx));
-  cudaError_t e = cudaMemcpy2DAsync(dev + kHaloL, static_cast<size_t>(px) * sizeof(T), host, static_cast<size_t>(sx) * sizeof(T),
-                                    static_cast<size_t>(sx) * sizeof(T), static_cast<size_t>(nrows), cudaMemcpyHostToDevice, st);
-  if (e != cudaSuccess) return e;
-  return static_cast<cudaError_t>(launch_fill_halo(dev, static_cast<int32_t>(sx), nrows, st));
-}
+// Plain copy of a job's lattice from the main part of its device rows (pitch px, after the kHaloL halo entries).
 template <typename T>
 cudaError_t lattice_download(T* host, const T* dev, int64_t sx, int64_t nrows, cudaStream_t st) {
   const int64_t px = lattice_pitch(static_cast<int32_t>(sx));
@@ -592,11 +610,13 @@ akmc_status upload_pot(akmc_ctx* ctx, size_t i, Potential& hp) {
 akmc_status setup_job(akmc_ctx* ctx, int32_t ji, JobDev& J, BlockDev* hb, int32_t* vsite, int32_t* vjob) {
   HostJob& j = ctx->jobs[static_cast<size_t>(ji)];
   const int32_t sx = 2 * static_cast<int32_t>(j.cfg.box[0]);
-  const int64_t nrows = j.cfg.box[1] * j.cfg.box[2];
   const size_t entries = static_cast<size_t>(lattice_entries(sx, static_cast<int32_t>(j.cfg.box[1]),
                                                              static_cast<int32_t>(j.cfg.box[2])));
   CK(dalloc(ctx->stream, &j.d_occ, entries));
-  CK(lattice_upload(j.d_occ, j.occ.data(), sx, nrows, ctx->stream));
+  {
+    const akmc_status st = load_lattice(ctx, ji, j.d_occ, j.occ.data(), false);
+    if (st != AKMC_OK) return st;
+  }
   if (j.has_eam) CK(dalloc(ctx->stream, &j.d_rho, entries));
   std::memset(&J, 0, sizeof(J));
   J.occ = j.d_occ;
@@ -925,6 +945,7 @@ AKMC_API akmc_status akmc_prepare(akmc_ctx* ctx) {
       RoundArgs ra{};
       ra.jobs = ctx->d_jobs;
       ra.pots = ctx->d_pots;
+      ra.geo = ctx->d_geo;
       const int e = launch_init_rho_jobs(ra, ctx->jl, ctx->stream);
       if (e) return fail(ctx, AKMC_ECUDA, std::string("init rho: ") + cuda_name(e));
     }
@@ -1088,13 +1109,10 @@ AKMC_API akmc_status akmc_load_occupancy(akmc_ctx* ctx, int32_t job, const uint8
   HostJob& j = ctx->jobs[static_cast<size_t>(job)];
   if (n_sites != j.nsites) return fail(ctx, AKMC_EINVAL, "n_sites does not match the job");
   CK(cudaSetDevice(ctx->cfg.device));
-  const int32_t sx = 2 * static_cast<int32_t>(j.cfg.box[0]);
-  CK(lattice_upload(j.d_occ, occ, sx, j.cfg.box[1] * j.cfg.box[2], ctx->stream));
-  int e = launch_collect_vacancies(j.d_occ, n_sites, sx, ctx->d_vac_site + j.vac0, ctx->d_vac_job + j.vac0, job,
-                                   static_cast<int32_t>(j.nvac), ctx->d_vac_count, ctx->d_status, ctx->stream);
-  if (e) return fail(ctx, AKMC_ECUDA, std::string("collect vacancies: ") + cuda_name(e));
+  const akmc_status ls = load_lattice(ctx, job, j.d_occ, occ, true);
+  if (ls != AKMC_OK) return ls;
   if (j.has_eam) {
-    e = launch_init_rho(j.d_occ, j.d_rho, 2 * static_cast<int32_t>(j.cfg.box[0]), static_cast<int32_t>(j.cfg.box[1]),
+    const int e = launch_init_rho(j.d_occ, j.d_rho, 2 * static_cast<int32_t>(j.cfg.box[0]), static_cast<int32_t>(j.cfg.box[1]),
                         static_cast<int32_t>(j.cfg.box[2]), ctx->d_pots + j.pot, ctx->d_geo, ctx->d_status,
                         ctx->stream);
     if (e) return fail(ctx, AKMC_ECUDA, std::string("init rho: ") + cuda_name(e));
@@ -1235,7 +1253,7 @@ static akmc_status build_rho_tables(akmc_ctx* ctx) {
     if (!j.has_eam || !j.live) continue;
     const int64_t sx = 2 * j.cfg.box[0], sy = j.cfg.box[1], sz = j.cfg.box[2];
     eam_jobs.push_back(static_cast<int32_t>(k));
-    tile0.push_back(tile0.back() + ((sx + 31) / 32) * ((sy + 7) / 8) * ((sz + 3) / 4));
+    tile0.push_back(tile0.back() + rho_tiles(sx, sy, sz));
   }
   CK(dalloc(ctx->stream, &ctx->d_tile0, tile0.size()));
   CK(dalloc(ctx->stream, &ctx->d_eam_jobs, std::max<size_t>(1, eam_jobs.size())));
@@ -1254,7 +1272,7 @@ static akmc_status setup_jobs_load(akmc_ctx* ctx) {
   if (ctx->d_stage) return AKMC_OK;
   const akmc_status rt = build_rho_tables(ctx);
   if (rt != AKMC_OK) return rt;
-  constexpr int64_t kChunk = 1 << 16;
+  constexpr int64_t kChunk = 1 << 14;  // sites, in whole rows
   std::vector<SiteChunk> ch;
   std::vector<int32_t> want;
   int64_t off = 0;
@@ -1264,14 +1282,15 @@ static akmc_status setup_jobs_load(akmc_ctx* ctx) {
       want.push_back(0);
       continue;
     }
-    for (int64_t s0 = 0; s0 < j.nsites; s0 += kChunk) {
+    const int64_t sx = 2 * j.cfg.box[0], rows = j.cfg.box[1] * j.cfg.box[2], per = std::max<int64_t>(1, kChunk / sx);
+    for (int64_t r0 = 0; r0 < rows; r0 += per) {
       SiteChunk c{};
       c.job = static_cast<int32_t>(k);
       c.vac0 = j.vac0;
       c.nvac = static_cast<int32_t>(j.nvac);
-      c.site0 = s0;
-      c.n = std::min(kChunk, j.nsites - s0);
-      c.stage0 = off + s0;
+      c.row0 = static_cast<int32_t>(r0);
+      c.nrows = static_cast<int32_t>(std::min(per, rows - r0));
+      c.stage0 = off + r0 * sx;
       ch.push_back(c);
     }
     off += j.nsites;

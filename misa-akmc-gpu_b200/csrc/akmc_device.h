@@ -215,13 +215,11 @@ int configure_hop_smem(size_t smem);
 int hop_ctas_per_sm(int eval_warps);  // CTAs of the hop kernels the register budget allows per SM
 // ev0/ev1 (cudaEvent_t or null) are recorded around the hop kernel.
 int launch_round(const RoundArgs& a, int hop_grid, size_t smem, void* stream, void* ev0, void* ev1);
-// Collects the vacancies of one job's lattice into its slice of the vacancy table and sets
-// kErrVacCount in *status unless exactly cap were found.
-int launch_collect_vacancies(const uint8_t* occ, int64_t n, int32_t sx, int32_t* vac_site, int32_t* vac_job,
-                             int32_t job, int32_t cap, int32_t* count, unsigned int* status, void* stream);
-// Refreshes the halo entries of every row of a lattice (halo layout, rows of sx sites).
-int launch_fill_halo(uint8_t* lat, int32_t sx, int64_t nrows, void* stream);
-int launch_fill_halo(int32_t* lat, int32_t sx, int64_t nrows, void* stream);
+// A lattice of nrows rows of sx sites from a staging buffer (rows back to back, on an even address) into its
+// device rows with their halos.  With vac_site, its vacancies go to the job's slice of the vacancy table, and
+// kErrVacCount is set in *status unless exactly cap were found.
+int launch_load_lattice(const uint8_t* stage, uint8_t* occ, int32_t sx, int64_t nrows, int32_t* vac_site, int32_t* vac_job,
+                        int32_t job, int32_t cap, int32_t* count, unsigned int* status, void* stream);
 int launch_api(const RoundArgs& a, size_t smem, void* stream);
 int launch_init_rho(uint8_t* occ, int32_t* rho, int32_t sx, int32_t sy, int32_t sz, const Potential* pot,
                     const Geometry* geo, unsigned int* status, void* stream);
@@ -232,11 +230,18 @@ int launch_flow(const RoundArgs& a, int grid, size_t smem, void* stream, void* e
 // Sets every block's remaining rounds to n before the launches of one akmc_run_rounds call.
 int launch_flow_begin(const RoundArgs& a, int64_t n, void* stream);
 
+// Tiles of the density build (one CTA takes one at a time).
+constexpr int kRhoTX = 64, kRhoTY = 16, kRhoTZ = 8;
+AK_HD int64_t rho_tiles(int64_t sx, int64_t sy, int64_t sz) {
+  return ((sx + kRhoTX - 1) / kRhoTX) * ((sy + kRhoTY - 1) / kRhoTY) * ((sz + kRhoTZ - 1) / kRhoTZ);
+}
+
 // Whole-context lattice transfers (akmc_load_occupancies / akmc_get_occupancies): the lattices
-// of all jobs back to back in a staging buffer, cut into chunks of one job each.
+// of all jobs back to back in a staging buffer, cut into chunks of whole rows of one job each.
 struct SiteChunk {
-  int32_t job, vac0, nvac, pad;
-  int64_t site0, n, stage0;  // first site in the job, sites, offset in the staging buffer
+  int32_t job, vac0, nvac;
+  int32_t row0, nrows, pad;  // rows of the job
+  int64_t stage0;            // offset in the staging buffer
 };
 struct JobsLoad {
   const uint8_t* stage_in;  // unused by the kernels (host side)
