@@ -111,12 +111,8 @@ struct akmc_ctx {
   unsigned long long* d_log_count = nullptr;
   unsigned int* d_status = nullptr;
   unsigned long long* d_counters = nullptr;
-  double* d_api_total = nullptr;
-  akmc_event* d_api_event = nullptr;
-  double* d_api_de = nullptr;
-  double* d_api_rates = nullptr;
-  int32_t* d_api_sites = nullptr;
-  int32_t* d_api_count = nullptr;
+  ApiOut* api = nullptr;  // answers of the per-hop entry points (host memory; from the first such call on)
+  bool settled = false;   // the last such call waited for the stream, and nothing was put on it since
   size_t smem = 0;
   int hop_grid = 0;
   int grid_sms = 0, grid_fit = 1, grid_resident = 1;  // SMs, CTAs per SM by shared memory / by registers
@@ -278,8 +274,7 @@ void free_device(akmc_ctx* ctx) {
   }
   void* ptrs[] = {ctx->d_jobs, ctx->d_blocks, ctx->d_vac_site, ctx->d_vac_job, ctx->d_blk_list, ctx->d_active,
                   ctx->d_n_active, ctx->d_pots, ctx->d_geo, ctx->d_log, ctx->d_log_count, ctx->d_status,
-                  ctx->d_counters, ctx->d_api_total, ctx->d_api_event, ctx->d_api_de, ctx->d_api_rates,
-                  ctx->d_api_sites, ctx->d_api_count};
+                  ctx->d_counters};
   for (void* p : ptrs) dfree(ctx->stream, p);
   ctx->d_jobs = nullptr;
   ctx->d_blocks = nullptr;
@@ -290,10 +285,8 @@ void free_device(akmc_ctx* ctx) {
   ctx->d_log_count = nullptr;
   ctx->d_status = nullptr;
   ctx->d_counters = nullptr;
-  ctx->d_api_total = nullptr;
-  ctx->d_api_event = nullptr;
-  ctx->d_api_de = ctx->d_api_rates = nullptr;
-  ctx->d_api_sites = ctx->d_api_count = nullptr;
+  if (ctx->api) cudaFreeHost(ctx->api);
+  ctx->api = nullptr;
   ctx->prepared = false;
 }
 
@@ -921,13 +914,6 @@ AKMC_API akmc_status akmc_prepare(akmc_ctx* ctx) {
   }
   CK(dalloc(ctx->stream, &ctx->d_flow, 7));
   CK(dalloc(ctx->stream, &ctx->d_log_count, 1));
-  CK(dalloc(ctx->stream, &ctx->d_api_total, 1));
-  CK(dalloc(ctx->stream, &ctx->d_api_event, 1));
-  CK(dalloc(ctx->stream, &ctx->d_api_de, static_cast<size_t>(kMaxV) * 8));
-  CK(dalloc(ctx->stream, &ctx->d_api_rates, static_cast<size_t>(kMaxV) * 8));
-  CK(dalloc(ctx->stream, &ctx->d_api_sites, static_cast<size_t>(kMaxV)));
-  CK(dalloc(ctx->stream, &ctx->d_api_count, 1));
-  CK(cudaMemsetAsync(ctx->d_api_count, 0, sizeof(int32_t), ctx->stream));
   if (ctx->cfg.event_log_capacity > 0) CK(dalloc(ctx->stream, &ctx->d_log, static_cast<size_t>(ctx->cfg.event_log_capacity)));
   CK(cudaMemcpyAsync(ctx->d_jobs, hj.data(), hj.size() * sizeof(JobDev), cudaMemcpyHostToDevice, ctx->stream));
   CK(cudaMemcpyAsync(ctx->d_blocks, hb.data(), hb.size() * sizeof(BlockDev), cudaMemcpyHostToDevice, ctx->stream));
@@ -974,12 +960,6 @@ AKMC_API akmc_status akmc_prepare(akmc_ctx* ctx) {
   a.flow_sweep_limit = ctx->cfg.flow_sweep_limit;
   a.api_job = -1;
   a.api_sector = -1;
-  a.api_total = ctx->d_api_total;
-  a.api_event = ctx->d_api_event;
-  a.api_de = ctx->d_api_de;
-  a.api_rates = ctx->d_api_rates;
-  a.api_sites = ctx->d_api_sites;
-  a.api_count = ctx->d_api_count;
   a.fstate = ctx->d_fstate;
   a.vslot = ctx->d_vslot;
   a.vcount = ctx->d_vcount;
@@ -1002,6 +982,7 @@ AKMC_API akmc_status akmc_prepare(akmc_ctx* ctx) {
 AKMC_API akmc_status akmc_admit_job(akmc_ctx* ctx, const akmc_job_config* cfg, const uint8_t* occ, int64_t n_sites,
                                     int32_t* job_id) {
   if (!ctx || !cfg || !occ) return AKMC_EINVAL;
+  ctx->settled = false;
   if (!ctx->prepared) return fail(ctx, AKMC_ESTATE, "akmc_admit_job needs a prepared context (akmc_add_job before it)");
   if (ctx->max_edge <= 0) return fail(ctx, AKMC_ESTATE, "the context was created without room for admitted jobs (max_jobs)");
   CK(cudaSetDevice(ctx->cfg.device));
@@ -1074,6 +1055,7 @@ AKMC_API akmc_status akmc_admit_job(akmc_ctx* ctx, const akmc_job_config* cfg, c
 
 AKMC_API akmc_status akmc_retire_job(akmc_ctx* ctx, int32_t job) {
   if (!ctx) return AKMC_EINVAL;
+  ctx->settled = false;
   if (!ctx->prepared) return fail(ctx, AKMC_ESTATE, "akmc_prepare first");
   if (job < 0 || job >= static_cast<int32_t>(ctx->jobs.size()) || !ctx->jobs[static_cast<size_t>(job)].live)
     return AKMC_ENOTFOUND;
@@ -1104,6 +1086,7 @@ AKMC_API akmc_status akmc_retire_job(akmc_ctx* ctx, int32_t job) {
 
 AKMC_API akmc_status akmc_load_occupancy(akmc_ctx* ctx, int32_t job, const uint8_t* occ, int64_t n_sites) {
   if (!ctx || !occ) return AKMC_EINVAL;
+  ctx->settled = false;
   if (!ctx->prepared) return fail(ctx, AKMC_ESTATE, "akmc_prepare first");
   if (!live_job(ctx, job)) return AKMC_ENOTFOUND;
   HostJob& j = ctx->jobs[static_cast<size_t>(job)];
@@ -1193,6 +1176,7 @@ AKMC_API akmc_status akmc_save_snapshot(akmc_ctx* ctx, int32_t job, uint8_t* buf
 
 AKMC_API akmc_status akmc_restore_snapshot(akmc_ctx* ctx, int32_t job, const uint8_t* buf, int64_t n) {
   if (!ctx || !buf) return AKMC_EINVAL;
+  ctx->settled = false;
   if (!ctx->prepared) return fail(ctx, AKMC_ESTATE, "akmc_prepare first");
   if (!live_job(ctx, job)) return AKMC_ENOTFOUND;
   const HostJob& j = ctx->jobs[static_cast<size_t>(job)];
@@ -1316,6 +1300,7 @@ static akmc_status setup_jobs_load(akmc_ctx* ctx) {
 
 AKMC_API akmc_status akmc_load_occupancies(akmc_ctx* ctx, const uint8_t* occ, int64_t total_sites) {
   if (!ctx || !occ) return AKMC_EINVAL;
+  ctx->settled = false;
   if (!ctx->prepared) return fail(ctx, AKMC_ESTATE, "akmc_prepare first");
   CK(cudaSetDevice(ctx->cfg.device));
   const akmc_status st = setup_jobs_load(ctx);
@@ -1333,6 +1318,7 @@ AKMC_API akmc_status akmc_load_occupancies(akmc_ctx* ctx, const uint8_t* occ, in
 
 AKMC_API akmc_status akmc_get_occupancies(akmc_ctx* ctx, uint8_t* out, int64_t total_sites) {
   if (!ctx || !out) return AKMC_EINVAL;
+  ctx->settled = false;
   if (!ctx->prepared) return fail(ctx, AKMC_ESTATE, "akmc_prepare first");
   CK(cudaSetDevice(ctx->cfg.device));
   const akmc_status st = setup_jobs_load(ctx);
@@ -1362,6 +1348,7 @@ AKMC_API akmc_status akmc_get_kernel_timing(akmc_ctx* ctx, double* hop_kernel_ms
 
 AKMC_API akmc_status akmc_run_rounds(akmc_ctx* ctx, int64_t n_rounds) {
   if (!ctx) return AKMC_EINVAL;
+  ctx->settled = false;
   if (!ctx->prepared) return fail(ctx, AKMC_ESTATE, "akmc_prepare first");
   if (n_rounds <= 0) return AKMC_OK;
   CK(cudaSetDevice(ctx->cfg.device));
@@ -1461,6 +1448,7 @@ AKMC_API akmc_status akmc_run_rounds(akmc_ctx* ctx, int64_t n_rounds) {
 
 AKMC_API akmc_status akmc_run_for(akmc_ctx* ctx, int64_t n_rounds, int64_t max_us) {
   if (!ctx) return AKMC_EINVAL;
+  ctx->settled = false;
   if (!ctx->prepared) return fail(ctx, AKMC_ESTATE, "akmc_prepare first");
   if (n_rounds <= 0) return AKMC_OK;
   if (max_us <= 0) return fail(ctx, AKMC_EINVAL, "max_us must be > 0");
@@ -1486,6 +1474,7 @@ int32_t* g_noalloc_base[kNoAllocDevices] = {};
 
 AKMC_API akmc_status akmc_run_rounds_noalloc(akmc_ctx* ctx, int64_t n_rounds) {
   if (!ctx) return AKMC_EINVAL;
+  ctx->settled = false;
   if (!ctx->prepared) return fail(ctx, AKMC_ESTATE, "akmc_prepare first");
   if (ctx->nblocks > kNoAllocMaxBlocks)
     return fail(ctx, AKMC_EINVAL, "akmc_run_rounds_noalloc: " + std::to_string(ctx->nblocks) +
@@ -1696,30 +1685,41 @@ AKMC_API akmc_status akmc_get_counters(akmc_ctx* ctx, int64_t* out8) {
   return AKMC_OK;
 }
 
+// One per-hop step: one launch and one wait; the answer is in ctx->api.
 static akmc_status api_step(akmc_ctx* ctx, int32_t job, int32_t sector_id, int32_t mode, double u) {
+  ctx->settled = false;
   if (!ctx->prepared) return fail(ctx, AKMC_ESTATE, "akmc_prepare first");
   if (!live_job(ctx, job)) return AKMC_ENOTFOUND;
-  if (ctx->jobs[static_cast<size_t>(job)].nblocks != 1)
-    return fail(ctx, AKMC_EINVAL, "the per-hop entry points drive single-domain jobs");
+  const HostJob& j = ctx->jobs[static_cast<size_t>(job)];
+  if (j.nblocks != 1) return fail(ctx, AKMC_EINVAL, "the per-hop entry points drive single-domain jobs");
   if (sector_id < 0 || sector_id > 7) return fail(ctx, AKMC_EINVAL, "sector id in [0, 7]");
   CK(cudaSetDevice(ctx->cfg.device));
+  if (!ctx->api) {
+    CK(cudaHostAlloc(reinterpret_cast<void**>(&ctx->api), sizeof(ApiOut), cudaHostAllocMapped));
+    std::memset(ctx->api, 0, sizeof(ApiOut));
+  }
   RoundArgs a = ctx->args;
   a.mode = mode;
   a.api_job = job;
   a.api_sector = sector_id;
+  a.api_vac0 = j.vac0;
+  a.api_nvac = static_cast<int32_t>(j.nvac);
   a.api_u = u;
+  CK(cudaHostGetDevicePointer(reinterpret_cast<void**>(&a.api), ctx->api, 0));
   a.log_cap = 0;
-  const int e = launch_api(a, ctx->smem, ctx->stream);
+  const int kind = j.cfg.energy_model == AKMC_MODEL_PAIRBOND ? 0 : j.cfg.precision == AKMC_FP32C ? 2 : 1;
+  const int e = launch_api(a, kind, ctx->smem, ctx->stream);
   if (e) return fail(ctx, AKMC_ECUDA, std::string("launch: ") + cuda_name(e));
-  return AKMC_OK;
+  CK(cudaStreamSynchronize(ctx->stream));
+  ctx->settled = true;
+  return ctx->api->status ? check_status(ctx) : AKMC_OK;  // errors of the step and of earlier asynchronous calls
 }
 
 AKMC_API akmc_status akmc_calculate(akmc_ctx* ctx, int32_t job, int32_t sector_id, double* total) {
   if (!ctx || !total) return AKMC_EINVAL;
-  akmc_status s = api_step(ctx, job, sector_id, kModeCalc, 0.0);
-  if (s) return s;
-  CK(cudaMemcpyAsync(total, ctx->d_api_total, sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
-  return akmc_sync(ctx);
+  const akmc_status s = api_step(ctx, job, sector_id, kModeCalc, 0.0);
+  if (ctx->settled) *total = ctx->api->total;
+  return s;
 }
 
 AKMC_API akmc_status akmc_get_calculated_rates(akmc_ctx* ctx, int32_t* sites, double* delta_e, double* rates,
@@ -1728,25 +1728,23 @@ AKMC_API akmc_status akmc_get_calculated_rates(akmc_ctx* ctx, int32_t* sites, do
   *n_out = 0;
   if (!ctx->prepared) return fail(ctx, AKMC_ESTATE, "akmc_prepare first");
   CK(cudaSetDevice(ctx->cfg.device));
-  int32_t n = 0;
-  CK(cudaMemcpyAsync(&n, ctx->d_api_count, sizeof(int32_t), cudaMemcpyDeviceToHost, ctx->stream));
-  CK(cudaStreamSynchronize(ctx->stream));
+  const ApiOut* o = ctx->api;
+  const int32_t n = o ? o->count : 0;
   *n_out = n;
   if (n > capacity) return fail(ctx, AKMC_EINVAL, "capacity below the sector's vacancy count");
   if (n == 0) return AKMC_OK;
-  CK(cudaMemcpyAsync(sites, ctx->d_api_sites, sizeof(int32_t) * n, cudaMemcpyDeviceToHost, ctx->stream));
-  CK(cudaMemcpyAsync(delta_e, ctx->d_api_de, sizeof(double) * 8 * n, cudaMemcpyDeviceToHost, ctx->stream));
-  CK(cudaMemcpyAsync(rates, ctx->d_api_rates, sizeof(double) * 8 * n, cudaMemcpyDeviceToHost, ctx->stream));
-  return akmc_sync(ctx);
+  std::memcpy(sites, o->sites, sizeof(int32_t) * static_cast<size_t>(n));
+  std::memcpy(delta_e, o->de, sizeof(double) * 8 * static_cast<size_t>(n));
+  std::memcpy(rates, o->rates, sizeof(double) * 8 * static_cast<size_t>(n));
+  return ctx->settled ? AKMC_OK : akmc_sync(ctx);  // errors of calls since the last per-hop one
 }
 
 AKMC_API akmc_status akmc_select_and_perform(akmc_ctx* ctx, int32_t job, int32_t sector_id, double u,
                                              akmc_event* ev) {
   if (!ctx || !ev) return AKMC_EINVAL;
-  akmc_status s = api_step(ctx, job, sector_id, kModeSelectPerform, u);
-  if (s) return s;
-  CK(cudaMemcpyAsync(ev, ctx->d_api_event, sizeof(akmc_event), cudaMemcpyDeviceToHost, ctx->stream));
-  return akmc_sync(ctx);
+  const akmc_status s = api_step(ctx, job, sector_id, kModeSelectPerform, u);
+  if (ctx->settled) *ev = ctx->api->event;
+  return s;
 }
 
 AKMC_API akmc_status akmc_eam_johnson(uint64_t seed, double lattice_const, double cutoff_radius,
@@ -1771,6 +1769,7 @@ AKMC_API akmc_status akmc_job_cluster_stats(akmc_ctx* ctx, int32_t job, int64_t*
                                             int64_t hist_len) {
   if (!ctx || !isolated_cu || hist_len < 0 || hist_len > AKMC_CLUSTER_MAX_BINS || (hist_len > 0 && !hist))
     return AKMC_EINVAL;
+  ctx->settled = false;
   if (!ctx->prepared) return fail(ctx, AKMC_ESTATE, "akmc_prepare first");
   if (!live_job(ctx, job)) return AKMC_ENOTFOUND;
   const HostJob& j = ctx->jobs[static_cast<size_t>(job)];

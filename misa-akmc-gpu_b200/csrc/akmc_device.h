@@ -160,6 +160,18 @@ enum : uint32_t {
 
 enum : int32_t { kModeRound = 0, kModeCalc = 1, kModeSelectPerform = 2 };
 
+// What a per-hop entry point answers, in host memory that the kernel writes: the caller waits for the stream and
+// reads it, without a copy.
+struct ApiOut {
+  double total;
+  uint32_t status;
+  int32_t count;            // the last akmc_calculate's vacancies
+  akmc_event event;
+  int32_t sites[kMaxV];     // their sites
+  double de[kMaxV * 8];     // ΔE of each jump
+  double rates[kMaxV * 8];  // its rates
+};
+
 struct RoundArgs {
   JobDev* jobs;
   int32_t njobs;
@@ -200,13 +212,9 @@ struct RoundArgs {
   int32_t eval_warps;           // CTA shape of the hop kernels: 8 or 4 evaluator warps
   // per-hop entry points
   int32_t api_job, api_sector;
+  int32_t api_vac0, api_nvac;  // the job's slice of the vacancy table
   double api_u;
-  double* api_total;
-  akmc_event* api_event;
-  double* api_de;         // kMaxV * 8: ΔE of each jump of the last akmc_calculate
-  double* api_rates;      // kMaxV * 8: its rates
-  int32_t* api_sites;     // kMaxV: vacancy sites (-1: left the sector)
-  int32_t* api_count;
+  ApiOut* api;
 };
 
 // Kernel launchers (akmc_kernels.cu).
@@ -220,7 +228,7 @@ int launch_round(const RoundArgs& a, int hop_grid, size_t smem, void* stream, vo
 // kErrVacCount is set in *status unless exactly cap were found.
 int launch_load_lattice(const uint8_t* stage, uint8_t* occ, int32_t sx, int64_t nrows, int32_t* vac_site, int32_t* vac_job,
                         int32_t job, int32_t cap, int32_t* count, unsigned int* status, void* stream);
-int launch_api(const RoundArgs& a, size_t smem, void* stream);
+int launch_api(const RoundArgs& a, int kind, size_t smem, void* stream);  // kind: 0 pair bond, 1 EAM FP64, 2 FP32-comp
 int launch_init_rho(uint8_t* occ, int32_t* rho, int32_t sx, int32_t sy, int32_t sz, const Potential* pot,
                     const Geometry* geo, unsigned int* status, void* stream);
 int launch_device_math(const double* x, int64_t n, double* e, double* l, void* stream);

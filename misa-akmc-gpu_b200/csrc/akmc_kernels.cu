@@ -989,7 +989,7 @@ __device__ __forceinline__ int run_block(const RoundArgs& a, Smem& sm, Round& C,
     ix[0] = sm.ix[tid & 63][0];
     ix[1] = sm.ix[tid & 63][1];
   }
-  double* const de_out = API && a.mode == kModeCalc ? a.api_de : nullptr;
+  double* const de_out = API && a.mode == kModeCalc ? a.api->de : nullptr;
   constexpr int D = eam ? 4 : 3;  // a hop changes the rates of vacancies within D cells of its origin
 
   // Density site i of 78 of a hop: jump b of parity p from the site with local index s and global
@@ -1391,19 +1391,19 @@ __device__ __forceinline__ int run_block(const RoundArgs& a, Smem& sm, Round& C,
         if (i == lane + 32) s1 = total;
       }
       if (API && a.mode == kModeCalc) {  // akmc_calculate: the sector's vacancies with their jump rates
-        if (tid < cnt) a.api_sites[tid] = sm.vpk[tid][1].w;
-        for (int i = tid; i < 8 * cnt; i += kThreads) a.api_rates[i] = (&sm.rates[0][0])[i];
+        if (tid < cnt) a.api->sites[tid] = sm.vpk[tid][1].w;
+        for (int i = tid; i < 8 * cnt; i += kThreads) a.api->rates[i] = (&sm.rates[0][0])[i];
         if (tid == kClk) {
-          *a.api_total = total;
-          *a.api_count = cnt;
+          a.api->total = total;
+          a.api->count = cnt;
         }
         break;
       }
       if (fabs(total) < DBL_EPSILON) {  // sublattice.inl:108-112
         if (tid == kClk) {
           if (API) {
-            a.api_event->from_site = -1;
-            a.api_event->total = total;
+            a.api->event.from_site = -1;
+            a.api->event.total = total;
           } else {
             sm.c_time = thr;
           }
@@ -1498,7 +1498,7 @@ __device__ __forceinline__ int run_block(const RoundArgs& a, Smem& sm, Round& C,
         if (!API && a.log_cap > 0) log_event(pb.w, nid, X, u, total, dt, nord, nd);
       }
       if (API && tid == kClk) {
-        akmc_event* e = a.api_event;
+        akmc_event* e = &a.api->event;
         e->round = 0;
         e->hop = C.hops;
         e->from_site = hop ? pb.w : -1;
@@ -1568,14 +1568,22 @@ __device__ __forceinline__ void carve(uint8_t* smem, int nreg, Smem*& sm, uint8_
   occ_s = occ_of(rho_s, nreg);
 }
 
-// One block whose sector's vacancies k_bucket listed (k_hop, k_api_block), CTA-wide.
-template <int KIND, int W, bool API>
-__device__ __forceinline__ void listed_block(const RoundArgs& a, int gb, int sec, uint8_t* smem) {
-  Smem& sm0 = *reinterpret_cast<Smem*>(smem);
+// The site's coordinates and whether it lies in the region's sector.
+__device__ __forceinline__ bool region_site(const Region& R, const JobDev& J, int32_t s, int& X, int& y, int& z) {
+  const int t = s / J.sx;
+  X = s - t * J.sx;
+  z = t / J.sy;
+  y = t - z * J.sy;
+  return static_cast<unsigned>((X >> 1) - R.slo[0]) < static_cast<unsigned>(R.w[0]) &&
+         static_cast<unsigned>(y - R.slo[1]) < static_cast<unsigned>(R.w[1]) &&
+         static_cast<unsigned>(z - R.slo[2]) < static_cast<unsigned>(R.w[2]);
+}
+
+// Block gb's record as round[0] (kernels whose blocks no sweep hands over); CTA-wide, no barrier.
+__device__ __forceinline__ void load_block(Smem& sm, const RoundArgs& a, int gb, int sec) {
   const int tid = threadIdx.x;
   const BlockDev& B = a.blocks[gb];
-  __syncthreads();  // the previous block's readers are done
-  Round& C = sm0.round[0];
+  Round& C = sm.round[0];
   if (tid == 0) {
     C.gb = gb;
     C.job = B.job;
@@ -1583,7 +1591,6 @@ __device__ __forceinline__ void listed_block(const RoundArgs& a, int gb, int sec
     C.r = B.round;
     C.hops = B.hops;
     C.evo = B.evo[sec];
-    sm0.fnv = min(B.cnt, kMaxV);
   } else if (tid >= 32 && tid < 35) {
     C.c0[tid - 32] = B.c0[tid - 32];
     C.c1[tid - 32] = B.c1[tid - 32];
@@ -1591,7 +1598,18 @@ __device__ __forceinline__ void listed_block(const RoundArgs& a, int gb, int sec
     const int q = tid - 64;
     C.str[q >> 2][q & 3] = q < 4 ? B.xs[q] : B.xt[q - 4];
   }
+}
+
+// One block whose sector's vacancies k_bucket listed (k_hop), CTA-wide.
+template <int KIND, int W>
+__device__ __forceinline__ void listed_block(const RoundArgs& a, int gb, int sec, uint8_t* smem) {
+  Smem& sm0 = *reinterpret_cast<Smem*>(smem);
+  const int tid = threadIdx.x;
+  __syncthreads();  // the previous block's readers are done
+  load_block(sm0, a, gb, sec);
+  if (tid == 0) sm0.fnv = min(a.blocks[gb].cnt, kMaxV);
   __syncthreads();
+  Round& C = sm0.round[0];
   load_job(sm0, a, C.job);
   Region R;
   make_region(C.c0, C.c1, sm0.job, sec, R);
@@ -1601,13 +1619,13 @@ __device__ __forceinline__ void listed_block(const RoundArgs& a, int gb, int sec
   carve(smem, R.n, sm, occ_s, rho_s);
   stage_region<KIND, W>(*sm, a, R, occ_s, rho_s);
   if (tid < sm->fnv) {
-    const JobDev& J = sm->job;
     const int v = a.blk_list[static_cast<int64_t>(gb) * kMaxV + tid];
     const int32_t s = a.vac_site[v];
-    const int t = s / J.sx;
-    put_record(*sm, R, tid, v, s, s - t * J.sx, t % J.sy, t / J.sy);
+    int X, y, z;
+    region_site(R, sm->job, s, X, y, z);
+    put_record(*sm, R, tid, v, s, X, y, z);
   }
-  run_block<KIND, W, API>(a, *sm, C, R, occ_s, rho_s, sec);
+  run_block<KIND, W, false>(a, *sm, C, R, occ_s, rho_s, sec);
 }
 
 __global__ void k_bucket(RoundArgs a) {
@@ -1617,8 +1635,7 @@ __global__ void k_bucket(RoundArgs a) {
   if (j < 0) return;  // a free entry of the vacancy table (a context with room for admitted jobs)
   const JobDev& J = a.jobs[j];
   if (J.done) return;
-  if (a.mode != kModeRound && j != a.api_job) return;
-  const int sec = a.mode == kModeRound ? sector_of_round(J.round) : a.api_sector;
+  const int sec = sector_of_round(J.round);
   const int s = a.vac_site[v];
   const int X = s % J.sx;
   const int t = s / J.sx;
@@ -1693,7 +1710,7 @@ __global__ void __launch_bounds__(Shape<W>::kThreads, Shape<W>::kCtasPerSm) k_ho
     const int gb = a.active[item];
     const BlockDev& B = a.blocks[gb];
     if (job_kind(a.jobs[B.job]) != KIND) continue;
-    listed_block<KIND, W, false>(a, gb, sector_of_round(B.round), smem);
+    listed_block<KIND, W>(a, gb, sector_of_round(B.round), smem);
   }
   cta_flush<W>(a, smem);
 }
@@ -2159,10 +2176,8 @@ __global__ void __launch_bounds__(Shape<W>::kThreads, Shape<W>::kCtasPerSm) k_fl
         stage_region<KIND, W>(*sm, a, R, occ_s, rho_s);
         if (tid < kFlowSlots && word != kNoVacancy) {
           const int32_t s = static_cast<int32_t>(word & 0xffffffffu);
-          const int t = s / sm->job.sx, X = s - t * sm->job.sx, z = t / sm->job.sy, y = t - z * sm->job.sy;
-          if (static_cast<unsigned>((X >> 1) - R.slo[0]) < static_cast<unsigned>(R.w[0]) &&
-              static_cast<unsigned>(y - R.slo[1]) < static_cast<unsigned>(R.w[1]) &&
-              static_cast<unsigned>(z - R.slo[2]) < static_cast<unsigned>(R.w[2])) {
+          int X, y, z;
+          if (region_site(R, sm->job, s, X, y, z)) {
             const int i = atomicAdd(&sm->fnv, 1);
             sm->fslot[i] = tid;
             put_record(*sm, R, i, static_cast<int>(word >> 32), s, X, y, z);
@@ -2357,32 +2372,61 @@ __global__ void k_finalize(RoundArgs a) {
   }
 }
 
-__global__ void __launch_bounds__(Shape<8>::kThreads, 1) k_api_block(RoundArgs a) {
+// One per-hop API step (akmc_calculate, akmc_select_and_perform) of a single-domain job in one launch: the CTA finds
+// the sector's vacancies itself and leaves the answer, the status word included, in host memory.
+template <int KIND>
+__global__ void __launch_bounds__(Shape<8>::kThreads, 1) k_api(RoundArgs a) {
+  constexpr int kThreads = Shape<8>::kThreads;
   extern __shared__ __align__(16) uint8_t smem[];
-  const JobDev& J = a.jobs[a.api_job];
-  if (*a.n_active == 0) {  // no vacancy in the sector
-    if (threadIdx.x == 0) {
+  Smem& sm0 = *reinterpret_cast<Smem*>(smem);
+  const int tid = threadIdx.x;
+  init_cta_smem(smem);
+  const int gb = a.jobs[a.api_job].block0;
+  load_block(sm0, a, gb, a.api_sector);
+  __syncthreads();
+  load_job(sm0, a, a.api_job);
+  Round& C = sm0.round[0];
+  Region R;
+  make_region(C.c0, C.c1, sm0.job, a.api_sector, R);
+  Smem* sm;
+  uint8_t* occ_s;
+  int32_t* rho_s;
+  carve(smem, R.n, sm, occ_s, rho_s);
+  for (int i = tid; i < a.api_nvac; i += kThreads) {
+    const int v = a.api_vac0 + i;
+    const int32_t s = a.vac_site[v];
+    int X, y, z;
+    if (!region_site(R, sm->job, s, X, y, z)) continue;
+    const int k = atomicAdd(&sm->fnv, 1);
+    if (k < kMaxV) put_record(*sm, R, k, v, s, X, y, z);
+  }
+  __syncthreads();
+  const int n = sm->fnv;
+  if (n > kMaxV) {
+    __syncthreads();
+    if (tid == 0) {
+      atomicOr(a.status, kErrVacOverflow);
+      sm->fnv = kMaxV;
+    }
+    __syncthreads();
+  }
+  if (n == 0) {  // no vacancy in the sector
+    if (tid == 0) {
+      a.api->total = 0.0;
       if (a.mode == kModeCalc) {
-        *a.api_total = 0.0;
-        *a.api_count = 0;
+        a.api->count = 0;
       } else {
-        a.api_event->from_site = -1;
-        a.api_event->total = 0.0;
+        a.api->event.from_site = -1;
+        a.api->event.total = 0.0;
       }
     }
-    return;
+  } else {
+    stage_region<KIND, 8>(*sm, a, R, occ_s, rho_s);
+    run_block<KIND, 8, true>(a, *sm, C, R, occ_s, rho_s, a.api_sector);
+    cta_flush<8>(a, smem);
   }
-  init_cta_smem(smem);
-  const int kind = job_kind(J);
-  if (kind == kPairBond) listed_block<kPairBond, 8, true>(a, J.block0, a.api_sector, smem);
-  else if (kind == kEam32) listed_block<kEam32, 8, true>(a, J.block0, a.api_sector, smem);
-  else listed_block<kEam64, 8, true>(a, J.block0, a.api_sector, smem);
-  cta_flush<8>(a, smem);
-}
-__global__ void k_api_reset(RoundArgs a) {
-  const JobDev& J = a.jobs[a.api_job];
-  a.blocks[J.block0].cnt = 0;
-  *a.n_active = 0;
+  __syncthreads();
+  if (tid == 0) a.api->status = *reinterpret_cast<volatile unsigned int*>(a.status);
 }
 
 // Density cache of a whole lattice: rho_i = sum over the 58 neighbours j within the cutoff of
@@ -2775,11 +2819,12 @@ int launch_round(const RoundArgs& a, int hop_grid, size_t smem, void* stream, vo
   return static_cast<int>(cudaGetLastError());
 }
 
-int launch_api(const RoundArgs& a, size_t smem, void* stream) {
+int launch_api(const RoundArgs& a, int kind, size_t smem, void* stream) {
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (a.nvac > 0) k_bucket<<<(a.nvac + 127) / 128, 128, 0, st>>>(a);
-  k_api_block<<<1, Shape<8>::kThreads, smem, st>>>(a);
-  k_api_reset<<<1, 1, 0, st>>>(a);
+  constexpr int T = Shape<8>::kThreads;
+  if (kind == kPairBond) k_api<kPairBond><<<1, T, smem, st>>>(a);
+  else if (kind == kEam32) k_api<kEam32><<<1, T, smem, st>>>(a);
+  else k_api<kEam64><<<1, T, smem, st>>>(a);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -2817,7 +2862,8 @@ int configure_hop_smem(size_t smem) {
       reinterpret_cast<const void*>(k_flow<kEam64, 8>),    reinterpret_cast<const void*>(k_flow<kEam32, 8>),
       reinterpret_cast<const void*>(k_flow<kPairBond, 8>), reinterpret_cast<const void*>(k_flow<kEam64, 4>),
       reinterpret_cast<const void*>(k_flow<kEam32, 4>),    reinterpret_cast<const void*>(k_flow<kPairBond, 4>),
-      reinterpret_cast<const void*>(k_api_block)};
+      reinterpret_cast<const void*>(k_api<kEam64>),        reinterpret_cast<const void*>(k_api<kEam32>),
+      reinterpret_cast<const void*>(k_api<kPairBond>)};
   cudaError_t e = cudaSuccess;
   for (const void* f : kernels)
     if (e == cudaSuccess) e = cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
