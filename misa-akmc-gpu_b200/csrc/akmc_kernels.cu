@@ -225,7 +225,8 @@ struct Smem {
   // the block's selection (0) and residence-time (1) streams: running state, the draws made
   // ahead, the state after each, and what the draws stand for (uniform, -ln uniform)
   uint64_t str[2][4];
-  uint64_t raw[2][kDrawRing], sts[kDrawRing][2][4];
+  uint64_t raw[2][kDrawRing];
+  alignas(16) uint64_t sts[kDrawRing][2][4];
   double du[kDrawRing], dl[kDrawRing];
   Round round[kMaxTake];   // rounds handed over by a sweep; [0] alone in the other kernels
   JobDev job;              // the job of the running block (job_key: its index), copied when it changes
@@ -622,6 +623,11 @@ __device__ __forceinline__ void jump_rates(Smem& sm, int set, const uint8_t* occ
 // moving Fe atom), by one warp; nothing for other targets.  Lane q sums sites i = q, q + 32, q + 64 of the
 // jump's list (jl: the list's packed entries); the 32 partials merge by a xor butterfly (16, 8, 4, 2, 1),
 // then the moving atom's own embedding change is added.
+// Jumps of the vacancy at local site l whose target holds a solute, one bit each; all lanes of a warp.
+__device__ __forceinline__ unsigned solute_jumps(const Smem& sm, const uint8_t* occ_s, int l) {
+  const int lane = threadIdx.x & 31;
+  return __ballot_sync(kFull, lane < 8 && occ_s[l + sm.d1[8 * (l & 1) + (lane & 7)].x] > kFe);
+}
 template <int KIND>
 __device__ __forceinline__ void solute_rate(Smem& sm, const uint8_t* occ_s, const int32_t* rho_s, int k, int l, int b,
                                             const Region& R, const Geometry& G, const FTab& FT, double* de_out) {
@@ -845,8 +851,9 @@ __device__ __forceinline__ void put_record(Smem& sm, const Region& R, int k, int
 // slot `slot`: the raw draw and the state after it.  Called by lanes 0 and 1 of one warp.
 __device__ __forceinline__ void draw_ahead(Smem& sm, uint64_t (&x)[4], int lane, int slot) {
   sm.raw[lane][slot] = xoshiro_next(x);
-#pragma unroll
-  for (int i = 0; i < 4; ++i) sm.sts[slot][lane][i] = x[i];
+  ulonglong2* const st = reinterpret_cast<ulonglong2*>(sm.sts[slot][lane]);
+  st[0] = make_ulonglong2(x[0], x[1]);
+  st[1] = make_ulonglong2(x[2], x[3]);
 }
 // What a batch's draws stand for, one draw a lane: the selection uniform in [0, 1) (lanes 0-7) and
 // -ln of the residence-time uniform in (0, 1] (lanes 8-15; sublattice.inl:118-120).
@@ -914,16 +921,17 @@ __device__ __forceinline__ int run_block(const RoundArgs& a, Smem& sm, Round& C,
   FT.kw0 = J.fwin0;
   FT.pot = &P;
   FT.status = a.status;
+  uint64_t dst[4] = {0, 0, 0, 0};  // last warp, lanes 0 and 1: a stream's running state
   if (warp == kEvalWarps - 1) {
     if (!API) {  // the first batch of draws, while the others order the vacancies and the copies fly
       if (lane < 2) {
-        uint64_t x[4];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) x[i] = C.str[lane][i];
+        for (int i = 0; i < 4; ++i) dst[i] = C.str[lane][i];
 #pragma unroll 1
-        for (int k = 0; k < kDrawBatch; ++k) draw_ahead(sm, x, lane, k);
+        for (int k = 0; k < kDrawBatch; ++k) draw_ahead(sm, dst, lane, k);
+        if (KIND == kPairBond)  // the pair-bond loop of one vacancy draws in warp 1
 #pragma unroll
-        for (int i = 0; i < 4; ++i) sm.str[lane][i] = x[i];
+          for (int i = 0; i < 4; ++i) sm.str[lane][i] = dst[i];
       }
       __syncwarp();
       draw_values(sm, lane, 0);
@@ -942,11 +950,6 @@ __device__ __forceinline__ int run_block(const RoundArgs& a, Smem& sm, Round& C,
       sm.nord[0] = n;
       sm.ctl_ok = 1;
       sm.ctl_stop = 0;
-      sm.c_nh = 0;
-      sm.c_nact = 0;
-      sm.c_evals = n;
-      sm.c_sel = 0;
-      sm.c_time = 0.0;
       if (need_win) {
         if (mbar_wait(&sm.mbar, sm.mbar_phase)) {
           sm.mbar_phase ^= 1u;
@@ -1036,18 +1039,21 @@ __device__ __forceinline__ int run_block(const RoundArgs& a, Smem& sm, Round& C,
     b = v0 > expected ? 0 : b;
     return b;
   };
-  // The clock thread: the selection used draw `it`; advances the sector's clock and decides
-  // whether its window is reached.  Returns the residence time.
+  // The clock thread's values of the block-round: the sector's clock, hops, n_act sum and evaluations, selections
+  // made; left in shared memory by clock_end.
+  double time = 0.0;
+  int64_t nh = 0, nact_sum = 0, evals = cnt;
+  int nsel = 0;
+  // The selection used draw `it`; advances the sector's clock and decides whether its window is reached.  Returns
+  // the residence time.
   auto clock_step = [&](int it, double total, bool hop, int n_act) -> double {
     const double dt = sm.dl[it & (kDrawRing - 1)] / total;
-    const double t = sm.c_time + dt;
-    int stop = t < thr ? 0 : 1;
-    sm.c_time = t;
-    sm.c_sel = it + 1;
+    time += dt;
+    int stop = time < thr ? 0 : 1;
+    nsel = it + 1;
     if (hop) {
-      sm.c_nact += n_act;
-      const int64_t nh = sm.c_nh + 1;
-      sm.c_nh = nh;
+      nact_sum += n_act;
+      nh += 1;
       if (nh >= a.hop_cap) {
         atomicOr(a.status, kErrHopCap);
         stop = 1;
@@ -1056,13 +1062,21 @@ __device__ __forceinline__ int run_block(const RoundArgs& a, Smem& sm, Round& C,
     sm.ctl_stop = stop;
     return dt;
   };
-  // The event record of the hop just counted (hop index C.hops + c_nh - 1).
-  auto log_event = [&](int from, int to, int X, double u, double total, double dt, int n_act, int nd) {
+  auto clock_end = [&]() {
+    if (tid != kClk) return;
+    sm.c_time = time;
+    sm.c_sel = nsel;
+    sm.c_nh = nh;
+    sm.c_nact = nact_sum;
+    sm.c_evals = evals;
+  };
+  // The event record of the hop-th hop of this block-round (from 1).
+  auto log_event = [&](int64_t hop, int from, int to, int X, double u, double total, double dt, int n_act, int nd) {
     const unsigned long long slot = atomicAdd(a.log_count, 1ull);
     if (slot < static_cast<unsigned long long>(a.log_cap)) {
       akmc_event* e = a.log + slot;
       e->round = round_now;
-      e->hop = C.hops + sm.c_nh - 1;
+      e->hop = C.hops + hop - 1;
       e->from_site = from;
       e->to_site = to;
       e->block = C.local;
@@ -1079,22 +1093,14 @@ __device__ __forceinline__ int run_block(const RoundArgs& a, Smem& sm, Round& C,
     }
   };
   // One draw of each stream ahead of its use, a batch after the one in use; the batch's values when
-  // it is complete.  Iteration `it`, by the last warp.
+  // it is complete.  Iteration `it`, by the last warp, whose lanes 0 and 1 hold the streams' states.
   auto draw_step = [&](int it) {
-    if (lane < 2) {
-      uint64_t x[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) x[i] = sm.str[lane][i];
-      draw_ahead(sm, x, lane, (it + kDrawBatch) & (kDrawRing - 1));
-#pragma unroll
-      for (int i = 0; i < 4; ++i) sm.str[lane][i] = x[i];
-    }
+    if (lane < 2) draw_ahead(sm, dst, lane, (it + kDrawBatch) & (kDrawRing - 1));
     if ((it & (kDrawBatch - 1)) == kDrawBatch - 1) {
       __syncwarp();
       draw_values(sm, lane, (it + 1) & (kDrawRing - 1));
     }
   };
-
   if (!API && cnt == 1 && !eam) {
     // One vacancy, pair bond: warp 0 runs the whole hop loop without a CTA barrier (32 lanes hold the 4
     // bond counts of all 8 jumps); warp 1 draws ahead, a batch at a time.  Only occupancies change: the
@@ -1129,8 +1135,6 @@ __device__ __forceinline__ int run_block(const RoundArgs& a, Smem& sm, Round& C,
     } else if (warp == 0) {
       const int4 pa = sm.vpk[0][0], pb = sm.vpk[0][1];
       int s = pa.x, lx = pa.y, ly = pa.z, lz = pa.w, gX = pb.x, gY = pb.y, gZ = pb.z, gid = pb.w;
-      double time = 0.0;
-      int64_t nh = 0, evals = 1;
       int it = 0, np = 1, meets = 0;
       if (lane == 0) path[0] = make_int2(s, gid);
       for (;; ++it) {
@@ -1171,10 +1175,7 @@ __device__ __forceinline__ int run_block(const RoundArgs& a, Smem& sm, Round& C,
             occ_s[snew] = kV;
             occ_s[s] = static_cast<uint8_t>(X);
             path[np] = make_int2(snew, nid);
-            if (a.log_cap > 0) {
-              sm.c_nh = nh;
-              log_event(gid, nid, X, u, total, dt, 1, nact ? 1 : 0);
-            }
+            if (a.log_cap > 0) log_event(nh, gid, nid, X, u, total, dt, 1, nact ? 1 : 0);
           }
           __syncwarp();
           s = snew;
@@ -1223,7 +1224,8 @@ __device__ __forceinline__ int run_block(const RoundArgs& a, Smem& sm, Round& C,
     //     target, then what the last hop left to do off the chain (its clock, the draws ahead, the
     //     write-through of its 78 densities and two occupancies);
     //  B  every warp selects, then the density deltas and dE terms at the vacancy's new site.
-    constexpr int kWt0 = kEvalWarps == 8 ? 96 : 64, kWtN = kEvalWarps == 8 ? 96 : 64;  // write-through threads
+    constexpr int kWt0 = 64, kWtN = kEvalWarps == 8 ? 96 : 64;  // write-through threads (densities)
+    constexpr int kOc = kEvalWarps == 8 ? 160 : 96;             // and of the two occupancies
     const int4 pa = sm.vpk[0][0], pb = sm.vpk[0][1];
     int s = pa.x, lx = pa.y, ly = pa.z, lz = pa.w, gX = pb.x, gY = pb.y, gZ = pb.z, gid = pb.w;
 #pragma unroll
@@ -1241,8 +1243,12 @@ __device__ __forceinline__ int run_block(const RoundArgs& a, Smem& sm, Round& C,
         if (nact) jump_rates<KIND>(sm, 0, occ_s, 0, s, warp, ix, nullptr);
       } else {
         if (nact) {
-#pragma unroll 1
-          for (int q = warp - 2; q < 8; q += kEvalWarps - 2) solute_rate<KIND>(sm, occ_s, rho_s, 0, s, q, R, *a.geo, FT, nullptr);
+          unsigned solutes = solute_jumps(sm, occ_s, s);
+          for (int q = 2; solutes; ++q) {  // the k-th of them to warp 2 + k
+            if ((q - 2) % (kEvalWarps - 2) == warp - 2)
+              solute_rate<KIND>(sm, occ_s, rho_s, 0, s, __ffs(static_cast<int>(solutes)) - 1, R, *a.geo, FT, nullptr);
+            solutes &= solutes - 1;
+          }
         }
         if (it > 0) {
           const int oX = gX, oY = gY, oZ = gZ, oid = gid;
@@ -1255,15 +1261,15 @@ __device__ __forceinline__ int run_block(const RoundArgs& a, Smem& sm, Round& C,
           if (tid == kClk) {
             const double dt = clock_step(it - 1, total, hop, 1);
             if (hop) {
-              sm.c_evals += nact ? 1 : 0;
-              if (a.log_cap > 0) log_event(oid, gid, X, u, total, dt, 1, nact ? 1 : 0);
+              evals += nact ? 1 : 0;
+              if (a.log_cap > 0) log_event(nh, oid, gid, X, u, total, dt, 1, nact ? 1 : 0);
             }
           }
           if (hop) {
             if (tid >= kWt0 && tid < kWt0 + kWtN)
               for (int i = tid - kWt0; i < kRefreshN; i += kWtN) refresh(i, os & 1, b, os, X, oX, oY, oZ, false);
-            if (tid == kCtl || tid == kCtl + 1) {
-              const bool to = tid == kCtl;
+            if (tid == kOc || tid == kOc + 1) {
+              const bool to = tid == kOc;
               put_occ(to ? gX : oX, to ? gY : oY, to ? gZ : oZ, to ? static_cast<uint8_t>(kV) : static_cast<uint8_t>(X));
             }
           }
@@ -1274,7 +1280,7 @@ __device__ __forceinline__ int run_block(const RoundArgs& a, Smem& sm, Round& C,
       AKMC_PHASE(2);
       if (it > 0 && sm.ctl_stop) break;
       if (!nact) {  // the sector is empty now: its clock jumps to the window
-        if (tid == kClk) sm.c_time = thr;
+        time = thr;
         break;
       }
       const double2* r = reinterpret_cast<const double2*>(sm.rates[0]);
@@ -1282,7 +1288,7 @@ __device__ __forceinline__ int run_block(const RoundArgs& a, Smem& sm, Round& C,
       u = sm.du[it & (kDrawRing - 1)];
       const int sel = select_one(r2, u, total);
       if (fabs(total) < DBL_EPSILON) {  // sublattice.inl:108-112
-        if (tid == kClk) sm.c_time = thr;
+        time = thr;
         break;
       }
       hop = sel >= 0;  // else: a selection that finds no jump advances the clock only
@@ -1312,6 +1318,7 @@ __device__ __forceinline__ int run_block(const RoundArgs& a, Smem& sm, Round& C,
       sm.vpk[0][0] = make_int4(s, lx, ly, lz);
       sm.vpk[0][1] = make_int4(gX, gY, gZ, gid);
     }
+    clock_end();
   } else {
     // vacancy k lies within D cells of the cell (qx, qy, qz) and in the sector
     auto dirty = [&](int k, int qx, int qy, int qz) -> bool {
@@ -1363,9 +1370,13 @@ __device__ __forceinline__ int run_block(const RoundArgs& a, Smem& sm, Round& C,
           }
           constexpr int kw = kEvalWarps == 8 ? 4 : 0;
           if (warp >= kw) {
-#pragma unroll 1
-            for (int n = warp - kw; n < (kb >= 0 ? 16 : 8); n += kEvalWarps - kw)
-              solute_rate<KIND>(sm, occ_s, rho_s, n < 8 ? ka : kb, n < 8 ? la : lb, n & 7, R, *a.geo, FT, de_out);
+            unsigned sol = solute_jumps(sm, occ_s, la) | (kb >= 0 ? solute_jumps(sm, occ_s, lb) << 8 : 0u);
+            for (int n = 0; sol; ++n) {  // the solute targets of both, one after another to these warps
+              const int q = __ffs(static_cast<int>(sol)) - 1;
+              if (n % (kEvalWarps - kw) == warp - kw)
+                solute_rate<KIND>(sm, occ_s, rho_s, q < 8 ? ka : kb, q < 8 ? la : lb, q & 7, R, *a.geo, FT, de_out);
+              sol &= sol - 1;
+            }
           }
           if (m0 | m1) __syncthreads();  // the term sets are written again
         }
@@ -1405,7 +1416,7 @@ __device__ __forceinline__ int run_block(const RoundArgs& a, Smem& sm, Round& C,
             a.api->event.from_site = -1;
             a.api->event.total = total;
           } else {
-            sm.c_time = thr;
+            time = thr;
           }
         }
         break;
@@ -1470,8 +1481,8 @@ __device__ __forceinline__ int run_block(const RoundArgs& a, Smem& sm, Round& C,
         if (tid == kClk) {
           if (API) {
             if (hop) {
-              sm.c_nh = 1;
-              sm.c_nact += nord;
+              nh = 1;
+              nact_sum += nord;
             }
             sm.ctl_stop = 1;  // the per-hop entry point stops after one selection
           } else {
@@ -1494,8 +1505,8 @@ __device__ __forceinline__ int run_block(const RoundArgs& a, Smem& sm, Round& C,
       }
       if (tid == kClk && hop) {
         const int nd = __popc(m0) + __popc(m1);
-        sm.c_evals += nd;
-        if (!API && a.log_cap > 0) log_event(pb.w, nid, X, u, total, dt, nord, nd);
+        evals += nd;
+        if (!API && a.log_cap > 0) log_event(nh, pb.w, nid, X, u, total, dt, nord, nd);
       }
       if (API && tid == kClk) {
         akmc_event* e = &a.api->event;
@@ -1515,6 +1526,7 @@ __device__ __forceinline__ int run_block(const RoundArgs& a, Smem& sm, Round& C,
       }
       if (sm.ctl_stop) break;
     }
+    clock_end();
   }
   __syncthreads();
   AKMC_PHASE(6);
