@@ -122,7 +122,7 @@ typedef struct akmc_context_config {
   int64_t event_log_capacity;  /* 0: no event log */
   int64_t hop_cap_per_round;   /* per block and round; 0: 1e7 */
   int64_t flow_sweep_limit;    /* AKMC_SCHEDULE_FLOW watchdog: sweeps per CTA and launch before
-                                  the launch gives up with AKMC_ETIMEOUT; 0: 2^24.  Rounds
+                                  the launch gives up with AKMC_ETIMEOUT; 0: 2^25.  Rounds
                                   already published stay complete; recover from a snapshot. */
   /* Room for jobs admitted after akmc_prepare (akmc_admit_job); max_jobs = 0: none.  The device
    * tables are sized at akmc_prepare for this many jobs, domain blocks and vacancies held at

@@ -130,7 +130,6 @@ struct akmc_ctx {
   int32_t* d_vcount = nullptr;
   int32_t* d_nbr = nullptr;
   unsigned char* d_tmaps = nullptr;  // per job slot: two 128-byte tensor maps
-  unsigned int* d_vsec = nullptr;
   int32_t* d_flow = nullptr;  // flow_need[3], flow_done[3], flow_idle
   // cluster statistics scratch: list, parent, size (one int32 per site of the largest job
   // measured so far), then n_list, the isolated count and the histogram
@@ -232,12 +231,11 @@ void free_device(akmc_ctx* ctx) {
   ctx->ev.clear();
   dfree(ctx->stream, ctx->d_vac_count);
   ctx->d_vac_count = nullptr;
-  void* flow_ptrs[] = {ctx->d_fstate, ctx->d_vslot, ctx->d_vcount, ctx->d_nbr, ctx->d_vsec, ctx->d_flow};
+  void* flow_ptrs[] = {ctx->d_fstate, ctx->d_vslot, ctx->d_vcount, ctx->d_nbr, ctx->d_flow};
   for (void* p : flow_ptrs) dfree(ctx->stream, p);
   ctx->d_fstate = nullptr;
   ctx->d_vslot = nullptr;
   ctx->d_vcount = ctx->d_nbr = ctx->d_flow = nullptr;
-  ctx->d_vsec = nullptr;
   dfree(ctx->stream, ctx->d_tmaps);
   ctx->d_tmaps = nullptr;
   dfree(ctx->stream, ctx->d_stage1);
@@ -428,7 +426,7 @@ AKMC_API akmc_status akmc_create(const akmc_context_config* cfg, akmc_ctx** out)
   if (cfg) ctx->cfg = *cfg;
   if (ctx->cfg.graph_rounds <= 0) ctx->cfg.graph_rounds = 32;
   if (ctx->cfg.hop_cap_per_round <= 0) ctx->cfg.hop_cap_per_round = 10000000;
-  if (ctx->cfg.flow_sweep_limit <= 0) ctx->cfg.flow_sweep_limit = int64_t(1) << 24;
+  if (ctx->cfg.flow_sweep_limit <= 0) ctx->cfg.flow_sweep_limit = int64_t(1) << 25;
   if (ctx->cfg.eval_warps == 0) ctx->cfg.eval_warps = 8;
   if ((ctx->cfg.eval_warps != 8 && ctx->cfg.eval_warps != 4) || ctx->cfg.flow_take < 0) {
     delete ctx;
@@ -903,7 +901,6 @@ AKMC_API akmc_status akmc_prepare(akmc_ctx* ctx) {
   CK(dalloc(ctx->stream, &ctx->d_vslot, ncap * kFlowSlots));
   CK(dalloc(ctx->stream, &ctx->d_vcount, ncap));
   CK(dalloc(ctx->stream, &ctx->d_nbr, ncap * kNbrStride));
-  CK(dalloc(ctx->stream, &ctx->d_vsec, ncap));
   {
     // every job slot's two tensor maps (filled for the jobs added so far; admitted jobs later)
     std::vector<unsigned char> tm(static_cast<size_t>(ctx->cap_jobs) * 256, 0);
@@ -964,7 +961,6 @@ AKMC_API akmc_status akmc_prepare(akmc_ctx* ctx) {
   a.vslot = ctx->d_vslot;
   a.vcount = ctx->d_vcount;
   a.nbr = ctx->d_nbr;
-  a.vsec = ctx->d_vsec;
   a.tmaps = ctx->d_tmaps;
   a.flow_need = ctx->d_flow;
   a.flow_done = ctx->d_flow + 3;

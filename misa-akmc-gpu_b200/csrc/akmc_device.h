@@ -17,7 +17,8 @@ constexpr int kTermN = 302;                       // distinct energy terms of a 
 constexpr int kTermSlots = 313;                   // + own and target embedding values, a zero, a trash term
 constexpr int kFootSlots = 256;                   // lanes that compute them
 constexpr int kShellNb = 58;                      // neighbours within the 5-shell cutoff
-constexpr int kNbrStride = 32;  // words per block of RoundArgs::nbr (one 128-byte line)
+constexpr int kNbrStride = 8;  // words per block of RoundArgs::nbr (one 32-byte sector)
+constexpr int kWordShift = 9;  // rounds in a block's word (RoundArgs::fstate)
 constexpr int kFlowSlots = 64;                    // vacancies held in one domain block's area
 
 // Packed neighbour entry: int8 dX | int8 dy << 8 | int8 dz << 16 | (sh_s | sh_t << 4) << 24,
@@ -146,6 +147,7 @@ struct BlockDev {
   int32_t budget_end;    // asynchronous schedule: the hop budget set the block's target (the job
                          // ends when the block reaches it)
   int32_t pad2;
+  int64_t step[8];       // asynchronous schedule, within a launch: rounds of each sector evo accounts for
 };
 
 enum : uint32_t {
@@ -194,21 +196,21 @@ struct RoundArgs {
   unsigned long long* counters;  // hops, evaluations, rounds, blocks, n_act sum, staged sites, written sites, -
   int64_t hop_cap;
   // asynchronous round schedule (k_flow)
-  unsigned long long* fstate;   // per block: rounds completed << 1, | 1 while a thread or CTA holds it
+  unsigned long long* fstate;   // per block: rounds completed << kWordShift, | 2 << s while a vacancy of its area
+                                // lies in sector s, | 1 while a thread or CTA holds it or it is at its target
   unsigned long long* vslot;    // per block, kFlowSlots words: id << 32 | site of each vacancy in its area
                                 // (all bits set: a free slot)
   int32_t* vcount;              // per block: fill counter while the slots are rebuilt
-  unsigned int* vsec;           // per block: bit s set while a vacancy of its area lies in sector s
   const void* tmaps;            // per job slot: two 128-byte tensor maps (occupancy, densities)
-  int32_t* nbr;                 // per block, kNbrStride words: the 27 neighbour blocks (offset
-                                // o = (dz+1)*9 + (dy+1)*3 + dx+1) and a flags word (k_flow_prep)
+  int32_t* nbr;                 // per block, kNbrStride words: index differences to the six face
+                                // neighbours, a flags word and the job (k_flow_prep)
   int32_t* flow_need;           // per energy kind: blocks with rounds to run in this launch
   int32_t* flow_done;           // per energy kind: blocks that reached their target
   int32_t* flow_idle;           // CTAs of the launch whose last sweep found no round to run
   int64_t flow_rounds;          // rounds this launch adds to every unfinished block
   int64_t flow_sweep_limit;     // sweeps per CTA before the launch gives up (kErrTimeout)
   int64_t time_budget_ns;       // > 0: the launch takes no new round after this long (akmc_run_for)
-  int32_t flow_take;            // rounds with vacancies a CTA takes per sweep (0: all it found)
+  int32_t flow_take;            // rounds with vacancies a CTA takes per sweep (0: by the idle CTAs)
   int32_t eval_warps;           // CTA shape of the hop kernels: 8 or 4 evaluator warps
   // per-hop entry points
   int32_t api_job, api_sector;

@@ -28,18 +28,12 @@ namespace {
 
 constexpr unsigned kFull = 0xffffffffu;
 constexpr int kStageRows = 4;  // rows of the staged region each warp has in flight
-// Blocks a k_flow thread may visit per sweep, until it takes one.  Measured on the 256^3 lattice
-// and the 512 batched boxes: 2 and 3 cost 1.7% and 4.5% on the 256^3 lattice and gain nothing
-// on the batched boxes.
-#ifndef AKMC_SWEEP_VISITS
-#define AKMC_SWEEP_VISITS 1
-#endif
-constexpr int kSweepVisits = AKMC_SWEEP_VISITS;
 // CTAs that look after a block at a time: a sweep visits at most nblocks * kSweepWatch / CTAs blocks (and one
 // per thread).  More only makes the visits wait on one another: with every thread of every CTA visiting, a
 // context of a few hundred blocks had each of its round words read hundreds of thousands of times a sweep.
 // 512 rounds of 180 blocks: 23.5 ms so, 11.7 with 16, 11.8 with 8, 13.1 with 4 (then blocks wait for a visit:
-// 56 and 113 ms with 2 and 1); 4096 blocks: the same from 8 on.
+// 56 and 113 ms with 2 and 1); 4096 blocks: the same from 8 on.  With cheaper visits (flow_ready) 8, 16 and 32
+// are within 1%.
 constexpr int kSweepWatch = 16;
 // Nanoseconds a k_flow CTA sleeps after a sweep that moved no block on (0: none).
 #ifndef AKMC_SWEEP_SLEEP_NS
@@ -1738,14 +1732,18 @@ __global__ void __launch_bounds__(Shape<W>::kThreads, Shape<W>::kCtasPerSm) k_ho
 // vacancies in its area in kFlowSlots slots; a hop that carries a vacancy into a
 // neighbour's area moves the id there.
 //
-// k_flow is persistent.  Each sweep a thread takes one block: while the block's next
-// round is ready and its sector holds no vacancy, the thread runs that round alone (the
-// clock jumps to the window, sublattice.inl:108-112); a ready round with vacancies is
-// handed to the CTA, which runs the hop loop for it.  A block is held with a lease while
-// anything works on it, and nothing waits while holding a lease.  The lease and the block's
-// completed rounds share one 64-bit word (fstate = rounds << 1 | leased): one compare-and-swap
-// reads the round and takes the lease, and one store after a fence publishes the rounds run
-// and frees the lease together.  B.round is refreshed from the word when the launch ends.
+// k_flow is persistent.  Each sweep a thread looks at one block.  A ready round whose sector holds
+// no vacancy is one compare-and-swap: the clock's jumps to the window (sublattice.inl:108-112) are
+// caught up when the sector next holds one, or when the launch ends (flow_clock).  A ready round
+// with vacancies is handed to the CTA, which runs the hop loop for it.  A block is held with a
+// lease while anything works on it, and nothing waits while holding a lease.
+//
+// A block's word (fstate = rounds << 9 | sector mask << 1 | lease) holds its completed rounds, a
+// bit for each sector that has a vacancy, and the lease, so that one compare-and-swap checks all
+// three: a neighbour that brought a vacancy into the sector after the word was read makes it fail.
+// One add after a fence publishes a round run and frees the lease.  A block at its target keeps
+// the lease bit, so a sweep reads nothing else of it.  B.round is refreshed from the word when the
+// launch ends.
 // A single-block job's rounds depend on nothing else, so the CTA that ran one runs the next
 // straight away when it holds no other round of the sweep (its hop budget is checked here, at
 // each time-step boundary).
@@ -1757,8 +1755,13 @@ __device__ __forceinline__ uint64_t globaltimer_ns() {
 }
 // Release/acquire fence at GPU scope (lighter than the sequentially consistent __threadfence).
 __device__ __forceinline__ void fence_acq_rel() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
-__device__ __forceinline__ void st_release_u64(unsigned long long* p, unsigned long long v) {
-  asm volatile("st.release.gpu.global.b64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+__device__ __forceinline__ void add_release_u64(unsigned long long* p, unsigned long long v) {
+  asm volatile("red.release.gpu.global.add.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+__device__ __forceinline__ unsigned long long ld_acquire_u64(const unsigned long long* p) {
+  unsigned long long v;
+  asm volatile("ld.acquire.gpu.global.b64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+  return v;
 }
 __device__ __forceinline__ unsigned long long ld_relaxed_u64(const unsigned long long* p) {
   unsigned long long v;
@@ -1771,40 +1774,35 @@ __device__ __forceinline__ unsigned int ld_relaxed_u32(const unsigned int* p) {
   return v;
 }
 
-// Rounds back to the latest earlier round of the neighbour at offset o = (dz+1)*9 + (dy+1)*3 + dx+1 whose
-// region meets this round's (phase = round mod 8), 0 if none ever does.  Per dimension a +1 neighbour's regions
-// meet ours only between our high half and its low half (block edges >= 8 cells, halos of 2), a -1 neighbour's
-// only between our low half and its high half.
 __host__ __device__ constexpr int flow_sector(int phase) {
   constexpr int ring[8] = {0, 7, 2, 5, 3, 4, 1, 6};  // sector_of_round
   return ring[phase & 7];
 }
-__host__ __device__ constexpr int flow_lag(int phase, int o) {
-  const int d[3] = {o % 3 - 1, (o / 3) % 3 - 1, o / 9 - 1};
-  for (int k = 1; k <= 8; ++k) {
-    bool meet = o != 13;
-    for (int a = 0; a < 3; ++a) {
-      const int hn = (flow_sector(phase) >> a) & 1, ht = (flow_sector(phase + 8 - k) >> a) & 1;
-      if (d[a] == 1) meet = meet && hn == 1 && ht == 0;
-      if (d[a] == -1) meet = meet && hn == 0 && ht == 1;
-    }
-    if (meet) return k;
-  }
-  return 0;
+// The neighbours a round waits for.  Per dimension a +1 neighbour's regions meet ours only between our high half
+// and its low half (block edges >= 8 cells, halos of 2), a -1 neighbour's only between our low half and its high
+// half.  So the round of sector s meets seven neighbours: those in the directions that s points to (bit a of s:
+// + in dimension a, else -), in any nonempty set m of the dimensions, each in the rounds whose sector differs from
+// s in every dimension of m.  Bits 4m..4m+3 of flow_lags: rounds back to the latest such round.
+__host__ __device__ constexpr uint32_t flow_lags(int phase) {
+  uint32_t v = 0;
+  for (int m = 1; m < 8; ++m)
+    for (int k = 7; k >= 1; --k)
+      if (((flow_sector(phase + 8 - k) ^ flow_sector(phase)) & m) == m)
+        v = (v & ~(15u << (4 * m))) | (static_cast<uint32_t>(k) << (4 * m));
+  return v;
 }
+__constant__ const uint32_t kFlowLags[8] = {flow_lags(0), flow_lags(1), flow_lags(2), flow_lags(3),
+                                            flow_lags(4), flow_lags(5), flow_lags(6), flow_lags(7)};
 
 __device__ __forceinline__ int wrapb(int v, int m) { return v < 0 ? v + m : (v >= m ? v - m : v); }
 
-// Global index of the neighbour of block local_id at offset o (o = (dz+1)*9 + (dy+1)*3 + dx+1).
-__device__ __forceinline__ int flow_neighbour(const JobDev& J, int local_id, int o) {
-  const int bx = local_id % J.nb[0], by = (local_id / J.nb[0]) % J.nb[1], bz = local_id / (J.nb[0] * J.nb[1]);
-  return J.block0 + wrapb(bx + o % 3 - 1, J.nb[0]) +
-         J.nb[0] * (wrapb(by + (o / 3) % 3 - 1, J.nb[1]) + J.nb[1] * wrapb(bz + o / 9 - 1, J.nb[2]));
+// Global index of the neighbour of block local_id one step (dir = -1 or 1) along dimension d.
+__device__ __forceinline__ int flow_neighbour(const JobDev& J, int local_id, int d, int dir) {
+  int b[3] = {local_id % J.nb[0], (local_id / J.nb[0]) % J.nb[1], local_id / (J.nb[0] * J.nb[1])};
+  b[d] = wrapb(b[d] + dir, J.nb[d]);
+  return J.block0 + b[0] + J.nb[0] * (b[1] + J.nb[1] * b[2]);
 }
 
-// Whether round r of the block may run.  The neighbours' round counters are read with
-// relaxed loads, all in flight at once, and a fence follows a positive answer (the acquire
-// pattern): the writes of the rounds waited for become visible to this thread.
 // A multi-block job with a hop budget ends at the end of the first time step at which the hops
 // of all its blocks reach the budget, so its round b at a time-step boundary (b = 8, 16, ...)
 // runs only once every block of the job has reached b; the blocks' hops at b (hops_at, written
@@ -1815,7 +1813,7 @@ __device__ int budget_gate(const RoundArgs& a, const JobDev& J, int64_t b) {
   if (J.hop_budget <= 0 || J.nblocks == 1 || b == 0 || (b & 7)) return 1;
   bool all = true;
   for (int k = 0; k < J.nblocks; ++k)
-    all &= static_cast<int64_t>(ld_relaxed_u64(&a.fstate[J.block0 + k]) >> 1) >= b;
+    all &= static_cast<int64_t>(ld_relaxed_u64(&a.fstate[J.block0 + k]) >> kWordShift) >= b;
   if (!all) return 0;
   fence_acq_rel();  // the hops_at written before those rounds were published
   const int slot = static_cast<int>((b >> 3) & 1);
@@ -1824,68 +1822,54 @@ __device__ int budget_gate(const RoundArgs& a, const JobDev& J, int64_t b) {
   return sum >= J.hop_budget ? 2 : 1;
 }
 
-// Flags word of a block's row of RoundArgs::nbr: the energy kind (kNbrFree for a free block
-// slot) and whether the job's hop budget gates its rounds at time-step boundaries (budget_gate).
+// A block's row of RoundArgs::nbr, one 32-byte sector: the index differences to its six face neighbours (-x, +x,
+// -y, +y, -z, +z; 0 where the dimension has one block), a flags word and the job.  Flags: the energy kind (kNbrFree
+// for a free block slot); kNbrGate: the job's hop budget gates its rounds at time-step boundaries (budget_gate);
 // kNbrSolo: a single-block job, whose rounds wait for no other block.
 constexpr int kNbrFree = 3, kNbrKindMask = 3, kNbrGate = 4, kNbrSolo = 8;
 
-// The neighbours' completed rounds relative to round r0 (P[o] = rounds - r0, clamped to
-// +-2^30; the block itself never holds it back: 2^30), read with relaxed loads, all in flight at
-// once, from the block's row of the neighbour table.  The caller fences after the loads (an
-// acquire) before it reads what those rounds wrote.  (Relative int32 counts keep the snapshot in
-// 27 registers.)
-constexpr int32_t kAhead = 1 << 30;
-// The block's row of the neighbour table: 27 neighbours and the flags word (y[27]).
-__device__ __forceinline__ void flow_row(const RoundArgs& a, int gb, int (&y)[28]) {
-  const int4* row = reinterpret_cast<const int4*>(a.nbr + static_cast<int64_t>(gb) * kNbrStride);
+// Whether the round the word w of block gb is at may run: the seven neighbours it meets have completed the rounds it
+// waits for.  Their words are read with relaxed loads, all in flight at once; the caller fences afterwards (an
+// acquire) before it reads what those rounds wrote.  Only the low halves are read: neighbours are within a few
+// rounds of each other, so the difference of 23 bits of the rounds is exact.
+// Bounded by the SM's path to L2: a sweep of 256 blocks that read all 26 neighbours' words and a 128-byte row of
+// their indices took 2.5K cycles for the rows and 3.8K for the words (256^3 lattice). One 32-byte
+// sector and seven words, and empty rounds passed over in the word alone instead of under a lease with their
+// record: 1024 rounds of the 256^3 lattice 27.9 -> 24.1 ms, 512 rounds of 180 pair-bond blocks 10.8 -> 10.0.
+__device__ __forceinline__ bool flow_ready(const RoundArgs& a, int gb, unsigned long long w, const int4& d0, const int4& d1) {
+  const int ph = static_cast<int>(w >> kWordShift) & 7, s = sector_of_round(ph);
+  const uint32_t lags = kFlowLags[ph];
+  const int d[3] = {s & 1 ? d0.y : d0.x, s & 2 ? d0.w : d0.z, s & 4 ? d1.y : d1.x};
+  int o[8];
+  uint32_t lo[8];
 #pragma unroll
-  for (int q = 0; q < 7; ++q) {
-    const int4 v = __ldcg(row + q);
-    y[4 * q] = v.x;
-    y[4 * q + 1] = v.y;
-    y[4 * q + 2] = v.z;
-    y[4 * q + 3] = v.w;
+  for (int m = 1; m < 8; ++m) {
+    o[m] = gb + (m & 1 ? d[0] : 0) + (m & 2 ? d[1] : 0) + (m & 4 ? d[2] : 0);
+    lo[m] = ld_relaxed_u32(reinterpret_cast<const unsigned int*>(&a.fstate[o[m]]));
   }
-}
-__device__ __forceinline__ void flow_snapshot(const RoundArgs& a, int gb, const int (&y)[28], int64_t r0,
-                                              int32_t (&P)[27]) {
-  // only the word's low 32 bits are read (27 registers in flight, not 54): neighbours of one job
-  // are within a few rounds of each other, so the difference taken modulo 2^31 is exact
-  const uint32_t base = static_cast<uint32_t>(r0) & 0x7fffffffu;
+  const uint32_t base = static_cast<uint32_t>(w) >> kWordShift << kWordShift;
+  bool ok = true;
 #pragma unroll
-  for (int o = 0; o < 27; ++o) {
-    if (y[o] == gb) {
-      P[o] = kAhead;
-    } else {
-      const uint32_t lo = ld_relaxed_u32(reinterpret_cast<const unsigned int*>(&a.fstate[y[o]]));
-      P[o] = static_cast<int32_t>(((lo >> 1) - base) << 1) >> 1;  // sign from bit 30
-    }
+  for (int m = 1; m < 8; ++m) {
+    const int ahead = static_cast<int32_t>((lo[m] >> kWordShift << kWordShift) - base) >> kWordShift;
+    ok = ok && (o[m] == gb || ahead + static_cast<int>((lags >> (4 * m)) & 15u) > 0);
   }
+  return ok;
 }
 
-// Rounds from r0 on that a snapshot relative to r0 lets run: the smallest d <= D such that some neighbour has
-// not completed the round that r0 + d waits for.  Round r0 + d, of phase (r0 + d) mod 8, waits for a neighbour
-// with lag k to have completed d - k + 1 rounds past r0; so for each phase (first reached after e rounds) and
-// neighbour, the first round held back is e + 8 max(0, floor((P + k + 7 - e) / 8)).  56 pairs of a phase and a
-// neighbour with a lag, five instructions each, for any number of rounds.
-template <int I>
-__device__ __forceinline__ int flow_limit_pair(const int32_t (&P)[27], const int (&e)[8], int D) {
-  constexpr int o = I / 8, ph = I % 8, k = flow_lag(ph, o);
-  if constexpr (k > 0) D = min(D, e[ph] + 8 * max(0, (P[o] + (k + 7) - e[ph]) >> 3));
-  return D;
+// A sector's clock e, which accounts for `from` of its rounds, after `to` of them when those between found no
+// vacancy (total = 0: the clock jumps to the window if it is behind, sublattice.inl:108-112).
+__device__ __forceinline__ double flow_clock(double e, int64_t from, int64_t to, double window) {
+  for (int64_t t = from; t < to; ++t) {
+    const double thr = static_cast<double>(t + 1) * window - e;
+    double sector_time = 0.0;
+    if (sector_time < thr) sector_time = thr;
+    e += sector_time;
+  }
+  return e;
 }
-template <int... I>
-__device__ __forceinline__ int flow_limit_all(const int32_t (&P)[27], const int (&e)[8], int D,
-                                              std::integer_sequence<int, I...>) {
-  ((D = flow_limit_pair<I>(P, e, D)), ...);
-  return D;
-}
-__device__ __forceinline__ int flow_limit(const int32_t (&P)[27], int64_t r0, int D) {
-  int e[8];
-#pragma unroll
-  for (int k = 0; k < 8; ++k) e[k] = (k - static_cast<int>(r0)) & 7;
-  return flow_limit_all(P, e, D, std::make_integer_sequence<int, 27 * 8>{});
-}
+// Rounds of the sector of phase p among a block's first r.
+__device__ __forceinline__ int64_t flow_steps(int64_t r, int p) { return (r + 7 - p) >> 3; }
 
 // Block whose area holds site s (the reference's rank split, as k_bucket) and the sector of that
 // block the site lies in.
@@ -1917,116 +1901,81 @@ __device__ void flow_give(const RoundArgs& a, int o, int v, int32_t site, int os
   for (int k = 0; k < kFlowSlots; ++k) {
     const int i = (v + k) & (kFlowSlots - 1);
     if (atomicCAS(slots + i, kNoVacancy, slot_word(v, site)) == kNoVacancy) {
-      atomicOr(&a.vsec[o], 1u << osec);
+      atomicOr(&a.fstate[o], 2ull << osec);
       return;
     }
   }
   atomicOr(a.status, kErrVacOverflow);
 }
 
-// Publishes the block's completed rounds (rn) and keeps (keep = 1) or frees the lease, with
-// one release store.  Release is cumulative: writes of other threads of the CTA that a barrier
-// ordered before this call are released too.  `reached`: this lease holder moved the
-// block onto its target (each block is counted once).
-__device__ __forceinline__ void flow_publish(const RoundArgs& a, int gb, int64_t rn, int keep, bool reached,
-                                             int kind) {
-  st_release_u64(&a.fstate[gb], (static_cast<unsigned long long>(rn) << 1) | static_cast<unsigned long long>(keep));
+// Adds n completed rounds to a held block's word and keeps (keep) or frees the lease, in one release: cumulative, so
+// writes of other threads of the CTA that a barrier ordered before this call are released too.  `reached`: this
+// lease holder moved the block onto its target (each block is counted once), where the lease stays.
+__device__ __forceinline__ void flow_publish(const RoundArgs& a, int gb, int64_t n, bool keep, bool reached, int kind) {
+  const unsigned long long v = (static_cast<unsigned long long>(n) << kWordShift) - (keep || reached ? 0 : 1);
+  if (v != 0) add_release_u64(&a.fstate[gb], v);
   if (reached) atomicAdd(&a.flow_done[kind], 1);
 }
 
-// Lease held, one thread, block gb of job `job` at round r0, with its next D rounds ready (flow_limit; 64 for a
-// single-block job): runs the ready rounds whose sectors hold no vacancy (the clock jumps to the window,
-// sublattice.inl:108-112), up to 64 in one batch, and leaves the block's round in *rn (the caller publishes it).
-// The sector mask read after the snapshot holds every vacancy those rounds can see (a round that could bring one
-// into such a sector overlaps it, so it is in the snapshot).  Returns true when it stops at a ready round with
-// vacancies, which is then described in *C (C null: in the next entry of sm.round, false when `take` are full);
-// false when the next round is not ready or the target is reached.  *reached: this call moved the block onto
-// its target (by running rounds, or by a budget moving the target down to r0); false for a block that was at its
-// target already (a stale sweep read).
-__device__ __forceinline__ bool flow_advance(const RoundArgs& a, Smem& sm, int gb, int job, int64_t r0, int D, Round* C,
+// Lease held, one thread, block gb of job `job`, w its word, its round ready: passes over the rounds whose sectors
+// hold no vacancy (one for a multi-block job; for a single-block job, whose rounds wait for nothing, all up to the
+// next that has some) and leaves the block's round in *rn (the caller publishes it).  Returns true when it stops at
+// a round with vacancies, which is then described in *C (C null: in the next entry of sm.round, false when `take`
+// are full); false when the target is reached, the next round has to be looked at anew, or a budget holds it back.
+// *reached: this call moved the block onto its target (by passing over rounds, or by a budget moving the target).
+__device__ __forceinline__ bool flow_advance(const RoundArgs& a, Smem& sm, int gb, int job, bool solo,
+                                             unsigned long long w, Round* C,
                                              int take, int64_t* rn, bool* reached) {
   BlockDev& B = a.blocks[gb];
   const JobDev& J = a.jobs[job];
+  const int64_t r0 = static_cast<int64_t>(w >> kWordShift);
   *rn = r0;
   *reached = false;
-  // one round of loads, all in flight together: the block's record (the lease is held: nothing else writes it),
-  // its sector mask and the job's constants
-  static_assert(sizeof(BlockDev) % 16 == 0 && offsetof(BlockDev, evo) % 16 == 0 && offsetof(BlockDev, xs) % 16 == 0 &&
-                    offsetof(BlockDev, c0) == 8 && offsetof(BlockDev, c1) == 20,
+  const unsigned mask = static_cast<unsigned>(w >> 1) & 255u;
+  int skip = 0;  // rounds from r0 on without vacancies, up to the limit above
+  while (skip < 8 && !((mask >> sector_of_round(r0 + skip)) & 1u)) ++skip;
+  if (!solo) skip = min(skip, 1);
+  const int sec = sector_of_round(r0 + skip);
+  // one round of loads, all in flight together: the block's record (the lease is held: nothing else writes it) and
+  // the job's constants
+  static_assert(sizeof(BlockDev) % 16 == 0 && offsetof(BlockDev, xs) % 16 == 0 && offsetof(BlockDev, c0) == 8 &&
+                    offsetof(BlockDev, c1) == 20,
                 "16-byte reads of the record");
   const int4* head = reinterpret_cast<const int4*>(&B);
   const int4 h0 = __ldcg(head), h1 = __ldcg(head + 1);  // job, local id, c0[0..1] | c0[2], c1
-  const int64_t t_old = __ldcg(&B.target);
+  int64_t target = __ldcg(&B.target);
   const int64_t hops = __ldcg(&B.hops);  // empty rounds add none
-  double2 ev[4];
   ulonglong2 st[4];
 #pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    ev[k] = __ldcg(reinterpret_cast<const double2*>(B.evo) + k);
-    st[k] = __ldcg(reinterpret_cast<const ulonglong2*>(B.xs) + k);
-  }
-  const unsigned occ_sec = __ldcg(&a.vsec[gb]);
+  for (int k = 0; k < 4; ++k) st[k] = __ldcg(reinterpret_cast<const ulonglong2*>(B.xs) + k);
+  const double evo = __ldcg(&B.evo[sec]);
+  const int64_t step = __ldcg(&B.step[sec]);
   const int nidle = __ldcg(a.flow_idle);
-  const int nbl = J.nblocks;
   const int64_t budget = J.hop_budget;
   const double window = J.window;
-  double evo[8];
-#pragma unroll
-  for (int k = 0; k < 8; ++k) evo[k] = k & 1 ? ev[k >> 1].y : ev[k >> 1].x;
-  if (r0 >= t_old) return false;
-  // a single-block job with a hop budget ends at the end of the first time step at which its
-  // hops reached the budget: once they have, its target moves down to the next boundary at or
-  // after r0 (never below r0)
-  int64_t target = t_old;
-  if (nbl == 1 && budget > 0 && hops >= budget) {
-    const int64_t b = (r0 + 7) & ~static_cast<int64_t>(7);
-    if (b < target) {
-      target = b;
-      B.target = b;
+  if (budget > 0) {
+    int64_t end = target;
+    if (solo) {
+      // a single-block job with a hop budget ends at the end of the first time step at which its
+      // hops reached the budget: once they have, its target moves down to the next boundary at or
+      // after r0 (never below r0)
+      if (hops >= budget) end = min(end, (r0 + 7) & ~static_cast<int64_t>(7));
+    } else {
+      const int g = budget_gate(a, J, r0);
+      if (g == 0) return false;
+      if (g == 2) end = r0;  // the job ends at this boundary: the block's target moves down to it
+    }
+    if (end < target) {
+      target = end;
+      B.target = end;
       B.budget_end = 1;
     }
   }
-  if (r0 >= target) {
-    *reached = true;
-    return false;
-  }
-  const int64_t last = min(target, r0 + D);
-  int64_t r = r0;
-  bool full = false;
-  double e = 0.0;
-  while (r < last) {
-    const int g = budget_gate(a, J, r);
-    if (g == 0) break;
-    if (g == 2) {  // the job ends at this boundary: the block's target moves down to it
-      B.target = r;
-      B.budget_end = 1;
-      target = r;
-      break;
-    }
-    const int sec = sector_of_round(r);
-    e = evo[0];
-#pragma unroll
-    for (int k = 1; k < 8; ++k) e = k == sec ? evo[k] : e;
-    if ((occ_sec >> sec) & 1u) {
-      full = true;
-      break;
-    }
-    const double thr = static_cast<double>((r >> 3) + 1) * window - e;
-    double sector_time = 0.0;
-    if (sector_time < thr) sector_time = thr;
-    const double ne = e + sector_time;
-#pragma unroll
-    for (int k = 0; k < 8; ++k) evo[k] = k == sec ? ne : evo[k];
-    ++r;
-    if ((r & 7) == 0) B.hops_at[(r >> 3) & 1] = hops;
-  }
-  if (r > r0) {
-#pragma unroll
-    for (int k = 0; k < 8; ++k) B.evo[k] = evo[k];
-  }
+  const int64_t r = min(skip < 8 ? r0 + skip : target, target);
+  if (!solo && budget > 0 && r > r0 && (r & 7) == 0) B.hops_at[(r >> 3) & 1] = hops;
   *rn = r;
-  *reached = r == target;  // the lease holder alone moves the target
-  if (!full) return false;
+  *reached = r >= target;  // the lease holder alone moves the target
+  if (*reached || (!solo && skip > 0)) return false;  // (here skip is 8 only without a vacancy: the target is reached)
   if (!C) {
     // Rounds a CTA takes per sweep: `take` when the context sets it.  Else every one its threads find while nearly
     // all CTAs have rounds to run (512 boxes: 22.5 ms for 256 rounds; 25.0 with two, 28.2 with one), but two
@@ -2045,7 +1994,7 @@ __device__ __forceinline__ bool flow_advance(const RoundArgs& a, Smem& sm, int g
   C->r = r;
   C->t = target;
   C->hops = hops;
-  C->evo = e;
+  C->evo = flow_clock(evo, step, r >> 3, window);
 #pragma unroll
   for (int k = 0; k < 4; ++k) {
     C->str[k >> 1][2 * (k & 1)] = st[k].x;
@@ -2073,10 +2022,9 @@ __global__ void __launch_bounds__(Shape<W>::kThreads, Shape<W>::kCtasPerSm) k_fl
   const int tid = threadIdx.x;
   init_cta_smem(smem);
   const int nb = a.nblocks;
-  const int watch = max(1, min(kThreads, static_cast<int>((static_cast<int64_t>(nb) * kSweepWatch) / gridDim.x)));
+  const int watch = max(1, min(min(kThreads, nb), static_cast<int>((static_cast<int64_t>(nb) * kSweepWatch) / gridDim.x)));
   int cursor = static_cast<int>((static_cast<int64_t>(blockIdx.x) * nb) / gridDim.x);
   const uint64_t t_begin = globaltimer_ns();  // a time-boxed launch takes no new round after its budget
-  if (tid == 0) sm0.flow_stop = 0;
 #ifdef AKMC_PHASE_PROFILE
   long long t_sweep = 0, t_hop = 0, n_sweep = 0, n_full = 0, t0 = 0;
 #endif
@@ -2089,9 +2037,8 @@ __global__ void __launch_bounds__(Shape<W>::kThreads, Shape<W>::kCtasPerSm) k_fl
       sm0.flow_progress = 0;
     }
     __syncthreads();
-    if (sm0.flow_stop) break;  // decided during the previous sweep
-    // thread 0 reads the launch's progress and status while the sweep's visits are in flight,
-    // and decides after its own visit whether the CTA stops after this sweep's rounds
+    // thread 0 reads the launch's progress and status before its visit, and decides after it whether the CTA
+    // stops after this sweep's rounds
     int need = 0, done = 0;
     unsigned st = 0;
     if (tid == 0) {
@@ -2100,50 +2047,45 @@ __global__ void __launch_bounds__(Shape<W>::kThreads, Shape<W>::kCtasPerSm) k_fl
       st = *reinterpret_cast<volatile unsigned*>(a.status);
     }
 
-    // sweep: thread tid looks after blocks (cursor + tid + k watch) mod nb, k < kSweepVisits,
-    // until it takes one: a visit that finds nothing to do ends after one or two round trips,
-    // while the sweep lasts as long as its slowest visit (one that takes a block)
-#pragma unroll 1
-    for (int vis = 0; vis < kSweepVisits; ++vis) {
-      const int off = tid + vis * watch;
-      if (tid >= watch || off >= nb) break;
-      int gb = cursor + off;
+    // sweep: thread tid looks after block (cursor + tid) mod nb.  One round of loads (the block's word and row) ends
+    // most visits to a block that is held, a second (the neighbours' words) those to one that waits.
+    if (tid < watch) {
+      int gb = cursor + tid;
       if (gb >= nb) gb -= nb;
-      // one round of loads decides whether to look closer: the block's word, target, job, and its
-      // row of the neighbour table with the flags (energy kind, free slot)
-      int y[28];
-      flow_row(a, gb, y);
-      const unsigned long long w = ld_relaxed_u64(&a.fstate[gb]);
-      const int64_t t0 = __ldcg(&a.blocks[gb].target);
-      const int bj = __ldcg(&a.blocks[gb].job);
-      const int64_t r = static_cast<int64_t>(w >> 1);
-      bool ok = (y[27] & kNbrKindMask) == KIND && !(w & 1ull) && r < t0;
-      int D = 64;  // ready rounds from r on
-      if (ok && !(y[27] & kNbrSolo)) {  // a second: the neighbours' rounds
-        int32_t P[27];
-        flow_snapshot(a, gb, y, r, P);
-        D = flow_limit(P, r, 64);
-        ok = D > 0;
-      }
-      // a multi-block job with a hop budget: its round at a time-step boundary waits for the job's
-      // other blocks (a job that ends there is taken, to mark it)
-      if (ok && (y[27] & kNbrGate) && budget_gate(a, a.jobs[bj], r) == 0) ok = false;
-      // the lease, then one fence: the snapshot's and the word's reads become acquires
-      if (ok && atomicCAS(&a.fstate[gb], w, w | 1ull) == w) {
-        fence_acq_rel();
-        int64_t rn = r;
-        bool reached = false;
-        const bool keep = flow_advance(a, sm0, gb, bj, r, D, nullptr, take, &rn, &reached);
-        if (rn > r) sm0.flow_progress = 1;
-        // a round handed over with none run before it: the word holds it and the lease already
-        if (!keep || rn > r) flow_publish(a, gb, rn, keep ? 1 : 0, reached, KIND);
-        break;
+      const int4* row = reinterpret_cast<const int4*>(a.nbr + static_cast<int64_t>(gb) * kNbrStride);
+      const int4 d0 = __ldg(row), d1 = __ldg(row + 1);
+      const unsigned long long w = ld_acquire_u64(&a.fstate[gb]);
+      if (!(w & 1ull) && (d1.z & kNbrKindMask) == KIND) {
+        const int64_t r = static_cast<int64_t>(w >> kWordShift);
+        const int64_t target = __ldcg(&a.blocks[gb].target);
+        bool ok = (d1.z & kNbrSolo) || flow_ready(a, gb, w, d0, d1);
+        // a multi-block job with a hop budget: its round at a time-step boundary waits for the job's
+        // other blocks (a job that ends there is taken, to mark it)
+        if (ok && (d1.z & kNbrGate) && budget_gate(a, a.jobs[d1.w], r) == 0) ok = false;
+        if (ok && !(d1.z & (kNbrSolo | kNbrGate)) && !((w >> (1 + sector_of_round(r))) & 1ull)) {
+          // no vacancy: the round is passed over, and the block keeps the lease bit at its target.  Nothing is read
+          // or written but the word, so there is nothing to fence: rounds that read what this block's or its
+          // neighbours' rounds wrote wait for those blocks themselves.
+          const bool end = r + 1 >= target;
+          if (atomicCAS(&a.fstate[gb], w, w + (1ull << kWordShift) + (end ? 1 : 0)) == w) {
+            sm0.flow_progress = 1;
+            if (end) atomicAdd(&a.flow_done[KIND], 1);
+          }
+        } else if (ok && atomicCAS(&a.fstate[gb], w, w | 1ull) == w) {
+          // the lease, then one fence: the reads of the words become acquires
+          fence_acq_rel();
+          int64_t rn = r;
+          bool reached = false;
+          const bool keep = flow_advance(a, sm0, gb, d1.w, (d1.z & kNbrSolo) != 0, w, nullptr, take, &rn, &reached);
+          if (rn > r) sm0.flow_progress = 1;
+          flow_publish(a, gb, rn - r, keep, reached, KIND);
+        }
       }
     }
     if (tid == 0) {
       int stop = done >= need || (st & (kErrVacOverflow | kErrRhoRange | kErrHopCap | kErrTimeout)) != 0;
       if (a.time_budget_ns > 0 && globaltimer_ns() - t_begin >= static_cast<uint64_t>(a.time_budget_ns)) stop = 1;
-      if (!stop && sweep + 1 >= a.flow_sweep_limit) {  // watchdog; the default 2^24 no launch of <= 1024 rounds needs
+      if (!stop && sweep + 1 >= a.flow_sweep_limit) {  // watchdog; the default 2^25 no launch of <= 1024 rounds needs
         atomicOr(a.status, kErrTimeout);
         stop = 1;
       }
@@ -2162,6 +2104,7 @@ __global__ void __launch_bounds__(Shape<W>::kThreads, Shape<W>::kCtasPerSm) k_fl
     // the hop loop for each round handed over; a single-block job's next rounds follow while
     // the launch's target allows (empty ones in between run on thread 0)
     const int ncand = min(sm0.flow_ncand, take);
+    const bool last = sm0.flow_stop;  // written again after the next sweep's first barrier only
     if (tid == 0 && (ncand == 0) != idle) {
       idle = ncand == 0;
       atomicAdd(a.flow_idle, idle ? 1 : -1);
@@ -2209,7 +2152,8 @@ __global__ void __launch_bounds__(Shape<W>::kThreads, Shape<W>::kCtasPerSm) k_fl
         // Vacancies carried into a neighbour's area change owner, the others' sites and sectors are kept up to
         // date (only if the round ran).  The sector's bit of the block's mask goes first and comes back for
         // each vacancy still in it.  With one vacancy, thread 0 does it all and publishes the round.
-        if (ran && tid == 0) atomicAnd(&a.vsec[gb], ~(1u << sec));
+        unsigned long long* const fw = a.fstate + gb;
+        if (ran && cnt != 1 && tid == 0) atomicAnd(fw, ~(2ull << sec));
         if (ran && cnt > 1) __syncthreads();
         if (ran && tid < cnt) {
           const int4 g = sm->vpk[tid][1];
@@ -2224,17 +2168,21 @@ __global__ void __launch_bounds__(Shape<W>::kThreads, Shape<W>::kCtasPerSm) k_fl
             o = owner_sector(sm->job, g.w, &osec);
           if (o == gb) {
             *reinterpret_cast<volatile unsigned long long*>(own) = slot_word(sm->vidx[tid], g.w);
-            atomicOr(&a.vsec[gb], 1u << osec);
+            if (cnt == 1 && osec != sec) atomicAnd(fw, ~(2ull << sec));
+            if (cnt > 1 || osec != sec) atomicOr(fw, 2ull << osec);
           } else {
             flow_give(a, o, sm->vidx[tid], g.w, osec);
             *reinterpret_cast<volatile unsigned long long*>(own) = kNoVacancy;
+            if (cnt == 1) atomicAnd(fw, ~(2ull << sec));
           }
         }
         if (ran && cnt > 1) __syncthreads();
         if (tid == 0) {
           // round C.r ran (it was below the target when handed over); the target is the lease
           // holder's to move, and it is this CTA
-          int64_t rn = C.r + 1;
+          const int64_t r1 = C.r + 1;
+          int64_t rn = r1;
+          a.blocks[gb].step[sec] = (C.r >> 3) + 1;
           if ((rn & 7) == 0) a.blocks[gb].hops_at[(rn >> 3) & 1] = C.hops;
           bool more = false, reached = rn >= C.t;
           const bool in_time =
@@ -2242,12 +2190,14 @@ __global__ void __launch_bounds__(Shape<W>::kThreads, Shape<W>::kCtasPerSm) k_fl
           if (!reached && sm->job.nblocks == 1 && c + 1 == ncand && in_time) {
             // a single-block job: its next rounds wait for nothing, so keep the lease and run on
             // -- when no other round this CTA took in the sweep is waiting for it
-            more = flow_advance(a, *sm, gb, C.job, rn, 64, &C, 0, &rn, &reached);
+            const unsigned long long w = ld_relaxed_u64(fw) + (1ull << kWordShift);
+            more = flow_advance(a, *sm, gb, C.job, true, w, &C, 0, &rn, &reached);
           }
+          const int64_t ran_rounds = rn - r1 + 1;
           sm->flow_progress = 1;
           sm->flow_more = more;
           sm->fnv = 0;
-          flow_publish(a, gb, rn, more ? 1 : 0, reached, KIND);
+          flow_publish(a, gb, ran_rounds, more, reached, KIND);
         }
         __syncthreads();
 #ifdef AKMC_PHASE_PROFILE
@@ -2262,8 +2212,9 @@ __global__ void __launch_bounds__(Shape<W>::kThreads, Shape<W>::kCtasPerSm) k_fl
 #ifdef AKMC_PHASE_PROFILE
     if (tid == 0) t_hop += clock64() - t0;
 #endif
+    if (last) break;
     if (AKMC_SWEEP_SLEEP_NS > 0 && !sm0.flow_progress) __nanosleep(AKMC_SWEEP_SLEEP_NS);
-    cursor += kSweepVisits * watch;
+    cursor += watch;
     if (cursor >= nb) cursor %= nb;
   }
   cta_flush<W>(a, smem);
@@ -2277,7 +2228,7 @@ __global__ void __launch_bounds__(Shape<W>::kThreads, Shape<W>::kCtasPerSm) k_fl
 #endif
 }
 
-// Per block: target round of this launch, lease and slots cleared; counts the blocks with
+// Per block: target round of this launch, word and row; counts the blocks with
 // rounds to run per energy kind.
 __global__ void k_flow_prep(RoundArgs a) {
   const int gb = blockIdx.x * blockDim.x + threadIdx.x;
@@ -2285,18 +2236,17 @@ __global__ void k_flow_prep(RoundArgs a) {
   BlockDev& B = a.blocks[gb];
   B.cnt = 0;
   a.vcount[gb] = 0;
-  a.vsec[gb] = 0;
   int32_t* row = a.nbr + static_cast<int64_t>(gb) * kNbrStride;
   if (B.job < 0) {  // a free block slot: nothing to run
     B.target = B.round;
-    a.fstate[gb] = static_cast<unsigned long long>(B.round) << 1;
-    for (int o = 0; o < 27; ++o) row[o] = gb;
-    row[27] = kNbrFree;
+    a.fstate[gb] = (static_cast<unsigned long long>(B.round) << kWordShift) | 1ull;
+    row[6] = kNbrFree;
     return;
   }
   const JobDev& J = a.jobs[B.job];
-  for (int o = 0; o < 27; ++o) row[o] = flow_neighbour(J, B.local_id, o);
-  row[27] = job_kind(J) | (J.nblocks == 1 ? kNbrSolo : J.hop_budget > 0 ? kNbrGate : 0);
+  for (int k = 0; k < 6; ++k) row[k] = flow_neighbour(J, B.local_id, k >> 1, k & 1 ? 1 : -1) - gb;
+  row[7] = B.job;
+  row[6] = job_kind(J) | (J.nblocks == 1 ? kNbrSolo : J.hop_budget > 0 ? kNbrGate : 0);
   // up to flow_rounds of the block's remaining rounds (hop budgets are checked by the kernel,
   // at time-step boundaries); a block sitting at a boundary records its hops there
   int64_t L = B.remaining < a.flow_rounds ? B.remaining : a.flow_rounds;
@@ -2306,7 +2256,8 @@ __global__ void k_flow_prep(RoundArgs a) {
   if (J.max_rounds > 0 && t > J.max_rounds) t = J.max_rounds > B.round ? J.max_rounds : B.round;
   B.remaining -= t - B.round;
   B.target = t;
-  a.fstate[gb] = static_cast<unsigned long long>(B.round) << 1;
+  for (int p = 0; p < 8; ++p) B.step[sector_of_round(p)] = flow_steps(B.round, p);
+  a.fstate[gb] = (static_cast<unsigned long long>(B.round) << kWordShift) | (t > B.round ? 0ull : 1ull);
   if (t > B.round) atomicAdd(&a.flow_need[job_kind(J)], 1);
 }
 
@@ -2323,17 +2274,25 @@ __global__ void k_flow_slots(RoundArgs a) {
     return;
   }
   a.vslot[static_cast<int64_t>(o) * kFlowSlots + slot] = slot_word(v, a.vac_site[v]);
-  atomicOr(&a.vsec[o], 1u << osec);
+  atomicOr(&a.fstate[o], 2ull << osec);
 }
 
-// After the flow kernels: job round and done flags as k_finalize leaves them.
+// After the flow kernels: the sectors' clocks caught up (8 threads a block, one a sector), job round and done flags as
+// k_finalize leaves them.
 __global__ void k_flow_finalize(RoundArgs a) {
-  const int gb = blockIdx.x * blockDim.x + threadIdx.x;
+  const int gb = (blockIdx.x * blockDim.x + threadIdx.x) >> 3, p = threadIdx.x & 7;
+  if (gb < a.nblocks && a.blocks[gb].job >= 0) {
+    BlockDev& B = a.blocks[gb];
+    const int sec = sector_of_round(p);
+    B.evo[sec] = flow_clock(B.evo[sec], B.step[sec], flow_steps(static_cast<int64_t>(a.fstate[gb] >> kWordShift), p),
+                            a.jobs[B.job].window);
+  }
+  if (p != 0) return;
   if (gb == 0 && a.time_budget_ns <= 0) atomicAdd(a.counters + 2, static_cast<unsigned long long>(a.flow_rounds));
   if (gb >= a.nblocks) return;
   BlockDev& B = a.blocks[gb];
   B.cnt = 0;
-  B.round = static_cast<int64_t>(a.fstate[gb] >> 1);
+  B.round = static_cast<int64_t>(a.fstate[gb] >> kWordShift);
   if (B.job < 0) return;
   // rounds of the call a time-boxed launch left to run go back to the block's remaining ones
   if (B.target > B.round) B.remaining += B.target - B.round;
@@ -2860,7 +2819,7 @@ int launch_flow(const RoundArgs& a, int grid, size_t smem, void* stream, void* e
   if (a.eval_warps == 4) launch_flows<4>(a, grid, smem, st);
   else launch_flows<8>(a, grid, smem, st);
   if (ev1) cudaEventRecord(static_cast<cudaEvent_t>(ev1), st);
-  k_flow_finalize<<<(a.nblocks + 127) / 128, 128, 0, st>>>(a);
+  k_flow_finalize<<<(a.nblocks + 15) / 16, 128, 0, st>>>(a);
   return static_cast<int>(cudaGetLastError());
 }
 
