@@ -111,7 +111,7 @@ struct akmc_ctx {
   unsigned long long* d_log_count = nullptr;
   unsigned int* d_status = nullptr;
   unsigned long long* d_counters = nullptr;
-  ApiOut* api = nullptr;  // answers of the per-hop entry points (host memory; from the first such call on)
+  ApiOut* api = nullptr;  // answers of the per-hop entry points and cluster statistics (api_buffer)
   bool settled = false;   // the last such call waited for the stream, and nothing was put on it since
   size_t smem = 0;
   int hop_grid = 0;
@@ -132,9 +132,9 @@ struct akmc_ctx {
   unsigned char* d_tmaps = nullptr;  // per job slot: two 128-byte tensor maps
   int32_t* d_flow = nullptr;  // flow_need[3], flow_done[3], flow_idle
   // cluster statistics scratch: list, parent, size (one int32 per site of the largest job
-  // measured so far), then n_list, the isolated count and the histogram
+  // measured so far) and the bits (one per site); then the counts (ClusterArgs::misc)
   int32_t* d_cl = nullptr;
-  int64_t cl_sites = 0;
+  int64_t cl_words = 0;
   unsigned long long* d_cl_misc = nullptr;
   // whole-context lattice transfers: staging buffer, chunk table, per-job vacancy counts,
   // density tiles of the EAM jobs (built at the first transfer)
@@ -245,7 +245,7 @@ void free_device(akmc_ctx* ctx) {
   dfree(ctx->stream, ctx->d_cl_misc);
   ctx->d_cl = nullptr;
   ctx->d_cl_misc = nullptr;
-  ctx->cl_sites = 0;
+  ctx->cl_words = 0;
   void* jl_ptrs[] = {ctx->d_stage, ctx->d_chunks, ctx->d_job_counts, ctx->d_job_want, ctx->d_tile0, ctx->d_eam_jobs};
   for (void* p : jl_ptrs) dfree(ctx->stream, p);
   ctx->d_stage = nullptr;
@@ -1681,6 +1681,16 @@ AKMC_API akmc_status akmc_get_counters(akmc_ctx* ctx, int64_t* out8) {
   return AKMC_OK;
 }
 
+// The host buffer that kernels answer in, from the first call that needs it on.
+static akmc_status api_buffer(akmc_ctx* ctx, ApiOut** dev) {
+  if (!ctx->api) {
+    CK(cudaHostAlloc(reinterpret_cast<void**>(&ctx->api), sizeof(ApiOut), cudaHostAllocMapped));
+    std::memset(ctx->api, 0, sizeof(ApiOut));
+  }
+  CK(cudaHostGetDevicePointer(reinterpret_cast<void**>(dev), ctx->api, 0));
+  return AKMC_OK;
+}
+
 // One per-hop step: one launch and one wait; the answer is in ctx->api.
 static akmc_status api_step(akmc_ctx* ctx, int32_t job, int32_t sector_id, int32_t mode, double u) {
   ctx->settled = false;
@@ -1690,10 +1700,6 @@ static akmc_status api_step(akmc_ctx* ctx, int32_t job, int32_t sector_id, int32
   if (j.nblocks != 1) return fail(ctx, AKMC_EINVAL, "the per-hop entry points drive single-domain jobs");
   if (sector_id < 0 || sector_id > 7) return fail(ctx, AKMC_EINVAL, "sector id in [0, 7]");
   CK(cudaSetDevice(ctx->cfg.device));
-  if (!ctx->api) {
-    CK(cudaHostAlloc(reinterpret_cast<void**>(&ctx->api), sizeof(ApiOut), cudaHostAllocMapped));
-    std::memset(ctx->api, 0, sizeof(ApiOut));
-  }
   RoundArgs a = ctx->args;
   a.mode = mode;
   a.api_job = job;
@@ -1701,7 +1707,8 @@ static akmc_status api_step(akmc_ctx* ctx, int32_t job, int32_t sector_id, int32
   a.api_vac0 = j.vac0;
   a.api_nvac = static_cast<int32_t>(j.nvac);
   a.api_u = u;
-  CK(cudaHostGetDevicePointer(reinterpret_cast<void**>(&a.api), ctx->api, 0));
+  const akmc_status st = api_buffer(ctx, &a.api);
+  if (st != AKMC_OK) return st;
   a.log_cap = 0;
   const int kind = j.cfg.energy_model == AKMC_MODEL_PAIRBOND ? 0 : j.cfg.precision == AKMC_FP32C ? 2 : 1;
   const int e = launch_api(a, kind, ctx->smem, ctx->stream);
@@ -1770,38 +1777,40 @@ AKMC_API akmc_status akmc_job_cluster_stats(akmc_ctx* ctx, int32_t job, int64_t*
   if (!live_job(ctx, job)) return AKMC_ENOTFOUND;
   const HostJob& j = ctx->jobs[static_cast<size_t>(job)];
   CK(cudaSetDevice(ctx->cfg.device));
-  if (ctx->cl_sites < j.nsites) {
-    CK(cudaStreamSynchronize(ctx->stream));
-    dfree(ctx->stream, ctx->d_cl);
-    ctx->d_cl = nullptr;
-    ctx->cl_sites = 0;
-    CK(dalloc(ctx->stream, &ctx->d_cl, static_cast<size_t>(3 * j.nsites)));
-    ctx->cl_sites = j.nsites;
-  }
-  if (!ctx->d_cl_misc) CK(dalloc(ctx->stream, &ctx->d_cl_misc, 2 + AKMC_CLUSTER_MAX_BINS));
   ClusterArgs c{};
-  c.occ = j.d_occ;
-  c.ns = j.nsites;
   c.sx = 2 * static_cast<int32_t>(j.cfg.box[0]);
   c.px = lattice_pitch(c.sx);
   c.sy = static_cast<int32_t>(j.cfg.box[1]);
   c.sz = static_cast<int32_t>(j.cfg.box[2]);
+  const int64_t words = 3 * j.nsites + cluster_words(c.sx, c.sy, c.sz);
+  if (ctx->cl_words < words) {
+    CK(cudaStreamSynchronize(ctx->stream));
+    dfree(ctx->stream, ctx->d_cl);
+    ctx->d_cl = nullptr;
+    ctx->cl_words = 0;
+    CK(dalloc(ctx->stream, &ctx->d_cl, static_cast<size_t>(words)));
+    ctx->cl_words = words;
+  }
+  if (!ctx->d_cl_misc) CK(dalloc(ctx->stream, &ctx->d_cl_misc, kClusterHist + AKMC_CLUSTER_MAX_BINS));
+  c.occ = j.d_occ;
   c.bins = hist_len > 0 ? static_cast<int32_t>(hist_len) : 1;
   c.list = ctx->d_cl;
   c.parent = ctx->d_cl + j.nsites;
   c.size = ctx->d_cl + 2 * j.nsites;
-  c.n_list = reinterpret_cast<unsigned int*>(ctx->d_cl_misc);
-  c.iso = ctx->d_cl_misc + 1;
-  c.hist = ctx->d_cl_misc + 2;
+  c.bits = reinterpret_cast<uint32_t*>(ctx->d_cl + 3 * j.nsites);
+  c.misc = ctx->d_cl_misc;
   c.status = ctx->d_status;
+  ApiOut* api = nullptr;
+  akmc_status st = api_buffer(ctx, &api);
+  if (st != AKMC_OK) return st;
+  c.out = api->cluster;
   const int e = launch_cluster_stats(c, ctx->stream);
   if (e) return fail(ctx, AKMC_ECUDA, std::string("launch: ") + cuda_name(e));
-  std::vector<unsigned long long> h(static_cast<size_t>(1 + c.bins));
-  CK(cudaMemcpyAsync(h.data(), c.iso, sizeof(unsigned long long) * h.size(), cudaMemcpyDeviceToHost, ctx->stream));
-  const akmc_status st = akmc_sync(ctx);
-  if (st != AKMC_OK) return st;
-  *isolated_cu = static_cast<int64_t>(h[0]);
-  for (int64_t k = 0; k < hist_len; ++k) hist[k] = static_cast<int64_t>(h[static_cast<size_t>(1 + k)]);
+  CK(cudaStreamSynchronize(ctx->stream));
+  const unsigned long long* const h = ctx->api->cluster;  // status, isolated atoms, histogram
+  if (h[0] && (st = check_status(ctx)) != AKMC_OK) return st;
+  *isolated_cu = static_cast<int64_t>(h[1]);
+  for (int64_t k = 0; k < hist_len; ++k) hist[k] = static_cast<int64_t>(h[2 + k]);
   return AKMC_OK;
 }
 

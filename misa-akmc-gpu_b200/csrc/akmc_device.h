@@ -162,8 +162,9 @@ enum : uint32_t {
 
 enum : int32_t { kModeRound = 0, kModeCalc = 1, kModeSelectPerform = 2 };
 
-// What a per-hop entry point answers, in host memory that the kernel writes: the caller waits for the stream and
-// reads it, without a copy.
+// What a per-hop entry point or the cluster statistics answer, in host memory that the kernels write: the caller
+// waits for the stream and reads it, without a copy.
+constexpr int kClusterHist = 2;
 struct ApiOut {
   double total;
   uint32_t status;
@@ -172,6 +173,7 @@ struct ApiOut {
   int32_t sites[kMaxV];     // their sites
   double de[kMaxV * 8];     // ΔE of each jump
   double rates[kMaxV * 8];  // its rates
+  unsigned long long cluster[2 + AKMC_CLUSTER_MAX_BINS];  // status, isolated atoms, histogram
 };
 
 struct RoundArgs {
@@ -269,19 +271,20 @@ int launch_load_jobs(const RoundArgs& a, const JobsLoad& L, void* stream);
 int launch_init_rho_jobs(const RoundArgs& a, const JobsLoad& L, void* stream);  // uses a.jobs, a.pots
 int launch_gather_jobs(const RoundArgs& a, const JobsLoad& L, void* stream);
 
-// Cu cluster statistics of one job's occupancy (akmc_cluster.cu).  list, parent and size hold
-// one int32 per site; iso and hist are cleared by the launch.
+// Cu cluster statistics of one job's occupancy (akmc_cluster.cu).  list, parent and size hold one int32 per site,
+// bits a bit per site in words of a row each; misc: the list's length and a ticket, the isolated atoms, then
+// the histogram (kClusterHist), all cleared by the launch; out: the status, the isolated atoms, the histogram.
+AK_HD int64_t cluster_words(int64_t sx, int64_t sy, int64_t sz) { return (sx + 31) / 32 * sy * sz; }
 struct ClusterArgs {
   const uint8_t* occ;  // halo layout
-  int64_t ns;
   int32_t sx, sy, sz, bins;
   int32_t px, pad;
+  uint32_t* bits;
   int32_t* list;
-  unsigned int* n_list;
   int32_t* parent;
   int32_t* size;
-  unsigned long long* iso;
-  unsigned long long* hist;
+  unsigned long long* misc;
+  unsigned long long* out;  // host memory
   unsigned int* status;
 };
 int launch_cluster_stats(const ClusterArgs& c, void* stream);
