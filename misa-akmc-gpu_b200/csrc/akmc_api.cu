@@ -100,6 +100,10 @@ struct akmc_ctx {
   // device state
   JobDev* d_jobs = nullptr;
   BlockDev* d_blocks = nullptr;
+  // the job and block records of round 0, in the second halves of d_jobs and d_blocks: a reloaded lattice starts
+  // from them by a copy on the device
+  JobDev* d_jobs0 = nullptr;
+  BlockDev* d_blocks0 = nullptr;
   int32_t* d_vac_site = nullptr;
   int32_t* d_vac_job = nullptr;
   int32_t* d_blk_list = nullptr;
@@ -276,6 +280,8 @@ void free_device(akmc_ctx* ctx) {
   for (void* p : ptrs) dfree(ctx->stream, p);
   ctx->d_jobs = nullptr;
   ctx->d_blocks = nullptr;
+  ctx->d_jobs0 = nullptr;
+  ctx->d_blocks0 = nullptr;
   ctx->d_vac_site = ctx->d_vac_job = ctx->d_blk_list = ctx->d_active = ctx->d_n_active = nullptr;
   ctx->d_pots = nullptr;
   ctx->d_geo = nullptr;
@@ -887,8 +893,10 @@ AKMC_API akmc_status akmc_prepare(akmc_ctx* ctx) {
   if (cb > nb) ctx->free_blocks.emplace_back(nb, cb);
   if (ctx->cap_vac > nv) ctx->free_vac.emplace_back(nv, ctx->cap_vac);
   const size_t ncap = static_cast<size_t>(cb);
-  CK(dalloc(ctx->stream, &ctx->d_jobs, hj.size()));
-  CK(dalloc(ctx->stream, &ctx->d_blocks, hb.size()));
+  CK(dalloc(ctx->stream, &ctx->d_jobs, 2 * hj.size()));
+  CK(dalloc(ctx->stream, &ctx->d_blocks, 2 * hb.size()));
+  ctx->d_jobs0 = ctx->d_jobs + hj.size();
+  ctx->d_blocks0 = ctx->d_blocks + hb.size();
   CK(dalloc(ctx->stream, &ctx->d_vac_site, vsite.size()));
   CK(dalloc(ctx->stream, &ctx->d_vac_job, vjob.size()));
   CK(dalloc(ctx->stream, &ctx->d_blk_list, ncap * kMaxV));
@@ -914,6 +922,8 @@ AKMC_API akmc_status akmc_prepare(akmc_ctx* ctx) {
   if (ctx->cfg.event_log_capacity > 0) CK(dalloc(ctx->stream, &ctx->d_log, static_cast<size_t>(ctx->cfg.event_log_capacity)));
   CK(cudaMemcpyAsync(ctx->d_jobs, hj.data(), hj.size() * sizeof(JobDev), cudaMemcpyHostToDevice, ctx->stream));
   CK(cudaMemcpyAsync(ctx->d_blocks, hb.data(), hb.size() * sizeof(BlockDev), cudaMemcpyHostToDevice, ctx->stream));
+  CK(cudaMemcpyAsync(ctx->d_jobs0, ctx->d_jobs, hj.size() * sizeof(JobDev), cudaMemcpyDeviceToDevice, ctx->stream));
+  CK(cudaMemcpyAsync(ctx->d_blocks0, ctx->d_blocks, hb.size() * sizeof(BlockDev), cudaMemcpyDeviceToDevice, ctx->stream));
   CK(cudaMemcpyAsync(ctx->d_vac_site, vsite.data(), vsite.size() * 4, cudaMemcpyHostToDevice, ctx->stream));
   CK(cudaMemcpyAsync(ctx->d_vac_job, vjob.data(), vjob.size() * 4, cudaMemcpyHostToDevice, ctx->stream));
   CK(cudaMemsetAsync(ctx->d_n_active, 0, 4, ctx->stream));
@@ -1027,9 +1037,10 @@ AKMC_API akmc_status akmc_admit_job(akmc_ctx* ctx, const akmc_job_config* cfg, c
   st = setup_job(ctx, slot, J, hb.data(), vsite.data(), vjob.data());
   if (st != AKMC_OK) return st;
   CK(cudaMemcpyAsync(ctx->d_tmaps + static_cast<size_t>(slot) * 256, h.tmap, 256, cudaMemcpyHostToDevice, ctx->stream));
-  CK(cudaMemcpyAsync(ctx->d_jobs + slot, &J, sizeof(J), cudaMemcpyHostToDevice, ctx->stream));
-  CK(cudaMemcpyAsync(ctx->d_blocks + h.block0, hb.data(), hb.size() * sizeof(BlockDev), cudaMemcpyHostToDevice,
-                     ctx->stream));
+  for (JobDev* p : {ctx->d_jobs, ctx->d_jobs0})
+    CK(cudaMemcpyAsync(p + slot, &J, sizeof(J), cudaMemcpyHostToDevice, ctx->stream));
+  for (BlockDev* p : {ctx->d_blocks, ctx->d_blocks0})
+    CK(cudaMemcpyAsync(p + h.block0, hb.data(), hb.size() * sizeof(BlockDev), cudaMemcpyHostToDevice, ctx->stream));
   if (h.nvac) {
     CK(cudaMemcpyAsync(ctx->d_vac_site + h.vac0, vsite.data(), vsite.size() * 4, cudaMemcpyHostToDevice, ctx->stream));
     CK(cudaMemcpyAsync(ctx->d_vac_job + h.vac0, vjob.data(), vjob.size() * 4, cudaMemcpyHostToDevice, ctx->stream));
@@ -1059,9 +1070,10 @@ AKMC_API akmc_status akmc_retire_job(akmc_ctx* ctx, int32_t job) {
   HostJob& h = ctx->jobs[static_cast<size_t>(job)];
   const JobDev J = free_job_record();
   const std::vector<BlockDev> hb(static_cast<size_t>(h.nblocks), free_block_record());
-  CK(cudaMemcpyAsync(ctx->d_jobs + job, &J, sizeof(J), cudaMemcpyHostToDevice, ctx->stream));
-  CK(cudaMemcpyAsync(ctx->d_blocks + h.block0, hb.data(), hb.size() * sizeof(BlockDev), cudaMemcpyHostToDevice,
-                     ctx->stream));
+  for (JobDev* p : {ctx->d_jobs, ctx->d_jobs0})
+    CK(cudaMemcpyAsync(p + job, &J, sizeof(J), cudaMemcpyHostToDevice, ctx->stream));
+  for (BlockDev* p : {ctx->d_blocks, ctx->d_blocks0})
+    CK(cudaMemcpyAsync(p + h.block0, hb.data(), hb.size() * sizeof(BlockDev), cudaMemcpyHostToDevice, ctx->stream));
   if (h.nvac) CK(cudaMemsetAsync(ctx->d_vac_job + h.vac0, 0xff, static_cast<size_t>(h.nvac) * 4, ctx->stream));
   dfree(ctx->stream, h.d_occ);
   dfree(ctx->stream, h.d_rho);
@@ -1096,10 +1108,9 @@ AKMC_API akmc_status akmc_load_occupancy(akmc_ctx* ctx, int32_t job, const uint8
                         ctx->stream);
     if (e) return fail(ctx, AKMC_ECUDA, std::string("init rho: ") + cuda_name(e));
   }
-  CK(cudaMemcpyAsync(ctx->d_jobs + job, &ctx->h_jobs[static_cast<size_t>(job)], sizeof(JobDev), cudaMemcpyHostToDevice,
-                     ctx->stream));
-  CK(cudaMemcpyAsync(ctx->d_blocks + j.block0, &ctx->h_blocks[static_cast<size_t>(j.block0)],
-                     static_cast<size_t>(j.nblocks) * sizeof(BlockDev), cudaMemcpyHostToDevice, ctx->stream));
+  CK(cudaMemcpyAsync(ctx->d_jobs + job, ctx->d_jobs0 + job, sizeof(JobDev), cudaMemcpyDeviceToDevice, ctx->stream));
+  CK(cudaMemcpyAsync(ctx->d_blocks + j.block0, ctx->d_blocks0 + j.block0, static_cast<size_t>(j.nblocks) * sizeof(BlockDev),
+                     cudaMemcpyDeviceToDevice, ctx->stream));
   return AKMC_OK;  // a wrong vacancy count is reported by the next synchronising call
 }
 
@@ -1305,10 +1316,9 @@ AKMC_API akmc_status akmc_load_occupancies(akmc_ctx* ctx, const uint8_t* occ, in
   CK(cudaMemcpyAsync(ctx->d_stage, occ, static_cast<size_t>(total_sites), cudaMemcpyHostToDevice, ctx->stream));
   const int e = launch_load_jobs(ctx->args, ctx->jl, ctx->stream);
   if (e) return fail(ctx, AKMC_ECUDA, std::string("load: ") + cuda_name(e));
-  CK(cudaMemcpyAsync(ctx->d_jobs, ctx->h_jobs.data(), ctx->h_jobs.size() * sizeof(JobDev), cudaMemcpyHostToDevice,
+  CK(cudaMemcpyAsync(ctx->d_jobs, ctx->d_jobs0, ctx->h_jobs.size() * sizeof(JobDev), cudaMemcpyDeviceToDevice, ctx->stream));
+  CK(cudaMemcpyAsync(ctx->d_blocks, ctx->d_blocks0, ctx->h_blocks.size() * sizeof(BlockDev), cudaMemcpyDeviceToDevice,
                      ctx->stream));
-  CK(cudaMemcpyAsync(ctx->d_blocks, ctx->h_blocks.data(), ctx->h_blocks.size() * sizeof(BlockDev),
-                     cudaMemcpyHostToDevice, ctx->stream));
   return AKMC_OK;  // a wrong vacancy count is reported by the next synchronising call
 }
 
@@ -1627,14 +1637,16 @@ AKMC_API akmc_status akmc_get_block_clocks(akmc_ctx* ctx, int32_t job, double* e
   const HostJob& j = ctx->jobs[static_cast<size_t>(job)];
   if (n_blocks != j.nblocks) return AKMC_EINVAL;
   if (!ctx->prepared) return fail(ctx, AKMC_ESTATE, "akmc_prepare first");
-  std::vector<BlockDev> hb(static_cast<size_t>(j.nblocks));
-  CK(cudaMemcpyAsync(hb.data(), ctx->d_blocks + j.block0, hb.size() * sizeof(BlockDev), cudaMemcpyDeviceToHost,
-                     ctx->stream));
+  CK(cudaSetDevice(ctx->cfg.device));
+  // gathered into the round-by-round schedule's list, which is filled anew in every round
+  double* const d_evo = reinterpret_cast<double*>(ctx->d_blk_list);
+  static_assert(kMaxV * sizeof(int32_t) >= 9 * sizeof(double), "nine words a block");
+  const int e = launch_gather_clocks(ctx->d_blocks + j.block0, n_blocks, d_evo, ctx->stream);
+  if (e) return fail(ctx, AKMC_ECUDA, std::string("launch: ") + cuda_name(e));
+  const size_t n = static_cast<size_t>(n_blocks);
+  CK(cudaMemcpyAsync(evo, d_evo, n * 8 * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
+  CK(cudaMemcpyAsync(hops, d_evo + 8 * n, n * sizeof(int64_t), cudaMemcpyDeviceToHost, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
-  for (int b = 0; b < j.nblocks; ++b) {
-    for (int k = 0; k < 8; ++k) evo[b * 8 + k] = hb[static_cast<size_t>(b)].evo[k];
-    hops[b] = hb[static_cast<size_t>(b)].hops;
-  }
   return AKMC_OK;
 }
 

@@ -269,6 +269,8 @@ struct JobsLoad {
 };
 int launch_load_jobs(const RoundArgs& a, const JobsLoad& L, void* stream);
 int launch_init_rho_jobs(const RoundArgs& a, const JobsLoad& L, void* stream);  // uses a.jobs, a.pots
+// n blocks' sector clocks (8 each), then their hops, packed into out.
+int launch_gather_clocks(const BlockDev* blocks, int32_t n, double* out, void* stream);
 int launch_gather_jobs(const RoundArgs& a, const JobsLoad& L, void* stream);
 
 // Cu cluster statistics of one job's occupancy (akmc_cluster.cu).  list, parent and size hold one int32 per site,

@@ -2733,6 +2733,15 @@ __global__ void k_check_counts(const int32_t* counts, const int32_t* want, int32
 }
 
 // Whole-context lattice read-back: the reverse copy into the staging buffer (rows of sx sites, an even number).
+// One thread a word: a read-out moves 72 bytes a block over PCIe, not its whole record.
+__global__ void k_gather_clocks(const BlockDev* __restrict__ blocks, int32_t n, double* __restrict__ out) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < 8 * n)
+    out[i] = blocks[i >> 3].evo[i & 7];
+  else if (i < 9 * n)
+    reinterpret_cast<int64_t*>(out)[i] = blocks[i - 8 * n].hops;
+}
+
 __global__ void k_gather(RoundArgs a, uint8_t* stage, const SiteChunk* chunks) {
   const SiteChunk c = chunks[blockIdx.x];
   const JobDev& J = a.jobs[c.job];
@@ -2841,6 +2850,10 @@ int configure_hop_smem(size_t smem) {
   return static_cast<int>(e);
 }
 
+int launch_gather_clocks(const BlockDev* blocks, int32_t n, double* out, void* stream) {
+  k_gather_clocks<<<(9 * n + 127) / 128, 128, 0, static_cast<cudaStream_t>(stream)>>>(blocks, n, out);
+  return static_cast<int>(cudaGetLastError());
+}
 int launch_init_rho(uint8_t* occ, int32_t* rho, int32_t sx, int32_t sy, int32_t sz, const Potential* pot,
                     const Geometry* geo, unsigned int* status, void* stream) {
   (void)status;

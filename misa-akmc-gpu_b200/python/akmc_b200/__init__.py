@@ -5,6 +5,7 @@ There is no CPU fallback: loading fails with an error when the library has not
 been built, and every non-zero status raises AkmcError.
 """
 import ctypes as C
+import math
 import os
 
 import numpy as np
@@ -317,7 +318,7 @@ def lib():
 
 
 def _ptr(a):
-    return a.ctypes.data_as(C.c_void_p)
+    return a.ctypes.data  # the callers hold the array during the call
 
 
 def _check(rc, ctx=None):
@@ -523,7 +524,10 @@ class Engine:
         return out
 
     def block_clocks(self, job=0):
-        nb = self.job_state(job)["n_blocks"]
+        if 0 <= job < len(self.jobs) and self.jobs[job] is not None:  # the device is not asked for it
+            nb = math.prod(max(1, b) for b in self.jobs[job][0].blocks)
+        else:
+            nb = self.job_state(job)["n_blocks"]
         evo = np.empty((nb, 8), np.float64)
         hops = np.empty(nb, np.int64)
         self._ck(lib().akmc_get_block_clocks(self.h, job, _ptr(evo), _ptr(hops), nb))
