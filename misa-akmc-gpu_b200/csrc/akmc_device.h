@@ -20,6 +20,7 @@ constexpr int kShellNb = 58;                      // neighbours within the 5-she
 constexpr int kNbrStride = 8;  // words per block of RoundArgs::nbr (one 32-byte sector)
 constexpr int kWordShift = 9;  // rounds in a block's word (RoundArgs::fstate)
 constexpr int kFlowSlots = 64;                    // vacancies held in one domain block's area
+constexpr int kSoloSlots = 512;                   // and in a context's only block (64 in each sector)
 
 // Packed neighbour entry: int8 dX | int8 dy << 8 | int8 dz << 16 | (sh_s | sh_t << 4) << 24,
 // dX in doubled-x site units; shell codes 0 = outside the cutoff, 1..5 shells, 6 = the site itself.
@@ -212,6 +213,7 @@ struct RoundArgs {
   int64_t flow_rounds;          // rounds this launch adds to every unfinished block
   int64_t flow_sweep_limit;     // sweeps per CTA before the launch gives up (kErrTimeout)
   int64_t time_budget_ns;       // > 0: the launch takes no new round after this long (akmc_run_for)
+  int32_t flow_slots;           // kFlowSlots, or kSoloSlots when the context holds one block
   int32_t flow_take;            // rounds with vacancies a CTA takes per sweep (0: by the idle CTAs)
   int32_t eval_warps;           // CTA shape of the hop kernels: 8 or 4 evaluator warps
   // per-hop entry points

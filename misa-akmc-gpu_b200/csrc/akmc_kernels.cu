@@ -226,7 +226,7 @@ struct Smem {
   JobDev job;              // the job of the running block (job_key: its index), copied when it changes
   int32_t job_key;
   int32_t fnv;             // vacancies of the running sector
-  int32_t fslot[kFlowSlots];  // and their slots (k_flow)
+  int32_t fslot[kMaxV];    // and their slots (k_flow)
   int32_t flow_ncand, flow_stop, flow_progress, flow_more;
   // run_block's clock thread: hops, n_act sum and evaluations of the block-round, selections made, the
   // sector's clock
@@ -1898,8 +1898,8 @@ __device__ __forceinline__ unsigned long long slot_word(int v, int32_t site) {
 // whole; a round of o that can see the vacancy waits for this block's round, which is published after both.
 __device__ void flow_give(const RoundArgs& a, int o, int v, int32_t site, int osec) {
   unsigned long long* const slots = a.vslot + static_cast<int64_t>(o) * kFlowSlots;
-  for (int k = 0; k < kFlowSlots; ++k) {
-    const int i = (v + k) & (kFlowSlots - 1);
+  for (int k = 0; k < a.flow_slots; ++k) {
+    const int i = (v + k) & (a.flow_slots - 1);
     if (atomicCAS(slots + i, kNoVacancy, slot_word(v, site)) == kNoVacancy) {
       atomicOr(&a.fstate[o], 2ull << osec);
       return;
@@ -2127,15 +2127,25 @@ __global__ void __launch_bounds__(Shape<W>::kThreads, Shape<W>::kCtasPerSm) k_fl
         int32_t* rho_s;
         carve(smem, R.n, sm, occ_s, rho_s);
         unsigned long long word = kNoVacancy;  // the block's vacancy slots, read while the region's copies are issued
-        if (tid < kFlowSlots) word = __ldcg(a.vslot + static_cast<int64_t>(gb) * kFlowSlots + tid);
+        const unsigned long long* const slots = a.vslot + static_cast<int64_t>(gb) * kFlowSlots;
+        constexpr int kReaders = kThreads - 32;  // not the last warp: the records' barrier leaves it out
+        static_assert(kReaders >= kFlowSlots, "one slot a thread at the usual number");
+        const int nslots = tid < kReaders ? a.flow_slots : 0;
+        if (tid < nslots) word = __ldcg(slots + tid);
         stage_region<KIND, W>(*sm, a, R, occ_s, rho_s);
-        if (tid < kFlowSlots && word != kNoVacancy) {
+        for (int k = tid; k < nslots; k += kReaders) {
+          if (k != tid) word = __ldcg(slots + k);
+          if (word == kNoVacancy) continue;
           const int32_t s = static_cast<int32_t>(word & 0xffffffffu);
           int X, y, z;
-          if (region_site(R, sm->job, s, X, y, z)) {
-            const int i = atomicAdd(&sm->fnv, 1);
-            sm->fslot[i] = tid;
+          if (!region_site(R, sm->job, s, X, y, z)) continue;
+          const int i = atomicAdd(&sm->fnv, 1);
+          if (i < kMaxV) {
+            sm->fslot[i] = k;
             put_record(*sm, R, i, static_cast<int>(word >> 32), s, X, y, z);
+          } else {  // more than a sector may hold
+            atomicSub(&sm->fnv, 1);
+            atomicOr(a.status, kErrVacOverflow);
           }
         }
 #ifdef AKMC_PHASE_PROFILE
@@ -2269,7 +2279,7 @@ __global__ void k_flow_slots(RoundArgs a) {
   int osec = 0;
   const int o = owner_sector(J, a.vac_site[v], &osec);
   const int slot = atomicAdd(&a.vcount[o], 1);
-  if (slot >= kFlowSlots) {
+  if (slot >= a.flow_slots) {
     atomicOr(a.status, kErrVacOverflow);
     return;
   }
@@ -2821,7 +2831,9 @@ int launch_flow_begin(const RoundArgs& a, int64_t n, void* stream) {
 int launch_flow(const RoundArgs& a, int grid, size_t smem, void* stream, void* ev0, void* ev1) {
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   cudaMemsetAsync(a.flow_need, 0, 7 * sizeof(int32_t), st);  // and flow_done, flow_idle behind it
-  cudaMemsetAsync(a.vslot, 0xff, static_cast<size_t>(a.nblocks) * kFlowSlots * sizeof(unsigned long long), st);
+  // (a context with one block uses the slots up to kSoloSlots past its first)
+  cudaMemsetAsync(a.vslot, 0xff,
+                  (static_cast<size_t>(a.nblocks - 1) * kFlowSlots + a.flow_slots) * sizeof(unsigned long long), st);
   k_flow_prep<<<(a.nblocks + 127) / 128, 128, 0, st>>>(a);
   if (a.nvac > 0) k_flow_slots<<<(a.nvac + 127) / 128, 128, 0, st>>>(a);
   if (ev0) cudaEventRecord(static_cast<cudaEvent_t>(ev0), st);
