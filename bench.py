@@ -737,7 +737,9 @@ def main():
     # once per step, then k_flow_prep, k_flow_slots, k_flow and k_flow_finalize
     sched = eng.round_schedule()
     sched_name = "flow" if sched == ak.SCHEDULE_FLOW else "rounds"
-    launches_per_step = (1 + 4 * ((R + 1023) // 1024)) if sched == ak.SCHEDULE_FLOW else 3 * R
+    # (one block's rounds run in one launch of that kernel under the automatic schedule)
+    persistent = sched == ak.SCHEDULE_FLOW or (args.workload == "serial" and args.schedule == "auto" and R >= 4)
+    launches_per_step = (1 + 4 * ((R + 1023) // 1024)) if persistent else 3 * R
 
     roofline = runner.roofline(eng, R, max(1, args.steps // 2), eam, args.workload)
     e_dt, e_hops, nbytes = runner.end_to_end(eng, lattices, R, args.steps, "e2e")

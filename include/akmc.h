@@ -209,7 +209,8 @@ AKMC_API akmc_status akmc_run_for(akmc_ctx* ctx, int64_t n_rounds, int64_t max_u
  * budget is checked inside the launch: the blocks of a multi-block budget job wait for one
  * another at each time-step boundary.  AUTO (default): FLOW when the context holds
  * more than one domain block and every block area starts with at most 32 vacancies, else
- * ROUNDS.  akmc_run_rounds_noalloc always runs ROUNDS. */
+ * ROUNDS.  For a context's only block the two are the same; under AUTO, reported as ROUNDS, a call
+ * of four rounds or more runs them in one launch.  akmc_run_rounds_noalloc always runs ROUNDS. */
 enum { AKMC_SCHEDULE_AUTO = 0, AKMC_SCHEDULE_ROUNDS = 1, AKMC_SCHEDULE_FLOW = 2 };
 AKMC_API akmc_status akmc_set_round_schedule(akmc_ctx* ctx, int32_t schedule);
 /* The schedule akmc_run_rounds uses (ROUNDS or FLOW), AUTO resolved; after akmc_prepare. */
@@ -237,11 +238,13 @@ AKMC_API akmc_status akmc_get_events(akmc_ctx* ctx, akmc_event* out, int64_t cap
  * [5] region sites staged into shared memory, [6] region sites written back, [7] reserved. */
 AKMC_API akmc_status akmc_get_counters(akmc_ctx* ctx, int64_t* out8);
 
-/* Cycle profile of the hop kernel's phases (thread 0, summed over blocks): [0] staging,
- * [1] list sort and table window, [2] first evaluations, [3] selection, [4] perform,
- * [5] re-evaluation and clock, [6] tail; EAM FP64 evaluation sub-phases: [8] site loop,
- * [9] butterfly, [10] own-embedding term, [11] rate.  All zero unless the library was
- * built with -DAKMC_PHASE_PROFILE. */
+/* Cycle profile of the hop kernels' phases (thread 0, summed over block-rounds): [0] staging,
+ * records and first draws, [1] the barrier after them, [2] the jump sums and rates (the first
+ * evaluation included), [4] dependency-driven: what precedes the hop loop (and, with several
+ * vacancies, selection and perform), [5] selection and dE terms, [6] tail, [7] dependency-driven:
+ * owner updates and publishing, [12] sweeps, [13] block-rounds, [14] number of sweeps, [15] of
+ * block-rounds; the others unused.  All zero unless the library was built with
+ * -DAKMC_PHASE_PROFILE. */
 AKMC_API akmc_status akmc_get_phase_cycles(akmc_ctx* ctx, int64_t* out16);
 
 /* Replaces the lattice of a prepared job (same box and vacancy count) and

@@ -12,7 +12,7 @@ The knobs, all of which leave every trajectory unchanged except the block edge (
 - threads per vacancy (eval_warps): the hop kernels evaluate a vacancy's 8 jumps with 8 warps
   (one jump each, one CTA per SM) or 4 warps (two jumps each, two CTAs per SM);
 - rounds per CTA (flow_take): how many ready rounds with vacancies a CTA of the
-  dependency-driven schedule takes per sweep (0: all it finds).
+  dependency-driven schedule takes per sweep (0: by how many CTAs are idle).
 
 The sector window is part of the model (3e-7 s, src/simulation.h:73-74), not a knob.
 
@@ -79,7 +79,7 @@ def tune_block_edge(jobs, lattices, eam, candidates=CANDIDATES, rounds=64, warmu
 
 
 def tune(jobs, lattices, eam, candidates=CANDIDATES, warps=WARPS, takes=TAKES, rounds=64, warmup=16, device=0):
-    """Staged search: the block edge with the default shape (8 warps, every round taken), then
+    """Staged search: the block edge with the default shape (8 warps, takes by the idle CTAs), then
     the other thread counts at that edge, then the round takes at the best (edge, warps).
     Returns ({"block_edge", "eval_warps", "flow_take"}, {"edge=E warps=W take=T": hops/s})."""
     edge, by_edge = tune_block_edge(jobs, lattices, eam, candidates, rounds, warmup, device)
