@@ -1728,6 +1728,7 @@ static akmc_status api_step(akmc_ctx* ctx, int32_t job, int32_t sector_id, int32
   a.mode = mode;
   a.api_job = job;
   a.api_sector = sector_id;
+  a.api_block = j.block0;
   a.api_vac0 = j.vac0;
   a.api_nvac = static_cast<int32_t>(j.nvac);
   a.api_u = u;

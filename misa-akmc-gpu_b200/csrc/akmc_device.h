@@ -218,7 +218,8 @@ struct RoundArgs {
   int32_t eval_warps;           // CTA shape of the hop kernels: 8 or 4 evaluator warps
   // per-hop entry points
   int32_t api_job, api_sector;
-  int32_t api_vac0, api_nvac;  // the job's slice of the vacancy table
+  int32_t api_block;           // the job's block
+  int32_t api_vac0, api_nvac;  // its slice of the vacancy table
   double api_u;
   ApiOut* api;
 };

@@ -2362,10 +2362,15 @@ __global__ void __launch_bounds__(Shape<8>::kThreads, 1) k_api(RoundArgs a) {
   Smem& sm0 = *reinterpret_cast<Smem*>(smem);
   const int tid = threadIdx.x;
   init_cta_smem(smem);
-  const int gb = a.jobs[a.api_job].block0;
-  load_block(sm0, a, gb, a.api_sector);
+  // one trip for the job's record, the block's and the vacancies' sites, not one each behind a barrier (a kernel of
+  // 8.0 us instead of 8.8 on 20^3 cells, pair bond)
+  int4 job = make_int4(0, 0, 0, 0);
+  if (tid < sizeof(JobDev) / 16) job = __ldcg(reinterpret_cast<const int4*>(a.jobs + a.api_job) + tid);
+  const int32_t first = tid < a.api_nvac ? __ldcg(a.vac_site + a.api_vac0 + tid) : 0;
+  load_block(sm0, a, a.api_block, a.api_sector);
+  if (tid < sizeof(JobDev) / 16) reinterpret_cast<int4*>(&sm0.job)[tid] = job;
   __syncthreads();
-  load_job(sm0, a, a.api_job);
+  if (tid == 0) sm0.job_key = a.api_job;
   Round& C = sm0.round[0];
   Region R;
   make_region(C.c0, C.c1, sm0.job, a.api_sector, R);
@@ -2375,7 +2380,7 @@ __global__ void __launch_bounds__(Shape<8>::kThreads, 1) k_api(RoundArgs a) {
   carve(smem, R.n, sm, occ_s, rho_s);
   for (int i = tid; i < a.api_nvac; i += kThreads) {
     const int v = a.api_vac0 + i;
-    const int32_t s = a.vac_site[v];
+    const int32_t s = i == tid ? first : a.vac_site[v];
     int X, y, z;
     if (!region_site(R, sm->job, s, X, y, z)) continue;
     const int k = atomicAdd(&sm->fnv, 1);
