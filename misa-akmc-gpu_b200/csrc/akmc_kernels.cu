@@ -2227,6 +2227,7 @@ __global__ void __launch_bounds__(Shape<W>::kThreads, Shape<W>::kCtasPerSm) k_fl
     cursor += watch;
     if (cursor >= nb) cursor %= nb;
   }
+  if (tid == 0 && idle) atomicAdd(a.flow_idle, -1);  // the next kind's kernel of the launch counts from zero
   cta_flush<W>(a, smem);
 #ifdef AKMC_PHASE_PROFILE
   if (tid == 0) {  // scheduler profile: [12] sweep cycles, [13] hop-loop cycles, [14] sweeps, [15] full rounds
