@@ -867,8 +867,12 @@ AKMC_API akmc_status akmc_prepare(akmc_ctx* ctx) {
   ctx->grid_resident = resident;
 
   // geometry and potentials
-  Geometry geo;
-  build_geometry(geo, 5);
+  // the lattice's tables depend on nothing else: built once (0.23 ms), by whichever thread comes first
+  static const Geometry geo = [] {
+    Geometry g;
+    build_geometry(g, 5);
+    return g;
+  }();
   CK(dalloc(ctx->stream, &ctx->d_geo, 1));
   CK(cudaMemcpyAsync(ctx->d_geo, &geo, sizeof(geo), cudaMemcpyHostToDevice, ctx->stream));
   std::vector<Potential> hp(ctx->pots.size());
