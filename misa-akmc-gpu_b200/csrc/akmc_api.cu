@@ -480,6 +480,27 @@ AKMC_API void* akmc_stream(akmc_ctx* ctx) { return ctx ? static_cast<void*>(ctx-
 
 namespace {
 
+// The first site from s on that holds a vacancy, n when there is none; a lattice of 33.5 M sites is searched at the
+// rate it is read (a byte at a time: 16 ms a pass).
+int64_t next_vacancy(const uint8_t* occ, int64_t s, int64_t n) {
+  const void* p = s < n ? std::memchr(occ + s, kV, static_cast<size_t>(n - s)) : nullptr;
+  return p ? static_cast<const uint8_t*>(p) - occ : n;
+}
+// The first site whose code is neither a vacancy nor an atom, n when there is none: such a code has a high bit or
+// two bits set, which a run of sites tests at once.
+int64_t first_invalid(const uint8_t* occ, int64_t n) {
+  static_assert(kV == 0 && kFe == 1 && kCu == 2 && kNi == 4 && kMn == 8, "one bit each");
+  constexpr int64_t kRun = 4096;
+  for (int64_t s0 = 0; s0 < n; s0 += kRun) {
+    const int64_t s1 = std::min(n, s0 + kRun);
+    uint8_t bad = 0;
+    for (int64_t s = s0; s < s1; ++s) bad |= static_cast<uint8_t>((occ[s] & (occ[s] - 1)) | (occ[s] & 0xf0));
+    for (int64_t s = s0; bad && s < s1; ++s)
+      if (occ[s] != kV && !is_atom(occ[s])) return s;
+  }
+  return n;
+}
+
 // A job's configuration and lattice checked and copied into j (akmc_add_job, akmc_admit_job).
 akmc_status check_job(akmc_ctx* ctx, const akmc_job_config* cfg, const uint8_t* occ, int64_t n_sites, HostJob& j) {
   j.cfg = *cfg;
@@ -510,10 +531,8 @@ akmc_status check_job(akmc_ctx* ctx, const akmc_job_config* cfg, const uint8_t* 
       return fail(ctx, AKMC_EINVAL, "the EAM path needs exactly the 5 BCC shells inside the cutoff");
   }
   j.occ.assign(occ, occ + n_sites);
-  for (int64_t s = 0; s < n_sites; ++s) {
-    if (occ[s] == kV) ++j.nvac;
-    else if (!is_atom(occ[s])) return fail(ctx, AKMC_EINVAL, "invalid occupancy code at site " + std::to_string(s));
-  }
+  const int64_t invalid = first_invalid(occ, n_sites);
+  if (invalid < n_sites) return fail(ctx, AKMC_EINVAL, "invalid occupancy code at site " + std::to_string(invalid));
   j.nblocks = (cfg->blocks[0] > 0 ? cfg->blocks[0] : 1) * (cfg->blocks[1] > 0 ? cfg->blocks[1] : 1) *
               (cfg->blocks[2] > 0 ? cfg->blocks[2] : 1);
   for (size_t k = 0; k + 1 < j.split[0].size(); ++k) {
@@ -524,8 +543,8 @@ akmc_status check_job(akmc_ctx* ctx, const akmc_job_config* cfg, const uint8_t* 
   // vacancies per block area (the dependency-driven schedule keeps each area's in 64 slots)
   std::vector<int32_t> per(static_cast<size_t>(j.nblocks), 0);
   const int nbx = static_cast<int>(j.split[0].size()) - 1, nby = static_cast<int>(j.split[1].size()) - 1;
-  for (int64_t s = 0; s < n_sites; ++s) {
-    if (occ[s] != kV) continue;
+  for (int64_t s = next_vacancy(occ, 0, n_sites); s < n_sites; s = next_vacancy(occ, s + 1, n_sites)) {
+    ++j.nvac;
     const int64_t X = s % (2 * cfg->box[0]), t = s / (2 * cfg->box[0]);
     const int64_t c[3] = {X >> 1, t % cfg->box[1], t / cfg->box[1]};
     int bi[3];
@@ -664,12 +683,11 @@ akmc_status setup_job(akmc_ctx* ctx, int32_t ji, JobDev& J, BlockDev* hb, int32_
     xoshiro_seed(B.xt, j.cfg.seed, kTagTime, static_cast<uint64_t>(b));
   }
   int32_t k = 0;
-  for (int64_t s = 0; s < j.nsites; ++s)
-    if (j.occ[static_cast<size_t>(s)] == kV) {
-      vsite[k] = static_cast<int32_t>(s);
-      vjob[k] = ji;
-      ++k;
-    }
+  for (int64_t s = next_vacancy(j.occ.data(), 0, j.nsites); s < j.nsites; s = next_vacancy(j.occ.data(), s + 1, j.nsites)) {
+    vsite[k] = static_cast<int32_t>(s);
+    vjob[k] = ji;
+    ++k;
+  }
   return AKMC_OK;
 }
 
