@@ -1132,16 +1132,23 @@ __device__ __forceinline__ int run_block(const RoundArgs& a, Smem& sm, Round& C,
       int it = 0, np = 1, meets = 0;
       if (lane == 0) path[0] = make_int2(s, gid);
       for (;; ++it) {
-        if (it > 0 && (it & (kDrawBatch - 1)) == 0) {  // the next batch of draws
-          asm volatile("bar.sync 2, 64;" ::: "memory");
-          ++meets;
-        }
         pair_rates(sm, occ_s, 0, s, R.LX, R.LX * R.LY, nullptr);
         __syncwarp();
         const double2* r = reinterpret_cast<const double2*>(sm.rates[0]);
         const double2 r2[4] = {r[0], r[1], r[2], r[3]};
-        const double u = sm.du[it & (kDrawRing - 1)];
         double total;
+        if (it > 0 && (it & (kDrawBatch - 1)) == 0) {
+          // the next batch of draws, once it is sure that one is used: the meeting lets warp 1 write over the
+          // batch before, which holds the streams' state after draw it - 1, the one a sector without events keeps
+          select_one(r2, 0.0, total);
+          if (fabs(total) < DBL_EPSILON) {
+            time = thr;
+            break;
+          }
+          asm volatile("bar.sync 2, 64;" ::: "memory");
+          ++meets;
+        }
+        const double u = sm.du[it & (kDrawRing - 1)];
         const int b = select_one(r2, u, total);
         if (fabs(total) < DBL_EPSILON) {  // sublattice.inl:108-112
           time = thr;
