@@ -283,7 +283,8 @@ AKMC_API akmc_status akmc_get_kernel_timing(akmc_ctx* ctx, double* hop_kernel_ms
  * sector loop, the RNG and the clock exactly as ABVIModel + SubLattice do.
  */
 /* calculate_GPU / first_calculate_GPU (gpu_simulate.h:33-35, gpu_simulate.hip:1211-1716):
- * rates of every vacancy in sector sector_id; returns their ordered sum. */
+ * rates of every vacancy in sector sector_id; returns their ordered sum.  A finished job has no
+ * events: 0, and akmc_select_and_perform selects none. */
 AKMC_API akmc_status akmc_calculate(akmc_ctx* ctx, int32_t job, int32_t sector_id, double* total);
 /* The jumps behind the last akmc_calculate, as the device vacancy records hold
  * them (d_vacancy_adv[].rates, gpu_simulate.hip:476-480): for each of the n_out

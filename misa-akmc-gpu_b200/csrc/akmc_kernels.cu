@@ -2386,7 +2386,8 @@ __global__ void __launch_bounds__(Shape<8>::kThreads, 1) k_api(RoundArgs a) {
   uint8_t* occ_s;
   int32_t* rho_s;
   carve(smem, R.n, sm, occ_s, rho_s);
-  for (int i = tid; i < a.api_nvac; i += kThreads) {
+  const int nvac = sm->job.done ? 0 : a.api_nvac;  // a finished job has no event left, as in the rounds
+  for (int i = tid; i < nvac; i += kThreads) {
     const int v = a.api_vac0 + i;
     const int32_t s = i == tid ? first : a.vac_site[v];
     int X, y, z;
