@@ -1775,11 +1775,6 @@ __device__ __forceinline__ unsigned long long ld_relaxed_u64(const unsigned long
   asm volatile("ld.relaxed.gpu.global.b64 %0, [%1];" : "=l"(v) : "l"(p));
   return v;
 }
-__device__ __forceinline__ unsigned int ld_relaxed_u32(const unsigned int* p) {
-  unsigned int v;
-  asm volatile("ld.relaxed.gpu.global.b32 %0, [%1];" : "=r"(v) : "l"(p));
-  return v;
-}
 
 __host__ __device__ constexpr int flow_sector(int phase) {
   constexpr int ring[8] = {0, 7, 2, 5, 3, 4, 1, 6};  // sector_of_round
@@ -1836,9 +1831,10 @@ __device__ int budget_gate(const RoundArgs& a, const JobDev& J, int64_t b) {
 constexpr int kNbrFree = 3, kNbrKindMask = 3, kNbrGate = 4, kNbrSolo = 8;
 
 // Whether the round the word w of block gb is at may run: the seven neighbours it meets have completed the rounds it
-// waits for.  Their words are read with relaxed loads, all in flight at once; the caller fences afterwards (an
-// acquire) before it reads what those rounds wrote.  Only the low halves are read: neighbours are within a few
-// rounds of each other, so the difference of 23 bits of the rounds is exact.
+// waits for.  Their words are read with relaxed loads, all in flight at once, as wide as every other access to them (the
+// loads pair with the publishing adds); the caller fences afterwards (an acquire) before it relies on anything those
+// rounds wrote.  Only the low halves are compared: neighbours are within a few rounds of each other, so the
+// difference of 23 bits of the rounds is exact.
 // Bounded by the SM's path to L2: a sweep of 256 blocks that read all 26 neighbours' words and a 128-byte row of
 // their indices took 2.5K cycles for the rows and 3.8K for the words (256^3 lattice). One 32-byte
 // sector and seven words, and empty rounds passed over in the word alone instead of under a lease with their
@@ -1852,7 +1848,7 @@ __device__ __forceinline__ bool flow_ready(const RoundArgs& a, int gb, unsigned 
 #pragma unroll
   for (int m = 1; m < 8; ++m) {
     o[m] = gb + (m & 1 ? d[0] : 0) + (m & 2 ? d[1] : 0) + (m & 4 ? d[2] : 0);
-    lo[m] = ld_relaxed_u32(reinterpret_cast<const unsigned int*>(&a.fstate[o[m]]));
+    lo[m] = static_cast<uint32_t>(ld_relaxed_u64(&a.fstate[o[m]]));
   }
   const uint32_t base = static_cast<uint32_t>(w) >> kWordShift << kWordShift;
   bool ok = true;
@@ -1957,7 +1953,7 @@ __device__ __forceinline__ bool flow_advance(const RoundArgs& a, Smem& sm, int g
   for (int k = 0; k < 4; ++k) st[k] = __ldcg(reinterpret_cast<const ulonglong2*>(B.xs) + k);
   const double evo = __ldcg(&B.evo[sec]);
   const int64_t step = __ldcg(&B.step[sec]);
-  const int nidle = __ldcg(a.flow_idle);
+  const int nidle = *reinterpret_cast<volatile int*>(a.flow_idle);
   const int64_t budget = J.hop_budget;
   const double window = J.window;
   if (budget > 0) {
@@ -2069,9 +2065,14 @@ __global__ void __launch_bounds__(Shape<W>::kThreads, Shape<W>::kCtasPerSm) k_fl
         // a multi-block job with a hop budget: its round at a time-step boundary waits for the job's
         // other blocks (a job that ends there is taken, to mark it)
         if (ok && (d1.z & kNbrGate) && budget_gate(a, a.jobs[d1.w], r) == 0) ok = false;
-        if (ok && !(d1.z & (kNbrSolo | kNbrGate)) && !((w >> (1 + sector_of_round(r))) & 1ull)) {
+        const bool empty = !(d1.z & kNbrSolo) && !((w >> (1 + sector_of_round(r))) & 1ull);
+        // A neighbour that carried a vacancy into this sector marked it in the word before it published the round that
+        // flow_ready saw.  The fence orders the two for this thread, so that the compare-and-swap below finds the mark
+        // and fails, whatever w was read as.  (It costs 1-2%: 256^3 lattice, 1024 rounds, 23.9 ms; 23.3-23.8 without.)
+        if (ok && empty) fence_acq_rel();
+        if (ok && empty && !(d1.z & kNbrGate)) {
           // no vacancy: the round is passed over, and the block keeps the lease bit at its target.  Nothing is read
-          // or written but the word, so there is nothing to fence: rounds that read what this block's or its
+          // or written but the word, so nothing else is fenced: rounds that read what this block's or its
           // neighbours' rounds wrote wait for those blocks themselves.
           const bool end = r + 1 >= target;
           if (atomicCAS(&a.fstate[gb], w, w + (1ull << kWordShift) + (end ? 1 : 0)) == w) {
@@ -2138,10 +2139,10 @@ __global__ void __launch_bounds__(Shape<W>::kThreads, Shape<W>::kCtasPerSm) k_fl
         constexpr int kReaders = kThreads - 32;  // not the last warp: the records' barrier leaves it out
         static_assert(kReaders >= kFlowSlots, "one slot a thread at the usual number");
         const int nslots = tid < kReaders ? a.flow_slots : 0;
-        if (tid < nslots) word = __ldcg(slots + tid);
+        if (tid < nslots) word = ld_relaxed_u64(slots + tid);  // a neighbour may be filling another of them
         stage_region<KIND, W>(*sm, a, R, occ_s, rho_s);
         for (int k = tid; k < nslots; k += kReaders) {
-          if (k != tid) word = __ldcg(slots + k);
+          if (k != tid) word = ld_relaxed_u64(slots + k);
           if (word == kNoVacancy) continue;
           const int32_t s = static_cast<int32_t>(word & 0xffffffffu);
           int X, y, z;
