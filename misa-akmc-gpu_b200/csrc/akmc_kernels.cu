@@ -177,8 +177,8 @@ constexpr int kDrawBatch = 8, kDrawRing = 2 * kDrawBatch;
 
 // Shared-memory working set of one CTA (followed by the staged region).
 struct Smem {
-  double e0[9];                 // migration energy prefactor by the moving atom's code
-  double b1[9 * 5], b2[9 * 5];  // pair-bond energies by the neighbour's code and the source's bond index
+  double e0[9];                   // migration energy prefactor by the moving atom's code
+  double b1[9 * 5], b2[9 * 5];    // pair-bond energies by the neighbour's code and the source's bond index
   union {                       // phi_XY(shell s) - phi_XY(shell t), index (X*4+Y)*64 + s*8 + t,
     double dphi64[4 * 4 * 64];  // in the precision of the kernel's kind
     float dphi32[4 * 4 * 64];
@@ -239,6 +239,12 @@ struct Smem {
   int32_t acc_job;
   unsigned long long acc_job_hops;
 };
+
+// A reloaded lattice may hold codes above 8, which no table has a row for: what is looked up for them as neighbours
+// lies within the working set.
+static_assert(offsetof(Smem, b2) + sizeof(double) * (255 * 5 + 5) <= sizeof(Smem) &&
+                  offsetof(Smem, dphi64) + sizeof(double) * ((3 * 4 + 96 + 1) * 64) <= sizeof(Smem),
+              "codes up to 255 (atom_index 96)");
 
 // --- bulk copy global -> shared with an mbarrier (cp.async.bulk, TMA unit) -----------
 __device__ __forceinline__ uint32_t smem_u32(const void* p) {
@@ -310,11 +316,10 @@ __device__ void load_tables(Smem& sm, const Potential& P, const Geometry& G, con
   }
   if (tid < 9) sm.e0[tid] = e0_of(static_cast<uint8_t>(tid));
   if (!eam) {
-    if (tid < 45) {  // codes 0, 1, 2, 4, 8 have a bond index; the other rows are never read
+    if (tid < 45) {  // codes that are no atom's (a reloaded lattice may hold some) bind as a vacancy
       const int code = tid / 5, i = tid % 5;
-      const bool used = (code & (code - 1)) == 0;
-      sm.b1[tid] = used ? P.b1[bond_index(static_cast<uint8_t>(code))][i] : 0.0;
-      sm.b2[tid] = used ? P.b2[bond_index(static_cast<uint8_t>(code))][i] : 0.0;
+      sm.b1[tid] = P.b1[bond_index(static_cast<uint8_t>(code))][i];
+      sm.b2[tid] = P.b2[bond_index(static_cast<uint8_t>(code))][i];
     }
     return;
   }
@@ -421,13 +426,18 @@ __device__ __forceinline__ FCell32 cell32(const FTab& T, int32_t r) {
   return c;
 }
 
-// The rate of a jump with energy change dE of atom Xc (0: the target is a vacancy), into the record of
-// vacancy k and jump b.
+// Codes 1, 2, 4 and 8 (the mask's bits), or 2, 4 and 8: one test, without a compare for each.
+__device__ __forceinline__ bool code_in(uint8_t c, uint32_t mask) { return c <= kMn && ((mask >> c) & 1u) != 0; }
+constexpr uint32_t kAtoms = 1u << kFe | 1u << kCu | 1u << kNi | 1u << kMn, kSolutes = kAtoms & ~(1u << kFe);
+
+// The rate of a jump with energy change dE onto a site with code Xc, into the record of vacancy k and jump b: 0 onto a
+// vacancy and onto a code that is no atom's (a reloaded lattice may hold some).
 __device__ __forceinline__ void put_rate(Smem& sm, int k, int b, uint8_t Xc, double dE, double* de_out) {
-  const double rate = arrhenius_rk(sm.job.nu, sm.job.kT, sm.job.rkT, sm.e0[Xc], dE);
-  sm.rates[k][b] = Xc ? rate : 0.0;
+  const bool atom = code_in(Xc, kAtoms);
+  const double rate = arrhenius_rk(sm.job.nu, sm.job.kT, sm.job.rkT, sm.e0[atom ? Xc : 0], dE);
+  sm.rates[k][b] = atom ? rate : 0.0;
   sm.vX[k][b] = Xc;
-  if (de_out) de_out[k * 8 + b] = Xc ? dE : 0.0;  // akmc_calculate only
+  if (de_out) de_out[k * 8 + b] = atom ? dE : 0.0;  // akmc_calculate only
 }
 
 // Pair bond: the rates of vacancy k at local site l, by one warp.  Lanes 4 b + 0..3 run the four bond
@@ -556,7 +566,7 @@ __device__ __forceinline__ void foot_terms(Smem& sm, int set, const uint8_t* occ
 }
 
 // Rates of jumps 4 half .. 4 half + 3 of vacancy k at local site l from term set `set`, by one warp, for
-// Fe targets and vacant ones; the other atoms' jumps are left to solute_rate.  Eight lanes take a jump:
+// Fe targets and those that hold no atom; solutes' jumps are left to solute_rate.  Eight lanes take a jump:
 // lane sub the partial sums sub + 8 g (g = 0..3) of the 32 interleaved ones (entries i = q, q + 32, q + 64
 // of the jump's list; ix: their terms, 10 bits each), merged in the order of the 32-lane xor butterfly
 // (16, 8, 4, 2, 1).  A vacancy's site adds 0.0, which leaves every partial sum as it is: a sum that
@@ -610,18 +620,17 @@ __device__ __forceinline__ void jump_rates(Smem& sm, int set, const uint8_t* occ
     }
     dE = static_cast<double>(EX + (x.s - x.c));
   }
-  if ((lane & 7) == 0 && Xc <= kFe) put_rate(sm, k, b, Xc, dE, de_out);
+  if ((lane & 7) == 0 && !code_in(Xc, kSolutes)) put_rate(sm, k, b, Xc, dE, de_out);
 }
 
-// Rate of jump b of vacancy k at local site l with a solute target (the shared terms are those of a
-// moving Fe atom), by one warp; nothing for other targets.  Lane q sums sites i = q, q + 32, q + 64 of the
-// jump's list (jl: the list's packed entries); the 32 partials merge by a xor butterfly (16, 8, 4, 2, 1),
-// then the moving atom's own embedding change is added.
 // Jumps of the vacancy at local site l whose target holds a solute, one bit each; all lanes of a warp.
 __device__ __forceinline__ unsigned solute_jumps(const Smem& sm, const uint8_t* occ_s, int l) {
   const int lane = threadIdx.x & 31;
-  return __ballot_sync(kFull, lane < 8 && occ_s[l + sm.d1[8 * (l & 1) + (lane & 7)].x] > kFe);
+  return __ballot_sync(kFull, lane < 8 && code_in(occ_s[l + sm.d1[8 * (l & 1) + (lane & 7)].x], kSolutes));
 }
+// Rate of jump b of vacancy k at local site l with a solute target (solute_jumps; the shared terms are those of a
+// moving Fe atom), by one warp.  Lane q sums sites i = q, q + 32, q + 64 of the jump's list; the 32 partials merge
+// by a xor butterfly (16, 8, 4, 2, 1), then the moving atom's own embedding change is added.
 template <int KIND>
 __device__ __forceinline__ void solute_rate(Smem& sm, const uint8_t* occ_s, const int32_t* rho_s, int k, int l, int b,
                                             const Region& R, const Geometry& G, const FTab& FT, double* de_out) {
@@ -629,7 +638,6 @@ __device__ __forceinline__ void solute_rate(Smem& sm, const uint8_t* occ_s, cons
   const int p = l & 1;
   const int tl = l + sm.d1[8 * p + b].x;
   const uint8_t Xc = occ_s[tl];
-  if (Xc <= kFe) return;  // uniform: Fe, or a vacancy
   const int X = atom_index(Xc);
   uint8_t o[3];
   int32_t r0[3], r1[3];
