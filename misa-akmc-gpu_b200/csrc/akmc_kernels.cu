@@ -359,20 +359,21 @@ __device__ void load_tables(Smem& sm, const Potential& P, const Geometry& G, con
 }
 
 
-// Cells outside the shared-memory window (rare): global memory, range-checked.
+// Cells outside the shared-memory window (rare): global memory, range-checked.  status null: a density off the table is
+// no error (the nearest end cell stands in).
 __device__ __noinline__ double F64_far(const double2* g64lo, const double2* g64hi, unsigned int* status, int32_t r,
                                        double p) {
   const int k = r >> kRhoCellShift;
   int kc = k;
   if (r < 0 || k > kTabN - 2) {
-    atomicOr(status, kErrRhoRange);
+    if (status) atomicOr(status, kErrRhoRange);
     kc = r < 0 ? 0 : kTabN - 2;
   }
   const double2 lo = __ldg(g64lo + kc), hi = __ldg(g64hi + kc);
   return cubic_d(lo.x, lo.y, hi.x, hi.y, p);
 }
 
-__device__ __forceinline__ double F64(const FTab& T, int32_t r) {
+__device__ __forceinline__ double F64(const FTab& T, int32_t r, unsigned int* status) {
   const int k = r >> kRhoCellShift;
   // p = (r mod 2^17) * 2^-17, built in the exponent field: 1 + m 2^-17 minus 1 (both exact)
   const double p = __hiloint2double(0x3FF00000 | ((r & kRhoFracMask) << 3), 0) - 1.0;
@@ -382,7 +383,7 @@ __device__ __forceinline__ double F64(const FTab& T, int32_t r) {
     const double2 hi = reinterpret_cast<const double2*>(T.win)[kFWin + kk];
     return cubic_d(lo.x, lo.y, hi.x, hi.y, p);
   }
-  return F64_far(T.pot->F64lo, T.pot->F64hi, T.status, r, p);
+  return F64_far(T.pot->F64lo, T.pot->F64hi, status, r, p);
 }
 
 // A cell known to lie inside the shared-memory window.
@@ -403,7 +404,7 @@ __device__ __forceinline__ FCell32 cell32win(const FTab& T, int32_t r) {
   return c;
 }
 
-__device__ __forceinline__ FCell32 cell32(const FTab& T, int32_t r) {
+__device__ __forceinline__ FCell32 cell32(const FTab& T, int32_t r, unsigned int* status) {
   const int k = r >> kRhoCellShift;
   const unsigned kk = static_cast<unsigned>(k - T.kw0);
   float4 a;
@@ -414,7 +415,7 @@ __device__ __forceinline__ FCell32 cell32(const FTab& T, int32_t r) {
   } else {
     int kc = k;
     if (r < 0 || k > kTabN - 2) {
-      atomicOr(T.status, kErrRhoRange);
+      if (status) atomicOr(status, kErrRhoRange);
       kc = r < 0 ? 0 : kTabN - 2;
     }
     a = __ldg(T.pot->F32a + kc);
@@ -526,6 +527,10 @@ __device__ __forceinline__ void foot_terms(Smem& sm, int set, const uint8_t* occ
   static_assert((kFWin & (kFWin - 1)) == 0, "one test for both cells");
   const bool win = static_cast<unsigned>(((rA >> kRhoCellShift) - FT.kw0) | ((rB >> kRhoCellShift) - FT.kw0)) <
                    static_cast<unsigned>(kFWin);
+  // A density itself is range-checked (hA = 0).  The terms are not: one that a jump of a Fe atom uses cannot leave the
+  // table when the density does not (the atom's own share is part of it), and one that no jump uses, its target being
+  // another atom or a vacancy, may: nothing reads it.
+  unsigned int* const status = c.hA == 0 ? FT.status : nullptr;
   const bool atom = o != kV;
   const int y = atom ? atom_index(static_cast<uint8_t>(o)) * 64 : 0;
   if (KIND == kEam64) {
@@ -534,8 +539,8 @@ __device__ __forceinline__ void foot_terms(Smem& sm, int set, const uint8_t* occ
       FA = F64win(FT, rA);
       FB = F64win(FT, rB);
     } else {
-      FA = F64(FT, rA);
-      FB = F64(FT, rB);
+      FA = F64(FT, rA, status);
+      FB = F64(FT, rB, nullptr);
     }
     const double F0 = __shfl_sync(kFull, FA, lead);
     const double tA = (FA - F0) + sm.dphi64[y + c.hA], tB = (FB - F0) + sm.dphi64[y + c.hB];
@@ -549,8 +554,8 @@ __device__ __forceinline__ void foot_terms(Smem& sm, int set, const uint8_t* occ
       a = F32part(cell32win(FT, rA), rA);
       bb = F32part(cell32win(FT, rB), rB);
     } else {
-      a = F32part(cell32(FT, rA), rA);
-      bb = F32part(cell32(FT, rB), rB);
+      a = F32part(cell32(FT, rA, status), rA);
+      bb = F32part(cell32(FT, rB, nullptr), rB);
     }
     F32Val f0;
     f0.hi = __shfl_sync(kFull, a.hi, lead);
@@ -670,9 +675,9 @@ __device__ __forceinline__ void solute_rate(Smem& sm, const uint8_t* occ_s, cons
 #pragma unroll
       for (int u = 0; u < 3; ++u) t[u] = in[u] ? F64win(FT, r1[u]) - F64win(FT, r0[u]) : 0.0;
     } else {
-      EX = F64(FT, rx1) - F64(FT, rx0);
+      EX = F64(FT, rx1, FT.status) - F64(FT, rx0, FT.status);
 #pragma unroll
-      for (int u = 0; u < 3; ++u) t[u] = in[u] ? F64(FT, r1[u]) - F64(FT, r0[u]) : 0.0;
+      for (int u = 0; u < 3; ++u) t[u] = in[u] ? F64(FT, r1[u], FT.status) - F64(FT, r0[u], FT.status) : 0.0;
     }
     // site term (F(r+d) - F(r)) + (phi_s - phi_t), summed in list order
     double acc = 0.0;
@@ -689,9 +694,9 @@ __device__ __forceinline__ void solute_rate(Smem& sm, const uint8_t* occ_s, cons
 #pragma unroll
       for (int u = 0; u < 3; ++u) t[u] = in[u] ? dF32(cell32win(FT, r1[u]), cell32win(FT, r0[u]), r1[u], r0[u]) : 0.f;
     } else {
-      EX = dF32(cell32(FT, rx1), cell32(FT, rx0), rx1, rx0);
+      EX = dF32(cell32(FT, rx1, FT.status), cell32(FT, rx0, FT.status), rx1, rx0);
 #pragma unroll
-      for (int u = 0; u < 3; ++u) t[u] = in[u] ? dF32(cell32(FT, r1[u]), cell32(FT, r0[u]), r1[u], r0[u]) : 0.f;
+      for (int u = 0; u < 3; ++u) t[u] = in[u] ? dF32(cell32(FT, r1[u], FT.status), cell32(FT, r0[u], FT.status), r1[u], r0[u]) : 0.f;
     }
     Comp32 acc;
     acc.s = 0.f;
