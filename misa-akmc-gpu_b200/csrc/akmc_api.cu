@@ -115,7 +115,8 @@ struct akmc_ctx {
   unsigned long long* d_log_count = nullptr;
   unsigned int* d_status = nullptr;
   unsigned long long* d_counters = nullptr;
-  ApiOut* api = nullptr;  // answers of the per-hop entry points and cluster statistics (api_buffer)
+  ApiOut* d_api = nullptr;  // the answer of a per-hop entry point on the device
+  ApiOut api{};             // and here, the last akmc_calculate's rates among it
   bool settled = false;   // the last such call waited for the stream, and nothing was put on it since
   size_t smem = 0;
   int hop_grid = 0;
@@ -137,7 +138,7 @@ struct akmc_ctx {
   unsigned char* d_tmaps = nullptr;  // per job slot: two 128-byte tensor maps
   int32_t* d_flow = nullptr;  // flow_need[3], flow_done[3], flow_idle
   // cluster statistics scratch: list, parent, size (one int32 per site of the largest job
-  // measured so far) and the bits (one per site); then the counts (ClusterArgs::misc)
+  // measured so far) and the bits (one per site); then the counts (ClusterArgs::misc) and the answer
   int32_t* d_cl = nullptr;
   int64_t cl_words = 0;
   unsigned long long* d_cl_misc = nullptr;
@@ -277,7 +278,7 @@ void free_device(akmc_ctx* ctx) {
   }
   void* ptrs[] = {ctx->d_jobs, ctx->d_blocks, ctx->d_vac_site, ctx->d_vac_job, ctx->d_blk_list, ctx->d_active,
                   ctx->d_n_active, ctx->d_pots, ctx->d_geo, ctx->d_log, ctx->d_log_count, ctx->d_status,
-                  ctx->d_counters};
+                  ctx->d_counters, ctx->d_api};
   for (void* p : ptrs) dfree(ctx->stream, p);
   ctx->d_jobs = nullptr;
   ctx->d_blocks = nullptr;
@@ -290,8 +291,7 @@ void free_device(akmc_ctx* ctx) {
   ctx->d_log_count = nullptr;
   ctx->d_status = nullptr;
   ctx->d_counters = nullptr;
-  if (ctx->api) cudaFreeHost(ctx->api);
-  ctx->api = nullptr;
+  ctx->d_api = nullptr;
   ctx->prepared = false;
 }
 
@@ -943,6 +943,8 @@ AKMC_API akmc_status akmc_prepare(akmc_ctx* ctx) {
   }
   CK(dalloc(ctx->stream, &ctx->d_flow, 7));
   CK(dalloc(ctx->stream, &ctx->d_log_count, 1));
+  CK(dalloc(ctx->stream, &ctx->d_api, 1));
+  CK(cudaMemsetAsync(ctx->d_api, 0, sizeof(ApiOut), ctx->stream));
   if (ctx->cfg.event_log_capacity > 0) CK(dalloc(ctx->stream, &ctx->d_log, static_cast<size_t>(ctx->cfg.event_log_capacity)));
   CK(cudaMemcpyAsync(ctx->d_jobs, hj.data(), hj.size() * sizeof(JobDev), cudaMemcpyHostToDevice, ctx->stream));
   CK(cudaMemcpyAsync(ctx->d_blocks, hb.data(), hb.size() * sizeof(BlockDev), cudaMemcpyHostToDevice, ctx->stream));
@@ -1727,17 +1729,10 @@ AKMC_API akmc_status akmc_get_counters(akmc_ctx* ctx, int64_t* out8) {
   return AKMC_OK;
 }
 
-// The host buffer that kernels answer in, from the first call that needs it on.
-static akmc_status api_buffer(akmc_ctx* ctx, ApiOut** dev) {
-  if (!ctx->api) {
-    CK(cudaHostAlloc(reinterpret_cast<void**>(&ctx->api), sizeof(ApiOut), cudaHostAllocMapped));
-    std::memset(ctx->api, 0, sizeof(ApiOut));
-  }
-  CK(cudaHostGetDevicePointer(reinterpret_cast<void**>(dev), ctx->api, 0));
-  return AKMC_OK;
-}
-
-// One per-hop step: one launch and one wait; the answer is in ctx->api.
+// One per-hop step: one launch and one copy, which waits; the answer is in ctx->api.  akmc_calculate on 20^3 cells takes
+// 31 us so, from a context's first call on, against 53 with three launches and two copies (and 105 the first).  A kernel
+// that answers in mapped host memory saves 8 to 12 us of copy, but pinning that memory takes 1.5 to 2.3 ms, and giving
+// it back 0.4 ms and a wait for everything that runs on the device.
 static akmc_status api_step(akmc_ctx* ctx, int32_t job, int32_t sector_id, int32_t mode, double u) {
   ctx->settled = false;
   if (!ctx->prepared) return fail(ctx, AKMC_ESTATE, "akmc_prepare first");
@@ -1754,21 +1749,22 @@ static akmc_status api_step(akmc_ctx* ctx, int32_t job, int32_t sector_id, int32
   a.api_vac0 = j.vac0;
   a.api_nvac = static_cast<int32_t>(j.nvac);
   a.api_u = u;
-  const akmc_status st = api_buffer(ctx, &a.api);
-  if (st != AKMC_OK) return st;
+  a.api = ctx->d_api;
   a.log_cap = 0;
   const int kind = j.cfg.energy_model == AKMC_MODEL_PAIRBOND ? 0 : j.cfg.precision == AKMC_FP32C ? 2 : 1;
   const int e = launch_api(a, kind, ctx->smem, ctx->stream);
   if (e) return fail(ctx, AKMC_ECUDA, std::string("launch: ") + cuda_name(e));
-  CK(cudaStreamSynchronize(ctx->stream));
+  // into pageable memory: the call returns when the copy, hence the kernel, is done
+  CK(cudaMemcpyAsync(&ctx->api, ctx->d_api, mode == kModeCalc ? sizeof(ApiOut) : offsetof(ApiOut, sites),
+                     cudaMemcpyDeviceToHost, ctx->stream));
   ctx->settled = true;
-  return ctx->api->status ? check_status(ctx) : AKMC_OK;  // errors of the step and of earlier asynchronous calls
+  return ctx->api.status ? check_status(ctx) : AKMC_OK;  // errors of the step and of earlier asynchronous calls
 }
 
 AKMC_API akmc_status akmc_calculate(akmc_ctx* ctx, int32_t job, int32_t sector_id, double* total) {
   if (!ctx || !total) return AKMC_EINVAL;
   const akmc_status s = api_step(ctx, job, sector_id, kModeCalc, 0.0);
-  if (ctx->settled) *total = ctx->api->total;
+  if (ctx->settled) *total = ctx->api.total;
   return s;
 }
 
@@ -1778,14 +1774,14 @@ AKMC_API akmc_status akmc_get_calculated_rates(akmc_ctx* ctx, int32_t* sites, do
   *n_out = 0;
   if (!ctx->prepared) return fail(ctx, AKMC_ESTATE, "akmc_prepare first");
   CK(cudaSetDevice(ctx->cfg.device));
-  const ApiOut* o = ctx->api;
-  const int32_t n = o ? o->count : 0;
+  const ApiOut& o = ctx->api;
+  const int32_t n = o.count;
   *n_out = n;
   if (n > capacity) return fail(ctx, AKMC_EINVAL, "capacity below the sector's vacancy count");
   if (n == 0) return AKMC_OK;
-  std::memcpy(sites, o->sites, sizeof(int32_t) * static_cast<size_t>(n));
-  std::memcpy(delta_e, o->de, sizeof(double) * 8 * static_cast<size_t>(n));
-  std::memcpy(rates, o->rates, sizeof(double) * 8 * static_cast<size_t>(n));
+  std::memcpy(sites, o.sites, sizeof(int32_t) * static_cast<size_t>(n));
+  std::memcpy(delta_e, o.de, sizeof(double) * 8 * static_cast<size_t>(n));
+  std::memcpy(rates, o.rates, sizeof(double) * 8 * static_cast<size_t>(n));
   return ctx->settled ? AKMC_OK : akmc_sync(ctx);  // errors of calls since the last per-hop one
 }
 
@@ -1793,7 +1789,7 @@ AKMC_API akmc_status akmc_select_and_perform(akmc_ctx* ctx, int32_t job, int32_t
                                              akmc_event* ev) {
   if (!ctx || !ev) return AKMC_EINVAL;
   const akmc_status s = api_step(ctx, job, sector_id, kModeSelectPerform, u);
-  if (ctx->settled) *ev = ctx->api->event;
+  if (ctx->settled) *ev = ctx->api.event;
   return s;
 }
 
@@ -1838,7 +1834,9 @@ AKMC_API akmc_status akmc_job_cluster_stats(akmc_ctx* ctx, int32_t job, int64_t*
     CK(dalloc(ctx->stream, &ctx->d_cl, static_cast<size_t>(words)));
     ctx->cl_words = words;
   }
-  if (!ctx->d_cl_misc) CK(dalloc(ctx->stream, &ctx->d_cl_misc, kClusterHist + AKMC_CLUSTER_MAX_BINS));
+  // what the kernels count in, then their answer: the status, the isolated atoms, the histogram
+  constexpr int kCounts = kClusterHist + AKMC_CLUSTER_MAX_BINS;
+  if (!ctx->d_cl_misc) CK(dalloc(ctx->stream, &ctx->d_cl_misc, 2 * kCounts));
   c.occ = j.d_occ;
   c.bins = hist_len > 0 ? static_cast<int32_t>(hist_len) : 1;
   c.list = ctx->d_cl;
@@ -1847,17 +1845,18 @@ AKMC_API akmc_status akmc_job_cluster_stats(akmc_ctx* ctx, int32_t job, int64_t*
   c.bits = reinterpret_cast<uint32_t*>(ctx->d_cl + 3 * j.nsites);
   c.misc = ctx->d_cl_misc;
   c.status = ctx->d_status;
-  ApiOut* api = nullptr;
-  akmc_status st = api_buffer(ctx, &api);
-  if (st != AKMC_OK) return st;
-  c.out = api->cluster;
+  c.out = ctx->d_cl_misc + kCounts;
   const int e = launch_cluster_stats(c, ctx->stream);
   if (e) return fail(ctx, AKMC_ECUDA, std::string("launch: ") + cuda_name(e));
+  std::vector<unsigned long long> h(static_cast<size_t>(2 + c.bins));
+  CK(cudaMemcpyAsync(h.data(), c.out, sizeof(unsigned long long) * h.size(), cudaMemcpyDeviceToHost, ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
-  const unsigned long long* const h = ctx->api->cluster;  // status, isolated atoms, histogram
-  if (h[0] && (st = check_status(ctx)) != AKMC_OK) return st;
+  if (h[0]) {
+    const akmc_status st = check_status(ctx);
+    if (st != AKMC_OK) return st;
+  }
   *isolated_cu = static_cast<int64_t>(h[1]);
-  for (int64_t k = 0; k < hist_len; ++k) hist[k] = static_cast<int64_t>(h[2 + k]);
+  for (int64_t k = 0; k < hist_len; ++k) hist[k] = static_cast<int64_t>(h[static_cast<size_t>(2 + k)]);
   return AKMC_OK;
 }
 

@@ -163,8 +163,8 @@ enum : uint32_t {
 
 enum : int32_t { kModeRound = 0, kModeCalc = 1, kModeSelectPerform = 2 };
 
-// What a per-hop entry point or the cluster statistics answer, in host memory that the kernels write: the caller
-// waits for the stream and reads it, without a copy.
+// What a per-hop entry point answers: written by its kernel, and read by the host in one copy, the first part alone after
+// a selection.
 constexpr int kClusterHist = 2;
 struct ApiOut {
   double total;
@@ -174,7 +174,6 @@ struct ApiOut {
   int32_t sites[kMaxV];     // their sites
   double de[kMaxV * 8];     // ΔE of each jump
   double rates[kMaxV * 8];  // its rates
-  unsigned long long cluster[2 + AKMC_CLUSTER_MAX_BINS];  // status, isolated atoms, histogram
 };
 
 struct RoundArgs {
@@ -289,7 +288,7 @@ struct ClusterArgs {
   int32_t* parent;
   int32_t* size;
   unsigned long long* misc;
-  unsigned long long* out;  // host memory
+  unsigned long long* out;
   unsigned int* status;
 };
 int launch_cluster_stats(const ClusterArgs& c, void* stream);

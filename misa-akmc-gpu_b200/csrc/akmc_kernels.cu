@@ -2376,7 +2376,7 @@ __global__ void k_finalize(RoundArgs a) {
 }
 
 // One per-hop API step (akmc_calculate, akmc_select_and_perform) of a single-domain job in one launch: the CTA finds
-// the sector's vacancies itself and leaves the answer, the status word included, in host memory.
+// the sector's vacancies itself and leaves the answer, the status word included, in one record.
 template <int KIND>
 __global__ void __launch_bounds__(Shape<8>::kThreads, 1) k_api(RoundArgs a) {
   constexpr int kThreads = Shape<8>::kThreads;
