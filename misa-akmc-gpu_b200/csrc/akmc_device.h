@@ -129,7 +129,8 @@ struct JobDev {
   int64_t hop_budget, max_rounds;
   double nu, kT, window;
   double rkT;         // RN(1 / kT): the rates' exponent arguments without a division
-  double pad;         // a multiple of 16 bytes: copied in 16-byte words
+  int32_t rich;       // most sites of its first lattice hold Cu, Ni or Mn (rich_share): a choice of speed, not of results
+  int32_t pad;        // a multiple of 16 bytes: copied in 16-byte words
 };
 
 struct BlockDev {
