@@ -36,6 +36,7 @@ struct HostJob {
   uint8_t* d_occ = nullptr;
   int32_t* d_rho = nullptr;
   CUtensorMap tmap[2];    // occupancy and density maps of the device lattice (JobDev::tma)
+  int64_t tiles(bool dense) const { return rho_tiles(2 * cfg.box[0], cfg.box[1], cfg.box[2], dense); }
 };
 
 struct DevPot {
@@ -508,6 +509,16 @@ int64_t first_invalid(const uint8_t* occ, int64_t n, int64_t* solutes) {
   return n;
 }
 
+// Whether the densities of a lattice like the job's first are built site by site: where its solutes are more than a
+// tenth of its sites, or the launch has fewer of the large tiles than the device SMs, which the small ones of the other
+// way fill.  A load of a lattice of 128^3 cells, by solutes against site by site: 154 and 206 us at 1.3 %, 208 and 206
+// at 8 %, 224 and 207 at 10 %, 258 and 206 at 50 %; 256^3 cells: 0.84 and 1.36 ms, 1.17 and 1.36, 1.27 and 1.36, 1.48
+// and 1.36; 20^3 cells (3 tiles): 65 and 58 us, 84 and 56, 86 and 56, 110 and 57; 48^3 (36): 66 and 56, 87 and 55,
+// 94 and 55, 116 and 56.
+bool rho_by_site(const akmc_ctx* ctx, const HostJob& j, int64_t launch_tiles) {
+  return j.nsolute + j.nvac > j.nsites / 10 || launch_tiles < ctx->grid_sms;
+}
+
 // The share of solutes from which on a job's several vacancies are evaluated jump by jump (rich_rates), by the CTA's
 // warps: where the two ways take the same time with 20 vacancies (8 warps, 128 rounds of 20^3 cells: 8.8 ms by shared
 // terms against 9.1 at 50 %, 8.7 against 8.4 at 60 %; 4 warps: 19.2 against 19.5 at 75 %, 23.1 against 19.8 at 100 %).
@@ -973,7 +984,7 @@ AKMC_API akmc_status akmc_prepare(akmc_ctx* ctx) {
   {  // density caches of every EAM job, one launch
     const akmc_status rt = build_rho_tables(ctx);
     if (rt != AKMC_OK) return rt;
-    if (ctx->jl.neam > 0) {
+    {
       RoundArgs ra{};
       ra.jobs = ctx->d_jobs;
       ra.pots = ctx->d_pots;
@@ -1088,7 +1099,7 @@ AKMC_API akmc_status akmc_admit_job(akmc_ctx* ctx, const akmc_job_config* cfg, c
   if (h.has_eam) {
     const int e = launch_init_rho(h.d_occ, h.d_rho, 2 * static_cast<int32_t>(h.cfg.box[0]),
                                   static_cast<int32_t>(h.cfg.box[1]), static_cast<int32_t>(h.cfg.box[2]),
-                                  ctx->d_pots + h.pot, ctx->d_geo, ctx->d_status, ctx->stream);
+                                  rho_by_site(ctx, h, h.tiles(false)), ctx->d_pots + h.pot, ctx->d_geo, ctx->stream);
     if (e) return fail(ctx, AKMC_ECUDA, std::string("init rho: ") + cuda_name(e));
   }
   ctx->h_jobs[static_cast<size_t>(slot)] = J;
@@ -1144,8 +1155,7 @@ AKMC_API akmc_status akmc_load_occupancy(akmc_ctx* ctx, int32_t job, const uint8
   if (ls != AKMC_OK) return ls;
   if (j.has_eam) {
     const int e = launch_init_rho(j.d_occ, j.d_rho, 2 * static_cast<int32_t>(j.cfg.box[0]), static_cast<int32_t>(j.cfg.box[1]),
-                        static_cast<int32_t>(j.cfg.box[2]), ctx->d_pots + j.pot, ctx->d_geo, ctx->d_status,
-                        ctx->stream);
+                        static_cast<int32_t>(j.cfg.box[2]), rho_by_site(ctx, j, j.tiles(false)), ctx->d_pots + j.pot, ctx->d_geo, ctx->stream);
     if (e) return fail(ctx, AKMC_ECUDA, std::string("init rho: ") + cuda_name(e));
   }
   CK(cudaMemcpyAsync(ctx->d_jobs + job, ctx->d_jobs0 + job, sizeof(JobDev), cudaMemcpyDeviceToDevice, ctx->stream));
@@ -1278,23 +1288,32 @@ AKMC_API akmc_status akmc_restore_snapshot(akmc_ctx* ctx, int32_t job, const uin
 static akmc_status build_rho_tables(akmc_ctx* ctx) {
   if (ctx->d_tile0) return AKMC_OK;
   std::vector<int32_t> eam_jobs;
-  std::vector<int64_t> tile0{0};
-  for (size_t k = 0; k < ctx->jobs.size(); ++k) {
-    const HostJob& j = ctx->jobs[k];
-    if (!j.has_eam || !j.live) continue;
-    const int64_t sx = 2 * j.cfg.box[0], sy = j.cfg.box[1], sz = j.cfg.box[2];
-    eam_jobs.push_back(static_cast<int32_t>(k));
-    tile0.push_back(tile0.back() + rho_tiles(sx, sy, sz));
+  std::vector<int64_t> tile0;
+  JobsLoad::RhoJobs* const rho = ctx->jl.rho;
+  int64_t all = 0;
+  for (const HostJob& j : ctx->jobs)
+    if (j.has_eam && j.live) all += j.tiles(false);
+  for (int dense = 0; dense < 2; ++dense) {
+    rho[dense].n = 0;
+    tile0.push_back(0);
+    for (size_t k = 0; k < ctx->jobs.size(); ++k) {
+      const HostJob& j = ctx->jobs[k];
+      if (!j.has_eam || !j.live || rho_by_site(ctx, j, all) != (dense != 0)) continue;
+      eam_jobs.push_back(static_cast<int32_t>(k));
+      tile0.push_back(tile0.back() + j.tiles(dense != 0));
+      ++rho[dense].n;
+    }
+    rho[dense].tiles = tile0.back();
   }
   CK(dalloc(ctx->stream, &ctx->d_tile0, tile0.size()));
   CK(dalloc(ctx->stream, &ctx->d_eam_jobs, std::max<size_t>(1, eam_jobs.size())));
   CK(cudaMemcpy(ctx->d_tile0, tile0.data(), tile0.size() * sizeof(int64_t), cudaMemcpyHostToDevice));
   if (!eam_jobs.empty())
     CK(cudaMemcpy(ctx->d_eam_jobs, eam_jobs.data(), eam_jobs.size() * sizeof(int32_t), cudaMemcpyHostToDevice));
-  ctx->jl.tile0 = ctx->d_tile0;
-  ctx->jl.eam_jobs = ctx->d_eam_jobs;
-  ctx->jl.neam = static_cast<int32_t>(eam_jobs.size());
-  ctx->jl.eam_tiles = tile0.back();
+  rho[0].tile0 = ctx->d_tile0;
+  rho[1].tile0 = ctx->d_tile0 + rho[0].n + 1;
+  rho[0].jobs = ctx->d_eam_jobs;
+  rho[1].jobs = ctx->d_eam_jobs + rho[0].n;
   return AKMC_OK;
 }
 

@@ -236,8 +236,8 @@ int launch_round(const RoundArgs& a, int hop_grid, size_t smem, void* stream, vo
 int launch_load_lattice(const uint8_t* stage, uint8_t* occ, int32_t sx, int64_t nrows, int32_t* vac_site, int32_t* vac_job,
                         int32_t job, int32_t cap, int32_t* count, unsigned int* status, void* stream);
 int launch_api(const RoundArgs& a, int kind, size_t smem, void* stream);  // kind: 0 pair bond, 1 EAM FP64, 2 FP32-comp
-int launch_init_rho(uint8_t* occ, int32_t* rho, int32_t sx, int32_t sy, int32_t sz, const Potential* pot,
-                    const Geometry* geo, unsigned int* status, void* stream);
+int launch_init_rho(uint8_t* occ, int32_t* rho, int32_t sx, int32_t sy, int32_t sz, bool dense, const Potential* pot,
+                    const Geometry* geo, void* stream);
 int launch_device_math(const double* x, int64_t n, double* e, double* l, void* stream);
 // n rounds of every unfinished block under the asynchronous schedule (no job may have a
 // hop budget); grid = persistent CTAs of the flow kernels.
@@ -245,10 +245,12 @@ int launch_flow(const RoundArgs& a, int grid, size_t smem, void* stream, void* e
 // Sets every block's remaining rounds to n before the launches of one akmc_run_rounds call.
 int launch_flow_begin(const RoundArgs& a, int64_t n, void* stream);
 
-// Tiles of the density build (one CTA takes one at a time).
+// Tiles of the density build (one CTA takes one at a time): summed by their solutes, or (a dense job's) site by site.
 constexpr int kRhoTX = 64, kRhoTY = 16, kRhoTZ = 8;
-AK_HD int64_t rho_tiles(int64_t sx, int64_t sy, int64_t sz) {
-  return ((sx + kRhoTX - 1) / kRhoTX) * ((sy + kRhoTY - 1) / kRhoTY) * ((sz + kRhoTZ - 1) / kRhoTZ);
+constexpr int kGatTX = 32, kGatTY = 8, kGatTZ = 4;
+AK_HD int64_t rho_tiles(int64_t sx, int64_t sy, int64_t sz, bool dense) {
+  const int tx = dense ? kGatTX : kRhoTX, ty = dense ? kGatTY : kRhoTY, tz = dense ? kGatTZ : kRhoTZ;
+  return ((sx + tx - 1) / tx) * ((sy + ty - 1) / ty) * ((sz + tz - 1) / tz);
 }
 
 // Whole-context lattice transfers (akmc_load_occupancies / akmc_get_occupancies): the lattices
@@ -265,10 +267,12 @@ struct JobsLoad {
   int32_t nchunks, njobs;
   int32_t* counts;          // vacancies found per job
   const int32_t* want;      // vacancies each job holds
-  const int64_t* tile0;     // density tiles of the EAM jobs, prefix (neam + 1)
-  const int32_t* eam_jobs;  // job index of each EAM job
-  int32_t neam;
-  int64_t eam_tiles;
+  struct RhoJobs {          // the EAM jobs whose tiles are summed by their solutes [0] or site by site [1]
+    const int64_t* tile0;   // their density tiles, prefix (n + 1)
+    const int32_t* jobs;    // their job indices
+    int32_t n;
+    int64_t tiles;
+  } rho[2];
 };
 int launch_load_jobs(const RoundArgs& a, const JobsLoad& L, void* stream);
 int launch_init_rho_jobs(const RoundArgs& a, const JobsLoad& L, void* stream);  // uses a.jobs, a.pots

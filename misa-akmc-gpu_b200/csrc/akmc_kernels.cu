@@ -19,6 +19,7 @@
 #include <algorithm>
 #include <cstddef>
 #include <cstdint>
+#include <type_traits>
 #include <utility>
 
 #include "akmc_device.h"
@@ -2475,10 +2476,10 @@ __global__ void __launch_bounds__(Shape<8>::kThreads, 1) k_api(RoundArgs a) {
 // site of the tile and its halo (4 sites in x, 2 rows in y and z) adds its difference to its 58 neighbours in
 // shared memory, a warp a site.  So the work is the reads (16 bytes a thread, 2.1 of them a site with the halo),
 // the writes and 58 additions per solute, not per site.  The additions are shared-memory atomics, a cycle a lane,
-// and bound it: the 256^3 lattice with 2.3% solutes takes 215 us, 650 us summed site by site.  A tile with more than
-// kRhoList such sites (12% of them) is still summed so (rho_gather), where the two meet: 128^3 cells take 34 us at
-// 1.3%, 65 at 5%, 105 at 10% and 130 site by site.
-constexpr int kGatTX = 32, kGatTY = 8, kGatTZ = 4, kRhoHX = 4, kRhoHY = 2, kRhoHZ = 2;
+// and bound it: the 256^3 lattice with 2.3% solutes takes 215 us.  A tile with more than kRhoList such sites (12% of
+// them) is summed site by site (rho_gather), part by part: a precipitate's, say.  A lattice that is rich in solutes
+// all over, or small, is left to k_init_rho<GatherSmem>, whose tiles are an eighth (rho_by_site).
+constexpr int kRhoHX = 4, kRhoHY = 2, kRhoHZ = 2;
 constexpr int kGatLX = kGatTX + 2 * kRhoHX, kGatLY = kGatTY + 2 * kRhoHY, kGatLZ = kGatTZ + 2 * kRhoHZ;
 
 struct RhoNb {
@@ -2678,21 +2679,40 @@ __device__ void rho_neighbours(const Geometry* geo, int32_t (&nb)[2][2]) {
     for (int u = 0; u < 2; ++u) nb[p][u] = lane + 32 * u < kShellNb ? __ldg(&geo->nbr[p][lane + 32 * u]) : 0;
 }
 
+// A dense job's tiles: summed site by site, many small ones (one CTA's share of a larger tile is gone through in turn).
+struct GatherSmem {
+  uint8_t tile[kGatLX * kGatLY * kGatLZ];
+  int32_t fqc[16 * 8];
+};
+__device__ void rho_tables(GatherSmem& m, const Potential* pot) {
+  __syncthreads();
+  rho_table(m.fqc, pot);
+}
+__device__ void rho_tile(const uint8_t* occ, int32_t* rho, int32_t sx, int32_t sy, int32_t sz, int32_t px, int64_t tix,
+                         GatherSmem& m, const int32_t (&)[2][2]) {
+  const int nx = (sx + kGatTX - 1) / kGatTX, ny = (sy + kGatTY - 1) / kGatTY;
+  const int64_t t = tix / nx;
+  rho_gather(occ, rho, sx, sy, sz, px, static_cast<int>(tix % nx) * kGatTX, static_cast<int>(t % ny) * kGatTY,
+             static_cast<int>(t / ny) * kGatTZ, m.tile, m.fqc);
+}
+
+template <typename M>
 __global__ void __launch_bounds__(256) k_init_rho(const uint8_t* occ, int32_t* rho, int32_t sx, int32_t sy,
                                                   int32_t sz, int32_t px, const Potential* pot, const Geometry* geo) {
-  __shared__ RhoSmem m;
+  __shared__ M m;
   int32_t nb[2][2];
   rho_neighbours(geo, nb);
   rho_tables(m, pot);
-  const int64_t ntiles = rho_tiles(sx, sy, sz);
+  const int64_t ntiles = rho_tiles(sx, sy, sz, std::is_same_v<M, GatherSmem>);
   for (int64_t tix = blockIdx.x; tix < ntiles; tix += gridDim.x) rho_tile(occ, rho, sx, sy, sz, px, tix, m, nb);
 }
 
-// The density build of every EAM job of a context in one launch: global tile t belongs to the
+// The density build of every EAM job of a context of one sort in one launch: global tile t belongs to the
 // job k with tile0[k] <= t < tile0[k + 1] (jobs[k] its index).
+template <typename M>
 __global__ void __launch_bounds__(256) k_init_rho_jobs(RoundArgs a, const int64_t* tile0, const int32_t* jobs,
                                                        int32_t njobs) {
-  __shared__ RhoSmem m;
+  __shared__ M m;
   int32_t nb[2][2];
   rho_neighbours(a.geo, nb);
   int pot = -1;
@@ -2925,12 +2945,12 @@ int launch_gather_clocks(const BlockDev* blocks, int32_t n, double* out, void* s
   k_gather_clocks<<<(9 * n + 127) / 128, 128, 0, static_cast<cudaStream_t>(stream)>>>(blocks, n, out);
   return static_cast<int>(cudaGetLastError());
 }
-int launch_init_rho(uint8_t* occ, int32_t* rho, int32_t sx, int32_t sy, int32_t sz, const Potential* pot,
-                    const Geometry* geo, unsigned int* status, void* stream) {
-  (void)status;
+int launch_init_rho(uint8_t* occ, int32_t* rho, int32_t sx, int32_t sy, int32_t sz, bool dense, const Potential* pot,
+                    const Geometry* geo, void* stream) {
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const int64_t blocks = std::min<int64_t>(rho_tiles(sx, sy, sz), 148 * 16);
-  k_init_rho<<<static_cast<int>(blocks), 256, 0, st>>>(occ, rho, sx, sy, sz, lattice_pitch(sx), pot, geo);
+  const int blocks = static_cast<int>(std::min<int64_t>(rho_tiles(sx, sy, sz, dense), 148 * 16));
+  if (dense) k_init_rho<GatherSmem><<<blocks, 256, 0, st>>>(occ, rho, sx, sy, sz, lattice_pitch(sx), pot, geo);
+  else k_init_rho<RhoSmem><<<blocks, 256, 0, st>>>(occ, rho, sx, sy, sz, lattice_pitch(sx), pot, geo);
   return static_cast<int>(cudaGetLastError());
 }
 
@@ -2939,9 +2959,11 @@ __global__ void k_check_vacancy_count(const int32_t* count, int32_t want, unsign
 }
 
 int launch_init_rho_jobs(const RoundArgs& a, const JobsLoad& L, void* stream) {
-  if (L.neam > 0)
-    k_init_rho_jobs<<<static_cast<int>(std::min<int64_t>(L.eam_tiles, 148 * 16)), 256, 0,
-                      static_cast<cudaStream_t>(stream)>>>(a, L.tile0, L.eam_jobs, L.neam);
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  auto blocks = [](const JobsLoad::RhoJobs& r) { return static_cast<int>(std::min<int64_t>(r.tiles, 148 * 16)); };
+  const JobsLoad::RhoJobs &s = L.rho[0], &d = L.rho[1];
+  if (s.n > 0) k_init_rho_jobs<RhoSmem><<<blocks(s), 256, 0, st>>>(a, s.tile0, s.jobs, s.n);
+  if (d.n > 0) k_init_rho_jobs<GatherSmem><<<blocks(d), 256, 0, st>>>(a, d.tile0, d.jobs, d.n);
   return static_cast<int>(cudaGetLastError());
 }
 
