@@ -389,6 +389,10 @@ def job_config(
     return c
 
 
+def _n_blocks(cfg):
+    return math.prod(max(1, b) for b in cfg.blocks)
+
+
 class Engine:
     """One akmc_ctx: a set of jobs advanced together on one GPU."""
 
@@ -415,6 +419,7 @@ class Engine:
         _check(lib().akmc_create(C.byref(cfg), C.byref(h)))
         self.h = h
         self.jobs = []
+        self.blocks = {}  # domain blocks of each live job, as it was added
 
     def close(self):
         if self.h:
@@ -441,6 +446,7 @@ class Engine:
         jid = C.c_int32(-1)
         self._ck(lib().akmc_add_job(self.h, C.byref(cfg), _ptr(occ), occ.size, C.byref(jid)))
         self.jobs.append((cfg, occ.size))
+        self.blocks[jid.value] = _n_blocks(cfg)
         return jid.value
 
     def prepare(self):
@@ -454,6 +460,7 @@ class Engine:
         while len(self.jobs) <= jid.value:
             self.jobs.append(None)
         self.jobs[jid.value] = (cfg, occ.size)
+        self.blocks[jid.value] = _n_blocks(cfg)
         return jid.value
 
     def run_for(self, n, max_us):
@@ -464,6 +471,7 @@ class Engine:
         """akmc_retire_job: frees the job's slots; its id may be given out again."""
         self._ck(lib().akmc_retire_job(self.h, job))
         self.jobs[job] = None
+        self.blocks.pop(job, None)
 
     def run_rounds(self, n):
         self._ck(lib().akmc_run_rounds(self.h, n))
@@ -524,9 +532,8 @@ class Engine:
         return out
 
     def block_clocks(self, job=0):
-        if 0 <= job < len(self.jobs) and self.jobs[job] is not None:  # the device is not asked for it
-            nb = math.prod(max(1, b) for b in self.jobs[job][0].blocks)
-        else:
+        nb = self.blocks.get(job)  # the device is not asked for it
+        if nb is None:
             nb = self.job_state(job)["n_blocks"]
         evo = np.empty((nb, 8), np.float64)
         hops = np.empty(nb, np.int64)
