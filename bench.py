@@ -342,7 +342,8 @@ class Runner:
         written = 4 * (ws - 2 * rh) + 2 * rh if eam else ws
         peak, peak_kind = peaks()
         achieved = bytes_alg / (hop_ms / 1e3) / 1e9 if hop_ms > 0 else 0.0
-        sched = "flow" if eng.round_schedule() == 2 else "rounds"
+        # a launch holds up to 1024 rounds, also those of a context's only block, whatever its schedule is called
+        sched = "flow" if eng.round_schedule() == 2 or launches < max(1, steps) * R else "rounds"
         traffic = traffic_per_launch(workload, sched, R)
         n = max(1, launches)
         return {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
@@ -735,13 +736,9 @@ def main():
     # kernels launched per timed step: round by round, k_bucket + k_hop + k_finalize per round
     # (captured in CUDA graphs); dependency-driven, per launch of up to 1024 rounds k_flow_begin
     # once per step, then k_flow_prep, k_flow_slots, k_flow and k_flow_finalize
-    sched = eng.round_schedule()
-    sched_name = "flow" if sched == ak.SCHEDULE_FLOW else "rounds"
-    # (one block's rounds run in one launch of that kernel under the automatic schedule)
-    persistent = sched == ak.SCHEDULE_FLOW or (args.workload == "serial" and args.schedule == "auto" and R >= 4)
-    launches_per_step = (1 + 4 * ((R + 1023) // 1024)) if persistent else 3 * R
-
+    sched_name = "flow" if eng.round_schedule() == ak.SCHEDULE_FLOW else "rounds"
     roofline = runner.roofline(eng, R, max(1, args.steps // 2), eam, args.workload)
+    launches_per_step = (1 + 4 * ((R + 1023) // 1024)) if roofline["kernel"] == "k_flow" else 3 * R
     e_dt, e_hops, nbytes = runner.end_to_end(eng, lattices, R, args.steps, "e2e")
     e_dt_all, e_hops_all = reduce_over_ranks(dist, e_dt, e_hops, "cuda")
     e2e = {"value": e_hops_all / e_dt_all, "unit": "hops/s", "h2d_bytes_per_step": nbytes,

@@ -1426,7 +1426,7 @@ AKMC_API akmc_status akmc_run_rounds(akmc_ctx* ctx, int64_t n_rounds) {
   // One block's rounds wait for nothing, so under either schedule they are the same rounds in the same order; the
   // persistent kernel runs them in one launch, without a bucketing and a finalizing kernel for each (256 rounds of a 20^3 box
   // with 20 vacancies: 19.0 -> 17.1 ms).
-  const bool solo = ctx->schedule == AKMC_SCHEDULE_AUTO && ctx->solo && !ctx->timing && n_rounds >= kSoloRounds;
+  const bool solo = ctx->schedule == AKMC_SCHEDULE_AUTO && ctx->solo && n_rounds >= kSoloRounds;
   const bool flow = ctx->schedule == AKMC_SCHEDULE_FLOW || (ctx->schedule == AKMC_SCHEDULE_AUTO && ctx->flow_ok) || solo;
   if (solo) a.flow_slots = kSoloSlots;
   if (flow) {
