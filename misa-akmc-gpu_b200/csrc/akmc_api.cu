@@ -19,6 +19,9 @@ using namespace akmc;
 
 namespace {
 
+// Sweeps per CTA and launch before a dependency-driven launch gives up, unless the context sets its own.
+constexpr int64_t kFlowSweepLimit = int64_t(1) << 25;
+
 struct HostJob {
   akmc_job_config cfg{};
   bool has_eam = false;
@@ -435,7 +438,7 @@ AKMC_API akmc_status akmc_create(const akmc_context_config* cfg, akmc_ctx** out)
   if (cfg) ctx->cfg = *cfg;
   if (ctx->cfg.graph_rounds <= 0) ctx->cfg.graph_rounds = 32;
   if (ctx->cfg.hop_cap_per_round <= 0) ctx->cfg.hop_cap_per_round = 10000000;
-  if (ctx->cfg.flow_sweep_limit <= 0) ctx->cfg.flow_sweep_limit = int64_t(1) << 25;
+  if (ctx->cfg.flow_sweep_limit <= 0) ctx->cfg.flow_sweep_limit = kFlowSweepLimit;
   if (ctx->cfg.eval_warps == 0) ctx->cfg.eval_warps = 8;
   if ((ctx->cfg.eval_warps != 8 && ctx->cfg.eval_warps != 4) || ctx->cfg.flow_take < 0) {
     delete ctx;
@@ -1428,7 +1431,10 @@ AKMC_API akmc_status akmc_run_rounds(akmc_ctx* ctx, int64_t n_rounds) {
   // with 20 vacancies: 19.0 -> 17.1 ms).
   const bool solo = ctx->schedule == AKMC_SCHEDULE_AUTO && ctx->solo && n_rounds >= kSoloRounds;
   const bool flow = ctx->schedule == AKMC_SCHEDULE_FLOW || (ctx->schedule == AKMC_SCHEDULE_AUTO && ctx->flow_ok) || solo;
-  if (solo) a.flow_slots = kSoloSlots;
+  if (solo) {
+    a.flow_slots = kSoloSlots;
+    a.flow_sweep_limit = std::max(a.flow_sweep_limit, kFlowSweepLimit);  // a caller's is for AKMC_SCHEDULE_FLOW
+  }
   if (flow) {
     // up to 1024 rounds per launch of the persistent flow kernels
     cudaEvent_t e0 = nullptr, e1 = nullptr;
