@@ -149,7 +149,7 @@ struct akmc_ctx {
   unsigned long long* d_cl_misc = nullptr;
   // whole-context lattice transfers: staging buffer, chunk table, per-job vacancy counts,
   // density tiles of the EAM jobs (built at the first transfer)
-  uint8_t* d_stage1 = nullptr;  // one lattice on its way into its device rows (load_lattice)
+  uint8_t* d_stage1 = nullptr;  // a pair-bond lattice on its way into its device rows (load_lattice)
   int64_t stage1_sites = 0;
   uint8_t* d_stage = nullptr;
   SiteChunk* d_chunks = nullptr;
@@ -198,25 +198,37 @@ void dfree(cudaStream_t s, void* p) {
   if (p) cudaFreeAsync(p, s);
 }
 
-// A job's lattice into its device rows: one plain copy into a staging buffer of the context (kept, and grown when
-// a larger lattice comes), then a kernel that lays the rows out with their halos.  With collect it also fills the
-// job's slice of the vacancy table (akmc_load_occupancy).  A strided copy straight into the rows measured 1.8 ms
-// for 131 x 117 rows of 300 sites, this 0.1 ms.
+// A job's lattice into its device rows: a plain copy into a staging buffer, then a kernel that lays the rows out with
+// their halos.  With collect it also fills the job's slice of the vacancy table (akmc_load_occupancy).  A strided copy
+// straight into the rows measured 1.8 ms for 131 x 117 rows of 300 sites, this 0.1 ms.  No memory beyond the job's own: an
+// EAM lattice is staged where its densities are built next (every caller builds them behind this); a pair-bond one, which
+// has none, through a buffer of the context, at most kStageSites at a time.
+constexpr int64_t kStageSites = int64_t(1) << 24;
 akmc_status load_lattice(akmc_ctx* ctx, int32_t job, uint8_t* d_occ, const uint8_t* occ, bool collect) {
   const HostJob& j = ctx->jobs[static_cast<size_t>(job)];
-  if (ctx->stage1_sites < j.nsites) {
-    dfree(ctx->stream, ctx->d_stage1);
-    ctx->d_stage1 = nullptr;
-    ctx->stage1_sites = 0;
-    CK(dalloc(ctx->stream, &ctx->d_stage1, static_cast<size_t>(j.nsites)));
-    ctx->stage1_sites = j.nsites;
+  uint8_t* stage = reinterpret_cast<uint8_t*>(j.d_rho);
+  int64_t sites = j.nsites;  // staged at a time
+  if (!stage) {
+    sites = std::min(sites, kStageSites);
+    if (ctx->stage1_sites < sites) {
+      dfree(ctx->stream, ctx->d_stage1);
+      ctx->d_stage1 = nullptr;
+      ctx->stage1_sites = 0;
+      CK(dalloc(ctx->stream, &ctx->d_stage1, static_cast<size_t>(sites)));
+      ctx->stage1_sites = sites;
+    }
+    stage = ctx->d_stage1;
   }
-  CK(cudaMemcpyAsync(ctx->d_stage1, occ, static_cast<size_t>(j.nsites), cudaMemcpyHostToDevice, ctx->stream));
-  const int e = launch_load_lattice(ctx->d_stage1, d_occ, 2 * static_cast<int32_t>(j.cfg.box[0]),
-                                    j.cfg.box[1] * j.cfg.box[2], collect ? ctx->d_vac_site + j.vac0 : nullptr,
-                                    collect ? ctx->d_vac_job + j.vac0 : nullptr, job, static_cast<int32_t>(j.nvac),
-                                    ctx->d_vac_count, ctx->d_status, ctx->stream);
-  if (e) return fail(ctx, AKMC_ECUDA, std::string("load lattice: ") + cuda_name(e));
+  const int32_t sx = 2 * static_cast<int32_t>(j.cfg.box[0]);
+  const int64_t rows = j.cfg.box[1] * j.cfg.box[2], per = sites / sx;
+  for (int64_t row0 = 0; row0 < rows; row0 += per) {
+    const int64_t n = std::min(per, rows - row0);
+    CK(cudaMemcpyAsync(stage, occ + row0 * sx, static_cast<size_t>(n * sx), cudaMemcpyHostToDevice, ctx->stream));
+    const int e = launch_load_lattice(stage, d_occ, sx, row0, n, rows, collect ? ctx->d_vac_site + j.vac0 : nullptr,
+                                      collect ? ctx->d_vac_job + j.vac0 : nullptr, job, static_cast<int32_t>(j.nvac),
+                                      ctx->d_vac_count, ctx->d_status, ctx->stream);
+    if (e) return fail(ctx, AKMC_ECUDA, std::string("load lattice: ") + cuda_name(e));
+  }
   return AKMC_OK;
 }
 
@@ -656,11 +668,11 @@ akmc_status setup_job(akmc_ctx* ctx, int32_t ji, JobDev& J, BlockDev* hb, int32_
   const size_t entries = static_cast<size_t>(lattice_entries(sx, static_cast<int32_t>(j.cfg.box[1]),
                                                              static_cast<int32_t>(j.cfg.box[2])));
   CK(dalloc(ctx->stream, &j.d_occ, entries));
+  if (j.has_eam) CK(dalloc(ctx->stream, &j.d_rho, entries));
   {
     const akmc_status st = load_lattice(ctx, ji, j.d_occ, j.occ.data(), false);
     if (st != AKMC_OK) return st;
   }
-  if (j.has_eam) CK(dalloc(ctx->stream, &j.d_rho, entries));
   std::memset(&J, 0, sizeof(J));
   J.occ = j.d_occ;
   J.rho = j.d_rho;

@@ -230,11 +230,12 @@ int configure_hop_smem(size_t smem);
 int hop_ctas_per_sm(int eval_warps);  // CTAs of the hop kernels the register budget allows per SM
 // ev0/ev1 (cudaEvent_t or null) are recorded around the hop kernel.
 int launch_round(const RoundArgs& a, int hop_grid, size_t smem, void* stream, void* ev0, void* ev1);
-// A lattice of nrows rows of sx sites from a staging buffer (rows back to back, on an even address) into its
-// device rows with their halos.  With vac_site, its vacancies go to the job's slice of the vacancy table, and
-// kErrVacCount is set in *status unless exactly cap were found.
-int launch_load_lattice(const uint8_t* stage, uint8_t* occ, int32_t sx, int64_t nrows, int32_t* vac_site, int32_t* vac_job,
-                        int32_t job, int32_t cap, int32_t* count, unsigned int* status, void* stream);
+// Rows row0 to row0 + n of a lattice of nrows rows of sx sites from a staging buffer (rows back to back, on an even
+// address) into its device rows with their halos.  With vac_site, their vacancies go to the job's slice of the vacancy
+// table, and kErrVacCount is set in *status unless exactly cap were found by the last row.
+int launch_load_lattice(const uint8_t* stage, uint8_t* occ, int32_t sx, int64_t row0, int64_t n, int64_t nrows,
+                        int32_t* vac_site, int32_t* vac_job, int32_t job, int32_t cap, int32_t* count,
+                        unsigned int* status, void* stream);
 int launch_api(const RoundArgs& a, int kind, size_t smem, void* stream);  // kind: 0 pair bond, 1 EAM FP64, 2 FP32-comp
 int launch_init_rho(uint8_t* occ, int32_t* rho, int32_t sx, int32_t sy, int32_t sz, bool dense, const Potential* pot,
                     const Geometry* geo, void* stream);

@@ -2772,10 +2772,10 @@ __device__ __forceinline__ void for_vacancies(const uint4& w4, int sx, int v, F 
   }
 }
 
-// A lattice from the staging buffer into a job's device rows, halos included; with vac_site its vacancies go to
-// the job's slice of the vacancy table (cap entries; count: vacancies found).
-__global__ void k_load_lattice(const uint8_t* __restrict__ stage, uint8_t* occ, int32_t sx, int32_t px, int64_t nrows,
-                               int32_t* vac_site, int32_t* vac_job, int32_t job, int32_t cap, int32_t* count) {
+// Rows of a lattice, row0 the first, from the staging buffer into a job's device rows, halos included; with vac_site
+// their vacancies go to the job's slice of the vacancy table (cap entries; count: vacancies found).
+__global__ void k_load_lattice(const uint8_t* __restrict__ stage, uint8_t* occ, int32_t sx, int32_t px, int64_t row0,
+                               int64_t nrows, int32_t* vac_site, int32_t* vac_job, int32_t job, int32_t cap, int32_t* count) {
   const int vpr = px / 16;
   const int64_t n = nrows * vpr;
   for (int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x; i < n;
@@ -2783,12 +2783,12 @@ __global__ void k_load_lattice(const uint8_t* __restrict__ stage, uint8_t* occ, 
     const int64_t row = i / vpr;
     const int v = static_cast<int>(i - row * vpr);
     const uint4 w = row_vector(stage + row * sx, sx, v);
-    *reinterpret_cast<uint4*>(occ + row * px + 16 * v) = w;
+    *reinterpret_cast<uint4*>(occ + (row0 + row) * px + 16 * v) = w;
     if (vac_site)
       for_vacancies(w, sx, v, [&](int x) {
         const int k = atomicAdd(count, 1);
         if (k < cap) {
-          vac_site[k] = static_cast<int32_t>(row * sx + x);
+          vac_site[k] = static_cast<int32_t>((row0 + row) * sx + x);
           vac_job[k] = job;
         }
       });
@@ -2982,14 +2982,15 @@ int launch_gather_jobs(const RoundArgs& a, const JobsLoad& L, void* stream) {
   return static_cast<int>(cudaGetLastError());
 }
 
-int launch_load_lattice(const uint8_t* stage, uint8_t* occ, int32_t sx, int64_t nrows, int32_t* vac_site, int32_t* vac_job,
-                        int32_t job, int32_t cap, int32_t* count, unsigned int* status, void* stream) {
+int launch_load_lattice(const uint8_t* stage, uint8_t* occ, int32_t sx, int64_t row0, int64_t n, int64_t nrows,
+                        int32_t* vac_site, int32_t* vac_job, int32_t job, int32_t cap, int32_t* count,
+                        unsigned int* status, void* stream) {
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int32_t px = lattice_pitch(sx);
-  const int blocks = static_cast<int>(std::min<int64_t>((nrows * (px / 16) + 255) / 256, 148 * 32));
-  if (vac_site) cudaMemsetAsync(count, 0, sizeof(int32_t), st);
-  k_load_lattice<<<blocks, 256, 0, st>>>(stage, occ, sx, px, nrows, vac_site, vac_job, job, cap, count);
-  if (vac_site) k_check_vacancy_count<<<1, 1, 0, st>>>(count, cap, status);
+  const int blocks = static_cast<int>(std::min<int64_t>((n * (px / 16) + 255) / 256, 148 * 32));
+  if (vac_site && row0 == 0) cudaMemsetAsync(count, 0, sizeof(int32_t), st);
+  k_load_lattice<<<blocks, 256, 0, st>>>(stage, occ, sx, px, row0, n, vac_site, vac_job, job, cap, count);
+  if (vac_site && row0 + n == nrows) k_check_vacancy_count<<<1, 1, 0, st>>>(count, cap, status);
   return static_cast<int>(cudaGetLastError());
 }
 
