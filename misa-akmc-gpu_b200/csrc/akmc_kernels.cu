@@ -433,10 +433,9 @@ __device__ __forceinline__ FCell32 cell32(const FTab& T, int32_t r, unsigned int
 __device__ __forceinline__ bool code_in(uint8_t c, uint32_t mask) { return c <= kMn && ((mask >> c) & 1u) != 0; }
 constexpr uint32_t kAtoms = 1u << kFe | 1u << kCu | 1u << kNi | 1u << kMn, kSolutes = kAtoms & ~(1u << kFe);
 
-// The rate of a jump with energy change dE onto a site with code Xc, into the record of vacancy k and jump b: 0 onto a
-// vacancy and onto a code that is no atom's (a reloaded lattice may hold some).
-__device__ __forceinline__ void put_rate(Smem& sm, int k, int b, uint8_t Xc, double dE, double* de_out) {
-  const bool atom = code_in(Xc, kAtoms);
+// The rate of a jump with energy change dE onto a site with code Xc, into the record of vacancy k and jump b: 0 unless
+// the code is an atom's (a vacancy's is not, nor are others that a reloaded lattice may hold).
+__device__ __forceinline__ void put_rate(Smem& sm, int k, int b, uint8_t Xc, bool atom, double dE, double* de_out) {
   const double rate = arrhenius_rk(sm.job.nu, sm.job.kT, sm.job.rkT, sm.e0[atom ? Xc : 0], dE);
   sm.rates[k][b] = atom ? rate : 0.0;
   sm.vX[k][b] = Xc;
@@ -477,7 +476,7 @@ __device__ __forceinline__ void pair_rates(Smem& sm, const uint8_t* occ_s, int k
   energy += t2[c[2] * 5];
   const double pair = energy + __shfl_down_sync(kFull, energy, 1);  // q0: e_before, q2: e_after
   const double after = __shfl_down_sync(kFull, pair, 2);
-  if (q == 0) put_rate(sm, k, b, Xc, after - pair, de_out);
+  if (q == 0) put_rate(sm, k, b, Xc, code_in(Xc, kAtoms), after - pair, de_out);
 }
 
 // FP32 F cell at density r: the node and the polynomial part of dF32.
@@ -627,7 +626,7 @@ __device__ __forceinline__ void jump_rates(Smem& sm, int set, const uint8_t* occ
     }
     dE = static_cast<double>(EX + (x.s - x.c));
   }
-  if ((lane & 7) == 0 && !code_in(Xc, kSolutes)) put_rate(sm, k, b, Xc, dE, de_out);
+  if ((lane & 7) == 0 && !code_in(Xc, kSolutes)) put_rate(sm, k, b, Xc, Xc == kFe, dE, de_out);
 }
 
 // Jumps of the vacancy at local site l whose target holds a solute, one bit each; all lanes of a warp.
@@ -715,7 +714,7 @@ __device__ __forceinline__ void solute_rate(Smem& sm, const uint8_t* occ_s, cons
     }
     dE = static_cast<double>(EX + (acc.s - acc.c));
   }
-  if (q == 0) put_rate(sm, k, b, Xc, dE, de_out);
+  if (q == 0) put_rate(sm, k, b, Xc, true, dE, de_out);
 }
 // Rates of the vacancies of masks m0 and m1 in a job rich in solutes, a warp a jump (W = 4: two), without the shared
 // terms: nearly every jump is summed on its own anyway, and all warps take part.  Vacancy ksel is at local site snew.
@@ -739,7 +738,7 @@ __device__ __noinline__ void rich_rates(Smem& sm, const uint8_t* occ_s, const in
     for (int b = threadIdx.x >> 5; b < 8; b += W) {
       const uint8_t Xc = occ_s[l + sm.d1[8 * (l & 1) + b].x];
       if (code_in(Xc, kAtoms)) solute_rate<KIND>(sm, occ_s, rho_s, k, l, b, LX, LY, *geo, FT, de_out);
-      else if ((threadIdx.x & 31) == 0) put_rate(sm, k, b, Xc, 0.0, de_out);
+      else if ((threadIdx.x & 31) == 0) put_rate(sm, k, b, Xc, false, 0.0, de_out);
     }
   }
 }
