@@ -68,6 +68,73 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_encode() {
   return fn;
 }
 
+// Pinned records that per-hop entry points and cluster statistics answer in, shared by a device's contexts.  A kernel
+// that writes its answer there saves the copy, 8 to 12 us a call, but pinning memory takes 1.5 to 2.3 ms, and giving it
+// back 0.4 ms and a wait for everything that runs on the device.  So one block of 16 is pinned by a device's first
+// akmc_prepare and kept; a context takes a record at its first such call and returns it at its end.  One that finds none
+// left has its answers copied from device memory.
+struct Answer {
+  ApiOut api;
+  unsigned long long cluster[kClusterHist + AKMC_CLUSTER_MAX_BINS];
+};
+constexpr int kAnswers = 16, kAnswerDevices = 16;
+struct AnswerPool {
+  std::mutex m;
+  Answer* block = nullptr;
+  unsigned long long id = 0;  // of the CUDA context that holds the block: a device reset takes it along
+  unsigned int used = 0;      // one bit a record
+} g_answers[kAnswerDevices];
+
+// The current CUDA context's id, unique in the process; 0 when the driver offers none.
+unsigned long long cuda_context_id() {
+  using GetId = CUresult (*)(CUcontext, unsigned long long*);
+  static const GetId fn = [] {
+    void* p = nullptr;
+    cudaDriverEntryPointQueryResult q{};
+    const bool ok = cudaGetDriverEntryPoint("cuCtxGetId", &p, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess;
+    return ok ? reinterpret_cast<GetId>(p) : nullptr;
+  }();
+  unsigned long long id = 0;
+  return fn && fn(nullptr, &id) == CUDA_SUCCESS ? id : 0;  // null: the current context
+}
+
+// The device's block is pinned, unless it cannot be (then the answers are copied).
+void pin_answers(int device) {
+  if (device < 0 || device >= kAnswerDevices) return;
+  AnswerPool& p = g_answers[device];
+  std::lock_guard<std::mutex> lk(p.m);
+  const unsigned long long id = cuda_context_id();
+  if (id == 0 || (p.block && p.id == id)) return;
+  p.block = nullptr;
+  p.used = 0;
+  if (cudaHostAlloc(reinterpret_cast<void**>(&p.block), kAnswers * sizeof(Answer), cudaHostAllocMapped) != cudaSuccess) {
+    cudaGetLastError();
+    p.block = nullptr;
+  }
+  p.id = id;
+}
+
+// A cleared record of the block that CUDA context `id` holds, null when there is none left.
+Answer* take_answer(int device, unsigned long long id) {
+  if (device < 0 || device >= kAnswerDevices || id == 0) return nullptr;
+  AnswerPool& p = g_answers[device];
+  std::lock_guard<std::mutex> lk(p.m);
+  if (!p.block || p.id != id) return nullptr;
+  for (int i = 0; i < kAnswers; ++i)
+    if (!((p.used >> i) & 1u)) {
+      p.used |= 1u << i;
+      std::memset(&p.block[i].api, 0, sizeof(ApiOut));
+      return p.block + i;
+    }
+  return nullptr;
+}
+void give_answer(int device, unsigned long long id, const Answer* a) {
+  if (!a) return;
+  AnswerPool& p = g_answers[device];
+  std::lock_guard<std::mutex> lk(p.m);
+  if (p.id == id) p.used &= ~(1u << (a - p.block));
+}
+
 // The tensor map of a job's device lattice array (halo layout, element size es): 3D tensor of
 // (pitch, sy, sz) entries, box = the job's widest staged region.  False if it cannot be encoded
 // (the job then stages by row copies).
@@ -122,6 +189,9 @@ struct akmc_ctx {
   unsigned long long* d_counters = nullptr;
   ApiOut* d_api = nullptr;  // the answer of a per-hop entry point on the device
   ApiOut api{};             // and here, the last akmc_calculate's rates among it
+  Answer* answer = nullptr;  // the pinned record it comes in, from the first such call on (take_answer)
+  bool asked = false;        // a record was asked for
+  unsigned long long cuda_id = 0;
   bool settled = false;   // the last such call waited for the stream, and nothing was put on it since
   size_t smem = 0;
   int hop_grid = 0;
@@ -309,6 +379,9 @@ void free_device(akmc_ctx* ctx) {
   ctx->d_status = nullptr;
   ctx->d_counters = nullptr;
   ctx->d_api = nullptr;
+  give_answer(ctx->cfg.device, ctx->cuda_id, ctx->answer);
+  ctx->answer = nullptr;
+  ctx->asked = false;
   ctx->prepared = false;
 }
 
@@ -983,6 +1056,8 @@ AKMC_API akmc_status akmc_prepare(akmc_ctx* ctx) {
   CK(dalloc(ctx->stream, &ctx->d_log_count, 1));
   CK(dalloc(ctx->stream, &ctx->d_api, 1));
   CK(cudaMemsetAsync(ctx->d_api, 0, sizeof(ApiOut), ctx->stream));
+  pin_answers(ctx->cfg.device);
+  ctx->cuda_id = cuda_context_id();
   if (ctx->cfg.event_log_capacity > 0) CK(dalloc(ctx->stream, &ctx->d_log, static_cast<size_t>(ctx->cfg.event_log_capacity)));
   CK(cudaMemcpyAsync(ctx->d_jobs, hj.data(), hj.size() * sizeof(JobDev), cudaMemcpyHostToDevice, ctx->stream));
   CK(cudaMemcpyAsync(ctx->d_blocks, hb.data(), hb.size() * sizeof(BlockDev), cudaMemcpyHostToDevice, ctx->stream));
@@ -1791,10 +1866,17 @@ AKMC_API akmc_status akmc_get_counters(akmc_ctx* ctx, int64_t* out8) {
   return AKMC_OK;
 }
 
-// One per-hop step: one launch and one copy, which waits; the answer is in ctx->api.  akmc_calculate on 20^3 cells takes
-// 31 us so, from a context's first call on, against 53 with three launches and two copies (and 105 the first).  A kernel
-// that answers in mapped host memory saves 8 to 12 us of copy, but pinning that memory takes 1.5 to 2.3 ms, and giving
-// it back 0.4 ms and a wait for everything that runs on the device.
+// The context's pinned record, null when there is none for it.
+static Answer* answer_of(akmc_ctx* ctx) {
+  if (!ctx->asked) {
+    ctx->asked = true;
+    ctx->answer = take_answer(ctx->cfg.device, ctx->cuda_id);
+  }
+  return ctx->answer;
+}
+
+// One per-hop step: one launch and one wait; the answer is in ctx->api.  akmc_calculate on 20^3 cells takes 22 us so,
+// 31 where the answer is copied, and 53 with three launches and two copies.
 static akmc_status api_step(akmc_ctx* ctx, int32_t job, int32_t sector_id, int32_t mode, double u) {
   ctx->settled = false;
   if (!ctx->prepared) return fail(ctx, AKMC_ESTATE, "akmc_prepare first");
@@ -1811,14 +1893,19 @@ static akmc_status api_step(akmc_ctx* ctx, int32_t job, int32_t sector_id, int32
   a.api_vac0 = j.vac0;
   a.api_nvac = static_cast<int32_t>(j.nvac);
   a.api_u = u;
-  a.api = ctx->d_api;
+  Answer* const pinned = answer_of(ctx);
+  a.api = pinned ? &pinned->api : ctx->d_api;
   a.log_cap = 0;
   const int kind = j.cfg.energy_model == AKMC_MODEL_PAIRBOND ? 0 : j.cfg.precision == AKMC_FP32C ? 2 : 1;
   const int e = launch_api(a, kind, ctx->smem, ctx->stream);
   if (e) return fail(ctx, AKMC_ECUDA, std::string("launch: ") + cuda_name(e));
-  // into pageable memory: the call returns when the copy, hence the kernel, is done
-  CK(cudaMemcpyAsync(&ctx->api, ctx->d_api, mode == kModeCalc ? sizeof(ApiOut) : offsetof(ApiOut, sites),
-                     cudaMemcpyDeviceToHost, ctx->stream));
+  const size_t n = mode == kModeCalc ? sizeof(ApiOut) : offsetof(ApiOut, sites);
+  if (pinned) {
+    CK(cudaStreamSynchronize(ctx->stream));
+    std::memcpy(&ctx->api, &pinned->api, n);
+  } else {  // into pageable memory: the call returns when the copy, hence the kernel, is done
+    CK(cudaMemcpyAsync(&ctx->api, ctx->d_api, n, cudaMemcpyDeviceToHost, ctx->stream));
+  }
   ctx->settled = true;
   return ctx->api.status ? check_status(ctx) : AKMC_OK;  // errors of the step and of earlier asynchronous calls
 }
@@ -1907,18 +1994,23 @@ AKMC_API akmc_status akmc_job_cluster_stats(akmc_ctx* ctx, int32_t job, int64_t*
   c.bits = reinterpret_cast<uint32_t*>(ctx->d_cl + 3 * j.nsites);
   c.misc = ctx->d_cl_misc;
   c.status = ctx->d_status;
-  c.out = ctx->d_cl_misc + kCounts;
+  Answer* const pinned = answer_of(ctx);
+  c.out = pinned ? pinned->cluster : ctx->d_cl_misc + kCounts;
   const int e = launch_cluster_stats(c, ctx->stream);
   if (e) return fail(ctx, AKMC_ECUDA, std::string("launch: ") + cuda_name(e));
-  std::vector<unsigned long long> h(static_cast<size_t>(2 + c.bins));
-  CK(cudaMemcpyAsync(h.data(), c.out, sizeof(unsigned long long) * h.size(), cudaMemcpyDeviceToHost, ctx->stream));
+  std::vector<unsigned long long> copied;
+  if (!pinned) {
+    copied.resize(static_cast<size_t>(2 + c.bins));
+    CK(cudaMemcpyAsync(copied.data(), c.out, sizeof(unsigned long long) * copied.size(), cudaMemcpyDeviceToHost, ctx->stream));
+  }
   CK(cudaStreamSynchronize(ctx->stream));
+  const unsigned long long* const h = pinned ? pinned->cluster : copied.data();
   if (h[0]) {
     const akmc_status st = check_status(ctx);
     if (st != AKMC_OK) return st;
   }
   *isolated_cu = static_cast<int64_t>(h[1]);
-  for (int64_t k = 0; k < hist_len; ++k) hist[k] = static_cast<int64_t>(h[static_cast<size_t>(2 + k)]);
+  for (int64_t k = 0; k < hist_len; ++k) hist[k] = static_cast<int64_t>(h[2 + k]);
   return AKMC_OK;
 }
 
