@@ -132,9 +132,9 @@ typedef struct akmc_context_config {
   int32_t max_block_edge;
   int64_t max_blocks;
   int64_t max_vacancies;
-  /* Launch shape of the hop kernels (autotuned by akmc_b200.autotune): eval_warps = warps that
-   * evaluate a vacancy's 8 jumps, 8 (one jump each, one CTA per SM; 0 = 8) or 4 (two jumps each,
-   * two CTAs per SM); flow_take = rounds with vacancies a CTA of the dependency-driven schedule
+  /* Launch shape of the hop kernels (autotuned by akmc_b200.autotune): eval_warps = warps of a
+   * CTA, which share the work on a vacancy's 8 jumps, 8 (one CTA per SM; 0 = 8) or 4 (two
+   * CTAs per SM); flow_take = rounds with vacancies a CTA of the dependency-driven schedule
    * takes per sweep (0: chosen by the kernel).  Results do not depend on either. */
   int32_t eval_warps;
   int32_t flow_take;
@@ -315,7 +315,7 @@ AKMC_API akmc_status akmc_cluster_stats(const uint8_t* occ, const int64_t box[3]
                                         int64_t hist_len);
 /* The same statistics of a job's resident lattice, computed on the device (the reference
  * computes them on the host from its hash sets, m_event_hook.cpp:17-55).  hist_len <=
- * AKMC_CLUSTER_MAX_BINS.  The first call for a job size allocates 12 bytes per site. */
+ * AKMC_CLUSTER_MAX_BINS.  The first call for a job size allocates 12 bytes and a bit per site. */
 #define AKMC_CLUSTER_MAX_BINS 4096
 AKMC_API akmc_status akmc_job_cluster_stats(akmc_ctx* ctx, int32_t job, int64_t* isolated_cu, int64_t* hist,
                                             int64_t hist_len);

@@ -91,8 +91,8 @@ unsigned long long cuda_context_id() {
   static const GetId fn = [] {
     void* p = nullptr;
     cudaDriverEntryPointQueryResult q{};
-    const bool ok = cudaGetDriverEntryPoint("cuCtxGetId", &p, cudaEnableDefault, &q) == cudaSuccess && q == cudaDriverEntryPointSuccess;
-    return ok ? reinterpret_cast<GetId>(p) : nullptr;
+    const cudaError_t e = cudaGetDriverEntryPoint("cuCtxGetId", &p, cudaEnableDefault, &q);
+    return e == cudaSuccess && q == cudaDriverEntryPointSuccess ? reinterpret_cast<GetId>(p) : nullptr;
   }();
   unsigned long long id = 0;
   return fn && fn(nullptr, &id) == CUDA_SUCCESS ? id : 0;  // null: the current context
@@ -777,7 +777,8 @@ akmc_status setup_job(akmc_ctx* ctx, int32_t ji, JobDev& J, BlockDev* hb, int32_
   J.nu = j.cfg.attempt_freq;
   J.kT = kBoltzmann * j.cfg.temperature;
   J.rkT = 1.0 / J.kT;
-  J.rich = static_cast<double>(j.nsites - j.niron - j.nvac) > rich_share(ctx->cfg.eval_warps) * static_cast<double>(j.nsites) ? 1 : 0;
+  const double solutes = static_cast<double>(j.nsites - j.niron - j.nvac);
+  J.rich = solutes > rich_share(ctx->cfg.eval_warps) * static_cast<double>(j.nsites) ? 1 : 0;
   J.fwin0 = ctx->pots[static_cast<size_t>(j.pot)].P.fwin0;
   J.window = j.cfg.sector_window;
   for (int b = 0; b < j.nblocks; ++b) {
@@ -1501,8 +1502,8 @@ AKMC_API akmc_status akmc_get_kernel_timing(akmc_ctx* ctx, double* hop_kernel_ms
 }
 
 // Rounds from which on a context with one block runs them in one launch of the persistent kernel.  Its seven launches
-// cost as much as three rounds' bucketing and finalizing: 1, 2 and 3 rounds took 107, 178 and 254 us against 99, 163
-// and 257 round by round, 4 and 8 289 and 497 against 326 and 704 (20 vacancies, FP64).
+// cost as much as two or three rounds' bucketing and finalizing: 1, 2 and 3 rounds took 152, 459 and 494 us against 138,
+// 462 and 511 round by round, 4, 8 and 32 532, 984 and 2650 against 565, 1080 and 2960 (20^3 cells, 20 vacancies, FP64).
 constexpr int64_t kSoloRounds = 4;
 AKMC_API akmc_status akmc_run_rounds(akmc_ctx* ctx, int64_t n_rounds) {
   if (!ctx) return AKMC_EINVAL;
@@ -1514,7 +1515,7 @@ AKMC_API akmc_status akmc_run_rounds(akmc_ctx* ctx, int64_t n_rounds) {
   a.mode = kModeRound;
   // One block's rounds wait for nothing, so under either schedule they are the same rounds in the same order; the
   // persistent kernel runs them in one launch, without a bucketing and a finalizing kernel for each (256 rounds of a 20^3 box
-  // with 20 vacancies: 19.0 -> 17.1 ms).
+  // with 20 vacancies: 21.9 -> 19.2 ms).
   const bool solo = ctx->schedule == AKMC_SCHEDULE_AUTO && ctx->solo && n_rounds >= kSoloRounds;
   const bool flow = ctx->schedule == AKMC_SCHEDULE_FLOW || (ctx->schedule == AKMC_SCHEDULE_AUTO && ctx->flow_ok) || solo;
   if (solo) {

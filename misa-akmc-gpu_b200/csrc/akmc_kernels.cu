@@ -6,10 +6,11 @@
 //              the block's active sector, append it to the block's list;
 //   k_hop      one CTA per active block: stage the sector plus a 2-cell halo (occupancy
 //              bytes and the int32 density cache) into shared memory and run the hop
-//              loop there.  Warp w evaluates jump directions w, w + W, ... of a vacancy (its
-//              32 lanes split the 76 sites of a jump); every warp forms the ordered total and
-//              selects for itself, and the hop's updates are spread over the warps; each hop
-//              writes its two occupancy bytes and 78 densities through to global memory;
+//              loop there.  EAM: all warps form the terms that a vacancy's 8 jumps share, two sum
+//              the jumps; pair bond: a warp evaluates a vacancy.  Every warp forms the ordered
+//              total and selects for itself, and the hop's updates are spread over the warps; each
+//              hop writes its two occupancy bytes and 78 densities through to global memory (one
+//              pair-bond vacancy: its path's sites, when its loop ends);
 //   k_finalize one thread per block: clock of blocks without vacancies, next round.
 // Concurrently active sectors are at least 4 cells apart, so the staged regions of
 // different blocks never overlap and no atomics are needed on the lattice.
@@ -48,7 +49,9 @@ enum : int { kPairBond = 0, kEam64 = 1, kEam32 = 2 };  // energy kinds, one kern
 // instructions, so its latency is what counts, and two CTAs per SM (128 registers a thread instead of 255,
 // so spills in the loop, and the other CTA's sweeps and hops on the same issue slots) measured slower: 40.6
 // against 33.5 ms for 1024 rounds of the 256^3 lattice end to end, 30.2 against 27.7 ms for 256 rounds of
-// 512 boxes.
+// 512 boxes.  Two CTAs of W = 4 (255 registers again) are within a few per cent of that where every SM has
+// rounds to run (512 boxes in 16-cell blocks: 48.5 against 47.9 M hops/s), and a third slower along a chain
+// (128 rounds of one block: 13.0 against 9.6 ms), so 8 is what a context gets that does not ask.
 template <int W>
 struct Shape {
   static_assert(8 % W == 0, "whole jump directions per warp");
@@ -635,8 +638,9 @@ __device__ __forceinline__ unsigned solute_jumps(const Smem& sm, const uint8_t* 
   return __ballot_sync(kFull, lane < 8 && code_in(occ_s[l + sm.d1[8 * (l & 1) + (lane & 7)].x], kSolutes));
 }
 // Rate of jump b of vacancy k at local site l with an atom as target, by one warp: for solutes (solute_jumps; the
-// shared terms are those of a moving Fe atom), and for every atom in a job rich in solutes.  Lane q sums sites i = q, q + 32, q + 64 of the jump's list; the 32 partials merge
-// by a xor butterfly (16, 8, 4, 2, 1), then the moving atom's own embedding change is added.
+// shared terms are those of a moving Fe atom), and for every atom in a job rich in solutes.  Lane q sums sites i = q,
+// q + 32, q + 64 of the jump's list; the 32 partials merge by a xor butterfly (16, 8, 4, 2, 1), then the moving atom's
+// own embedding change is added.
 template <int KIND>
 __device__ __forceinline__ void solute_rate(Smem& sm, const uint8_t* occ_s, const int32_t* rho_s, int k, int l, int b,
                                             int LX, int LY, const Geometry& G, const FTab& FT, double* de_out) {
@@ -2112,7 +2116,7 @@ __global__ void __launch_bounds__(Shape<W>::kThreads, Shape<W>::kCtasPerSm) k_fl
         const bool empty = !(d1.z & kNbrSolo) && !((w >> (1 + sector_of_round(r))) & 1ull);
         // A neighbour that carried a vacancy into this sector marked it in the word before it published the round that
         // flow_ready saw.  The fence orders the two for this thread, so that the compare-and-swap below finds the mark
-        // and fails, whatever w was read as.  (It costs 1-2%: 256^3 lattice, 1024 rounds, 23.9 ms; 23.3-23.8 without.)
+        // and fails, whatever w was read as.  (It costs 2-3%: 1024 rounds of the resident 256^3 lattice took 21.9 ms without it, 22.4 with.)
         if (ok && empty) fence_acq_rel();
         if (ok && empty && !(d1.z & kNbrGate)) {
           // no vacancy: the round is passed over, and the block keeps the lease bit at its target.  Nothing is read
@@ -2820,7 +2824,6 @@ __global__ void k_check_counts(const int32_t* counts, const int32_t* want, int32
   if (j < njobs && counts[j] != want[j]) atomicOr(status, kErrVacCount);
 }
 
-// Whole-context lattice read-back: the reverse copy into the staging buffer (rows of sx sites, an even number).
 // One thread a word: a read-out moves 72 bytes a block over PCIe, not its whole record.
 __global__ void k_gather_clocks(const BlockDev* __restrict__ blocks, int32_t n, double* __restrict__ out) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -2830,6 +2833,7 @@ __global__ void k_gather_clocks(const BlockDev* __restrict__ blocks, int32_t n, 
     reinterpret_cast<int64_t*>(out)[i] = blocks[i - 8 * n].hops;
 }
 
+// Whole-context lattice read-back: the reverse copy into the staging buffer (rows of sx sites, an even number).
 __global__ void k_gather(RoundArgs a, uint8_t* stage, const SiteChunk* chunks) {
   const SiteChunk c = chunks[blockIdx.x];
   const JobDev& J = a.jobs[c.job];

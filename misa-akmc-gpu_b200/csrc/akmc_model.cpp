@@ -18,21 +18,12 @@ const int kNN1[2][8][3] = {
     {{-1, 0, 0}, {-1, 0, 1}, {-1, 1, 0}, {-1, 1, 1}, {1, 0, 0}, {1, 0, 1}, {1, 1, 0}, {1, 1, 1}}};
 // 2nn offsets in PeriodLatticeList::get2nn2 order (src/lattice/period_lattice_list.cpp:234-256).
 const int kNN2[6][3] = {{-2, 0, 0}, {0, -1, 0}, {0, 0, -1}, {0, 0, 1}, {0, 1, 0}, {2, 0, 0}};
-// BCC shells within 2a: squared distance in (a/2)^2 units.
-const int kShellD2[5] = {3, 4, 8, 11, 12};
-constexpr int kSelf = 6;
-
 // squared distance between site (X0, 0, 0) and (X0 + dX, dy, dz) in (a/2)^2 units;
 // corner sites (X even) sit at (X, 2y, 2z), centre sites at (X, 2y + 1, 2z + 1).
 int dist2(int X0, int dX, int dy, int dz) {
   const int p0 = X0 & 1, p1 = (X0 + dX) & 1;
   const int hy = 2 * dy + p1 - p0, hz = 2 * dz + p1 - p0;
   return dX * dX + hy * hy + hz * hz;
-}
-int shell_code(int d2, int nsh) {
-  for (int i = 0; i < nsh; ++i)
-    if (kShellD2[i] == d2) return i + 1;
-  return 0;
 }
 
 }  // namespace

@@ -9,6 +9,15 @@
 
 namespace akmc {
 
+// BCC shells within 2a: squared distance in (a/2)^2 units.  Codes 1..5, 6 = the site itself, 0 = none.
+constexpr int kShellD2[5] = {3, 4, 8, 11, 12};
+constexpr int kSelf = 6;
+inline int shell_code(int d2, int nsh) {
+  for (int i = 0; i < nsh; ++i)
+    if (kShellD2[i] == d2) return i + 1;
+  return 0;
+}
+
 int shells_within(double lattice_const, double cutoff);
 void build_geometry(Geometry& g, int nshells);
 // The foot_* and term tables of a geometry whose jump lists are filled (called by build_geometry).

@@ -6,19 +6,6 @@
 
 namespace akmc {
 
-namespace {
-
-// BCC shells within 2a: squared distance in (a/2)^2 units; code 1..5, 6 = the site itself, 0 = none.
-const int kShellD2[5] = {3, 4, 8, 11, 12};
-constexpr int kSelf = 6;
-int shell_code(int d2, int nsh) {
-  for (int i = 0; i < nsh; ++i)
-    if (kShellD2[i] == d2) return i + 1;
-  return 0;
-}
-
-}  // namespace
-
 // The lanes that form the dE terms of a vacancy's 8 jumps (Geometry::foot_*), in half lattice
 // constants around the vacancy: the same for both x parities but for the site ids' own offsets.
 void build_terms(Geometry& g, int nsh) {

@@ -9,8 +9,8 @@ The knobs, all of which leave every trajectory unchanged except the block edge (
   regions that most hops never touch.  A box of edge n gets ceil(n / edge) blocks per dimension,
   at most n // 8 (blocks are at least 8 cells).  Different blocks give different (equally valid)
   trajectories, so the choice is made once, before the run it serves;
-- threads per vacancy (eval_warps): the hop kernels evaluate a vacancy's 8 jumps with 8 warps
-  (one jump each, one CTA per SM) or 4 warps (two jumps each, two CTAs per SM);
+- threads per vacancy (eval_warps): the hop kernels' CTAs have 8 warps (one CTA per SM) or 4
+  (two CTAs per SM), which share the work on a vacancy's 8 jumps;
 - rounds per CTA (flow_take): how many ready rounds with vacancies a CTA of the
   dependency-driven schedule takes per sweep (0: by how many CTAs are idle).
 
