@@ -6,8 +6,8 @@
 // copying the lattice out.
 //
 //   k_cu_bits     one pass over the occupancy bytes (32 sites a thread, two 16-byte loads) into a
-//                 bit per site: the only pass over the whole lattice.  33.5 MB in 9.4 us out of L2,
-//                 where a sampled lattice mostly lies, in 10.4 from DRAM (3.5 TB/s).
+//                 bit per site: the only pass over the whole lattice.  33.5 MB in 7.8 us out of L2,
+//                 where a sampled lattice mostly lies, in 9.0 from DRAM (4.1 TB/s).
 //   k_cu_classify 32 sites a thread from their own bits and those of the seven rows around: the Cu
 //                 atoms without a Cu first neighbour are counted, the others are listed and start
 //                 as their own roots.  All in L2 (a bit a site).
@@ -19,7 +19,7 @@
 // At dilute concentrations nine Cu atoms in ten are isolated, and only the rest is written to the
 // scattered list, parent and size entries.  33.5 M sites, 1.34 % Cu: collecting every Cu atom and
 // testing its neighbours byte by byte took 56 + 35 us, sizes and histogram 15 + 18 us, the whole
-// call 165 us; now 9 + 16 us, 12 us for the union, 10 us for the histogram, and the call 61 us.
+// call 165 us; now 8 + 15 us, 11 us for the union, 8 us for the histogram, and the call 61 us.
 // The partition, hence every count, does not depend on the order the threads run in.
 #include <algorithm>
 #include <cstdint>
