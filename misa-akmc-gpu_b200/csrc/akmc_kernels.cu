@@ -246,7 +246,7 @@ struct Smem {
 
 // A reloaded lattice may hold codes above 8, which no table has a row for: what is looked up for them as neighbours
 // lies within the working set.
-static_assert(offsetof(Smem, b2) + sizeof(double) * (255 * 5 + 5) <= sizeof(Smem) &&
+static_assert(offsetof(Smem, b2) + sizeof(double) * (255 * 5 + 9) <= sizeof(Smem) &&
                   offsetof(Smem, dphi64) + sizeof(double) * ((3 * 4 + 96 + 1) * 64) <= sizeof(Smem),
               "codes up to 255 (atom_index 96)");
 
@@ -2560,7 +2560,8 @@ __device__ void rho_gather(const uint8_t* occ, int32_t* rho, int32_t sx, int32_t
       gy -= gy >= sy ? sy : 0;
       gz -= gz >= sz ? sz : 0;
     }
-    tile[i] = __ldg(occ + kHaloL + gx + static_cast<int64_t>(px) * (gy + static_cast<int64_t>(sy) * gz));
+    const uint8_t c = __ldg(occ + kHaloL + gx + static_cast<int64_t>(px) * (gy + static_cast<int64_t>(sy) * gz));
+    tile[i] = c < 16 ? c : static_cast<uint8_t>(kV);  // the f table's rows; no code above 8 is an atom's
   }
   __syncthreads();
   // each warp takes sites of one x parity (both parities' sums are unrolled code): warp w

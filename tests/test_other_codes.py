@@ -1,7 +1,8 @@
 """GPU: a reloaded lattice with sites that hold no atom's code (3, 5, 6 or 7), beside a vacancy.
 
 Such a site never jumps: its rate is 0, and the run leaves it where it is.  With the pair-bond model it binds as a vacancy
-does, so the other jumps' energies are those of the same lattice with a vacancy there.
+does, so the other jumps' energies are those of the same lattice with a vacancy there.  Densities count it as none, up to
+the largest code a byte holds, both ways they are built.
 """
 import numpy as np
 import pytest
@@ -44,3 +45,28 @@ def test_a_site_without_an_atoms_code_never_jumps(model, precision, code):
         eng.sync()
         end = eng.occupancy(0)
         assert end[odd] == code and (end == 0).sum() == 1 and (end == ak.FE).sum() == len(iron) - 2
+
+
+@pytest.mark.parametrize("edge,blocks", [(16, 1), (96, 4)])  # built site by site; by its solutes
+def test_densities_do_not_count_other_codes(edge, blocks):
+    import akmc_b200 as ak
+
+    box, n = (edge,) * 3, 2 * edge ** 3
+    with ak.Engine() as eng:
+        one = np.full(n, ak.FE, np.uint8)
+        one[0] = 0
+        eng.add_job(ak.job_config(box, blocks=(blocks,) * 3, eam=ak.eam_johnson(42)), one)
+        eng.prepare()
+        codes = np.arange(256, dtype=np.int64)
+        others = codes[(codes > 0) & ~np.isin(codes, [ak.FE, ak.CU, ak.NI, ak.MN])].astype(np.uint8)
+        at = 1 + np.arange(len(others)) * (n // 300)
+        other, vacant = one.copy(), one.copy()
+        other[at], vacant[at] = others, 0
+        eng.load_occupancy(0, other)
+        eng.sync()
+        rho = eng.rho(0)
+        assert np.array_equal(eng.occupancy(0), other)
+        eng.load_occupancy(0, vacant)
+        with pytest.raises(ak.AkmcError):  # more vacancies than the job holds; its densities are built all the same
+            eng.sync()
+        assert np.array_equal(eng.rho(0), rho)
