@@ -164,8 +164,8 @@ enum : uint32_t {
 
 enum : int32_t { kModeRound = 0, kModeCalc = 1, kModeSelectPerform = 2 };
 
-// What a per-hop entry point answers: written by its kernel, and read by the host in one copy, the first part alone after
-// a selection.
+// What a per-hop entry point answers: written by its kernel in a pinned record or in device memory, and copied by the
+// host, the first part alone after a selection.
 constexpr int kClusterHist = 2;
 struct ApiOut {
   double total;
@@ -246,7 +246,7 @@ int launch_flow(const RoundArgs& a, int grid, size_t smem, void* stream, void* e
 // Sets every block's remaining rounds to n before the launches of one akmc_run_rounds call.
 int launch_flow_begin(const RoundArgs& a, int64_t n, void* stream);
 
-// Tiles of the density build (one CTA takes one at a time): summed by their solutes, or (a dense job's) site by site.
+// Tiles of the density build (one CTA takes one at a time): summed by their solutes, or site by site (dense).
 constexpr int kRhoTX = 64, kRhoTY = 16, kRhoTZ = 8;
 constexpr int kGatTX = 32, kGatTY = 8, kGatTZ = 4;
 AK_HD int64_t rho_tiles(int64_t sx, int64_t sy, int64_t sz, bool dense) {

@@ -701,7 +701,8 @@ __device__ __forceinline__ void solute_rate(Smem& sm, const uint8_t* occ_s, cons
     } else {
       EX = dF32(cell32(FT, rx1, FT.status), cell32(FT, rx0, FT.status), rx1, rx0);
 #pragma unroll
-      for (int u = 0; u < 3; ++u) t[u] = in[u] ? dF32(cell32(FT, r1[u], FT.status), cell32(FT, r0[u], FT.status), r1[u], r0[u]) : 0.f;
+      for (int u = 0; u < 3; ++u)
+        t[u] = in[u] ? dF32(cell32(FT, r1[u], FT.status), cell32(FT, r0[u], FT.status), r1[u], r0[u]) : 0.f;
     }
     Comp32 acc;
     acc.s = 0.f;
@@ -1291,7 +1292,8 @@ __device__ __forceinline__ int run_block(const RoundArgs& a, Smem& sm, Round& C,
           unsigned solutes = solute_jumps(sm, occ_s, s);
           for (int q = 2; solutes; ++q) {  // the k-th of them to warp 2 + k
             if ((q - 2) % (kEvalWarps - 2) == warp - 2)
-              solute_rate<KIND>(sm, occ_s, rho_s, 0, s, __ffs(static_cast<int>(solutes)) - 1, R.LX, R.LY, *a.geo, FT, nullptr);
+              solute_rate<KIND>(sm, occ_s, rho_s, 0, s, __ffs(static_cast<int>(solutes)) - 1, R.LX, R.LY, *a.geo, FT,
+                                nullptr);
             solutes &= solutes - 1;
           }
         }
@@ -1423,7 +1425,8 @@ __device__ __forceinline__ int run_block(const RoundArgs& a, Smem& sm, Round& C,
             for (int n = 0; sol; ++n) {  // the solute targets of both, one after another to these warps
               const int q = __ffs(static_cast<int>(sol)) - 1;
               if (n % (kEvalWarps - kw) == warp - kw)
-                solute_rate<KIND>(sm, occ_s, rho_s, q < 8 ? ka : kb, q < 8 ? la : lb, q & 7, R.LX, R.LY, *a.geo, FT, de_out);
+                solute_rate<KIND>(sm, occ_s, rho_s, q < 8 ? ka : kb, q < 8 ? la : lb, q & 7, R.LX, R.LY, *a.geo, FT,
+                                  de_out);
               sol &= sol - 1;
             }
           }
@@ -2116,7 +2119,8 @@ __global__ void __launch_bounds__(Shape<W>::kThreads, Shape<W>::kCtasPerSm) k_fl
         const bool empty = !(d1.z & kNbrSolo) && !((w >> (1 + sector_of_round(r))) & 1ull);
         // A neighbour that carried a vacancy into this sector marked it in the word before it published the round that
         // flow_ready saw.  The fence orders the two for this thread, so that the compare-and-swap below finds the mark
-        // and fails, whatever w was read as.  (It costs 2-3%: 1024 rounds of the resident 256^3 lattice took 21.9 ms without it, 22.4 with.)
+        // and fails, whatever w was read as.  (It costs 2-3%: 1024 rounds of the resident 256^3 lattice took 21.9 ms
+        // without it, 22.4 with.)
         if (ok && empty) fence_acq_rel();
         if (ok && empty && !(d1.z & kNbrGate)) {
           // no vacancy: the round is passed over, and the block keeps the lease bit at its target.  Nothing is read
