@@ -273,9 +273,9 @@ AKMC_API akmc_status akmc_save_snapshot(akmc_ctx* ctx, int32_t job, uint8_t* buf
 AKMC_API akmc_status akmc_restore_snapshot(akmc_ctx* ctx, int32_t job, const uint8_t* buf, int64_t n);
 
 /* Kernel timing mode: while enabled, akmc_run_rounds puts CUDA events around each launch of
- * the hop kernel on the context stream (round by round, without a CUDA graph; one launch for up to 1024
- * rounds where they run in one); akmc_get_kernel_timing returns their summed time and the
- * launch count.  The rounds run in the same kernels as without it. */
+ * the hop kernel on the context stream (a launch a round, without a CUDA graph, or one for up to
+ * 1024 rounds where they run in one); akmc_get_kernel_timing returns their summed time and
+ * the launch count.  The rounds run in the same kernels as without it. */
 AKMC_API akmc_status akmc_set_kernel_timing(akmc_ctx* ctx, int32_t enable);
 AKMC_API akmc_status akmc_get_kernel_timing(akmc_ctx* ctx, double* hop_kernel_ms, int64_t* hop_launches);
 

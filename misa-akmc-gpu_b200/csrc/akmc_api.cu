@@ -1245,7 +1245,8 @@ AKMC_API akmc_status akmc_load_occupancy(akmc_ctx* ctx, int32_t job, const uint8
   if (ls != AKMC_OK) return ls;
   if (j.has_eam) {
     const int e = launch_init_rho(j.d_occ, j.d_rho, 2 * static_cast<int32_t>(j.cfg.box[0]), static_cast<int32_t>(j.cfg.box[1]),
-                        static_cast<int32_t>(j.cfg.box[2]), rho_by_site(ctx, j, j.tiles(false)), ctx->d_pots + j.pot, ctx->d_geo, ctx->stream);
+                        static_cast<int32_t>(j.cfg.box[2]), rho_by_site(ctx, j, j.tiles(false)), ctx->d_pots + j.pot,
+                        ctx->d_geo, ctx->stream);
     if (e) return fail(ctx, AKMC_ECUDA, std::string("init rho: ") + cuda_name(e));
   }
   CK(cudaMemcpyAsync(ctx->d_jobs + job, ctx->d_jobs0 + job, sizeof(JobDev), cudaMemcpyDeviceToDevice, ctx->stream));
@@ -2002,7 +2003,8 @@ AKMC_API akmc_status akmc_job_cluster_stats(akmc_ctx* ctx, int32_t job, int64_t*
   std::vector<unsigned long long> copied;
   if (!pinned) {
     copied.resize(static_cast<size_t>(2 + c.bins));
-    CK(cudaMemcpyAsync(copied.data(), c.out, sizeof(unsigned long long) * copied.size(), cudaMemcpyDeviceToHost, ctx->stream));
+    CK(cudaMemcpyAsync(copied.data(), c.out, sizeof(unsigned long long) * copied.size(), cudaMemcpyDeviceToHost,
+                       ctx->stream));
   }
   CK(cudaStreamSynchronize(ctx->stream));
   const unsigned long long* const h = pinned ? pinned->cluster : copied.data();
